@@ -30,8 +30,11 @@ szp = np.ctypeslib.ndpointer(dtype=np.uintp, flags="C_CONTIGUOUS")
 
 
 # Where the reference project's sources are looked for: $REF_ROOT, else a checkout named
-# `reference` beside this repository.  Only the build of the compiled reference reads them.
+# `reference` beside this repository; "" where that folder holds no sources.  Only the build of the
+# compiled reference reads them.
 REF_ROOT = os.environ.get("REF_ROOT") or os.path.normpath(os.path.join(HERE, os.pardir, os.pardir, "reference"))
+if not os.path.isdir(os.path.join(REF_ROOT, "src")):
+    REF_ROOT = ""
 
 
 def build(ref: bool = False) -> None:
