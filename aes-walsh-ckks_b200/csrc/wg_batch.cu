@@ -56,6 +56,8 @@ struct KsPlan {
     double mac_bytes, modup_bytes, moddown_bytes, combine_bytes;
     bool fused;   // ModUp / ModDown fused with the NTT column phases (Context::ntt_fusion)
     int max_src;  // widest digit (fused ModUp shared memory)
+    int max_dst;  // most destination limbs of a digit
+    int max_limbs;  // most Q limbs of a switch
 };
 
 size_t batch_keyswitch_words(const Context& c, const KsItem* items, size_t n) {
@@ -74,7 +76,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     std::vector<GatherJob> gather;
     std::vector<NttEpiJob> contrib_epi;
     KsPlan p{};
-    p.fused = c.fuse(2 * n);  // the ModDown launch has two jobs per switch
+    p.fused = c.fuse();
     // MAC groups: consecutive switches with the same key, level and digit layout (up to
     // kMacGroup), one job per QP limb; [group_begin, it) is the open group
     size_t group_begin = 0;
@@ -110,6 +112,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
         const KsItem& x = items[it];
         const size_t level = x.level, L = level + 1, T = L + K, B = c.parts_at(level);
         if (level >= nq) fail(kInvalid, "batched keyswitch: invalid ciphertext level");
+        p.max_limbs = std::max(p.max_limbs, (int)L);
         if (x.key->key_level < level) fail(kRuntime, "keyswitch: switch key level is below ciphertext level");
         if (x.key->parts < B) fail(kRuntime, "keyswitch: insufficient key partitions");
         uint64_t* coeff = ws;
@@ -122,6 +125,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
             modup.push_back({c.d_modup + level * c.dnum + j, coeff, digits + j * T * N});
             const ModUpDesc& d = c.modup[level][j];
             p.max_src = std::max(p.max_src, d.src_count);
+            p.max_dst = std::max(p.max_dst, d.dst_count);
             p.modup_bytes += 8.0 * N * (d.src_count + d.dst_count);
             const size_t s0 = j * c.alpha, s1 = std::min(s0 + c.alpha, L);
             for (size_t l = 0; l < T; ++l) {
@@ -143,7 +147,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
             }
         for (int poly = 0; poly < 2; ++poly) {
             moddown.push_back({acc + (poly * T + L) * N, contrib + poly * L * N, c.fold_inv[level],
-                               c.fold_inv_s[level], (int)L, 0});
+                               c.fold_inv_s[level], (int)L, 0, c.fold_fp[level]});
             if (!p.fused)
                 for (size_t qi = 0; qi < L; ++qi) {
                     uint64_t* ptr = contrib + (poly * L + qi) * N;
@@ -202,14 +206,14 @@ static void run_keyswitch(const Context& c, const KsPlan& p, const JobTable& t, 
         // inverse row phase -> [inverse column phase, ModUp, forward column phase] -> forward
         // row phase; the same around ModDown (wg_ksfuse.cu)
         ntt_jobs_phase(c, t.at(p.intt_in), p.n_intt_in, false, false, s);
-        modup_ntt_jobs(c, t.at(p.modup), p.n_modup, p.max_src, p.modup_bytes, s);
+        modup_ntt_jobs(c, t.at(p.modup), p.n_modup, p.max_src, p.max_dst, p.modup_bytes, s);
         ntt_jobs_phase(c, t.at(p.ntt_digits), p.n_ntt_digits, true, false, s);
         {
             Probe probe(kClsKeyMac, p.mac_bytes, s);
             kb_mac_group<<<grid_for(c, p.n_mac), kT, 0, s>>>(t.at(p.mac), p.n_mac, c.d_mod, (int)c.nq, N);
         }
         ntt_jobs_phase(c, t.at(p.intt_p), p.n_intt_p, false, false, s);
-        moddown_ntt_jobs(c, t.at(p.moddown), p.n_moddown, p.moddown_bytes, s);
+        moddown_ntt_jobs(c, t.at(p.moddown), p.n_moddown, p.max_limbs, p.moddown_bytes, s);
         ntt_rows_epilogue_jobs(c, t.at(p.contrib_epi), p.n_contrib_epi, p.contrib_epi_bytes, s);
         if (p.n_gather) {
             Probe probe(kClsCombine, 8.0 * N * 4.0 * p.n_gather, s);
@@ -253,6 +257,24 @@ void batch_keyswitch(Context& c, const KsItem* items, size_t n, cudaStream_t s) 
     run_keyswitch(c, p, t, s);
 }
 
+void batch_rescale(Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, cudaStream_t s) {
+    if (level == 0 || level >= c.nq) fail(kInvalid, "ckks_rescale: invalid level");
+    constexpr size_t kChunk = 64;  // bounds the scratch for the remainders
+    for (size_t k0 = 0; k0 < npolys; k0 += kChunk) {
+        const size_t n = std::min(kChunk, npolys - k0);
+        const size_t words = (level + 1) * c.N;  // the remainders and the dropped limb's row phase
+        uint64_t* ws = c.batch_buffers(s).arena(c, n * words, s);
+        RescaleJobs rs;
+        rs.dropped = RescaleJobs::kCoefficients;
+        for (size_t k = 0; k < n; ++k)
+            rs.add(polys + (k0 + k) * stride, level, ws + k * words, ws + k * words + level * c.N);
+        JobTable t;
+        rs.plan(c, t);
+        t.upload(c, s);
+        rs.run(c, t, s);
+    }
+}
+
 // ------------------------------------------------------------------------------------------
 // Batched mul + relin + rescale + rotate
 // ------------------------------------------------------------------------------------------
@@ -275,7 +297,7 @@ static size_t pipeline_words(const Context& c, size_t count, const size_t* level
     size_t c2_words = 0, rem_words = 0;
     for (size_t i = 0; i < count; ++i) {
         c2_words += (levels[i] + 1) * N;
-        rem_words += 2 * levels[i] * N;
+        rem_words += 2 * (levels[i] + 1) * N;  // remainders and the dropped limb's row phase
         relin_items[i].level = levels[i];
         if (galois[i]) {
             KsItem it;
@@ -303,6 +325,7 @@ static void plan_pipeline(const Context& c, PipelinePlan& P, size_t count, const
     std::vector<KsItem> relin_items(count), rot_items;
     std::vector<TensorJob> tensor;
     RescaleJobs& rs = P.rescale.emplace();
+    rs.dropped = RescaleJobs::kCallers;
     uint64_t* c2p = c2base;
     uint64_t* remp = rembase;
     for (size_t i = 0; i < count; ++i) {
@@ -322,8 +345,8 @@ static void plan_pipeline(const Context& c, PipelinePlan& P, size_t count, const
         ri.galois = 0;
         c2p += L * N;
         for (int poly = 0; poly < 2; ++poly) {
-            rs.add(poly ? xa[i] : xb[i], lv, remp);
-            remp += lv * N;
+            rs.add(poly ? xa[i] : xb[i], lv, remp, remp + lv * N);
+            remp += (lv + 1) * N;
         }
         if (galois[i]) {
             KsItem it;

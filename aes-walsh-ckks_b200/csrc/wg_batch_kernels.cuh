@@ -238,16 +238,25 @@ dim3 grid_wide(const Context& c, size_t njobs) {
 // The launches of one batched rescale (ckks_rescale, src/ckks/operations/arith/ckks_rescale.cpp:
 // 68-148) over polynomials of any levels: add() records a polynomial x at level lv with lv
 // remainder limbs of scratch, plan() puts the job tables into a JobTable, run() launches.
-// Fused (Context::fuse over the polynomials): the inverse row phase of the dropped limbs, one
+// Fused (Context::fuse): the inverse row phase of the dropped limbs, one
 // fused launch (inverse column phase, rounded remainders, forward column phase; k_rescale_ntt)
 // and the forward row phase with the finish step as its epilogue (k_ntt_rows_epi): 3 launches.
 // Without: inverse NTT, kb_rescale_prep, forward NTT, kb_rescale_finish: 6 launches.  Same words.
+//
+// The limb that a rescale drops from a caller's polynomial ends as it always did, since the caller
+// can read it: as its canonical coefficients, or, in batches that fill the device, as the lazily
+// reduced words of its inverse row phase.  The latter row phase therefore runs in word arithmetic
+// also for the moduli of the FP64 path (one limb per polynomial); the former needs `spare`, N words
+// the row phase writes to.  Polynomials of the library's own (spare null, kOwn) leave anything.
 struct RescaleJobs {
+    enum Dropped { kOwn, kCallers, kCoefficients };
     struct Poly {
         uint64_t* x;
         size_t lv;
         uint64_t* rem;
+        uint64_t* spare;
     };
+    Dropped dropped = kOwn;
     std::vector<Poly> polys;
     bool fused = false;
     std::vector<NttJob> drop, rem_ntt;
@@ -255,6 +264,7 @@ struct RescaleJobs {
     std::vector<RescaleFinishJob> fin;
     std::vector<RescaleNttJob> cols;
     std::vector<NttEpiJob> rows;
+    int max_lv = 0;
     double prep_bytes = 0.0, fin_bytes = 0.0;
     const NttJob *jd = nullptr, *jr = nullptr;
     const RescalePrepJob* jp = nullptr;
@@ -263,20 +273,24 @@ struct RescaleJobs {
     const NttEpiJob* je = nullptr;
 
     bool empty() const { return polys.empty(); }
-    void add(uint64_t* x, size_t lv, uint64_t* rem) { polys.push_back({x, lv, rem}); }
-    // builds the jobs (fused when the batch fills the device: Context::fuse) into t
+    void add(uint64_t* x, size_t lv, uint64_t* rem, uint64_t* spare = nullptr) { polys.push_back({x, lv, rem, spare}); }
+    // builds the jobs (fused or not: Context::fuse) into t
     void plan(const Context& c, JobTable& t) {
         const size_t N = c.N;
-        fused = c.fuse(polys.size());
+        fused = c.fuse();
+        const bool rows_words = dropped == kCallers && c.fills(polys.size());
+        const bool coefficients = dropped != kOwn && !rows_words;
         for (const Poly& pl : polys) {
             const size_t lv = pl.lv;
+            max_lv = std::max(max_lv, (int)lv);
             uint64_t* x = pl.x;
             uint64_t* rem = pl.rem;
             const uint64_t* rc = c.rs_host.data() + c.rs_host_off[lv];
             uint64_t* dl = x + lv * N;
-            drop.push_back({dl, dl, (int)lv, 0});
+            uint64_t* rows_to = fused && coefficients ? pl.spare : dl;
+            drop.push_back({dl, rows_to, (int)lv, fused && rows_words});
             if (fused) {
-                cols.push_back({dl, rem, c.rs_one_s[lv], (int)lv, 0});
+                cols.push_back({rows_to, rem, c.rs_one_s[lv], (int)lv, rows_words, coefficients ? dl : nullptr});
                 for (size_t q = 0; q < lv; ++q)
                     rows.push_back({rem + q * N, nullptr, x + q * N, x + q * N, rc[lv + q], rc[2 * lv + q], (int)q,
                                     kEpiRescale});
@@ -305,7 +319,7 @@ struct RescaleJobs {
         const size_t N = c.N;
         if (fused) {
             ntt_jobs_phase(c, t.at(jd), (int)drop.size(), false, false, s);
-            rescale_ntt_jobs(c, t.at(jc), (int)cols.size(), prep_bytes, s);
+            rescale_ntt_jobs(c, t.at(jc), (int)cols.size(), max_lv, prep_bytes, s);
             ntt_rows_epilogue_jobs(c, t.at(je), (int)rows.size(), ntt_epilogue_bytes(rows, N), s);
         } else {
             ntt_jobs(c, t.at(jd), (int)drop.size(), false, s);

@@ -120,8 +120,8 @@ void q0p0_switch(Context& c, size_t count, uint64_t* const* b, uint64_t* const* 
             mac.push_back({key.d_data, a[ci], dg, acc, 2 * N, 1, 1, 1, (int)c.alpha, 0, i});
         intt_p.push_back({acc + N, acc + N, (int)nq, 0});
         intt_p.push_back({acc + 3 * N, acc + 3 * N, (int)nq, 0});
-        md.push_back({acc + N, ct, c.fold_inv[0], c.fold_inv_s[0], 1, 0});
-        md.push_back({acc + 3 * N, ct + N, c.fold_inv[0], c.fold_inv_s[0], 1, 0});
+        md.push_back({acc + N, ct, c.fold_inv[0], c.fold_inv_s[0], 1, 0, c.fold_fp[0]});
+        md.push_back({acc + 3 * N, ct + N, c.fold_inv[0], c.fold_inv_s[0], 1, 0, c.fold_fp[0]});
         ntt_c.push_back({ct, ct, 0, 0});
         ntt_c.push_back({ct + N, ct + N, 0, 0});
         comb.push_back({acc, ct, b[ci], a[ci], b[ci], a[ci], 1, 1, 0, 1, 0, 0});

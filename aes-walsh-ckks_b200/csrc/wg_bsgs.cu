@@ -437,7 +437,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
 
     JobTable t;
     // 1. hoist
-    const bool fused = c.fuse(2 * count);  // the pair ModDown launch: two jobs per ciphertext
+    const bool fused = c.fuse();
     int max_src = 1;
     for (size_t j = 0; j < B; ++j) max_src = std::max(max_src, c.modup[level][j].src_count);
     std::vector<NttJob> intt_a, ntt_dig;
@@ -512,7 +512,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
                 uint64_t* p = in_a + (L + pi) * N;
                 intt_pg.push_back({p, p, (int)(nq + pi), 0});
             }
-            md_single.push_back({in_a + L * N, cs, c.fold_inv[level], c.fold_inv_s[level], (int)L, 0});
+            md_single.push_back({in_a + L * N, cs, c.fold_inv[level], c.fold_inv_s[level], (int)L, 0, c.fold_fp[level]});
             for (size_t qi = 0; qi < L; ++qi) {
                 if (fused) {
                     // key term = inner a - ModDown: the subtraction as the row phase's epilogue
@@ -581,7 +581,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
             uint64_t* o = out + ci * slotw + poly * T * N;
             uint64_t* cf = cfinal + (ci * 2 + poly) * L * N;
             for (size_t pi = 0; pi < K; ++pi) intt_po.push_back({o + (L + pi) * N, o + (L + pi) * N, (int)(nq + pi), 0});
-            md_pair.push_back({o + L * N, cf, c.fold_inv[level], c.fold_inv_s[level], (int)L, 0});
+            md_pair.push_back({o + L * N, cf, c.fold_inv[level], c.fold_inv_s[level], (int)L, 0, c.fold_fp[level]});
             uint64_t* dst = poly ? b[ci] : a[ci];  // out holds a at offset 0, b at T*N
             for (size_t qi = 0; qi < L; ++qi) {
                 if (fused) {
@@ -594,11 +594,14 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
         }
     }
     RescaleJobs rescale_jobs;
+    rescale_jobs.dropped = RescaleJobs::kCallers;
     if (st.rescale) {
         if (level == 0) fail(kInvalid, "ckks_rescale: invalid level");
         for (size_t ci = 0; ci < count; ++ci)
-            for (int poly = 0; poly < 2; ++poly)
-                rescale_jobs.add(poly ? a[ci] : b[ci], level, rem + (ci * 2 + poly) * level * N);
+            for (int poly = 0; poly < 2; ++poly) {
+                uint64_t* r = rem + (ci * 2 + poly) * L * N;  // level remainders, then the dropped limb's row phase
+                rescale_jobs.add(poly ? a[ci] : b[ci], level, r, r + level * N);
+            }
     }
 
     // Baby slot 0 holds (a, b) with zero P limbs: copy Q limbs, clear P limbs.
@@ -639,7 +642,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
     if (fused) {
         // inverse row phase, [inverse columns, ModUp, forward columns], forward row phase
         ntt_jobs_phase(c, t.at(j_intt_a), (int)intt_a.size(), false, false, s);
-        modup_ntt_jobs(c, t.at(j_modup), (int)modup.size(), max_src, 8.0 * N * (double)(count * B * T), s);
+        modup_ntt_jobs(c, t.at(j_modup), (int)modup.size(), max_src, (int)T, 8.0 * N * (double)(count * B * T), s);
         ntt_jobs_phase(c, t.at(j_ntt_dig), (int)ntt_dig.size(), true, false, s);
     } else {
         ntt_jobs(c, t.at(j_intt_a), (int)intt_a.size(), false, s);
@@ -667,10 +670,10 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
     // 4.
     if (!md_single.empty() && fused) {
         ntt_jobs_phase(c, t.at(j_intt_pg), (int)intt_pg.size(), false, false, s);
-        moddown_ntt_jobs(c, t.at(j_mds), (int)md_single.size(), 8.0 * N * (K + L) * md_single.size(), s, false);
+        moddown_ntt_jobs(c, t.at(j_mds), (int)md_single.size(), (int)L, 8.0 * N * (K + L) * md_single.size(), s, false);
         ntt_rows_epilogue_jobs(c, t.at(j_cs_epi), (int)cs_epi.size(), ntt_epilogue_bytes(cs_epi, N), s);
         ntt_jobs_phase(c, t.at(j_intt_kt), (int)intt_kt.size(), false, false, s);
-        modup_ntt_jobs(c, t.at(j_modup2), (int)modup2.size(), max_src, 8.0 * N * (double)(md_single.size() * B * T),
+        modup_ntt_jobs(c, t.at(j_modup2), (int)modup2.size(), max_src, (int)T, 8.0 * N * (double)(md_single.size() * B * T),
                        s);
         ntt_jobs_phase(c, t.at(j_ntt_dig2), (int)ntt_dig2.size(), true, false, s);
         Probe probe(kClsKeyMac, mac2_bytes, s);
@@ -705,7 +708,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
     // 6.
     if (fused) {
         ntt_jobs_phase(c, t.at(j_intt_po), (int)intt_po.size(), false, false, s);
-        moddown_ntt_jobs(c, t.at(j_mdp), (int)md_pair.size(), 8.0 * N * (K + L) * md_pair.size(), s);
+        moddown_ntt_jobs(c, t.at(j_mdp), (int)md_pair.size(), (int)L, 8.0 * N * (K + L) * md_pair.size(), s);
         ntt_rows_epilogue_jobs(c, t.at(j_cf_epi), (int)cf_epi.size(), ntt_epilogue_bytes(cf_epi, N), s);
     } else {
         ntt_jobs(c, t.at(j_intt_po), (int)intt_po.size(), false, s);
@@ -759,7 +762,7 @@ void rotate_many_batch(Context& c, size_t level, size_t count, const uint64_t* c
     uint64_t* arena = c.batch_buffers(s).arena(c, count * per_ct, s);
     auto modq = [&](size_t limb) { return (int)(limb < L ? limb : nq + (limb - L)); };
 
-    const bool fused = c.fuse(count * B);  // the ModUp launch: one job per digit
+    const bool fused = c.fuse();
     int max_src = 1;
     for (size_t j = 0; j < B; ++j) max_src = std::max(max_src, c.modup[level][j].src_count);
     std::vector<NttJob> intt_a, ntt_dig, intt_p, ntt_c;
@@ -805,7 +808,7 @@ void rotate_many_batch(Context& c, size_t level, size_t count, const uint64_t* c
                     intt_p.push_back({p, p, (int)(nq + pi), 0});
                 }
                 md.push_back({acc + (poly * T + L) * N, cr + poly * L * N, c.fold_inv[level], c.fold_inv_s[level],
-                              (int)L, 0});
+                              (int)L, 0, c.fold_fp[level]});
                 if (!fused)
                     for (size_t qi = 0; qi < L; ++qi)
                         ntt_c.push_back({cr + (poly * L + qi) * N, cr + (poly * L + qi) * N, (int)qi, 0});
@@ -842,7 +845,7 @@ void rotate_many_batch(Context& c, size_t level, size_t count, const uint64_t* c
     modup_bytes *= count;
     if (fused) {
         ntt_jobs_phase(c, t.at(j1), (int)intt_a.size(), false, false, s);
-        modup_ntt_jobs(c, t.at(j2), (int)modup.size(), max_src, modup_bytes, s);
+        modup_ntt_jobs(c, t.at(j2), (int)modup.size(), max_src, (int)T, modup_bytes, s);
         ntt_jobs_phase(c, t.at(j3), (int)ntt_dig.size(), true, false, s);
     } else {
         ntt_jobs(c, t.at(j1), (int)intt_a.size(), false, s);
@@ -859,7 +862,7 @@ void rotate_many_batch(Context& c, size_t level, size_t count, const uint64_t* c
         }
         if (fused) {
             ntt_jobs_phase(c, t.at(j5), (int)intt_p.size(), false, false, s);
-            moddown_ntt_jobs(c, t.at(j6), (int)md.size(), 8.0 * N * (K + L) * md.size(), s);
+            moddown_ntt_jobs(c, t.at(j6), (int)md.size(), (int)L, 8.0 * N * (K + L) * md.size(), s);
             ntt_rows_epilogue_jobs(c, t.at(j10), (int)c_epi.size(), ntt_epilogue_bytes(c_epi, N), s);
             Probe probe(kClsCombine, 8.0 * N * 4.0 * gath.size(), s);
             kb_gather<<<grid_for(c, gath.size()), kT, 0, s>>>(t.at(j9), (int)gath.size(), c.logN);

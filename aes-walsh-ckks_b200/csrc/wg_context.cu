@@ -227,7 +227,8 @@ Context::~Context() {
     for (auto& kv : batches) kv.second.release();
     cudaFree(d_modup);
     cudaFree(d_mod);
-    cudaFree(d_tw);
+    for (uint64_t* t : d_tw) cudaFree(t);
+    cudaFree(d_tw_words);
     cudaFree(d_tables);
 }
 
@@ -309,15 +310,31 @@ Context* create_context(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
         }
     };
     dev_alloc((void**)&c->d_mod, nm * sizeof(Modulus));
-    dev_alloc((void**)&c->d_tw, H.tw.size() * 8);
     c->tables_words = H.words.size() + 1;
     dev_alloc((void**)&c->d_tables, c->tables_words * 8);
     check_cuda(cudaMemcpy(c->d_mod, c->mods.data(), nm * sizeof(Modulus), cudaMemcpyHostToDevice), "upload moduli");
     {
-        // interleaved (w, Shoup w) pairs per modulus and direction, as the NTT kernels read them
+        // twiddle pairs per modulus and direction, as the NTT kernels read them
         std::vector<ntt::TwPair> pairs(nm * 2 * N);
-        for (size_t i = 0; i < nm; ++i) ntt::interleave_twiddles(N, H.tw.data() + i * 4 * N, pairs.data() + i * 2 * N);
-        check_cuda(cudaMemcpy(c->d_tw, pairs.data(), pairs.size() * sizeof(ntt::TwPair), cudaMemcpyHostToDevice),
+        auto upload = [&](uint64_t*& d, int eb) {
+            for (size_t i = 0; i < nm; ++i)
+                for (size_t dir = 0; dir < 2; ++dir) {
+                    const uint64_t* w = H.tw.data() + (i * 4 + 2 * dir) * N;
+                    ntt::twiddle_pairs(N, H.mods[i].q, w, w + N, eb, false, pairs.data() + (i * 2 + dir) * N);
+                }
+            dev_alloc((void**)&d, pairs.size() * sizeof(ntt::TwPair));
+            check_cuda(cudaMemcpy(d, pairs.data(), pairs.size() * sizeof(ntt::TwPair), cudaMemcpyHostToDevice),
+                       "upload twiddles");
+        };
+        upload(c->d_tw[0], 3);
+        upload(c->d_tw[1], 4);
+        for (int eb = 3; eb <= 4; ++eb)
+            for (size_t i = 0; i < nq; ++i) {
+                const uint64_t* w = H.tw.data() + (i * 4 + 2) * N;
+                ntt::twiddle_pairs(N, H.mods[i].q, w, w + N, eb, true, pairs.data() + ((eb - 3) * nq + i) * N);
+            }
+        dev_alloc((void**)&c->d_tw_words, 2 * nq * N * sizeof(ntt::TwPair));
+        check_cuda(cudaMemcpy(c->d_tw_words, pairs.data(), 2 * nq * N * sizeof(ntt::TwPair), cudaMemcpyHostToDevice),
                    "upload twiddles");
     }
     check_cuda(cudaMemcpy(c->d_tables, H.words.data(), H.words.size() * 8, cudaMemcpyHostToDevice),
@@ -340,14 +357,18 @@ Context* create_context(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
             d.corr = T + o.corr;
             d.dst_limb = reinterpret_cast<const int*>(T + o.dst_limb);
             d.dst_mod = reinterpret_cast<const int*>(T + o.dst_mod);
+            d.scale_fp = reinterpret_cast<const ntt::TwPair*>(T + o.scale_fp);
+            d.qhat_fp = reinterpret_cast<const ntt::TwPair*>(T + o.qhat_fp);
             c->modup[level].push_back(d);
         }
     }
     c->fold_inv.resize(nq);
     c->fold_inv_s.resize(nq);
+    c->fold_fp.resize(nq);
     for (size_t level = 0; level < nq; ++level) {
         c->fold_inv[level] = T + H.fold_inv[level];
         c->fold_inv_s[level] = T + H.fold_inv_s[level];
+        c->fold_fp[level] = reinterpret_cast<const ntt::TwPair*>(T + H.fold_fp[level]);
     }
     {
         std::vector<ModUpDesc> flat(nq * dnum);

@@ -72,6 +72,10 @@ struct ModUpDesc {
     const uint64_t* corr;      // [dst][src+1]
     const int* dst_limb;       // QP limb index written for each dst
     const int* dst_mod;        // modulus index (into Context::d_mod) for each dst
+    // for the fused kernels, FP64 factor pairs (fp::term_factor): N^-1 qhat_inv per source limb and
+    // qhat per (dst, src), zero where the source's / destination's modulus is not below 2^50
+    const ntt::TwPair* scale_fp;
+    const ntt::TwPair* qhat_fp;
 };
 
 struct KeyEntry {
@@ -140,19 +144,23 @@ struct Context {
     std::vector<uint64_t> q, p;
     std::vector<Modulus> mods;       // nq + np entries (P after Q)
     Modulus* d_mod = nullptr;
-    uint64_t* d_tw = nullptr;        // [mod][2][N] (w, Shoup w) pairs: forward, inverse (ntt::TwPair)
+    // twiddle pairs [mod][2][N] (forward, inverse; ntt::twiddle_pairs) for 8 and 16 residues per thread
+    uint64_t* d_tw[2] = {nullptr, nullptr};
+    // [8 / 16 residues][Q limb][N]: the inverse's (w, Shoup w) pairs of every Q limb (NttJob::words)
+    ntt::TwPair* d_tw_words = nullptr;
+    const ntt::TwPair* twiddles(int eb) const { return reinterpret_cast<const ntt::TwPair*>(d_tw[eb - 3]); }
     int ntt_variant[2][2] = {{0, 0}, {0, 0}};  // NTT geometry per [direction][phase: rows, columns]
     // Key switches and rescales can run their base changes fused with the adjacent NTT column
     // phases and their final element-wise steps in the last row phase's epilogue (wg_ksfuse.cu,
-    // k_ntt_rows_epi).  0: always the separate launches; 1: fused when the launch fills the
-    // device (fuse()); 2: always fused.  The words are the same in every mode.
+    // k_ntt_rows_epi).  0: the separate launches; 1, 2: fused.  The words are the same in every mode.
     int ntt_fusion = 1;
     int sm_count = 148;  // multiprocessors of the device
-    // Whether a step over `jobs` jobs runs fused: the fused kernels give one CTA of 128 threads
-    // per (job, 1024-coefficient column tile) and hold several source tiles in shared memory, so
-    // they only pay when the launch fills the device at least twice; smaller calls (a single
-    // ciphertext) keep the separate, wider launches.
-    bool fuse(size_t jobs) const {
+    // Whether the batched steps run fused.  Launches too small to fill the device divide their
+    // jobs' output limbs over several CTAs (split_of, wg_ksfuse.cu), so the fused sequence is the
+    // shorter one at every size.
+    bool fuse() const { return ntt_fusion != 0; }
+    // Whether a step over `jobs` jobs counts as one that fills the device (RescaleJobs).
+    bool fills(size_t jobs) const {
         return ntt_fusion == 2 || (ntt_fusion == 1 && jobs * (N >= 1024 ? N / 1024 : 1) >= 2 * (size_t)sm_count);
     }
     NttTuning tuning{};
@@ -162,6 +170,7 @@ struct Context {
     size_t tables_words = 0;
     // folded ModDown constants per level: [qi][pi] inverse and Shoup
     std::vector<const uint64_t*> fold_inv, fold_inv_s;
+    std::vector<const ntt::TwPair*> fold_fp;  // the inverses as FP64 factor pairs
     const double* d_p_inv = nullptr; // [pi] 1.0 / p
     // rescale constants per dropped limb d: arrays of d entries (Shoup of 1, p^-1 and its
     // Shoup companion, floor(p/2) mod q_i)
@@ -275,7 +284,7 @@ struct NttJob {
     const uint64_t* src;
     uint64_t* dst;
     int mod;
-    int pad;
+    int words;  // inverse row phase of a Q limb only: run in word arithmetic whatever the modulus
 };
 void ntt_jobs(const Context& c, const NttJob* d_jobs, int njobs, bool forward, cudaStream_t s);
 // Time every NTT geometry on the context's device and keep the fastest per direction and phase
@@ -309,17 +318,21 @@ struct ModDownNttJob {
     const uint64_t* inv_s;
     int L;
     int pad;
+    const ntt::TwPair* inv_fp;  // the same table as FP64 factor pairs (Context::fold_fp)
 };
 // Rescale of one polynomial at level lv (ckks_rescale): drop holds its last limb after the
 // inverse row phase; the kernel finishes that inverse transform, forms the rounded remainder
 // for every lower limb and writes it to rem (lv limbs) after the forward column phase.  rc: the
-// device rescale constants of level lv (one_s, inv_p, inv_p_s, half; lv words each).
+// device rescale constants of level lv (one_s, inv_p, inv_p_s, half; lv words each).  keep: where the
+// limb's canonical coefficients go as well (not drop itself: blocks that share a job read it), or
+// null.  words: the row phase ran in word arithmetic (NttJob::words).
 struct RescaleNttJob {
     const uint64_t* drop;
     uint64_t* rem;
     const uint64_t* rc;
     int lv;
-    int pad;
+    int words;
+    uint64_t* keep;
 };
 // The forward row phase of job-table limbs with an element-wise epilogue (NttEpiJob, wg_ntt.cuh).
 using ntt::NttEpiJob;
@@ -334,15 +347,17 @@ inline double ntt_epilogue_bytes(const std::vector<NttEpiJob>& jobs, size_t N) {
         words += 2.0 + (j.kind == kEpiCombine ? 1.0 : 0.0) + ((j.kind == kEpiRescale || j.c0) ? 1.0 : 0.0);
     return 8.0 * (double)N * words;
 }
-void rescale_ntt_jobs(const Context& c, const RescaleNttJob* d_jobs, int njobs, double bytes, cudaStream_t s);
+// max_out: the most output limbs of a job (how far a small launch divides its jobs, split_of).
+void rescale_ntt_jobs(const Context& c, const RescaleNttJob* d_jobs, int njobs, int max_out, double bytes,
+                      cudaStream_t s);
 
 // max_src: the largest source-limb count of the jobs (shared-memory size).
-void modup_ntt_jobs(const Context& c, const ModUpNttJob* d_jobs, int njobs, int max_src, double bytes,
+void modup_ntt_jobs(const Context& c, const ModUpNttJob* d_jobs, int njobs, int max_src, int max_out, double bytes,
                     cudaStream_t s);
 // fma_alpha: the alpha estimate rounded as fused multiply-adds (the key switch's pair ModDown)
 // or as multiplies then adds (the single-polynomial ModDown of the QP linear transform).
-void moddown_ntt_jobs(const Context& c, const ModDownNttJob* d_jobs, int njobs, double bytes, cudaStream_t s,
-                      bool fma_alpha = true);
+void moddown_ntt_jobs(const Context& c, const ModDownNttJob* d_jobs, int njobs, int max_out, double bytes,
+                      cudaStream_t s, bool fma_alpha = true);
 
 // NTT over `polys` polynomials of `limbs` limbs each, `poly_stride` words apart.
 void ntt_forward(const Context& c, uint64_t* data, int limbs, int polys, size_t poly_stride,

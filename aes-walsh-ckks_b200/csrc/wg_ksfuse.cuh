@@ -20,9 +20,18 @@
 //            phase that follows finishes the rescale in its epilogue, k_ntt_rows_epi).
 //
 // The butterflies, reductions and FP64 sums are those of the unfused kernels in the same
-// order, so the words written equal the ones the separate launches write.  Thread t owns tile
-// elements t + k * THREADS (k < 8) in every element-wise step, so those steps need no barrier
-// between them; the column rounds are separated by barriers as in k_ntt_phase.
+// order, so the words written equal the ones the separate launches write.
+//
+// A thread owns the same 8 elements of the tile in the inverse phase's last round as in the forward
+// phase's first (make_plan), so between the two transforms everything is its own: the finished
+// source limbs wait in shared memory slots that only their thread touches (slot k * THREADS + t: no
+// barrier, no bank conflict, no padding), and a base change's values go from registers straight
+// into the forward rounds.  Only the rounds' exchanges use the padded tile and barriers.
+//
+// Limbs whose modulus is below fp::kLimit run in FP64 (wg_fp.cuh): their slots hold doubles, from
+// the inverse row phase's words to those the forward row phase continues from.  A scaled source
+// (ModUp), P residue (ModDown) or dropped limb (rescale) is then the same canonical residue as
+// its word, as a double (SourceKinds, fp_src: a bit per source limb for the form its slots hold).
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -41,46 +50,41 @@ template <int LOGN>
 struct Geom {
     using Fwd = ntt::Phase<LOGN, true, true, 3, false, kTile>;
     using Inv = ntt::Phase<LOGN, false, true, 3, false, kTile>;
+    template <int RD>
+    using FwdRound = ntt::Round<LOGN, true, true, 3, false, RD, kTile>;
+    template <int RD>
+    using InvRound = ntt::Round<LOGN, false, true, 3, false, RD, kTile>;
     static constexpr int N = 1 << LOGN;
     static constexpr int TILE = Fwd::TILE;
     static constexpr int THREADS = Fwd::THREADS;
     static constexpr int E = 8;
-    static constexpr int SUBS = Fwd::SUBS;
-    static constexpr int PAD = TILE + TILE / 16;  // words of one padded tile
+    static constexpr int PAD = TILE + TILE / 16;  // words of the padded exchange tile
     static constexpr int TILES = N / TILE;
     static constexpr int ROUNDS = Fwd::ROUNDS;
     static_assert(Fwd::TILE == Inv::TILE && Fwd::THREADS == Inv::THREADS, "one tile shape for both directions");
 };
 
-template <int LOGN>
-WG_HD size_t col_offset(int tile, int e) {
-    return ntt::tile_offset<LOGN, true, true, 3, false, kTile>(tile, e);
-}
-
-// Load thread t's elements of one limb's column tile.
-template <int LOGN>
-WG_HD void load_tile(uint64_t* sm, const uint64_t* __restrict__ limb, int tile, int t) {
-    using G = Geom<LOGN>;
-#pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        const int e = t + k * G::THREADS;
-        sm[ntt::pad16(e)] = limb[col_offset<LOGN>(tile, e)];
-    }
+// Offset in the limb of thread t's element 0 in a round; element k is limb_step(k) further.
+template <class R>
+WG_HD size_t limb_offset(int tile, int t) {
+    using P = typename R::P;
+    const int e = R::element(P::sub_of(t), P::o_of(t));
+    return ((size_t)(e / P::SUBS) << P::NB2) + (size_t)tile * P::SUBS + e % P::SUBS;
 }
 
 #if defined(__CUDACC__)
-// The same load as an asynchronous copy (cp.async, 8 bytes per element) that lands in shared
-// memory without passing through registers, so a CTA can have all its source tiles in flight at
-// once; completion is awaited per commit group (cp_async_wait_upto) before a barrier.
+// Thread t's elements (first inverse round) of one limb into its slots, as asynchronous copies
+// (cp.async, 8 bytes each) that pass no register, so a CTA can have all its source limbs in flight at
+// once; completion is awaited per commit group (cp_async_wait_upto), by the thread alone.
 template <int LOGN>
-__device__ __forceinline__ void load_tile_async(uint64_t* sm, const uint64_t* __restrict__ limb, int tile, int t) {
+__device__ __forceinline__ void load_slots_async(uint64_t* slots, const uint64_t* __restrict__ limb, int tile, int t) {
     using G = Geom<LOGN>;
+    using R = typename G::template InvRound<0>;
+    const uint64_t* p = limb + limb_offset<R>(tile, t);
 #pragma unroll
     for (int k = 0; k < G::E; ++k) {
-        const int e = t + k * G::THREADS;
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(sm + ntt::pad16(e));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(limb + col_offset<LOGN>(tile, e))
-                     : "memory");
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(slots + k * G::THREADS + t);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(p + R::limb_step(k)) : "memory");
     }
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -103,52 +107,70 @@ __device__ __forceinline__ void cp_async_wait_upto(int pending) {
 }
 #endif
 
-// Store thread t's elements of the tile to one limb (no reduction: the forward transform's row
-// phase continues from these words).
-template <int LOGN>
-WG_HD void store_tile(const uint64_t* sm, uint64_t* __restrict__ limb, int tile, int t) {
-    using G = Geom<LOGN>;
+// Thread t's elements of a limb's tile in round R, and back (no reduction: the forward transform's
+// row phase continues from these words).
+template <class R>
+WG_HD void load_limb(uint64_t* w, const uint64_t* __restrict__ limb, int tile, int t) {
+    const uint64_t* p = limb + limb_offset<R>(tile, t);
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        const int e = t + k * G::THREADS;
-        limb[col_offset<LOGN>(tile, e)] = sm[ntt::pad16(e)];
-    }
+    for (int k = 0; k < R::E; ++k) w[k] = p[R::limb_step(k)];
 }
-
-// Round RD of the column phase for thread t (a barrier must follow each round).
-template <int LOGN, bool FWD, int RD, bool LAZY>
-WG_HD void col_round(uint64_t* sm, int tile, int t, uint64_t q, const ntt::TwPair* __restrict__ tw) {
-    using P = ntt::Phase<LOGN, FWD, true, 3, false, kTile>;
-    ntt::ntt_round<LOGN, FWD, true, 3, false, RD, LAZY, kTile>(sm, t % P::SUBS, t / P::SUBS, tile, q, tw);
-}
-
-// Last step of the inverse transform for thread t's elements: multiply by N^-1 (canonical).
-template <int LOGN>
-WG_HD void scale_n_inv(uint64_t* sm, int t, const Modulus& m) {
-    using G = Geom<LOGN>;
+template <class R>
+WG_HD void store_limb(const uint64_t* w, uint64_t* __restrict__ limb, int tile, int t) {
+    uint64_t* p = limb + limb_offset<R>(tile, t);
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        uint64_t& v = sm[ntt::pad16(t + k * G::THREADS)];
-        v = mul_shoup(v, m.n_inv, m.n_inv_shoup, m.q);
-    }
+    for (int k = 0; k < R::E; ++k) p[R::limb_step(k)] = w[k];
 }
 
-// ModUp, source limb i of the digit (coefficients in tile sm_i, canonical): scale by
-// qhat_inv_i in place and add the FP64 estimate term to thread t's alpha sums, in the order of
-// modup_coeff_w.  (modup_coeff_w first reduces its input below q; the inverse transform's
-// N^-1 step already leaves it canonical, so that reduction is the identity here.)
-template <int LOGN, class Desc>
-WG_HD void modup_scale(uint64_t* sm_i, int t, const Desc& d, int i, uint64_t qi, double* alpha) {
-    using G = Geom<LOGN>;
+// Per source limb (bits): its slots hold doubles; its modulus is of the FP64 path but not below
+// fp::kNoReduce.
+struct SourceKinds {
+    unsigned fp64 = 0, wide = 0;
+    WG_HD void set(int i, uint64_t q) {
+        if (q < fp::kLimit) fp64 |= 1u << i;
+        if (q < fp::kLimit && q >= fp::kNoReduce) wide |= 1u << i;
+    }
+};
+
+// A slot's word as an integer, whichever form it holds.
+WG_HD uint64_t slot_word(uint64_t x, bool fp64) { return fp64 ? fp::to_word(fp::bits_double(x)) : x; }
+
+// Last step of an FP64 inverse transform: multiply by the factor pair (N^-1, or N^-1 with a base
+// change's constant) to the canonical residue.
+WG_HD void scale_fp(double* v, double w, double wq, double q) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = fp::lift(fp::mulmod(v[k], w, wq, q), q);
+}
+
+// Last step of the inverse transform: multiply by N^-1 (canonical).
+WG_HD void scale_n_inv(uint64_t* v, const Modulus& m) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = mul_shoup(v[k], m.n_inv, m.n_inv_shoup, m.q);
+}
+
+// ModUp, source limb i of the digit (canonical coefficients): scale by qhat_inv_i in place and add
+// the FP64 estimate term to the alpha sums, in the order of modup_coeff_w.  (modup_coeff_w first
+// reduces its input below q; the inverse transform's N^-1 step already leaves it canonical, so that
+// reduction is the identity here.)
+template <class Desc>
+WG_HD void modup_scale(uint64_t* v, const Desc& d, int i, uint64_t qi, double* alpha) {
     const uint64_t w = WG_LDG(d.qhat_inv + i), ws = WG_LDG(d.qhat_inv_s + i);
     const double inv = WG_LDG(d.src_inv + i);
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        uint64_t& v = sm_i[ntt::pad16(t + k * G::THREADS)];
-        const uint64_t s = mul_shoup(v, w, ws, qi);
-        v = s;
-        alpha[k] = dadd(alpha[k], dmul(u2d(s), inv));
+    for (int k = 0; k < 8; ++k) {
+        v[k] = mul_shoup(v[k], w, ws, qi);
+        alpha[k] = dadd(alpha[k], dmul(u2d(v[k]), inv));
     }
+}
+
+// The same for an FP64 source, from the inverse rounds' values: N^-1 and qhat_inv_i in one factor.
+template <class Desc>
+WG_HD void modup_scale_fp(double* v, const Desc& d, int i, double qi, double* alpha) {
+    const ntt::TwPair f = d.scale_fp[i];
+    scale_fp(v, fp::bits_double(f.w), fp::bits_double(f.ws), qi);
+    const double inv = WG_LDG(d.src_inv + i);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) alpha[k] = dadd(alpha[k], dmul(v[k], inv));
 }
 
 WG_HD uint32_t hps_count(double alpha, int n) {
@@ -156,12 +178,12 @@ WG_HD uint32_t hps_count(double alpha, int n) {
     return (uint32_t)(h > (uint64_t)n ? (uint64_t)n : h);
 }
 
-// ModUp destination dst of the digit: thread t's coefficients into the work tile.
-// src_tiles holds the n scaled source tiles (stride PAD); W >= n bounds the digit width so the
+// ModUp destination dst of the digit: thread t's coefficients.
+// src holds the n scaled sources' slots (TILE words each); W >= n bounds the digit width so the
 // dst row of constants stays in registers.
 template <int LOGN, int W, class Desc>
-WG_HD void modup_value(uint64_t* work, const uint64_t* src_tiles, int t, const Desc& d, int dst, uint64_t m,
-                       const uint32_t* hps) {
+WG_HD void modup_value(uint64_t* v, const uint64_t* src, int t, const Desc& d, int dst, uint64_t m, const uint32_t* hps,
+                       unsigned fp_src) {
     using G = Geom<LOGN>;
     const int n = d.src_count;
     const uint64_t* row = d.qhat + (size_t)dst * n;
@@ -175,45 +197,120 @@ WG_HD void modup_value(uint64_t* work, const uint64_t* src_tiles, int t, const D
     }
 #pragma unroll
     for (int k = 0; k < G::E; ++k) {
-        const int pe = ntt::pad16(t + k * G::THREADS);
         uint64_t acc = 0;
 #pragma unroll
         for (int i = 0; i < W; ++i)
-            if (i < n) acc = add_mod(acc, mul_shoup(src_tiles[(size_t)i * G::PAD + pe], w[i], ws[i], m), m);
-        work[pe] = sub_mod(acc, WG_LDG(corr + hps[k]), m);
+            if (i < n)
+                acc = add_mod(acc, mul_shoup(slot_word(src[i * G::TILE + k * G::THREADS + t], fp_src >> i & 1), w[i], ws[i], m),
+                              m);
+        v[k] = sub_mod(acc, WG_LDG(corr + hps[k]), m);
     }
 }
 
-// ModDown: FP64 estimate of thread t's coefficients over the K P tiles, in the order of
+// Sums of products s w of thread t's source elements s, modulo a destination q of the FP64 path.
+//   q < fp::kNoReduce: exact sums with one reduction (fp::Dot), 4 FP64 instructions a term; a word
+//     source (61 bits) is two terms, s = s1 2^31 + s0 with the factors w and 2^31 w; a 43- to 50-bit
+//     FP64 source would overflow the sum and adds its reduced product instead.
+//   larger q: an FP64 source adds the reduced product through its factor pair (w, w / q), a word
+//     source a lazy Shoup product in [0, 2q), centred; each term adds at most q in magnitude, and the
+//     sum is brought back to q / 2 after every fourth, so it stays below 5.5 q < 2^53.
+// `f` is the term's table entry: (w, w / q), or (w, 2^31 w) for a word source (fp::kWordSplit).
+struct SumFp {
+    fp::Dot d[8];
+    WG_HD void start(int k, double v) {
+        d[k].clear();
+        d[k].l = v;
+    }
+    template <int LOGN>
+    WG_HD void add(const uint64_t* slots, int t, bool fp64, bool wide, ntt::TwPair f, uint64_t w, uint64_t ws, int term,
+                   const Modulus& m) {
+        using G = Geom<LOGN>;
+        const double f0 = fp::bits_double(f.w), f1 = fp::bits_double(f.ws);
+        const bool dot = m.q < fp::kNoReduce;
+        slots += t;
+        if (fp64 && dot && !wide) {
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) d[k].add(fp::bits_double(slots[k * G::THREADS]), f0);
+        } else if (fp64) {
+#pragma unroll
+            for (int k = 0; k < G::E; ++k)
+                d[k].l = dadd(d[k].l, fp::mulmod(fp::bits_double(slots[k * G::THREADS]), f0, f1, m.qd));
+        } else if (dot) {
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) {
+                const uint64_t s = slots[k * G::THREADS];
+                d[k].add(fp::from_word(s & 0x7fffffffu), f0);
+                d[k].add(fp::from_word(s >> 31), f1);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) {
+                const uint64_t r = mul_shoup_lazy(slots[k * G::THREADS], w, ws, m.q);
+                d[k].l = dadd(d[k].l, dadd(fp::from_word(r), -m.qd));
+            }
+        }
+        if (!dot && (term & 3) == 3) {
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) d[k].l = fp::reduce(d[k].l, m.qd, m.inv_q);
+        }
+    }
+    WG_HD void finish(double* v, const Modulus& m) const {
+        const bool dot = m.q < fp::kNoReduce;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = dot ? d[k].value(m.qd, m.inv_q) : d[k].l;
+    }
+};
+static_assert(2 * kMaxDigitWidth <= fp::kDotTerms && 2 * kMaxPLimbs <= fp::kDotTerms, "a base change is one exact sum");
+
+// ModUp destination dst of the FP64 path: thread t's coefficients, unreduced.
+template <int LOGN, class Desc>
+WG_HD void modup_value_fp(double* v, const uint64_t* src, int t, const Desc& d, int dst, const Modulus& m,
+                          const uint32_t* hps, SourceKinds kinds) {
+    using G = Geom<LOGN>;
+    const int n = d.src_count;
+    const uint64_t* corr = d.corr + (size_t)dst * (n + 1);
+    SumFp sum;
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) sum.start(k, -fp::from_word(WG_LDG(corr + hps[k])));
+    for (int i = 0; i < n; ++i) {
+        const size_t at = (size_t)dst * n + i;
+        sum.add<LOGN>(src + i * G::TILE, t, kinds.fp64 >> i & 1, kinds.wide >> i & 1, d.qhat_fp[at], d.qhat[at],
+                      d.qhat_s[at], i, m);
+    }
+    sum.finish(v, m);
+}
+
+// ModDown: FP64 estimate of thread t's coefficients over the K P limbs, in the order of
 // moddown_all_limbs_k; FMA: rounded as a fused multiply-add (the pair ModDown's compiled form)
-// or as a multiply then an add (the single-polynomial ModDown's).  The tiles hold canonical
+// or as a multiply then an add (the single-polynomial ModDown's).  The slots hold canonical
 // residues (the inverse transform's N^-1 step), so moddown_all_limbs_k's reduction of its input
 // below p is the identity here and is left out.  KW >= K keeps the constants in registers.
 template <int LOGN, int KW, bool FMA = true>
-WG_HD void moddown_hps(const uint64_t* p_tiles, int t, const Modulus* __restrict__ pmods, int K, uint32_t* hps) {
+WG_HD void moddown_hps(const uint64_t* src, int t, const Modulus* __restrict__ pmods, int K, uint32_t* hps,
+                       unsigned fp_src) {
     using G = Geom<LOGN>;
     double inv[KW];
 #pragma unroll
     for (int pi = 0; pi < KW; ++pi) inv[pi] = pi < K ? pmods[pi].inv_q : 0.0;
 #pragma unroll
     for (int k = 0; k < G::E; ++k) {
-        const int pe = ntt::pad16(t + k * G::THREADS);
         double alpha = 0.0;
 #pragma unroll
         for (int pi = 0; pi < KW; ++pi)
             if (pi < K) {
-                const uint64_t s = p_tiles[(size_t)pi * G::PAD + pe];
-                alpha = FMA ? dfma(u2d(s), inv[pi], alpha) : dadd(alpha, dmul(u2d(s), inv[pi]));
+                const uint64_t x = src[pi * G::TILE + k * G::THREADS + t];
+                const double s = fp_src >> pi & 1 ? fp::bits_double(x) : u2d(x);
+                alpha = FMA ? dfma(s, inv[pi], alpha) : dadd(alpha, dmul(s, inv[pi]));
             }
         hps[k] = hps_count(alpha, K);
     }
 }
 
-// ModDown contribution for Q limb qi: thread t's coefficients into the work tile (canonical P
-// residues as for moddown_hps; KW >= K).
+// ModDown contribution for Q limb qi: thread t's coefficients (canonical P residues as for
+// moddown_hps; KW >= K).
 template <int LOGN, int KW>
-WG_HD void moddown_value(uint64_t* work, const uint64_t* p_tiles, int t, int K, uint64_t q,
-                         const uint64_t* __restrict__ iv, const uint64_t* __restrict__ ivs, const uint32_t* hps) {
+WG_HD void moddown_value(uint64_t* v, const uint64_t* src, int t, int K, uint64_t q, const uint64_t* __restrict__ iv,
+                         const uint64_t* __restrict__ ivs, const uint32_t* hps, unsigned fp_src) {
     using G = Geom<LOGN>;
     uint64_t w[KW], ws[KW];
 #pragma unroll
@@ -223,28 +320,66 @@ WG_HD void moddown_value(uint64_t* work, const uint64_t* p_tiles, int t, int K, 
     }
 #pragma unroll
     for (int k = 0; k < G::E; ++k) {
-        const int pe = ntt::pad16(t + k * G::THREADS);
         uint64_t acc = 0;
 #pragma unroll
         for (int pi = 0; pi < KW; ++pi)
-            if (pi < K) acc = add_mod(acc, mul_shoup(p_tiles[(size_t)pi * G::PAD + pe], w[pi], ws[pi], q), q);
-        work[pe] = sub_mod(acc, (uint64_t)hps[k], q);
+            if (pi < K)
+                acc = add_mod(acc, mul_shoup(slot_word(src[pi * G::TILE + k * G::THREADS + t], fp_src >> pi & 1), w[pi],
+                                             ws[pi], q), q);
+        v[k] = sub_mod(acc, (uint64_t)hps[k], q);
     }
 }
 
-// Rescale: thread t's rounded remainders of the dropped limb (coefficients in drop, canonical,
-// modulus p) for target limb q into the work tile, as kb_rescale_prep forms them
+// The same for a Q limb of the FP64 path, unreduced.
+template <int LOGN>
+WG_HD void moddown_value_fp(double* v, const uint64_t* src, int t, int K, const Modulus& m,
+                            const uint64_t* __restrict__ iv, const uint64_t* __restrict__ ivs,
+                            const ntt::TwPair* __restrict__ ivf, const uint32_t* hps, SourceKinds kinds) {
+    using G = Geom<LOGN>;
+    SumFp sum;
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) sum.start(k, -fp::from_word(hps[k]));
+    for (int pi = 0; pi < K; ++pi)
+        sum.add<LOGN>(src + pi * G::TILE, t, kinds.fp64 >> pi & 1, kinds.wide >> pi & 1, ivf[pi], iv[pi], ivs[pi], pi, m);
+    sum.finish(v, m);
+}
+
+// Rescale: thread t's rounded remainders of the dropped limb (slots, canonical, modulus p) for
+// target limb q, as kb_rescale_prep forms them
 // (ckks_rescale, src/ckks/operations/arith/ckks_rescale.cpp:68-148).
 template <int LOGN>
-WG_HD void rescale_value(uint64_t* work, const uint64_t* drop, int t, uint64_t p, uint64_t q, uint64_t one_s,
-                         uint64_t half) {
+WG_HD void rescale_value(uint64_t* v, const uint64_t* drop, int t, uint64_t p, uint64_t q, uint64_t one_s, uint64_t half,
+                         bool fp_drop) {
     using G = Geom<LOGN>;
 #pragma unroll
     for (int k = 0; k < G::E; ++k) {
-        const int pe = ntt::pad16(t + k * G::THREADS);
-        uint64_t shift = drop[pe] + (p >> 1);
+        uint64_t shift = slot_word(drop[k * G::THREADS + t], fp_drop) + (p >> 1);
         if (shift >= p) shift -= p;
-        work[pe] = sub_mod(reduce_shoup(shift, q, one_s), half, q);
+        v[k] = sub_mod(reduce_shoup(shift, q, one_s), half, q);
+    }
+}
+
+// The same for a target limb of the FP64 path: unreduced, at most 2 q in magnitude.
+template <int LOGN>
+WG_HD void rescale_value_fp(double* v, const uint64_t* drop, int t, uint64_t p, const Modulus& m, uint64_t one_s,
+                            uint64_t half, bool fp_drop) {
+    using G = Geom<LOGN>;
+    const double h = fp::from_word(half);
+    const double pd = u2d(p), hp = u2d(p >> 1);
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) {
+        const uint64_t x = drop[k * G::THREADS + t];
+        double r;
+        if (fp_drop) {
+            double shift = dadd(fp::bits_double(x), hp);
+            if (shift >= pd) shift = dadd(shift, -pd);
+            r = fp::reduce(shift, m.qd, m.inv_q);
+        } else {
+            uint64_t shift = x + (p >> 1);
+            if (shift >= p) shift -= p;
+            r = fp::from_word(shift - umulhi(shift, one_s) * m.q);  // in [0, 2q)
+        }
+        v[k] = dadd(r, -h);
     }
 }
 

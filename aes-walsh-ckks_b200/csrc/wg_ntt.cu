@@ -8,17 +8,22 @@
 // Device organisation (N = 2^n, n = n1 + n2, n1 = floor(n/2)):
 //   * the transform runs as two phases; the "column" phase owns the n1 high index bits, the
 //     "row" phase the n2 low bits.  Forward = columns then rows, inverse = rows then columns.
-//   * a CTA stages a 2048-element tile (or the whole limb for N < 2048) in shared memory with
-//     one pad word every 16 words, so strided 64-bit accesses stay at two wavefronts per warp;
-//   * each thread carries 8 or 16 elements (the geometry's EB) through up to three or four
-//     radix-2 stages in registers per round (one shared-memory round trip per round);
+//   * a CTA owns a 2048-element tile (or the whole limb for N < 2048); each thread carries 8 or 16
+//     elements (the geometry's EB) through up to three or four radix-2 stages in registers per
+//     round, from device memory into the first round and from the last one back;
+//   * between rounds the CTA exchanges them in shared memory with one pad word every 16 words, so
+//     strided 64-bit accesses stay at two wavefronts per warp;
 //   * twiddles come as (w, Shoup w) pairs, one 16-byte load each, either staged in shared
 //     memory per CTA or read from the L2-resident table directly (the geometry's STAGED);
 //   * grid.y indexes limbs and grid.z polynomials, so one launch covers a whole ciphertext
 //     batch; each limb picks its modulus through a LimbMap (Q limbs, P limbs or a mix).
-// Butterflies are Harvey/Shoup with lazy ranges: forward values stay in [0, 4q) (or, for moduli
-// below 2^58, grow by at most 2q per stage without reduction, see kLazyForwardLimit), inverse
-// in [0, 2q); the last phase canonicalises (forward) or scales by N^-1 with Shoup (inverse).
+// Moduli below 2^50 (fp::kLimit) run in FP64: signed integers in doubles, exact products through
+// the fused multiply-add's rounding error (wg_fp.cuh, ntt::FpArith), 8 FP64 instructions a
+// butterfly against about 30 integer ones; between the phases a limb holds the doubles' bits.
+// Larger moduli use Harvey/Shoup butterflies on words with lazy ranges: forward values stay in
+// [0, 4q) (or, for moduli below 2^58, grow by at most 2q per stage without reduction, see
+// kLazyForwardLimit), inverse in [0, 2q).  The last phase canonicalises (forward) or scales by
+// N^-1 (inverse), so both give the same words.
 // Every geometry performs the same butterflies on the same values, so all of them give the
 // same words; which one runs is chosen per (direction, phase) by timing them on the device
 // when a context is created (ntt_autotune).
@@ -34,10 +39,61 @@ namespace wg {
 namespace {
 using namespace ntt;
 
-template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, bool LAZY, int... RD>
-__device__ __forceinline__ void ntt_rounds(std::integer_sequence<int, RD...>, uint64_t* sm, int sub, int o, int tile,
-                                           uint64_t q, const TwPair* tw) {
-    ((ntt_round<LOGN, FWD, COLS, EB, STAGED, RD, LAZY>(sm, sub, o, tile, q, tw), __syncthreads()), ...);
+// The rounds of one phase on a thread's elements, exchanged through `sm` in between: v enters in the
+// first round's places and leaves in the last one's.  `sm` may still be read by others on entry.
+template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int TL, int RD, class Arith>
+__device__ __forceinline__ void ntt_round(uint64_t* sm, typename Arith::V* v, int sub, int o, int tile,
+                                          const Arith& ar, const TwPair* tw) {
+    if constexpr (RD > 0) {
+        __syncthreads();
+        Round<LOGN, FWD, COLS, EB, STAGED, RD - 1, TL>::template scatter<Arith>(sm, sub, o, v);
+        __syncthreads();
+        Round<LOGN, FWD, COLS, EB, STAGED, RD, TL>::template gather<Arith>(sm, sub, o, v);
+    }
+    Round<LOGN, FWD, COLS, EB, STAGED, RD, TL>::stages(v, sub, o, tile, ar, tw);
+}
+template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int TL, class Arith, int... RD>
+__device__ __forceinline__ void ntt_rounds(std::integer_sequence<int, RD...>, uint64_t* sm, typename Arith::V* v,
+                                           int sub, int o, int tile, const Arith& ar, const TwPair* tw) {
+    (ntt_round<LOGN, FWD, COLS, EB, STAGED, TL, RD>(sm, v, sub, o, tile, ar, tw), ...);
+}
+
+// A thread's elements of a round to and from one limb.  A run of consecutive words (the row phase's
+// last bits) goes in whole 32-byte sectors where the limb is aligned to them: a word at a time, every
+// access of a warp would touch 32 sectors for a quarter of each.
+template <class R>
+__device__ __forceinline__ void load_words(const uint64_t* __restrict__ p, uint64_t* w) {
+    if (R::RUN && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < R::E; j += 4)
+            asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];\n"
+                         : "=l"(w[j]), "=l"(w[j + 1]), "=l"(w[j + 2]), "=l"(w[j + 3])
+                         : "l"(p + j)
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < R::E; ++j) w[j] = p[R::limb_step(j)];
+    }
+}
+template <class R>
+__device__ __forceinline__ void store_words(uint64_t* __restrict__ p, const uint64_t* w) {
+    if (R::RUN && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < R::E; j += 4)
+            asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};\n" ::"l"(p + j), "l"(w[j]), "l"(w[j + 1]),
+                         "l"(w[j + 2]), "l"(w[j + 3])
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < R::E; ++j) p[R::limb_step(j)] = w[j];
+    }
+}
+
+// Words of a word-arithmetic limb on their way out of its last phase.
+__device__ __forceinline__ uint64_t word_store(bool last, bool fwd, uint64_t v, const Modulus& m) {
+    if (!last) return v;
+    if (!fwd) return mul_shoup(v, m.n_inv, m.n_inv_shoup, m.q);
+    return m.q < kLazyForwardLimit ? reduce64(v, m) : red4q(v, m.q);
 }
 
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED>
@@ -53,6 +109,26 @@ constexpr int min_blocks() {
     return 4;
 }
 
+// The twiddle pairs a CTA reads, copied to shared memory in twiddle_src order.
+template <int LOGN, bool FWD, bool COLS, int EB>
+__device__ __forceinline__ void stage_twiddles(const TwPair* __restrict__ tw, TwPair* tw_s, int tile, int t) {
+    using P = Phase<LOGN, FWD, COLS, EB, true>;
+    const ulonglong2* src2 = reinterpret_cast<const ulonglong2*>(tw);
+    ulonglong2* dst2 = reinterpret_cast<ulonglong2*>(tw_s);
+    if (COLS) {
+        for (int e = t; e < P::TW; e += P::THREADS) dst2[e] = __ldg(src2 + e);
+    } else {
+        // row-stage k: SUBS * 2^k contiguous table entries
+#pragma unroll
+        for (int k = 0; k < P::MB; ++k) {
+            const int cnt = P::SUBS << k;
+            const int dst = P::SUBS * ((1 << k) - 1);
+            const size_t src = ((size_t)1 << (P::NB1 + k)) + (size_t)tile * cnt;
+            for (int e = t; e < cnt; e += P::THREADS) dst2[dst + e] = __ldg(src2 + src + e);
+        }
+    }
+}
+
 // Addressing of one limb: either a strided batch (blockIdx.y = limb, blockIdx.z = polynomial,
 // modulus from a LimbMap) or an entry of a job table (blockIdx.y + 65535 * blockIdx.z).  The
 // first phase may read from a different buffer than it writes (src -> dst); the second phase
@@ -60,18 +136,20 @@ constexpr int min_blocks() {
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, bool TABLE>
 __global__ void __launch_bounds__(Phase<LOGN, FWD, COLS, EB, STAGED>::THREADS, min_blocks<EB>())
     k_ntt_phase(uint64_t* __restrict__ data, size_t poly_stride, LimbMap map, const NttJob* __restrict__ jobs,
-                int njobs, const Modulus* __restrict__ mods, const TwPair* __restrict__ tw_base) {
+                int njobs, const Modulus* __restrict__ mods, const TwPair* __restrict__ tw_base,
+                const TwPair* __restrict__ tw_words) {
     using P = Phase<LOGN, FWD, COLS, EB, STAGED>;
     constexpr int N = P::N;
     constexpr int E = P::E;
     constexpr bool FIRST = FWD ? COLS : !COLS;
     extern __shared__ __align__(16) uint64_t smem[];
-    uint64_t* sm = smem;                                                             // data tile, padded
-    TwPair* tw_s = reinterpret_cast<TwPair*>(smem + P::TILE + P::TILE / 16);        // staged twiddles
+    uint64_t* sm = smem;                                                       // exchange tile, padded
+    TwPair* tw_s = reinterpret_cast<TwPair*>(smem + P::TILE + P::TILE / 16);  // staged twiddles
 
-    const uint64_t* __restrict__ xin;
-    uint64_t* __restrict__ x;
+    const uint64_t* xin;
+    uint64_t* x;
     int mi;
+    bool words = false;
     if (TABLE) {
         const int j = blockIdx.y + 65535 * blockIdx.z;
         if (j >= njobs) return;
@@ -79,64 +157,45 @@ __global__ void __launch_bounds__(Phase<LOGN, FWD, COLS, EB, STAGED>::THREADS, m
         x = job.dst;
         xin = FIRST ? job.src : job.dst;
         mi = job.mod;
+        words = !FWD && !COLS && job.words != 0;
     } else {
         const int limb = blockIdx.y;
         x = data + (size_t)blockIdx.z * poly_stride + (size_t)limb * N;
         xin = x;
         mi = map(limb);
     }
-    const uint64_t q = mods[mi].q;
-    const TwPair* tw = tw_base + (size_t)mi * 2 * N + (FWD ? 0 : N);
+    const Modulus m = mods[mi];
+    const bool fp64 = m.q < fp::kLimit && !words;
+    const TwPair* tw = words ? tw_words + (size_t)mi * N : tw_base + (size_t)mi * 2 * N + (FWD ? 0 : N);
     const int tile = blockIdx.x;
-    const int t = threadIdx.x;
-
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int e = t + k * P::THREADS;
-        sm[pad16(e)] = xin[tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, e)];
-    }
+    const int t = threadIdx.x, sub = P::sub_of(t), o = P::o_of(t);
+    using Begin = Round<LOGN, FWD, COLS, EB, STAGED, 0>;
+    using End = Round<LOGN, FWD, COLS, EB, STAGED, P::ROUNDS - 1>;
+    uint64_t w[E];
+    load_words<Begin>(xin + tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, Begin::element(sub, o)), w);
     if (STAGED) {
-        const ulonglong2* src2 = reinterpret_cast<const ulonglong2*>(tw);
-        ulonglong2* dst2 = reinterpret_cast<ulonglong2*>(tw_s);
-        if (COLS) {
-            for (int e = t; e < P::TW; e += P::THREADS) dst2[e] = __ldg(src2 + e);
-        } else {
-            // row-stage k: SUBS * 2^k contiguous table entries (twiddle_src order)
-#pragma unroll
-            for (int k = 0; k < P::MB; ++k) {
-                const int cnt = P::SUBS << k;
-                const int dst = P::SUBS * ((1 << k) - 1);
-                const size_t src = ((size_t)1 << (P::NB1 + k)) + (size_t)tile * cnt;
-                for (int e = t; e < cnt; e += P::THREADS) dst2[dst + e] = __ldg(src2 + src + e);
-            }
-        }
+        stage_twiddles<LOGN, FWD, COLS, EB>(tw, tw_s, tile, t);
+        __syncthreads();
     }
-    __syncthreads();
-
-    const int sub = COLS ? t % P::SUBS : t >> P::OB;
-    const int o = COLS ? t / P::SUBS : t & ((1 << P::OB) - 1);
     const TwPair* twr = STAGED ? tw_s : tw;
-    // forward transforms under kLazyForwardLimit skip the per-butterfly reduction (uniform per CTA)
-    const bool lazy = FWD && q < kLazyForwardLimit;
-    if (lazy)
-        ntt_rounds<LOGN, FWD, COLS, EB, STAGED, true>(std::make_integer_sequence<int, P::ROUNDS>{}, sm, sub, o, tile,
-                                                      q, twr);
-    else
-        ntt_rounds<LOGN, FWD, COLS, EB, STAGED, false>(std::make_integer_sequence<int, P::ROUNDS>{}, sm, sub, o, tile,
-                                                       q, twr);
-
-    uint64_t n_inv = 0, n_inv_s = 0;
-    if (P::LAST && !FWD) {
-        n_inv = mods[mi].n_inv;
-        n_inv_s = mods[mi].n_inv_shoup;
-    }
+    constexpr auto rounds = std::make_integer_sequence<int, P::ROUNDS>{};
+    if (fp64) {
+        double v[E];
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int e = t + k * P::THREADS;
-        uint64_t val = sm[pad16(e)];
-        if (P::LAST) val = FWD ? (lazy ? reduce64(val, mods[mi]) : red4q(val, q)) : mul_shoup(val, n_inv, n_inv_s, q);
-        x[tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, e)] = val;
+        for (int j = 0; j < E; ++j) v[j] = fp::bits_double(fp_load(FIRST, w[j], m));
+        ntt_rounds<LOGN, FWD, COLS, EB, STAGED, kMaxTile>(rounds, sm, v, sub, o, tile, fp_arith(m), twr);
+#pragma unroll
+        for (int j = 0; j < E; ++j) w[j] = fp_store(P::LAST, FWD, fp::double_bits(v[j]), m);
+    } else {
+        // forward transforms under kLazyForwardLimit skip the per-butterfly reduction
+        if (FWD && m.q < kLazyForwardLimit)
+            ntt_rounds<LOGN, FWD, COLS, EB, STAGED, kMaxTile>(rounds, sm, w, sub, o, tile, WordArith<FWD>{m.q}, twr);
+        else
+            ntt_rounds<LOGN, FWD, COLS, EB, STAGED, kMaxTile>(rounds, sm, w, sub, o, tile, WordArith<false>{m.q}, twr);
+#pragma unroll
+        for (int j = 0; j < E; ++j) w[j] = word_store(P::LAST, FWD, w[j], m);
     }
+    store_words<End>(x + tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, End::element(sub, o)), w);
 }
 
 // The forward row phase of one job-table limb with an element-wise epilogue (NttEpiJob): the
@@ -200,42 +259,44 @@ __global__ void __launch_bounds__(Phase<LOGN, true, false, EB, STAGED>::THREADS,
         }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int e = t + k * P::THREADS;
-        sm[pad16(e)] = job.data[tile_offset<LOGN, true, false, EB, STAGED>(tile, e)];
-    }
+    using Begin = Round<LOGN, true, false, EB, STAGED, 0>;
+    using End = Round<LOGN, true, false, EB, STAGED, P::ROUNDS - 1>;
+    const int sub = P::sub_of(t), o = P::o_of(t);
+    uint64_t w[E];
+    load_words<Begin>(job.data + base + Begin::element(sub, o), w);
     if (STAGED) {
-        const ulonglong2* src2 = reinterpret_cast<const ulonglong2*>(tw);
-        ulonglong2* dst2 = reinterpret_cast<ulonglong2*>(tw_s);
-#pragma unroll
-        for (int k = 0; k < P::MB; ++k) {
-            const int cnt = P::SUBS << k;
-            const int dst = P::SUBS * ((1 << k) - 1);
-            const size_t src = ((size_t)1 << (P::NB1 + k)) + (size_t)tile * cnt;
-            for (int e = t; e < cnt; e += P::THREADS) dst2[dst + e] = __ldg(src2 + src + e);
-        }
+        stage_twiddles<LOGN, true, false, EB>(tw, tw_s, tile, t);
+        __syncthreads();
     }
-    __syncthreads();
-    const int sub = t >> P::OB;
-    const int o = t & ((1 << P::OB) - 1);
     const TwPair* twr = STAGED ? tw_s : tw;
-    const bool lazy = m.q < kLazyForwardLimit;
-    if (lazy)
-        ntt_rounds<LOGN, true, false, EB, STAGED, true>(std::make_integer_sequence<int, P::ROUNDS>{}, sm, sub, o, tile,
-                                                       m.q, twr);
-    else
-        ntt_rounds<LOGN, true, false, EB, STAGED, false>(std::make_integer_sequence<int, P::ROUNDS>{}, sm, sub, o,
-                                                        tile, m.q, twr);
+    constexpr auto rounds = std::make_integer_sequence<int, P::ROUNDS>{};
+    const bool fp64 = m.q < fp::kLimit;
+    // the last round's values through the tile once more, so that the epilogue's accesses are
+    // consecutive over a warp as its operands' copies are
+    if (fp64) {
+        double v[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = fp::bits_double(w[j]);
+        ntt_rounds<LOGN, true, false, EB, STAGED, kMaxTile>(rounds, sm, v, sub, o, tile, fp_arith(m), twr);
+        __syncthreads();
+        End::template scatter<FpArith>(sm, sub, o, v);
+    } else {
+        if (m.q < kLazyForwardLimit)
+            ntt_rounds<LOGN, true, false, EB, STAGED, kMaxTile>(rounds, sm, w, sub, o, tile, WordArith<true>{m.q}, twr);
+        else
+            ntt_rounds<LOGN, true, false, EB, STAGED, kMaxTile>(rounds, sm, w, sub, o, tile, WordArith<false>{m.q}, twr);
+        __syncthreads();
+        End::template scatter<WordArith<false>>(sm, sub, o, w);
+    }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    const uint64_t q = m.q;
+    const FpEpilogue c = fp64 ? fp_epilogue(job, m) : FpEpilogue{};
 #pragma unroll
     for (int k = 0; k < E; ++k) {
         const int e = t + k * P::THREADS;
-        const uint64_t raw = sm[pad16(e)];
-        const uint64_t v = lazy ? reduce64(raw, m) : red4q(raw, q);
-        job.out[base + e] = epilogue_value(job, need_acc ? acc_s[e] : 0, need_in ? in_s[e] : 0, v, q);
+        const uint64_t x = sm[pad16(e)], acc = need_acc ? acc_s[e] : 0, in = need_in ? in_s[e] : 0;
+        job.out[base + e] = fp64 ? fp_epilogue_value(job, c, acc, in, x, m)
+                                 : epilogue_value(job, acc, in, word_store(true, true, x, m), m.q);
     }
 }
 
@@ -249,8 +310,7 @@ void launch_rows_epi(const Context& c, const NttEpiJob* jobs, int njobs, cudaStr
     }();
     (void)opted;
     const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
-    k_ntt_rows_epi<LOGN, EB, STAGED><<<grid, P::THREADS, sm, s>>>(jobs, njobs, c.d_mod,
-                                                                  reinterpret_cast<const TwPair*>(c.d_tw));
+    k_ntt_rows_epi<LOGN, EB, STAGED><<<grid, P::THREADS, sm, s>>>(jobs, njobs, c.d_mod, c.twiddles(EB));
 }
 
 template <int LOGN>
@@ -279,7 +339,7 @@ void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t 
                  const NttJob* jobs, int njobs, cudaStream_t s) {
     using P = Phase<LOGN, FWD, COLS, EB, STAGED>;
     constexpr size_t sm = smem_bytes<LOGN, FWD, COLS, EB, STAGED>();
-    const TwPair* tw = reinterpret_cast<const TwPair*>(c.d_tw);
+    const TwPair* tw = c.twiddles(EB);
     if (jobs) {
         enable_smem<LOGN, FWD, COLS, EB, STAGED, true>();
         const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
@@ -287,13 +347,14 @@ void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t 
         // per residue for each of the two phases (16 N B per limb-transform)
         Probe probe(kClsNtt, 8.0 * P::N * njobs, s);
         k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, true><<<grid, P::THREADS, sm, s>>>(nullptr, 0, map, jobs, njobs,
-                                                                                   c.d_mod, tw);
+                                                                                   c.d_mod, tw,
+                                                                                   c.d_tw_words + (EB - 3) * c.nq * c.N);
     } else {
         enable_smem<LOGN, FWD, COLS, EB, STAGED, false>();
         const dim3 grid(P::N / P::TILE, limbs, polys);
         Probe probe(kClsNtt, 8.0 * P::N * limbs * polys, s);
         k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, false><<<grid, P::THREADS, sm, s>>>(data, stride, map, nullptr, 0,
-                                                                                    c.d_mod, tw);
+                                                                                    c.d_mod, tw, nullptr);
     }
 }
 

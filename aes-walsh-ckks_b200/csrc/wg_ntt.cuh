@@ -6,15 +6,17 @@
 #include <utility>
 
 #include "wg_arith.cuh"
+#include "wg_fp.cuh"
 
 namespace wg {
 namespace ntt {
 
 constexpr int kMaxTile = 2048;
 
-// One entry of the interleaved twiddle table: the twiddle and its Shoup constant side by side,
-// so a butterfly fetches both with one 16-byte load.  Table layout per modulus:
-// [forward pairs (N)][inverse pairs (N)].
+// One entry of the interleaved twiddle table: the twiddle and its Shoup constant (for the moduli of
+// the FP64 path: the doubles w and w / q, twiddle_pairs) side by side, so a butterfly fetches both
+// with one 16-byte load.  Table layout per modulus:
+// [forward pairs (N)][inverse pairs (N)], one table per residues-per-thread (twiddle_pairs).
 struct alignas(16) TwPair {
     uint64_t w, ws;
 };
@@ -32,7 +34,10 @@ WG_HD int insert_zero(int v, int g) {
 }
 
 // Bits handled by one round: up to EB stage bits (in processing order) plus filler bits (the
-// lowest free bits) so every thread always owns 2^EB elements.
+// lowest free bits) so every thread always owns 2^EB elements.  The forward transform's rounds go
+// down from the highest bit in groups of EB, the last one taking what is left; the inverse's rounds
+// are the same groups from the last to the first, so a thread owns the same elements in the
+// inverse's last round as in the forward's first.
 struct RoundPlan {
     int ns;
     int sb[4];  // stage bits, processing order
@@ -43,9 +48,10 @@ struct RoundPlan {
 template <int MB, bool FWD, int EB>
 WG_HDC constexpr RoundPlan make_plan(int rd) {
     RoundPlan p{0, {0, 0, 0, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}};
+    const int fr = FWD ? rd : (MB + EB - 1) / EB - 1 - rd;  // the forward round with the same group
     for (int k = 0; k < EB; ++k) {
-        const int b = FWD ? MB - 1 - EB * rd - k : EB * rd + k;
-        if (b >= 0 && b < MB) p.sb[p.ns++] = b;
+        const int b = MB - 1 - EB * fr - (FWD ? k : EB - 1 - k);
+        if (b >= 0) p.sb[p.ns++] = b;
     }
     int mask = 0;
     for (int k = 0; k < p.ns; ++k) mask |= 1 << p.sb[k];
@@ -66,7 +72,9 @@ WG_HDC constexpr RoundPlan make_plan(int rd) {
 
 // Geometry of one phase of an N = 2^LOGN transform.
 //   EB:     a thread carries 2^EB residues through each round (3: radix-8 rounds of up to three
-//           stages; 4: radix-16 rounds of up to four), so a round is one shared-memory round trip;
+//           stages; 4: radix-16 rounds of up to four).  They come from device memory into the first
+//           round's registers and leave from the last one's; between rounds the CTA exchanges them
+//           through shared memory;
 //   STAGED: the CTA first copies the twiddle pairs it will read into shared memory; otherwise
 //           the rounds read them from the (L2-resident) global table directly, which leaves
 //           shared memory to the data tile and admits more CTAs per SM.
@@ -84,6 +92,8 @@ struct Phase {
     static constexpr int OB = MB - EB;
     static constexpr int ROUNDS = (MB + EB - 1) / EB;
     static constexpr bool LAST = FWD ? !COLS : COLS;
+    WG_HD static int sub_of(int t) { return COLS ? t % SUBS : t >> OB; }
+    WG_HD static int o_of(int t) { return COLS ? t / SUBS : t & ((1 << OB) - 1); }
     // Twiddle pairs one CTA reads (staged in shared memory when STAGED): the column phase reads
     // table entries [0, 2^NB1); the row phase reads, for row-stage k, SUBS * 2^k contiguous
     // entries.
@@ -120,85 +130,175 @@ WG_HDC constexpr int round_bits(const RoundPlan& p, int j) {
 constexpr uint64_t kLazyForwardLimit = uint64_t{1} << 58;
 static_assert((4 + 2 * 16) < (1 << (64 - 58)), "lazy forward bound: 36 q < 2^64 for q < 2^58");
 
-// One round (up to EB radix-2 stages) for thread (sub, o) of tile `tile`.  `tw` is the CTA's
-// staged block (STAGED, twiddle_src order) or the modulus's table of this direction.  LAZY
-// (forward only, q < kLazyForwardLimit) keeps the upper value unreduced through the round.
+// The arithmetic of a round: the value a thread carries (as the word kept in shared memory), the
+// butterflies of both directions, and the reductions a round needs at its stages' starts.
 //
-// The thread's elements are base | round_bits(j), with base's bits disjoint from the group
-// positions, so every index splits into a runtime part (one per round, or one per stage for
-// twiddles) plus a compile-time offset: pad16 and shifts distribute over disjoint bit sets.
-// Loads then use immediate offsets, and butterflies of a stage that share a twiddle load it
-// once (same address).
-template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int RD, bool LAZY = false, int TL = kMaxTile>
-WG_HD void ntt_round(uint64_t* sm, int sub, int o, int tile, uint64_t q, const TwPair* __restrict__ tw) {
-    using P = Phase<LOGN, FWD, COLS, EB, STAGED, TL>;
-    constexpr int E = P::E;
-    constexpr RoundPlan plan = make_plan<P::MB, FWD, EB>(RD);
-    const uint64_t two_q = q << 1;
-    int base = o;
-#pragma unroll
-    for (int k = 0; k < EB; ++k) base = insert_zero(base, plan.g[k]);
-    // element index e = COLS ? h * SUBS + sub : (sub << MB) | h, with h = base | round_bits(j)
-    const int e_base = COLS ? base * P::SUBS + sub : (sub << P::MB) | base;
-    uint64_t* row = sm + pad16(e_base);
-    uint64_t v[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-        const int c = COLS ? round_bits<EB>(plan, j) * P::SUBS : round_bits<EB>(plan, j);
-        v[j] = row[pad16(c)];
+// WordArith: 64-bit words, Harvey / Shoup; LAZY (forward only, q < kLazyForwardLimit) keeps the
+// upper value unreduced through the round.
+template <bool LAZY>
+struct WordArith {
+    using V = uint64_t;
+    uint64_t q;
+    WG_HD static V of_bits(uint64_t x) { return x; }
+    WG_HD static uint64_t bits(V v) { return v; }
+    template <bool FWD, int EB, int RD>
+    WG_HD void before_stage(V*, int) const {}
+    WG_HD void forward(V& a, V& b, uint64_t w, uint64_t ws) const {
+        const uint64_t two_q = q << 1;
+        uint64_t t = a;
+        if (!LAZY && t >= two_q) t -= two_q;
+        const uint64_t u = mul_shoup_lazy(b, w, ws, q);
+        a = t + u;
+        b = t + two_q - u;
     }
+    WG_HD void inverse(V& a, V& b, uint64_t w, uint64_t ws) const {
+        const uint64_t two_q = q << 1;
+        const uint64_t t = a, u = b;
+        uint64_t sum = t + u;
+        if (sum >= two_q) sum -= two_q;
+        a = sum;
+        b = mul_shoup_lazy(t - u + two_q, w, ws, q);
+    }
+};
+
+// FpArith: signed integers in FP64 (wg_fp.cuh), q < fp::kLimit; the twiddle pair is (w, w / q).
+// Bounds, in units of q, with values up to B q entering a product leaving at most 1/2 + B q 2^-55
+// (at most 5/8 for B q <= 2^52):
+//   forward, q < kNoReduce (2^42): each stage adds at most 5/8; inputs below 17 q (the base
+//     changes of wg_ksfuse.cuh; 4 q elsewhere) stay below 17 + 16 x 5/8 = 27 q < 2^47.
+//   forward, larger q (`red`): the rounds reduce to 1/2 every six (EB = 3) or four stages;
+//     b -> b + 1/2 + b / 32 takes 1/2 to 3.85 in six stages, below the 4 q <= 2^52 a product takes.
+//   inverse, q < kNoReduce: a sum doubles per stage; words below 4 q entering, and values reduced
+//     to 1/2 between the two phases, stay below 4 x 2^8 q <= 2^52 through 8 stages.
+//   inverse, larger q: values reduced to 1/2 at the start of a round and, for EB = 4, before its
+//     third stage; at most three stages follow, and the sums stay below 4 q <= 2^52.
+struct FpArith {
+    using V = double;
+    double q, inv_q;
+    bool red;  // q >= kNoReduce
+    WG_HD static V of_bits(uint64_t x) { return fp::bits_double(x); }
+    WG_HD static uint64_t bits(V v) { return fp::double_bits(v); }
+    template <bool FWD, int EB, int RD>
+    WG_HD void before_stage(V* v, int s) const {
+        const bool due = FWD ? (s == 0 && (EB == 4 || RD % 2 == 0)) : (s == 0 || (EB == 4 && s == 2));
+        if (due && red) {
 #pragma unroll
-    for (int s = 0; s < plan.ns; ++s) {
-        const int b = plan.sb[s];
-        const int jb = plan.jb[s];
-        // The table index of a pair is (1 << (n-1-gb)) + (x >> (gb+1)) for its global index x
-        // and stage bit gb; relative to the staged block (or to the table) it is:
-        const int kr = P::NB2 - 1 - b;  // row-stage of bit b
-        const size_t base_idx =
-            COLS ? (size_t)(1 << (P::NB1 - 1 - b))
-                 : (STAGED ? (size_t)(P::SUBS * ((1 << kr) - 1) + (sub << kr))
-                           : ((size_t)1 << (P::NB1 + kr)) + (size_t)tile * P::SUBS * ((size_t)1 << kr) +
-                                 (size_t)(sub << kr));
-        const TwPair* tw_st = tw + base_idx + (base >> (b + 1));
+            for (int j = 0; j < (1 << EB); ++j) v[j] = fp::reduce(v[j], q, inv_q);
+        }
+    }
+    WG_HD void forward(V& a, V& b, uint64_t w, uint64_t ws) const {
+        const double t = a, u = fp::mulmod(b, fp::bits_double(w), fp::bits_double(ws), q);
+        a = dadd(t, u);
+        b = dadd(t, -u);
+    }
+    WG_HD void inverse(V& a, V& b, uint64_t w, uint64_t ws) const {
+        const double t = a, u = b;
+        a = dadd(t, u);
+        b = fp::mulmod(dadd(t, -u), fp::bits_double(w), fp::bits_double(ws), q);
+    }
+};
+WG_HD FpArith fp_arith(const Modulus& m) { return FpArith{m.qd, m.inv_q, m.q >= fp::kNoReduce}; }
+
+// Thread (sub, o)'s elements in round RD: base | round_bits(j) within its sub-transform, with base's
+// bits disjoint from the group positions, so every index splits into a runtime part (one per round,
+// or one per stage for twiddles) plus a compile-time offset: pad16, shifts and the tile's offsets
+// distribute over disjoint bit sets.  Accesses then use immediate offsets, and butterflies of a
+// stage that share a twiddle load it once (same address).
+template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int RD, int TL = kMaxTile>
+struct Round {
+    using P = Phase<LOGN, FWD, COLS, EB, STAGED, TL>;
+    static constexpr int E = P::E;
+    // the elements of a thread are consecutive words of the limb
+    static constexpr bool RUN = !COLS && make_plan<P::MB, FWD, EB>(RD).g[EB - 1] == EB - 1;
+    WG_HD static int base(int o) {
+        constexpr RoundPlan plan = make_plan<P::MB, FWD, EB>(RD);
 #pragma unroll
-        for (int j = 0; j < E; ++j) {
-            if ((j >> jb) & 1) continue;
-            const int j1 = j | (1 << jb);
-            const int k = round_bits<EB>(plan, j) >> (b + 1);
+        for (int k = 0; k < EB; ++k) o = insert_zero(o, plan.g[k]);
+        return o;
+    }
+    WG_HD static int element(int sub, int o) { return COLS ? base(o) * P::SUBS + sub : (sub << P::MB) | base(o); }
+    // offsets of element j from element(): in the tile, and in the limb
+    WG_HDC static constexpr int tile_step(int j) {
+        return round_bits<EB>(make_plan<P::MB, FWD, EB>(RD), j) * (COLS ? P::SUBS : 1);
+    }
+    WG_HDC static constexpr size_t limb_step(int j) {
+        return (size_t)round_bits<EB>(make_plan<P::MB, FWD, EB>(RD), j) << (COLS ? P::NB2 : 0);
+    }
+    template <class Arith>
+    WG_HD static void scatter(uint64_t* sm, int sub, int o, const typename Arith::V* v) {
+        uint64_t* row = sm + pad16(element(sub, o));
+#pragma unroll
+        for (int j = 0; j < E; ++j) row[pad16(tile_step(j))] = Arith::bits(v[j]);
+    }
+    template <class Arith>
+    WG_HD static void gather(const uint64_t* sm, int sub, int o, typename Arith::V* v) {
+        const uint64_t* row = sm + pad16(element(sub, o));
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = Arith::of_bits(row[pad16(tile_step(j))]);
+    }
+    // The round's stages (up to EB radix-2 stages) on the thread's elements.  `tw` is the CTA's
+    // staged block (STAGED, twiddle_src order) or the modulus's table of this direction.
+    template <class Arith>
+    WG_HD static void stages(typename Arith::V* v, int sub, int o, int tile, const Arith& ar,
+                             const TwPair* __restrict__ tw) {
+        constexpr RoundPlan plan = make_plan<P::MB, FWD, EB>(RD);
+        const int b0 = base(o);
+#pragma unroll
+        for (int s = 0; s < plan.ns; ++s) {
+            ar.template before_stage<FWD, EB, RD>(v, s);
+            const int b = plan.sb[s];
+            const int jb = plan.jb[s];
+            // The table index of a pair is (1 << (n-1-gb)) + (x >> (gb+1)) for its global index x
+            // and stage bit gb; relative to the staged block (or to the table) it is:
+            const int kr = P::NB2 - 1 - b;  // row-stage of bit b
+            const size_t base_idx =
+                COLS ? (size_t)(1 << (P::NB1 - 1 - b))
+                     : (STAGED ? (size_t)(P::SUBS * ((1 << kr) - 1) + (sub << kr))
+                               : ((size_t)1 << (P::NB1 + kr)) + (size_t)tile * P::SUBS * ((size_t)1 << kr) +
+                                     (size_t)(sub << kr));
+            // (in the round of the lowest bits the table is in row_order: thread-minor)
+            const TwPair* tw_st = tw + base_idx + (RUN ? o : b0 >> (b + 1));
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                if ((j >> jb) & 1) continue;
+                const int j1 = j | (1 << jb);
+                const int k = (round_bits<EB>(plan, j) >> (b + 1)) << (RUN ? P::OB : 0);
 #if defined(__CUDA_ARCH__)
-            uint64_t w, ws;
-            if (STAGED) {
-                const TwPair tp = tw_st[k];
-                w = tp.w;
-                ws = tp.ws;
-            } else {
-                const ulonglong2 tp = __ldg(reinterpret_cast<const ulonglong2*>(tw_st + k));
-                w = tp.x;
-                ws = tp.y;
-            }
+                uint64_t w, ws;
+                if (STAGED) {
+                    const TwPair tp = tw_st[k];
+                    w = tp.w;
+                    ws = tp.ws;
+                } else {
+                    const ulonglong2 tp = __ldg(reinterpret_cast<const ulonglong2*>(tw_st + k));
+                    w = tp.x;
+                    ws = tp.y;
+                }
 #else
-            const uint64_t w = tw_st[k].w, ws = tw_st[k].ws;
+                const uint64_t w = tw_st[k].w, ws = tw_st[k].ws;
 #endif
-            if (FWD) {
-                uint64_t t = v[j];
-                if (!LAZY && t >= two_q) t -= two_q;
-                const uint64_t u = mul_shoup_lazy(v[j1], w, ws, q);
-                v[j] = t + u;
-                v[j1] = t + two_q - u;
-            } else {
-                const uint64_t t = v[j], u = v[j1];
-                uint64_t sum = t + u;
-                if (sum >= two_q) sum -= two_q;
-                v[j] = sum;
-                v[j1] = mul_shoup_lazy(t - u + two_q, w, ws, q);
+                if (FWD)
+                    ar.forward(v[j], v[j1], w, ws);
+                else
+                    ar.inverse(v[j], v[j1], w, ws);
             }
         }
     }
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-        const int c = COLS ? round_bits<EB>(plan, j) * P::SUBS : round_bits<EB>(plan, j);
-        row[pad16(c)] = v[j];
-    }
+};
+
+// Words of an FP64 transform on their way in and out of a phase.  Between the two phases (and the
+// fused kernels' steps) a limb holds the bits of the doubles; the inverse transform's first phase
+// reduces them there when its rounds do not (q < kNoReduce).
+WG_HD uint64_t fp_load(bool first, uint64_t x, const Modulus& m) {
+    if (!first) return x;
+    if (x >> 52) x = reduce64(x, m);  // words of 4 q and more, which the forward transform accepts
+    return fp::double_bits(fp::from_word(x));
+}
+WG_HD uint64_t fp_store(bool last, bool fwd, uint64_t x, const Modulus& m) {
+    const double v = fp::bits_double(x);
+    if (!last) return !fwd && m.q < fp::kNoReduce ? fp::double_bits(fp::reduce(v, m.qd, m.inv_q)) : x;
+    if (fwd) return fp::canonical(v, m.qd, m.inv_q);
+    return fp::to_word(fp::lift(fp::mulmod(v, m.n_inv_w, m.n_inv_wq, m.qd), m.qd));
 }
 
 // The forward row phase of one limb (data: after the forward column phase, read only) with an
@@ -248,11 +348,58 @@ WG_HD size_t tile_offset(int tile, int e) {
     return (size_t)tile * P::TILE + e;
 }
 
-// Interleaved twiddle table (TwPair layout above) from the split one [fwd, fwd_shoup, inv,
-// inv_shoup][N] of one modulus.
-inline void interleave_twiddles(size_t N, const uint64_t* split, TwPair* out) {
-    for (size_t d = 0; d < 2; ++d)
-        for (size_t i = 0; i < N; ++i) out[d * N + i] = TwPair{split[2 * d * N + i], split[(2 * d + 1) * N + i]};
+// The epilogue of an FP64 transform: v is the unreduced value of the last row phase's word.  The
+// rescale's product runs in FP64 as well; the combine keeps the word arithmetic, because `in` may
+// hold a word in [q, 2q) (a product with a single Barrett correction) that add_mod carries on.
+struct FpEpilogue {
+    double w, wq;
+};
+WG_HD FpEpilogue fp_epilogue(const NttEpiJob& j, const Modulus& m) {
+    FpEpilogue c{0.0, 0.0};
+    if (j.kind == kEpiRescale) fp::factor_of(j.c0, m.qd, m.inv_q, c.w, c.wq);
+    return c;
+}
+WG_HD uint64_t fp_epilogue_value(const NttEpiJob& j, const FpEpilogue& c, uint64_t acc, uint64_t in, uint64_t x,
+                                 const Modulus& m) {
+    const double v = fp::reduce(fp::bits_double(x), m.qd, m.inv_q);
+    if (j.kind == kEpiRescale) {
+        // |in - v| <= 2.5 q < 2^52: the product is below q in magnitude (factor_of)
+        const double d = dadd(fp::from_word(in), -v);
+        return fp::to_word(fp::lift(fp::mulmod(d, c.w, c.wq, m.qd), m.qd));
+    }
+    return epilogue_value(j, acc, in, fp::to_word(fp::lift(v, m.qd)), m.q);
+}
+
+// The place of twiddle x of a row (of the 2^kr of row-stage kr = NB2 - 1 - b) in the table.  In the
+// round of a row's lowest bits thread o uses the 2^(eb-1-b) consecutive twiddles from o << (eb-1-b),
+// so over a warp each of these loads would touch a 128-byte line per lane; there they stand
+// thread-minor.
+inline size_t row_order(int nb2, int eb, int b, size_t x) {
+    const int last = nb2 - eb * ((nb2 + eb - 1) / eb - 1);  // stages of that round
+    if (b >= last) return x;
+    const int kb = eb - 1 - b, ob = nb2 - eb;
+    return ((x & (((size_t)1 << kb) - 1)) << ob) | (x >> kb);
+}
+
+// The table a modulus q is transformed with by the geometries of 2^eb residues per thread, one
+// direction, from the split (w, Shoup w) words: the factor pairs (w, w / q) as bits of doubles for the
+// moduli of the FP64 path (unless `words`), the words otherwise; rows in row_order.
+inline void twiddle_pairs(size_t N, uint64_t q, const uint64_t* w, const uint64_t* ws, int eb, bool words, TwPair* out) {
+    const bool fp64 = q < fp::kLimit && !words;
+    const int n = floor_log2((unsigned)N), nb1 = n / 2, nb2 = n - nb1;
+    auto put = [&](size_t to, size_t from) {
+        double f = 0, fq = 0;
+        if (fp64) fp::factor(w[from], q, f, fq);
+        out[to] = fp64 ? TwPair{fp::double_bits(f), fp::double_bits(fq)} : TwPair{w[from], ws[from]};
+    };
+    for (size_t i = 0; i < ((size_t)1 << nb1); ++i) put(i, i);
+    for (int kr = 0; kr < nb2; ++kr) {
+        const size_t stage = (size_t)1 << (nb1 + kr);
+        for (size_t i = 0; i < stage; ++i) {
+            const size_t row = i >> kr, x = i & (((size_t)1 << kr) - 1);
+            put(stage + (row << kr) + row_order(nb2, eb, nb2 - 1 - kr, x), stage + i);
+        }
+    }
 }
 
 }  // namespace ntt

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "wg_fp.cuh"
 #include "wg_internal.hpp"
 #include "wg_tables.hpp"
 
@@ -30,6 +31,15 @@ struct TableImage {
             words.push_back(w);
         }
         return off;
+    }
+    // FP64 factor pairs of residues v[i] modulo q[i], 16-byte aligned, for products with source limbs
+    // modulo p[i % p.size()]; zero for the moduli that the FP64 path does not take
+    size_t put_factors(const std::vector<uint64_t>& v, const std::vector<uint64_t>& q, const std::vector<uint64_t>& p) {
+        if (words.size() & 1) words.push_back(0);
+        std::vector<double> d(2 * v.size(), 0.0);
+        for (size_t i = 0; i < v.size(); ++i)
+            if (q[i] < fp::kLimit) fp::term_factor(v[i], p[i % p.size()], q[i], d[2 * i], d[2 * i + 1]);
+        return put(d);
     }
     size_t put(const std::vector<int>& v) {  // two ints per word
         const size_t off = words.size();
@@ -69,6 +79,8 @@ HostTables build_tables(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
         host::ntt_tables(N, m, t, t + N, t + 2 * N, t + 3 * N, md.n_inv);
         md.n_inv_shoup = host::shoup(md.n_inv, m);
         md.inv_q = 1.0 / (double)m;
+        md.qd = (double)m;
+        fp::factor(md.n_inv, m, md.n_inv_w, md.n_inv_wq);
     }
 
     TableImage img{H.words};
@@ -135,12 +147,18 @@ HostTables build_tables(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
             o.corr = img.put(corr);
             o.dst_limb = img.put(dst_limb);
             o.dst_mod = img.put(dst_mod);
+            std::vector<uint64_t> scale(sc), qhat_q(dc * sc);
+            for (size_t i = 0; i < sc; ++i) scale[i] = host::mulmod(H.mods[s0 + i].n_inv, qhat_inv[i], src[i]);
+            for (size_t t = 0; t < dc; ++t) std::fill_n(qhat_q.begin() + t * sc, sc, dst[t]);
+            o.scale_fp = img.put_factors(scale, src, src);
+            o.qhat_fp = img.put_factors(qhat, qhat_q, src);
             H.modup[level].push_back(o);
         }
     }
     // Folded ModDown constants per level.
     H.fold_inv.resize(nq);
     H.fold_inv_s.resize(nq);
+    H.fold_fp.resize(nq);
     for (size_t level = 0; level < nq; ++level) {
         std::vector<uint64_t> inv((level + 1) * np), inv_s((level + 1) * np);
         for (size_t qi = 0; qi <= level; ++qi)
@@ -151,6 +169,9 @@ HostTables build_tables(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
             }
         H.fold_inv[level] = img.put(inv);
         H.fold_inv_s[level] = img.put(inv_s);
+        std::vector<uint64_t> of((level + 1) * np);
+        for (size_t qi = 0; qi <= level; ++qi) std::fill_n(of.begin() + qi * np, np, q[qi]);
+        H.fold_fp[level] = img.put_factors(inv, of, std::vector<uint64_t>(p, p + np));
     }
     // Rescale constants per dropped limb.
     H.rescale.assign(nq, 0);

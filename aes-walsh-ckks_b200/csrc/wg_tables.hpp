@@ -13,6 +13,7 @@ namespace wg {
 struct ModUpOffsets {
     int src_count, dst_count, src_first;
     size_t qhat_inv, qhat_inv_s, src_inv, qhat, qhat_s, corr, dst_limb, dst_mod;
+    size_t scale_fp, qhat_fp;  // FP64 factor pairs: [src] N^-1 qhat_inv, [dst][src] qhat
 };
 
 struct HostTables {
@@ -22,7 +23,8 @@ struct HostTables {
     std::vector<uint64_t> tw;                      // [mod][4][N]
     std::vector<uint64_t> words;                   // small tables, addressed by word offsets
     std::vector<std::vector<ModUpOffsets>> modup;  // [level][part]
-    std::vector<size_t> fold_inv, fold_inv_s;      // [level] -> [(level+1)][np]
+    // [level] -> [(level+1)][np]; fold_fp: the same values as FP64 factor pairs
+    std::vector<size_t> fold_inv, fold_inv_s, fold_fp;
     std::vector<size_t> rescale;                   // [d] -> one_s[d], inv_p[d], inv_p_s[d], half[d]
 };
 

@@ -160,10 +160,9 @@ int wg_ntt_set_geometry(wg_context* ctx, int direction, int phase, int geometry)
  * epilogue of the last forward row phase.  ckks_hybrid_key_switch_inplace
  * (src/ckks/operations/keyswitch/ckks_keyswitch.cpp:1330-1641) and ckks_rescale
  * (src/ckks/operations/arith/ckks_rescale.cpp:68-148) compute the same words step by step.
- * mode 1 (the default) fuses a step when its launch fills the device at least twice (the fused
- * kernels run one 128-thread block per job and 1024-coefficient column tile), so a single
- * ciphertext keeps the wider separate launches; mode 2 always fuses, mode 0 never.  The words
- * are identical in every mode. */
+ * Launches too small to fill the device divide a job's output limbs over several blocks.  mode 1
+ * (the default) and mode 2 fuse, mode 0 runs the separate launches.  The words are identical in
+ * every mode. */
 int wg_set_ntt_fusion(wg_context* ctx, int mode);
 
 /* Hybrid key switch of key_term at `level` with the installed key (kind, rotation):

@@ -5,7 +5,9 @@
 // thread, so the index logic, butterflies, HPS base changes and tables can be checked against
 // the oracle without a GPU.  Shared-memory rounds are separated exactly where the kernels put
 // __syncthreads().  Not part of the product library.
+#include <array>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 #include <stdexcept>
 #include <vector>
@@ -31,27 +33,62 @@ struct HostModUp {
     const double* src_inv;
     const uint64_t *qhat, *qhat_s, *corr;
     const int *dst_limb, *dst_mod;
+    const ntt::TwPair *scale_fp, *qhat_fp;
 };
 
 struct Emu {
     HostTables H;
     int logN;
     std::vector<std::vector<HostModUp>> modup;
-    std::vector<ntt::TwPair> tw;  // interleaved table of every modulus: [mod][fwd N, inv N]
+    std::vector<ntt::TwPair> tw;  // twiddle pairs of every modulus: [mod][fwd N, inv N]
 };
 
-template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, bool LAZY, int... RD>
-void rounds(std::integer_sequence<int, RD...>, uint64_t* sm, int tile, uint64_t q, const ntt::TwPair* tw) {
-    using P = ntt::Phase<LOGN, FWD, COLS, EB, STAGED>;
-    auto one = [&](auto rd_const) {
-        constexpr int R = decltype(rd_const)::value;
-        for (int t = 0; t < P::THREADS; ++t) {
-            const int sub = COLS ? t % P::SUBS : t >> P::OB;
-            const int o = COLS ? t / P::SUBS : t & ((1 << P::OB) - 1);
-            ntt::ntt_round<LOGN, FWD, COLS, EB, STAGED, R, LAZY>(sm, sub, o, tile, q, tw);
-        }
-    };
-    (one(std::integral_constant<int, RD>{}), ...);
+// The rounds of one phase over a CTA: v[t] are thread t's elements, exchanged through the padded tile
+// where the kernels do (ntt_round, wg_ntt.cu).
+template <class Arith, int E>
+using Lanes = std::vector<std::array<typename Arith::V, E>>;
+
+template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int TL, int RD, class Arith>
+void one_round(uint64_t* sm, Lanes<Arith, 1 << EB>& v, int tile, const Arith& ar, const ntt::TwPair* tw) {
+    using R = ntt::Round<LOGN, FWD, COLS, EB, STAGED, RD, TL>;
+    using P = typename R::P;
+    if constexpr (RD > 0) {
+        for (int t = 0; t < P::THREADS; ++t)
+            ntt::Round<LOGN, FWD, COLS, EB, STAGED, RD - 1, TL>::template scatter<Arith>(sm, P::sub_of(t), P::o_of(t),
+                                                                                       v[t].data());
+        for (int t = 0; t < P::THREADS; ++t) R::template gather<Arith>(sm, P::sub_of(t), P::o_of(t), v[t].data());
+    }
+    for (int t = 0; t < P::THREADS; ++t) R::stages(v[t].data(), P::sub_of(t), P::o_of(t), tile, ar, tw);
+}
+template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int TL, class Arith, int... RD>
+void rounds(std::integer_sequence<int, RD...>, uint64_t* sm, Lanes<Arith, 1 << EB>& v, int tile, const Arith& ar,
+            const ntt::TwPair* tw) {
+    (one_round<LOGN, FWD, COLS, EB, STAGED, TL, RD>(sm, v, tile, ar, tw), ...);
+}
+
+// A limb's tile through one phase: `in` maps a word of the limb to the rounds' bits, `out` back.
+template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int TL, class Arith, class In, class Out>
+void tile_phase(uint64_t* x, int tile, const Arith& ar, const ntt::TwPair* tw, In in, Out out) {
+    using P = ntt::Phase<LOGN, FWD, COLS, EB, STAGED, TL>;
+    using Begin = ntt::Round<LOGN, FWD, COLS, EB, STAGED, 0, TL>;
+    using End = ntt::Round<LOGN, FWD, COLS, EB, STAGED, P::ROUNDS - 1, TL>;
+    std::vector<uint64_t> sm(P::TILE + P::TILE / 16);
+    Lanes<Arith, 1 << EB> v(P::THREADS);
+    for (int t = 0; t < P::THREADS; ++t) {
+        const uint64_t* p = x + ntt::tile_offset<LOGN, FWD, COLS, EB, STAGED, TL>(tile, Begin::element(P::sub_of(t), P::o_of(t)));
+        for (int j = 0; j < P::E; ++j) v[t][j] = Arith::of_bits(in(p[Begin::limb_step(j)]));
+    }
+    rounds<LOGN, FWD, COLS, EB, STAGED, TL>(std::make_integer_sequence<int, P::ROUNDS>{}, sm.data(), v, tile, ar, tw);
+    for (int t = 0; t < P::THREADS; ++t) {
+        uint64_t* p = x + ntt::tile_offset<LOGN, FWD, COLS, EB, STAGED, TL>(tile, End::element(P::sub_of(t), P::o_of(t)));
+        for (int j = 0; j < P::E; ++j) p[End::limb_step(j)] = out(Arith::bits(v[t][j]));
+    }
+}
+
+uint64_t word_store(bool last, bool fwd, uint64_t v, const Modulus& m) {
+    if (!last) return v;
+    if (!fwd) return mul_shoup(v, m.n_inv, m.n_inv_shoup, m.q);
+    return m.q < ntt::kLazyForwardLimit ? reduce64(v, m) : red4q(v, m.q);
 }
 
 // NTT geometry the emulated phases use (the device's kNttGeometries order: 0 = 8 residues per
@@ -59,42 +96,42 @@ void rounds(std::integer_sequence<int, RD...>, uint64_t* sm, int tile, uint64_t 
 int g_geometry = 0;
 
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED>
-void phase(const Emu& E, uint64_t* x, int mi) {
+void phase(const Emu& E, uint64_t* x, int mi, bool epilogue) {
     using P = ntt::Phase<LOGN, FWD, COLS, EB, STAGED>;
     const size_t N = P::N;
-    std::vector<ntt::TwPair> table(2 * N);
-    ntt::interleave_twiddles(N, E.H.tw.data() + (size_t)mi * 4 * N, table.data());
-    const ntt::TwPair* tw = table.data() + (FWD ? 0 : N);
+    std::vector<ntt::TwPair> table(N);
+    const uint64_t* w = E.H.tw.data() + ((size_t)mi * 4 + (FWD ? 0 : 2)) * N;
+    ntt::twiddle_pairs(N, E.H.mods[mi].q, w, w + N, EB, false, table.data());
+    const ntt::TwPair* tw = table.data();
     const Modulus& md = E.H.mods[mi];
-    std::vector<uint64_t> sm(P::TILE + P::TILE / 16);
+    const bool fp64 = md.q < fp::kLimit, lazy = FWD && md.q < ntt::kLazyForwardLimit;
+    const bool first = FWD ? COLS : !COLS;
     std::vector<ntt::TwPair> tw_s(P::TW);
+    const auto out = [&](uint64_t v) { return word_store(P::LAST, FWD, v, md); };
+    const auto same = [](uint64_t v) { return v; };
     for (int tile = 0; tile < (int)(N / P::TILE); ++tile) {
-        for (int e = 0; e < P::TILE; ++e) sm[ntt::pad16(e)] = x[ntt::tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, e)];
         if (STAGED)
             for (int e = 0; e < P::TW; ++e) tw_s[e] = tw[ntt::twiddle_src<LOGN, FWD, COLS, EB, STAGED>(tile, e)];
         const ntt::TwPair* twr = STAGED ? tw_s.data() : tw;
-        const bool lazy = FWD && md.q < ntt::kLazyForwardLimit;
-        if (lazy)
-            rounds<LOGN, FWD, COLS, EB, STAGED, true>(std::make_integer_sequence<int, P::ROUNDS>{}, sm.data(), tile, md.q,
-                                                      twr);
+        if (fp64)
+            tile_phase<LOGN, FWD, COLS, EB, STAGED, ntt::kMaxTile>(
+                x, tile, ntt::fp_arith(md), twr, [&](uint64_t v) { return ntt::fp_load(first, v, md); },
+                [&](uint64_t v) { return epilogue ? v : ntt::fp_store(P::LAST, FWD, v, md); });
+        else if (lazy)
+            tile_phase<LOGN, FWD, COLS, EB, STAGED, ntt::kMaxTile>(x, tile, ntt::WordArith<true>{md.q}, twr, same, out);
         else
-            rounds<LOGN, FWD, COLS, EB, STAGED, false>(std::make_integer_sequence<int, P::ROUNDS>{}, sm.data(), tile,
-                                                       md.q, twr);
-        for (int e = 0; e < P::TILE; ++e) {
-            uint64_t v = sm[ntt::pad16(e)];
-            if (P::LAST) v = FWD ? (lazy ? reduce64(v, md) : red4q(v, md.q)) : mul_shoup(v, md.n_inv, md.n_inv_shoup, md.q);
-            x[ntt::tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, e)] = v;
-        }
+            tile_phase<LOGN, FWD, COLS, EB, STAGED, ntt::kMaxTile>(x, tile, ntt::WordArith<false>{md.q}, twr, same, out);
     }
 }
 
+// epilogue: leave an FP64 limb's last words to the caller's epilogue (k_ntt_rows_epi)
 template <int LOGN, bool FWD, bool COLS>
-void phase_geom(const Emu& E, uint64_t* x, int mi) {
+void phase_geom(const Emu& E, uint64_t* x, int mi, bool epilogue = false) {
     switch (g_geometry) {
-        case 0: phase<LOGN, FWD, COLS, 3, true>(E, x, mi); break;
-        case 1: phase<LOGN, FWD, COLS, 3, false>(E, x, mi); break;
-        case 2: phase<LOGN, FWD, COLS, 4, true>(E, x, mi); break;
-        default: phase<LOGN, FWD, COLS, 4, false>(E, x, mi); break;
+        case 0: phase<LOGN, FWD, COLS, 3, true>(E, x, mi, epilogue); break;
+        case 1: phase<LOGN, FWD, COLS, 3, false>(E, x, mi, epilogue); break;
+        case 2: phase<LOGN, FWD, COLS, 4, true>(E, x, mi, epilogue); break;
+        default: phase<LOGN, FWD, COLS, 4, false>(E, x, mi, epilogue); break;
     }
 }
 
@@ -125,34 +162,70 @@ void ntt_one(const Emu& E, uint64_t* x, int mi, bool fwd) {
 // Key switches and rescales run the fused sequences of wg_ksfuse.cu (Context::ntt_fusion).
 int g_fused = 0;
 
-template <int LOGN, bool FWD, bool LAZY, int... RD>
-void col_rounds(std::integer_sequence<int, RD...>, uint64_t* sm, int tile, uint64_t q, const ntt::TwPair* tw) {
+bool is_fp(const Emu& E, int mi) { return E.H.mods[mi].q < fp::kLimit; }
+
+template <int LOGN, bool FWD, class Arith>
+void columns(Lanes<Arith, 8>& v, int tile, const Arith& ar, const ntt::TwPair* tw) {
     using G = ksf::Geom<LOGN>;
-    auto one = [&](auto rd_const) {
-        constexpr int R = decltype(rd_const)::value;
-        for (int t = 0; t < G::THREADS; ++t) ksf::col_round<LOGN, FWD, R, LAZY>(sm, tile, t, q, tw);
-    };
-    (one(std::integral_constant<int, RD>{}), ...);
+    std::vector<uint64_t> sm(G::PAD);
+    rounds<LOGN, FWD, true, 3, false, ksf::kTile>(std::make_integer_sequence<int, G::ROUNDS>{}, sm.data(), v, tile, ar, tw);
 }
 
-template <int LOGN>
-void inverse_cols(const Emu& E, uint64_t* sm, int tile, int mi) {
+// inverse_slots (wg_ksfuse.cu) of one source limb whose words thread t has at slots[k * THREADS + t].
+template <int LOGN, class ScaleFp, class ScaleWords>
+void inverse_slots(const Emu& E, uint64_t* slots, int tile, int mi, ScaleFp scale_f, ScaleWords scale_w) {
     using G = ksf::Geom<LOGN>;
     const Modulus& m = E.H.mods[mi];
-    col_rounds<LOGN, false, false>(std::make_integer_sequence<int, G::ROUNDS>{}, sm, tile, m.q,
-                                   E.tw.data() + (size_t)mi * 2 * G::N + G::N);
-    for (int t = 0; t < G::THREADS; ++t) ksf::scale_n_inv<LOGN>(sm, t, m);
-}
-
-template <int LOGN>
-void forward_cols(const Emu& E, uint64_t* sm, int tile, int mi) {
-    using G = ksf::Geom<LOGN>;
-    const uint64_t q = E.H.mods[mi].q;
-    const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * G::N;
-    if (q < ntt::kLazyForwardLimit)
-        col_rounds<LOGN, true, true>(std::make_integer_sequence<int, G::ROUNDS>{}, sm, tile, q, tw);
+    const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * G::N + G::N;
+    auto run = [&](const auto& ar, auto scale) {
+        using A = std::decay_t<decltype(ar)>;
+        Lanes<A, 8> v(G::THREADS);
+        for (int t = 0; t < G::THREADS; ++t)
+            for (int k = 0; k < G::E; ++k) v[t][k] = A::of_bits(slots[k * G::THREADS + t]);
+        columns<LOGN, false>(v, tile, ar, tw);
+        for (int t = 0; t < G::THREADS; ++t) {
+            scale(v[t].data(), t);
+            for (int k = 0; k < G::E; ++k) slots[k * G::THREADS + t] = A::bits(v[t][k]);
+        }
+    };
+    if (is_fp(E, mi))
+        run(ntt::fp_arith(m), scale_f);
     else
-        col_rounds<LOGN, true, false>(std::make_integer_sequence<int, G::ROUNDS>{}, sm, tile, q, tw);
+        run(ntt::WordArith<false>{m.q}, scale_w);
+}
+template <int LOGN>
+void load_slots(uint64_t* slots, const uint64_t* limb, int tile) {
+    using G = ksf::Geom<LOGN>;
+    for (int t = 0; t < G::THREADS; ++t) {
+        uint64_t w[8];
+        ksf::load_limb<typename G::template InvRound<0>>(w, limb, tile, t);
+        for (int k = 0; k < G::E; ++k) slots[k * G::THREADS + t] = w[k];
+    }
+}
+// forward_limb (wg_ksfuse.cu).
+template <int LOGN, class ValueFp, class ValueWords>
+void forward_limb(const Emu& E, uint64_t* limb, int tile, int mi, ValueFp value_f, ValueWords value_w) {
+    using G = ksf::Geom<LOGN>;
+    using End = typename G::template FwdRound<G::ROUNDS - 1>;
+    const Modulus& m = E.H.mods[mi];
+    const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * G::N;
+    auto run = [&](const auto& ar, auto value) {
+        using A = std::decay_t<decltype(ar)>;
+        Lanes<A, 8> v(G::THREADS);
+        for (int t = 0; t < G::THREADS; ++t) value(v[t].data(), t);
+        columns<LOGN, true>(v, tile, ar, tw);
+        for (int t = 0; t < G::THREADS; ++t) {
+            uint64_t w[8];
+            for (int k = 0; k < G::E; ++k) w[k] = A::bits(v[t][k]);
+            ksf::store_limb<End>(w, limb, tile, t);
+        }
+    };
+    if (is_fp(E, mi))
+        run(ntt::fp_arith(m), value_f);
+    else if (m.q < ntt::kLazyForwardLimit)
+        run(ntt::WordArith<true>{m.q}, value_w);
+    else
+        run(ntt::WordArith<false>{m.q}, value_w);
 }
 
 // k_modup_ntt over every column tile of one digit.
@@ -160,27 +233,37 @@ template <int LOGN>
 void modup_fused(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t* digit) {
     using G = ksf::Geom<LOGN>;
     const int n = d.src_count;
-    std::vector<uint64_t> smem((size_t)(n + 1) * G::PAD);
-    uint64_t* work = smem.data() + (size_t)n * G::PAD;
+    std::vector<uint64_t> slots((size_t)n * G::TILE);
     for (int tile = 0; tile < G::TILES; ++tile) {
         std::vector<double> alpha((size_t)G::THREADS * G::E, 0.0);
+        ksf::SourceKinds kinds;
         for (int i = 0; i < n; ++i) {
             const int mi = d.src_first + i;
-            uint64_t* sm = smem.data() + (size_t)i * G::PAD;
-            for (int t = 0; t < G::THREADS; ++t) ksf::load_tile<LOGN>(sm, src + (size_t)mi * G::N, tile, t);
-            inverse_cols<LOGN>(E, sm, tile, mi);
-            for (int t = 0; t < G::THREADS; ++t)
-                ksf::modup_scale<LOGN>(sm, t, d, i, E.H.mods[mi].q, alpha.data() + (size_t)t * G::E);
+            const Modulus& m = E.H.mods[mi];
+            uint64_t* sl = slots.data() + (size_t)i * G::TILE;
+            kinds.set(i, m.q);
+            load_slots<LOGN>(sl, src + (size_t)mi * G::N, tile);
+            inverse_slots<LOGN>(
+                E, sl, tile, mi,
+                [&](double* v, int t) { ksf::modup_scale_fp(v, d, i, m.qd, alpha.data() + (size_t)t * G::E); },
+                [&](uint64_t* v, int t) {
+                    ksf::scale_n_inv(v, m);
+                    ksf::modup_scale(v, d, i, m.q, alpha.data() + (size_t)t * G::E);
+                });
         }
         std::vector<uint32_t> hps((size_t)G::THREADS * G::E);
         for (size_t k = 0; k < hps.size(); ++k) hps[k] = ksf::hps_count(alpha[k], n);
         for (int dst = 0; dst < d.dst_count; ++dst) {
             const int mi = d.dst_mod[dst];
-            for (int t = 0; t < G::THREADS; ++t)
-                ksf::modup_value<LOGN, 16>(work, smem.data(), t, d, dst, E.H.mods[mi].q, hps.data() + (size_t)t * G::E);
-            forward_cols<LOGN>(E, work, tile, mi);
-            for (int t = 0; t < G::THREADS; ++t)
-                ksf::store_tile<LOGN>(work, digit + (size_t)d.dst_limb[dst] * G::N, tile, t);
+            const Modulus& m = E.H.mods[mi];
+            forward_limb<LOGN>(
+                E, digit + (size_t)d.dst_limb[dst] * G::N, tile, mi,
+                [&](double* v, int t) {
+                    ksf::modup_value_fp<LOGN>(v, slots.data(), t, d, dst, m, hps.data() + (size_t)t * G::E, kinds);
+                },
+                [&](uint64_t* v, int t) {
+                    ksf::modup_value<LOGN, 16>(v, slots.data(), t, d, dst, m.q, hps.data() + (size_t)t * G::E, kinds.fp64);
+                });
         }
     }
 }
@@ -188,27 +271,37 @@ void modup_fused(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t
 // k_moddown_ntt over every column tile of one accumulator polynomial.
 template <int LOGN>
 void moddown_fused(const Emu& E, const uint64_t* src_p, uint64_t* out, int L, const uint64_t* inv,
-                   const uint64_t* inv_s) {
+                   const uint64_t* inv_s, const ntt::TwPair* inv_fp) {
     using G = ksf::Geom<LOGN>;
     const int K = (int)E.H.np, nq = (int)E.H.nq;
     const Modulus* pmods = E.H.mods.data() + nq;
-    std::vector<uint64_t> smem((size_t)(K + 1) * G::PAD);
-    uint64_t* work = smem.data() + (size_t)K * G::PAD;
+    std::vector<uint64_t> slots((size_t)K * G::TILE);
+    ksf::SourceKinds kinds;
+    for (int pi = 0; pi < K; ++pi) kinds.set(pi, pmods[pi].q);
     for (int tile = 0; tile < G::TILES; ++tile) {
         for (int pi = 0; pi < K; ++pi) {
-            uint64_t* sm = smem.data() + (size_t)pi * G::PAD;
-            for (int t = 0; t < G::THREADS; ++t) ksf::load_tile<LOGN>(sm, src_p + (size_t)pi * G::N, tile, t);
-            inverse_cols<LOGN>(E, sm, tile, nq + pi);
+            const Modulus& m = pmods[pi];
+            uint64_t* sl = slots.data() + (size_t)pi * G::TILE;
+            load_slots<LOGN>(sl, src_p + (size_t)pi * G::N, tile);
+            inverse_slots<LOGN>(
+                E, sl, tile, nq + pi, [&](double* v, int) { ksf::scale_fp(v, m.n_inv_w, m.n_inv_wq, m.qd); },
+                [&](uint64_t* v, int) { ksf::scale_n_inv(v, m); });
         }
         std::vector<uint32_t> hps((size_t)G::THREADS * G::E);
         for (int t = 0; t < G::THREADS; ++t)
-            ksf::moddown_hps<LOGN, 16>(smem.data(), t, pmods, K, hps.data() + (size_t)t * G::E);
+            ksf::moddown_hps<LOGN, 16>(slots.data(), t, pmods, K, hps.data() + (size_t)t * G::E, kinds.fp64);
         for (int qi = 0; qi < L; ++qi) {
-            for (int t = 0; t < G::THREADS; ++t)
-                ksf::moddown_value<LOGN, 16>(work, smem.data(), t, K, E.H.mods[qi].q, inv + (size_t)qi * K,
-                                             inv_s + (size_t)qi * K, hps.data() + (size_t)t * G::E);
-            forward_cols<LOGN>(E, work, tile, qi);
-            for (int t = 0; t < G::THREADS; ++t) ksf::store_tile<LOGN>(work, out + (size_t)qi * G::N, tile, t);
+            const Modulus& m = E.H.mods[qi];
+            const uint64_t *iv = inv + (size_t)qi * K, *ivs = inv_s + (size_t)qi * K;
+            forward_limb<LOGN>(
+                E, out + (size_t)qi * G::N, tile, qi,
+                [&](double* v, int t) {
+                    ksf::moddown_value_fp<LOGN>(v, slots.data(), t, K, m, iv, ivs, inv_fp + (size_t)qi * K,
+                                                hps.data() + (size_t)t * G::E, kinds);
+                },
+                [&](uint64_t* v, int t) {
+                    ksf::moddown_value<LOGN, 16>(v, slots.data(), t, K, m.q, iv, ivs, hps.data() + (size_t)t * G::E, kinds.fp64);
+                });
         }
     }
 }
@@ -219,8 +312,16 @@ template <int LOGN>
 void rows_epi(const Emu& E, const ntt::NttEpiJob& j) {
     const size_t N = (size_t)1 << LOGN;
     std::vector<uint64_t> v(j.data, j.data + N);
-    phase_geom<LOGN, true, false>(E, v.data(), j.mod);
-    for (size_t off = 0; off < N; ++off) ntt::ntt_epilogue(j, off, v[off], E.H.mods[j.mod].q);
+    phase_geom<LOGN, true, false>(E, v.data(), j.mod, true);
+    const Modulus& m = E.H.mods[j.mod];
+    if (is_fp(E, j.mod)) {
+        const ntt::FpEpilogue c = ntt::fp_epilogue(j, m);
+        for (size_t off = 0; off < N; ++off)
+            j.out[off] = ntt::fp_epilogue_value(j, c, j.kind == ntt::kEpiCombine ? j.acc[off] : 0,
+                                                j.kind == ntt::kEpiRescale || j.c0 ? j.in[off] : 0, v[off], m);
+        return;
+    }
+    for (size_t off = 0; off < N; ++off) ntt::ntt_epilogue(j, off, v[off], m.q);
 }
 
 // k_rescale_ntt over every column tile of one polynomial (dropped limb after the inverse row
@@ -228,18 +329,23 @@ void rows_epi(const Emu& E, const ntt::NttEpiJob& j) {
 template <int LOGN>
 void rescale_fused(const Emu& E, const uint64_t* drop, uint64_t* rem, int lv, const uint64_t* rc) {
     using G = ksf::Geom<LOGN>;
-    std::vector<uint64_t> smem((size_t)2 * G::PAD);
-    uint64_t* dl = smem.data();
-    uint64_t* work = smem.data() + G::PAD;
-    const uint64_t p = E.H.mods[lv].q;
+    std::vector<uint64_t> slots(G::TILE);
+    const Modulus& mp = E.H.mods[lv];
     for (int tile = 0; tile < G::TILES; ++tile) {
-        for (int t = 0; t < G::THREADS; ++t) ksf::load_tile<LOGN>(dl, drop, tile, t);
-        inverse_cols<LOGN>(E, dl, tile, lv);
+        load_slots<LOGN>(slots.data(), drop, tile);
+        inverse_slots<LOGN>(
+            E, slots.data(), tile, lv, [&](double* v, int) { ksf::scale_fp(v, mp.n_inv_w, mp.n_inv_wq, mp.qd); },
+            [&](uint64_t* v, int) { ksf::scale_n_inv(v, mp); });
         for (int qi = 0; qi < lv; ++qi) {
-            for (int t = 0; t < G::THREADS; ++t)
-                ksf::rescale_value<LOGN>(work, dl, t, p, E.H.mods[qi].q, rc[qi], rc[3 * lv + qi]);
-            forward_cols<LOGN>(E, work, tile, qi);
-            for (int t = 0; t < G::THREADS; ++t) ksf::store_tile<LOGN>(work, rem + (size_t)qi * G::N, tile, t);
+            const Modulus& m = E.H.mods[qi];
+            forward_limb<LOGN>(
+                E, rem + (size_t)qi * G::N, tile, qi,
+                [&](double* v, int t) {
+                    ksf::rescale_value_fp<LOGN>(v, slots.data(), t, mp.q, m, rc[qi], rc[3 * lv + qi], is_fp(E, lv));
+                },
+                [&](uint64_t* v, int t) {
+                    ksf::rescale_value<LOGN>(v, slots.data(), t, mp.q, m.q, rc[qi], rc[3 * lv + qi], is_fp(E, lv));
+                });
         }
     }
 }
@@ -293,11 +399,16 @@ void* emu_create(uint64_t N, const uint64_t* q, size_t nq, const uint64_t* p, si
             d.corr = T + o.corr;
             d.dst_limb = reinterpret_cast<const int*>(T + o.dst_limb);
             d.dst_mod = reinterpret_cast<const int*>(T + o.dst_mod);
+            d.scale_fp = reinterpret_cast<const ntt::TwPair*>(T + o.scale_fp);
+            d.qhat_fp = reinterpret_cast<const ntt::TwPair*>(T + o.qhat_fp);
             E->modup[l].push_back(d);
         }
     E->tw.resize((nq + np) * 2 * N);
     for (size_t m = 0; m < nq + np; ++m)
-        ntt::interleave_twiddles(N, E->H.tw.data() + m * 4 * N, E->tw.data() + m * 2 * N);
+        for (size_t dir = 0; dir < 2; ++dir) {
+            const uint64_t* w = E->H.tw.data() + (m * 4 + 2 * dir) * N;
+            ntt::twiddle_pairs(N, E->H.mods[m].q, w, w + N, 3, false, E->tw.data() + (m * 2 + dir) * N);
+        }
     return E;
 }
 
@@ -359,7 +470,8 @@ void emu_keyswitch(void* h, size_t level, const uint64_t* key_term, const uint64
                 EMU_LOGN_SWITCH(E.logN, phase_one<LG>(E, acc + (poly * T + L + pi) * N, (int)(nq + pi), false, false));
         for (int poly = 0; poly < 2; ++poly)
             EMU_LOGN_SWITCH(E.logN, moddown_fused<LG>(E, acc + (poly * T + L) * N, contrib + poly * L * N, (int)L,
-                                                      W + E.H.fold_inv[level], W + E.H.fold_inv_s[level]));
+                                                      W + E.H.fold_inv[level], W + E.H.fold_inv_s[level],
+                                                      reinterpret_cast<const ntt::TwPair*>(W + E.H.fold_fp[level])));
         // forward row phase of the contributions with the combine as its epilogue (outputs over
         // the accumulators' Q limbs when an automorphism follows)
         const bool gal = galois != 0;
@@ -460,6 +572,17 @@ void emu_mont_mul(uint64_t q, const uint64_t* x, const uint64_t* y, size_t n, ui
     uint64_t inv = q;  // q q = 1 (mod 8): three correct bits, doubled by each step
     for (int k = 0; k < 5; ++k) inv *= 2 - q * inv;
     for (size_t i = 0; i < n; ++i) out[i] = mont_mul(x[i], y[i], q, 0 - inv);
+}
+
+// fp::mulmod on n pairs (a[i] any integer-valued double, w[i] a residue): the representative and,
+// in word[i], the canonical word of it.
+void emu_fp_mulmod(uint64_t q, const double* a, const uint64_t* w, size_t n, double* out, uint64_t* word) {
+    for (size_t i = 0; i < n; ++i) {
+        double fw, fwq;
+        fp::factor(w[i], q, fw, fwq);
+        out[i] = fp::mulmod(a[i], fw, fwq, (double)q);
+        word[i] = fp::canonical(out[i], (double)q, 1.0 / (double)q);
+    }
 }
 
 // reduce128 on n values (hi[i], lo[i]) modulo q

@@ -1,0 +1,192 @@
+"""The FP64 arithmetic of moduli below 2^50 (csrc/wg_fp.cuh): the product, the transforms at the
+edges of their ranges, and key switches whose digits mix FP64 and word moduli.
+
+The CPU tests run the kernels' bodies through the emulation; the GPU tests run the kernels.  All
+of it is exact: every comparison is word for word.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from test_emulation import emu, u64p  # noqa: F401
+
+f64p = np.ctypeslib.ndpointer(dtype=np.float64, flags="C_CONTIGUOUS")
+
+
+def _prime(below, N, step=-1):
+    """The nearest prime = 1 (mod 2N) below (or, step = 1, above) `below`."""
+    q = below // (2 * N) * (2 * N) + 1
+    if step < 0 and q >= below:
+        q -= 2 * N
+    if step > 0 and q <= below:
+        q += 2 * N
+    while not all(pow(b, q - 1, q) == 1 for b in (2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37)):
+        q += step * 2 * N
+    return q
+
+
+def _edges(N):
+    """Moduli on both sides of the path's limit (2^50) and of its reduction limit (2^42), and a small one."""
+    return [_prime(1 << 50, N), _prime(1 << 50, N, 1), _prime(1 << 42, N), _prime(1 << 42, N, 1), _prime(1 << 27, N)]
+
+
+@pytest.mark.parametrize("q", [_prime(1 << 50, 1 << 15), _prime(1 << 42, 1 << 15, 1), 274876334081, 12289])
+def test_product_is_exact_and_bounded(emu, q):  # noqa: F811
+    emu.emu_fp_mulmod.argtypes = [C.c_uint64, f64p, u64p, C.c_size_t, f64p, u64p]
+    rng = np.random.default_rng(q % 1000003)
+    a = [int(v) for v in rng.integers(-(1 << 52), 1 << 52, 4000)] + [int(v) for v in rng.integers(-q, q, 4000)]
+    w = [int(v) for v in rng.integers(0, q, 8000)]
+    for av in (0, 1, -1, q, -q, (1 << 52), -(1 << 52), (1 << 52) - 1, 4 * q - 1):
+        for wv in (0, 1, q - 1, q // 2, q // 2 + 1, q // 2 - 1, q // 3):
+            if abs(av) <= 1 << 52:
+                a.append(av)
+                w.append(wv)
+    x, y = np.array(a, np.float64), np.array(w, np.uint64)
+    out, word = np.zeros(len(a)), np.zeros(len(a), np.uint64)
+    emu.emu_fp_mulmod(q, x, y, len(a), out, word)
+    for i in range(len(a)):
+        assert out[i] == int(out[i]) and (int(out[i]) - a[i] * w[i]) % q == 0, (a[i], w[i])
+        assert 8 * abs(int(out[i])) <= 5 * q, (a[i], w[i])
+        assert int(word[i]) == a[i] * w[i] % q
+
+
+def _extreme_polys(q, N, rng):
+    """Residue polynomials that drive the lazy sums to their bounds, with words up to 4q - 1."""
+    top = np.full(N, q - 1, np.uint64)
+    alt = top.copy()
+    alt[::2] = 0
+    wide = rng.integers(0, 4 * q, N, dtype=np.uint64)
+    return [top, alt, rng.integers(0, q, N, dtype=np.uint64), wide, np.full(N, 4 * q - 1, np.uint64)]
+
+
+@pytest.mark.parametrize("logN", [10, 15, 16])
+@pytest.mark.parametrize("geometry", [0, 3])
+def test_emulated_transforms_at_the_edges(oracle_mod, emu, logN, geometry):  # noqa: F811
+    N = 1 << logN
+    q = np.array(_edges(N), np.uint64)
+    p = np.array([_prime(1 << 60, N)], np.uint64)
+    o = oracle_mod.OracleCtx(N, q, p, 1)
+    h = emu.emu_create(N, q, len(q), p, 1, 1)
+    emu.emu_set_ntt_geometry(geometry)
+    try:
+        rng = np.random.default_rng(logN)
+        polys = [_extreme_polys(int(m), N, rng) for m in q]
+        for k in range(5):
+            x = np.concatenate([pl[k] for pl in polys])
+            canon = x % np.repeat(q, N)
+            y = x.copy()
+            emu.emu_ntt(h, y, len(q), 0, 0, 0)
+            want = o.ntt(canon)
+            assert (y == want).all(), k
+            emu.emu_ntt(h, y, len(q), 0, 0, 1)
+            assert (y == canon).all(), k
+            # the forward transform takes words far above 4 q of a lazily reduced modulus
+            if k == 2:
+                y = rng.integers(0, 1 << 63, x.size, dtype=np.uint64)
+                want = o.ntt(y % np.repeat(q, N))
+                emu.emu_ntt(h, y, len(q), 0, 0, 0)
+                assert (y == want).all()
+            y = canon.copy()
+            emu.emu_ntt(h, y, len(q), 0, 0, 1)
+            emu.emu_ntt(h, y, len(q), 0, 0, 0)
+            assert (y == canon).all(), k
+    finally:
+        emu.emu_set_ntt_geometry(0)
+        emu.emu_destroy(h)
+
+
+# digits of eight 50-bit limbs over nine 50-bit P limbs (the sums' bound, every width of the ModDown);
+# digits and P limbs that mix FP64 and word moduli in both roles
+MIXED = [dict(logN=10, q_bits=[50] * 8, p_bits=[50] * 9, dnum=1),
+         dict(logN=10, q_bits=[50, 61, 42, 55, 38, 61, 50], p_bits=[61, 50, 58, 38, 60], dnum=2),
+         dict(logN=11, q_bits=[31, 27, 30, 50], p_bits=[32, 50], dnum=4)]
+
+
+@pytest.mark.parametrize("prm", MIXED)
+def test_emulated_mixed_key_switches(oracle_mod, emu, prm):  # noqa: F811
+    O, N = oracle_mod, 1 << prm["logN"]
+    p, q = O.find_primes(prm["p_bits"], prm["q_bits"], N)
+    o = O.OracleCtx(N, q, p, prm["dnum"])
+    h = emu.emu_create(N, q, len(q), p, len(p), prm["dnum"])
+    try:
+        L = len(q)
+        rk = o.rotation_key(o.ternary(64, 3), 3, 11)
+        for fused in (0, 1):
+            emu.emu_set_keyswitch_fusion(fused)
+            for level in (L - 1, L // 2, 1):
+                b, a = o.uniform(level + 1, 9), o.uniform(level + 1, 10)
+                ob, oa = o.rotate(level, b, a, rk, 3)
+                eb, ea = b.copy(), a.copy()
+                emu.emu_keyswitch(h, level, a.copy(), rk, L - 1, eb, ea, 1, 0, o.galois(3))
+                assert (eb == ob).all() and (ea == oa).all(), (fused, level)
+                (ref,) = o.rescale(level, [b])
+                xs = b.copy()
+                emu.emu_rescale(h, level, xs)
+                assert (xs[: level * N] == ref).all(), (fused, level)
+    finally:
+        emu.emu_set_keyswitch_fusion(0)
+        emu.emu_destroy(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("logN", [10, 11, 12, 13, 14, 15, 16])
+def test_transforms_at_the_edges(wg, oracle_mod, logN):
+    import torch
+
+    N = 1 << logN
+    q = np.array(_edges(N), np.uint64)
+    p = np.array([_prime(1 << 60, N)], np.uint64)
+    o, ctx = oracle_mod.OracleCtx(N, q, p, 1), wg.Context(N, q, p, 1)
+    rng = np.random.default_rng(logN)
+    polys = [_extreme_polys(int(m), N, rng) for m in q]
+    for geometry in range(4):
+        for d in range(2):
+            for ph in range(2):
+                ctx.set_ntt_geometry(d, ph, geometry)
+        for k in range(5):
+            x = np.concatenate([pl[k] for pl in polys])
+            canon = x % np.repeat(q, N)
+            dx = wg.to_device(x)
+            ctx.ntt_forward(dx, len(q))
+            torch.cuda.synchronize()
+            assert (wg.to_host(dx) == o.ntt(canon)).all(), (geometry, k)
+            ctx.ntt_inverse(dx, len(q))
+            dy = wg.to_device(canon)
+            ctx.ntt_inverse(dy, len(q))
+            ctx.ntt_forward(dy, len(q))
+            torch.cuda.synchronize()
+            assert (wg.to_host(dx) == canon).all() and (wg.to_host(dy) == canon).all(), (geometry, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fusion", [0, 2])
+@pytest.mark.parametrize("prm", MIXED)
+def test_mixed_key_switches(wg, oracle_mod, prm, fusion):
+    import torch
+
+    O, N = oracle_mod, 1 << prm["logN"]
+    p, q = O.find_primes(prm["p_bits"], prm["q_bits"], N)
+    o, ctx = O.OracleCtx(N, q, p, prm["dnum"]), wg.Context(N, q, p, prm["dnum"])
+    ctx.set_ntt_fusion(fusion)
+    L = len(q)
+    s = o.ternary(64, 3)
+    rk, rl = o.rotation_key(s, 3, 11), o.relin_key(s, 13)
+    ctx.set_key(wg.WG_KEY_ROTATION, rk, rotation=3)
+    ctx.set_key(wg.WG_KEY_RELIN, rl)
+    for level in (L - 1, L // 2, 1):
+        n = (level + 1) * N
+        b, a, c2 = o.uniform(level + 1, 9), o.uniform(level + 1, 10), o.uniform(level + 1, 12)
+        db, da, dc = wg.to_device(b), wg.to_device(a), wg.to_device(c2)
+        ctx.rotate(level, db, da, 3)
+        ob, oa = o.rotate(level, b, a, rk, 3)
+        e0, e1 = wg.to_device(b), wg.to_device(a)
+        ctx.relin(level, e0, e1, dc)
+        r0, r1 = o.relin(level, b, a, c2, rl)
+        torch.cuda.synchronize()
+        assert (wg.to_host(db) == ob).all() and (wg.to_host(da) == oa).all(), level
+        assert (wg.to_host(e0)[:n] == r0).all() and (wg.to_host(e1)[:n] == r1).all(), level
+        ctx.rescale(level, e0)
+        (ref,) = o.rescale(level, [r0])
+        torch.cuda.synchronize()
+        assert (wg.to_host(e0)[: level * N] == ref).all(), level
