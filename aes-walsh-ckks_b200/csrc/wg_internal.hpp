@@ -150,6 +150,7 @@ struct Context {
     ntt::TwPair* d_tw_words = nullptr;
     const ntt::TwPair* twiddles(int eb) const { return reinterpret_cast<const ntt::TwPair*>(d_tw[eb - 3]); }
     int ntt_variant[2][2] = {{0, 0}, {0, 0}};  // NTT geometry per [direction][phase: rows, columns]
+    int ntt_pinned[2] = {0, 0};                // phases of the direction whose geometry the caller pinned (bits)
     // Key switches and rescales can run their base changes fused with the adjacent NTT column
     // phases and their final element-wise steps in the last row phase's epilogue (wg_ksfuse.cu,
     // k_ntt_rows_epi).  0: the separate launches; 1, 2: fused.  The words are the same in every mode.

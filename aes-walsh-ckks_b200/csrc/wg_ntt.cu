@@ -198,6 +198,151 @@ __global__ void __launch_bounds__(Phase<LOGN, FWD, COLS, EB, STAGED>::THREADS, m
     store_words<End>(x + tile_offset<LOGN, FWD, COLS, EB, STAGED>(tile, End::element(sub, o)), w);
 }
 
+// A whole transform of one limb per cluster (Whole, wg_ntt.cuh): both phases' rounds with the results
+// of the first handed over in distributed shared memory, so a limb crosses device memory once each
+// way instead of twice and a small batch pays one launch.
+// `between` is applied to the first phase's values on their way to the second's tiles.
+template <int LOGN, bool FWD, class Arith, class Between>
+__device__ __forceinline__ void whole_transform(uint64_t* first, uint64_t* second, typename Arith::V* v, int tile, int t,
+                                                const Arith& ar, const TwPair* tw, Between between) {
+    using W = Whole<LOGN>;
+    using P1 = typename W::template Ph<FWD, FWD>;
+    using P2 = typename W::template Ph<FWD, !FWD>;
+    using End = Round<LOGN, FWD, FWD, 3, false, P1::ROUNDS - 1, W::TL>;
+    using Begin = Round<LOGN, FWD, !FWD, 3, false, 0, W::TL>;
+    ntt_rounds<LOGN, FWD, FWD, 3, false, W::TL>(std::make_integer_sequence<int, P1::ROUNDS>{}, first, v, P1::sub_of(t),
+                                                P1::o_of(t), tile, ar, tw);
+    if (W::CTAS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // every CTA has started
+    const int e0 = End::element(P1::sub_of(t), P1::o_of(t));
+#pragma unroll
+    for (int j = 0; j < End::E; ++j) {
+        const HandOver h = hand_over<LOGN, FWD>(tile, e0 + End::tile_step(j));
+        const uint64_t w = between(Arith::bits(v[j]));
+        if (W::CTAS > 1) {
+            const unsigned local = (unsigned)__cvta_generic_to_shared(second + pad16(h.at));
+            unsigned remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(local), "r"(h.cta));
+            asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(remote), "l"(w) : "memory");
+        } else {
+            second[pad16(h.at)] = w;
+        }
+    }
+    if (W::CTAS > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    Begin::template gather<Arith>(second, P2::sub_of(t), P2::o_of(t), v);
+    // no CTA writes to `second` any more, but its own threads still read: the rounds exchange in `first`
+    ntt_rounds<LOGN, FWD, !FWD, 3, false, W::TL>(std::make_integer_sequence<int, P2::ROUNDS>{}, first, v, P2::sub_of(t),
+                                                 P2::o_of(t), tile, ar, tw);
+}
+
+template <int LOGN>
+constexpr size_t whole_smem() {
+    return 2 * 8 * (size_t)Whole<LOGN>::PAD;
+}
+
+template <int LOGN, bool FWD, bool TABLE>
+__global__ void __launch_bounds__(Whole<LOGN>::template Ph<FWD, true>::THREADS,
+                                  1024 / Whole<LOGN>::template Ph<FWD, true>::THREADS)
+    k_ntt_whole(uint64_t* __restrict__ data, size_t poly_stride, LimbMap map, const NttJob* __restrict__ jobs, int njobs,
+                const Modulus* __restrict__ mods, const TwPair* __restrict__ tw_base) {
+    using W = Whole<LOGN>;
+    using P1 = typename W::template Ph<FWD, FWD>;
+    using P2 = typename W::template Ph<FWD, !FWD>;
+    using Begin = Round<LOGN, FWD, FWD, 3, false, 0, W::TL>;
+    using End = Round<LOGN, FWD, !FWD, 3, false, P2::ROUNDS - 1, W::TL>;
+    constexpr int E = 8;
+    extern __shared__ __align__(16) uint64_t smem[];
+    uint64_t* first = smem;
+    uint64_t* second = smem + W::PAD;
+    const uint64_t* xin;
+    uint64_t* x;
+    int mi;
+    if (TABLE) {
+        const int j = blockIdx.y + 65535 * blockIdx.z;
+        if (j >= njobs) return;  // the same for every CTA of a cluster
+        const NttJob job = jobs[j];
+        x = job.dst;
+        xin = job.src;
+        mi = job.mod;
+    } else {
+        const int limb = blockIdx.y;
+        x = data + (size_t)blockIdx.z * poly_stride + (size_t)limb * W::N;
+        xin = x;
+        mi = map(limb);
+    }
+    if (W::CTAS > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+    const Modulus m = mods[mi];
+    const TwPair* tw = tw_base + (size_t)mi * 2 * W::N + (FWD ? 0 : W::N);
+    const int tile = blockIdx.x, t = threadIdx.x;
+    uint64_t w[E];
+    load_words<Begin>(
+        xin + tile_offset<LOGN, FWD, FWD, 3, false, W::TL>(tile, Begin::element(P1::sub_of(t), P1::o_of(t))), w);
+    if (m.q < fp::kLimit) {
+        double v[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = fp::bits_double(fp_load(true, w[j], m));
+        whole_transform<LOGN, FWD>(first, second, v, tile, t, fp_arith(m), tw,
+                                   [&](uint64_t b) { return fp_store(false, FWD, b, m); });
+#pragma unroll
+        for (int j = 0; j < E; ++j) w[j] = fp_store(true, FWD, fp::double_bits(v[j]), m);
+    } else {
+        const auto same = [](uint64_t b) { return b; };
+        if (FWD && m.q < kLazyForwardLimit)
+            whole_transform<LOGN, FWD>(first, second, w, tile, t, WordArith<FWD>{m.q}, tw, same);
+        else
+            whole_transform<LOGN, FWD>(first, second, w, tile, t, WordArith<false>{m.q}, tw, same);
+#pragma unroll
+        for (int j = 0; j < E; ++j) w[j] = word_store(true, FWD, w[j], m);
+    }
+    store_words<End>(
+        x + tile_offset<LOGN, FWD, !FWD, 3, false, W::TL>(tile, End::element(P2::sub_of(t), P2::o_of(t))), w);
+}
+
+template <int LOGN, bool FWD, bool TABLE>
+void launch_whole(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,
+                  const NttJob* jobs, int njobs, cudaStream_t s) {
+    using W = Whole<LOGN>;
+    static const bool opted = [] {
+        cudaFuncSetAttribute(k_ntt_whole<LOGN, FWD, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)whole_smem<LOGN>());
+        return true;
+    }();
+    (void)opted;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = TABLE ? dim3(W::CTAS, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535)
+                        : dim3(W::CTAS, limbs, polys);
+    cfg.blockDim = dim3(W::template Ph<FWD, true>::THREADS);
+    cfg.dynamicSmemBytes = whole_smem<LOGN>();
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = W::CTAS;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    // algorithmic bytes: every residue read once and written once
+    Probe probe(kClsNtt, 16.0 * W::N * (TABLE ? njobs : (double)limbs * polys), s);
+    check_cuda(cudaLaunchKernelEx(&cfg, k_ntt_whole<LOGN, FWD, TABLE>, data, stride, map, jobs, njobs,
+                                  (const Modulus*)c.d_mod, c.twiddles(3)),
+               "ntt launch");
+}
+
+template <int LOGN>
+void whole_dispatch(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,
+                    const NttJob* jobs, int njobs, bool fwd, cudaStream_t s) {
+    if (jobs) {
+        if (fwd) launch_whole<LOGN, true, true>(c, data, limbs, polys, stride, map, jobs, njobs, s);
+        else launch_whole<LOGN, false, true>(c, data, limbs, polys, stride, map, jobs, njobs, s);
+    } else {
+        if (fwd) launch_whole<LOGN, true, false>(c, data, limbs, polys, stride, map, jobs, njobs, s);
+        else launch_whole<LOGN, false, false>(c, data, limbs, polys, stride, map, jobs, njobs, s);
+    }
+}
+
 // The forward row phase of one job-table limb with an element-wise epilogue (NttEpiJob): the
 // same rounds and final reduction as k_ntt_phase<LOGN, true, false, ...>, then the epilogue in
 // place of the store.  The epilogue's operands (acc, in: the tile's contiguous words) are
@@ -401,6 +546,22 @@ void dispatch(const Context& c, uint64_t* data, int limbs, int polys, size_t str
     if (jobs ? njobs <= 0 : (limbs <= 0 || polys <= 0)) return;
     if (!jobs && (polys > 65535 || limbs > 65535)) fail(kInvalid, "ntt: too many limbs or polynomials in one batch");
     const int d = fwd ? 0 : 1;
+    // One launch per transform for the rings whose limb a cluster of small CTAs covers, while the batch
+    // is about one wave of clusters.  Measured at 38-bit moduli, one launch / two phases, in us: 2^14:
+    // 10 / 12 (32 limbs), 14 / 16 (64), 20 / 20 (96), 42 / 38 (256); 2^13: 9 / 12 (64), 13 / 17 (128),
+    // 22 / 24 (256); 2^12: 9 / 12 (128), 18 / 22 (512).  At 2^15 clusters of 8 CTAs of 512 threads
+    // leave most SMs waiting (29 / 24 at 64 limbs, 189 / 132 at 512), so larger rings take the phases.
+    const size_t words = (size_t)(jobs ? njobs : limbs * (size_t)polys) * c.N;
+    if (!c.ntt_pinned[d] && (c.logN <= 12 || (c.logN <= kWholeMaxLog && words <= ((size_t)1 << 20)))) {
+        switch (c.logN) {
+            case 10: whole_dispatch<10>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
+            case 11: whole_dispatch<11>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
+            case 12: whole_dispatch<12>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
+            case 13: whole_dispatch<13>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
+            default: whole_dispatch<14>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
+        }
+        return;
+    }
     // forward: columns then rows; inverse: rows then columns
     const bool first_cols = fwd;
     phase_dispatch(c, fwd, first_cols, c.ntt_variant[d][first_cols ? 1 : 0], data, limbs, polys, stride, map, jobs,

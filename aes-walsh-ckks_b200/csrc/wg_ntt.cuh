@@ -370,6 +370,37 @@ WG_HD uint64_t fp_epilogue_value(const NttEpiJob& j, const FpEpilogue& c, uint64
     return epilogue_value(j, acc, in, fp::to_word(fp::lift(v, m.qd)), m.q);
 }
 
+// A whole transform in one launch: the limb's TL-element tiles of both phases belong to the CTAs of
+// one cluster, which hand the first phase's results to the second through distributed shared memory.
+// Tile element e of the first phase goes to element `at` of CTA `cta`'s second-phase tile.
+constexpr int kWholeMaxLog = 14;
+template <int LOGN>
+struct Whole {
+    static_assert(LOGN <= kWholeMaxLog, "a cluster has at most 8 CTAs");
+    static constexpr int N = 1 << LOGN;
+    static constexpr int TL = N < kMaxTile ? N : kMaxTile;
+    static constexpr int CTAS = N / TL;  // the cluster: 1 to 8 CTAs
+    template <bool FWD, bool COLS>
+    using Ph = Phase<LOGN, FWD, COLS, 3, false, TL>;
+    static constexpr int COLUMNS = Ph<true, true>::SUBS;  // columns, and rows, of a CTA's tiles
+    static constexpr int ROWS = Ph<true, false>::SUBS;
+    static constexpr int NB2 = Ph<true, true>::NB2;
+    static constexpr int PAD = TL + TL / 16;
+};
+struct HandOver {
+    int cta, at;
+};
+template <int LOGN, bool FWD>
+WG_HD HandOver hand_over(int tile, int e) {
+    using W = Whole<LOGN>;
+    if (FWD) {  // columns to rows
+        const int h = e / W::COLUMNS, c = tile * W::COLUMNS + e % W::COLUMNS;
+        return {h / W::ROWS, (h % W::ROWS) << W::NB2 | c};
+    }
+    const int h = tile * W::ROWS + (e >> W::NB2), c = e & ((1 << W::NB2) - 1);
+    return {c / W::COLUMNS, h * W::COLUMNS + c % W::COLUMNS};
+}
+
 // The place of twiddle x of a row (of the 2^kr of row-stage kr = NB2 - 1 - b) in the table.  In the
 // round of a row's lowest bits thread o uses the 2^(eb-1-b) consecutive twiddles from o << (eb-1-b),
 // so over a warp each of these loads would touch a 128-byte line per lane; there they stand

@@ -362,6 +362,67 @@ void phase_one(const Emu& E, uint64_t* x, int mi, bool fwd, bool cols) {
     }
 }
 
+// k_ntt_whole of one limb: every CTA of the cluster runs the first phase on its tile, hands the
+// results over (HandOver), then runs the second.
+template <int LOGN, bool FWD, class Arith>
+void whole_limb(const Emu& E, uint64_t* x, int mi, const Arith& ar) {
+    using W = ntt::Whole<LOGN>;
+    using P1 = typename W::template Ph<FWD, FWD>;
+    using P2 = typename W::template Ph<FWD, !FWD>;
+    using Begin1 = ntt::Round<LOGN, FWD, FWD, 3, false, 0, W::TL>;
+    using End1 = ntt::Round<LOGN, FWD, FWD, 3, false, P1::ROUNDS - 1, W::TL>;
+    using Begin2 = ntt::Round<LOGN, FWD, !FWD, 3, false, 0, W::TL>;
+    using End2 = ntt::Round<LOGN, FWD, !FWD, 3, false, P2::ROUNDS - 1, W::TL>;
+    const Modulus& m = E.H.mods[mi];
+    const bool fp64 = is_fp(E, mi);
+    const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * W::N + (FWD ? 0 : W::N);
+    std::vector<uint64_t> first(W::PAD), second((size_t)W::CTAS * W::PAD, ~uint64_t{0});
+    for (int tile = 0; tile < W::CTAS; ++tile) {
+        Lanes<Arith, 8> v(P1::THREADS);
+        for (int t = 0; t < P1::THREADS; ++t) {
+            const uint64_t* p = x + ntt::tile_offset<LOGN, FWD, FWD, 3, false, W::TL>(
+                                        tile, Begin1::element(P1::sub_of(t), P1::o_of(t)));
+            for (int j = 0; j < 8; ++j) {
+                const uint64_t w = p[Begin1::limb_step(j)];
+                v[t][j] = Arith::of_bits(fp64 ? ntt::fp_load(true, w, m) : w);
+            }
+        }
+        rounds<LOGN, FWD, FWD, 3, false, W::TL>(std::make_integer_sequence<int, P1::ROUNDS>{}, first.data(), v, tile, ar, tw);
+        for (int t = 0; t < P1::THREADS; ++t)
+            for (int j = 0; j < 8; ++j) {
+                const ntt::HandOver h = ntt::hand_over<LOGN, FWD>(
+                    tile, End1::element(P1::sub_of(t), P1::o_of(t)) + End1::tile_step(j));
+                const uint64_t w = Arith::bits(v[t][j]);
+                second[(size_t)h.cta * W::PAD + ntt::pad16(h.at)] = fp64 ? ntt::fp_store(false, FWD, w, m) : w;
+            }
+    }
+    for (int tile = 0; tile < W::CTAS; ++tile) {
+        Lanes<Arith, 8> v(P2::THREADS);
+        for (int t = 0; t < P2::THREADS; ++t)
+            Begin2::template gather<Arith>(second.data() + (size_t)tile * W::PAD, P2::sub_of(t), P2::o_of(t), v[t].data());
+        rounds<LOGN, FWD, !FWD, 3, false, W::TL>(std::make_integer_sequence<int, P2::ROUNDS>{}, first.data(), v, tile, ar, tw);
+        for (int t = 0; t < P2::THREADS; ++t) {
+            uint64_t* p = x + ntt::tile_offset<LOGN, FWD, !FWD, 3, false, W::TL>(
+                                  tile, End2::element(P2::sub_of(t), P2::o_of(t)));
+            for (int j = 0; j < 8; ++j) {
+                const uint64_t w = Arith::bits(v[t][j]);
+                p[End2::limb_step(j)] = fp64 ? ntt::fp_store(true, FWD, w, m) : word_store(true, FWD, w, m);
+            }
+        }
+    }
+}
+template <int LOGN>
+void whole_ntt(const Emu& E, uint64_t* x, int mi, bool fwd) {
+    const Modulus& m = E.H.mods[mi];
+    if (is_fp(E, mi))
+        fwd ? whole_limb<LOGN, true>(E, x, mi, ntt::fp_arith(m)) : whole_limb<LOGN, false>(E, x, mi, ntt::fp_arith(m));
+    else if (fwd && m.q < ntt::kLazyForwardLimit)
+        whole_limb<LOGN, true>(E, x, mi, ntt::WordArith<true>{m.q});
+    else
+        fwd ? whole_limb<LOGN, true>(E, x, mi, ntt::WordArith<false>{m.q})
+            : whole_limb<LOGN, false>(E, x, mi, ntt::WordArith<false>{m.q});
+}
+
 #define EMU_LOGN_SWITCH(logN, CALL)                                        \
     do switch (logN) {                                                     \
         case 10: { constexpr int LG = 10; CALL; } break;                   \
@@ -422,6 +483,23 @@ void emu_ntt(void* h, uint64_t* poly, size_t limbs, size_t first, int basis, int
     const Emu& E = *static_cast<Emu*>(h);
     for (size_t l = 0; l < limbs; ++l)
         ntt_one(E, poly + l * E.H.N, (int)((basis ? E.H.nq : 0) + first + l), !inverse);
+}
+
+// The same through the one-launch transforms.
+void emu_ntt_whole(void* h, uint64_t* poly, size_t limbs, size_t first, int basis, int inverse) {
+    const Emu& E = *static_cast<Emu*>(h);
+    for (size_t l = 0; l < limbs; ++l) {
+        uint64_t* x = poly + l * E.H.N;
+        const int mi = (int)((basis ? E.H.nq : 0) + first + l);
+        switch (E.logN) {
+            case 10: whole_ntt<10>(E, x, mi, !inverse); break;
+            case 11: whole_ntt<11>(E, x, mi, !inverse); break;
+            case 12: whole_ntt<12>(E, x, mi, !inverse); break;
+            case 13: whole_ntt<13>(E, x, mi, !inverse); break;
+            case 14: whole_ntt<14>(E, x, mi, !inverse); break;
+            default: throw std::invalid_argument("emu: ring too large for the one-launch transform");
+        }
+    }
 }
 
 // The device keyswitch() sequence, stage by stage, with the same buffers.

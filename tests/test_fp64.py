@@ -96,6 +96,27 @@ def test_emulated_transforms_at_the_edges(oracle_mod, emu, logN, geometry):  # n
         emu.emu_destroy(h)
 
 
+@pytest.mark.parametrize("logN", [10, 11, 12, 13, 14])
+def test_emulated_whole_transforms(oracle_mod, emu, logN):  # noqa: F811
+    """The one-launch transform (1 to 8 CTAs a cluster) in each arithmetic: FP64 with and without
+    reductions inside, lazy words and fully reduced words."""
+    N = 1 << logN
+    q = np.array([_prime(1 << 50, N), _prime(1 << 38, N), _prime(1 << 55, N), _prime(1 << 61, N)], np.uint64)
+    o = oracle_mod.OracleCtx(N, q[:3], q[3:], 1)
+    h = emu.emu_create(N, q[:3].copy(), 3, q[3:].copy(), 1, 1)
+    emu.emu_ntt_whole.argtypes = emu.emu_ntt.argtypes
+    try:
+        for basis, mods in ((0, q[:3]), (1, q[3:])):
+            x = np.concatenate([np.random.default_rng(int(m) % 1000).integers(0, int(m), N, dtype=np.uint64) for m in mods])
+            y = x.copy()
+            emu.emu_ntt_whole(h, y, len(mods), 0, basis, 0)
+            assert (y == o.ntt(x, which=basis)).all(), basis
+            emu.emu_ntt_whole(h, y, len(mods), 0, basis, 1)
+            assert (y == x).all(), basis
+    finally:
+        emu.emu_destroy(h)
+
+
 # digits of eight 50-bit limbs over nine 50-bit P limbs (the sums' bound, every width of the ModDown);
 # digits and P limbs that mix FP64 and word moduli in both roles
 MIXED = [dict(logN=10, q_bits=[50] * 8, p_bits=[50] * 9, dnum=1),
@@ -140,7 +161,7 @@ def test_transforms_at_the_edges(wg, oracle_mod, logN):
     o, ctx = oracle_mod.OracleCtx(N, q, p, 1), wg.Context(N, q, p, 1)
     rng = np.random.default_rng(logN)
     polys = [_extreme_polys(int(m), N, rng) for m in q]
-    for geometry in range(4):
+    for geometry in range(-1, 4):  # -1: unpinned (the one-launch transform up to 2^14)
         for d in range(2):
             for ph in range(2):
                 ctx.set_ntt_geometry(d, ph, geometry)
