@@ -36,9 +36,10 @@ struct Modulus {
     uint64_t n_inv;      // N^{-1} mod q
     uint64_t n_inv_shoup;
     double inv_q;        // 1.0 / (double)q
-    // for q < fp::kLimit: (double)q, and N^{-1} as an FP64 factor (wg_fp.cuh)
+    // for q < fp::kLimit: (double)q, and N^{-1} and 2^-64 mod q as FP64 factors (wg_fp.cuh)
     double qd;
     double n_inv_w, n_inv_wq;
+    double r_inv_w, r_inv_wq;
 };
 
 WG_HD uint64_t umulhi(uint64_t a, uint64_t b) {

@@ -106,22 +106,31 @@ __global__ void __launch_bounds__(kT) kb_mac(const MacJob* jobs, int n, const Mo
               j->acc, N, j->i, coeff);
 }
 
-// acc_{a,b}[i] = sum_parts REDC(digit_part[i] * key_part_{a,b}[i]) for the NC switches of a group,
-// parts accumulated in order as in mac_accumulate (wg_keyswitch.cuh).  NC is a compile-time
-// count so that every digit load of a part is unconditional and all of them are in flight at once.
-template <int NC>
-__device__ __forceinline__ void mac_group(const MacGroupJob* j, const Modulus* mods, int nq, size_t N) {
+// acc_{a,b}[i] = sum_parts REDC(digit_part[i] * key_part_{a,b}[i]) for switches [c0, c0 + NC) of a
+// group, parts accumulated in order as in mac_accumulate (wg_keyswitch.cuh).  NC is a compile-time
+// count so that every digit load of a part is unconditional and all of them are in flight at once;
+// a group of more than kMacPass switches takes two passes, the second finding the key words in L1,
+// which keeps the sums in 64 registers and four blocks on an SM.
+// FP: the modulus is below fp::kLimit and the sums run in FP64 (mac_words_fp); 16 FP64 instructions
+// per part and switch against two Montgomery products, which leaves the kernel to its loads.
+constexpr int kMacPass = 4;
+template <int NC, bool FP>
+__device__ __forceinline__ void mac_group(const MacGroupJob* j, int c0, const Modulus& m, size_t N) {
     const size_t coeff = (size_t)blockIdx.x * kT + threadIdx.x;
     const int i = j->i, L = j->L, K = j->K, T = L + K;
     const bool is_p = i >= L;
-    const Modulus& m = mods[is_p ? nq + (i - L) : i];
     const uint64_t q = m.q, qninv = m.qninv;
+    const double qd = m.qd, inv_q = m.inv_q;
     const size_t key_limbs = (size_t)j->key_level + 1 + K;
     const size_t klimb = is_p ? (size_t)j->key_level + 1 + (i - L) : (size_t)i;
     const size_t at = (size_t)i * N + coeff;
     uint64_t acc_a[NC], acc_b[NC];
+    double sum_a[NC], sum_b[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) acc_a[c] = acc_b[c] = 0;
+    for (int c = 0; c < NC; ++c) {
+        acc_a[c] = acc_b[c] = 0;
+        sum_a[c] = sum_b[c] = 0.0;
+    }
     for (int p = 0; p < j->parts; ++p) {
         const int s0 = p * j->alpha, s1 = s0 + j->alpha < L ? s0 + j->alpha : L;
         const bool own = !is_p && i >= s0 && i < s1;
@@ -129,17 +138,39 @@ __device__ __forceinline__ void mac_group(const MacGroupJob* j, const Modulus* m
         const uint64_t kb = j->key[(((size_t)p * 2 + 1) * key_limbs + klimb) * N + coeff];
         uint64_t d[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) d[c] = own ? j->key_term[c][at] : j->digits[c][p * j->part_stride + at];
+        for (int c = 0; c < NC; ++c) d[c] = own ? j->key_term[c0 + c][at] : j->digits[c0 + c][p * j->part_stride + at];
+        if (FP) {
+            const fp::Factor fa = fp::key_factor(ka, inv_q), fb = fp::key_factor(kb, inv_q);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            acc_a[c] = add_mod(acc_a[c], mont_mul(d[c], ka, q, qninv), q);
-            acc_b[c] = add_mod(acc_b[c], mont_mul(d[c], kb, q, qninv), q);
+            for (int c = 0; c < NC; ++c) {
+                const double x = fp::from_word(d[c]);
+                sum_a[c] = fp::mont_sum_bound(dadd(sum_a[c], fp::mulmod(x, fa.w, fa.wq, qd)), p, m);
+                sum_b[c] = fp::mont_sum_bound(dadd(sum_b[c], fp::mulmod(x, fb.w, fb.wq, qd)), p, m);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                acc_a[c] = add_mod(acc_a[c], mont_mul(d[c], ka, q, qninv), q);
+                acc_b[c] = add_mod(acc_b[c], mont_mul(d[c], kb, q, qninv), q);
+            }
         }
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        j->acc[c][at] = acc_a[c];
-        j->acc[c][(size_t)T * N + at] = acc_b[c];
+        j->acc[c0 + c][at] = FP ? fp::mont_sum_word(sum_a[c], m) : acc_a[c];
+        j->acc[c0 + c][(size_t)T * N + at] = FP ? fp::mont_sum_word(sum_b[c], m) : acc_b[c];
+    }
+}
+template <bool FP>
+__device__ __forceinline__ void mac_passes(const MacGroupJob* j, const Modulus& m, size_t N) {
+    static_assert(kMacPass == 4, "one case per pass size");
+    for (int c0 = 0; c0 < j->n; c0 += kMacPass) {
+        switch (j->n - c0) {  // the same for every thread of the block
+            case 1: mac_group<1, FP>(j, c0, m, N); break;
+            case 2: mac_group<2, FP>(j, c0, m, N); break;
+            case 3: mac_group<3, FP>(j, c0, m, N); break;
+            default: mac_group<4, FP>(j, c0, m, N); break;
+        }
     }
 }
 
@@ -147,17 +178,11 @@ __global__ void __launch_bounds__(kT, 3) kb_mac_group(const MacGroupJob* jobs, i
                                                       size_t N) {
     const MacGroupJob* j = job_of(jobs, n);
     if (!j) return;
-    static_assert(kMacGroup == 8, "one case per group size");
-    switch (j->n) {  // the same for every thread of the block
-        case 1: mac_group<1>(j, mods, nq, N); break;
-        case 2: mac_group<2>(j, mods, nq, N); break;
-        case 3: mac_group<3>(j, mods, nq, N); break;
-        case 4: mac_group<4>(j, mods, nq, N); break;
-        case 5: mac_group<5>(j, mods, nq, N); break;
-        case 6: mac_group<6>(j, mods, nq, N); break;
-        case 7: mac_group<7>(j, mods, nq, N); break;
-        default: mac_group<8>(j, mods, nq, N); break;
-    }
+    const Modulus& m = mods[j->i >= j->L ? nq + (j->i - j->L) : j->i];
+    if (m.q < fp::kLimit)
+        mac_passes<true>(j, m, N);
+    else
+        mac_passes<false>(j, m, N);
 }
 
 __global__ void __launch_bounds__(kT) kb_moddown(const ModDownJob* jobs, int n, const Modulus* mods, int nq, int K,

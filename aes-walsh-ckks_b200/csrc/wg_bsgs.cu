@@ -120,30 +120,42 @@ struct AccumJob {
     int ngiants, i, pad0, pad1;
 };
 
-// NC (the ciphertexts of the job) is a compile-time count so that every digit load of a part is
-// unconditional and all of them are in flight at once.
-template <int NC>
-__device__ __forceinline__ void baby_step(const BabyJob* j, const CtRef* __restrict__ cts,
+// The b sum of a baby step whose input word b is not below q: add_mod keeps such a word's excess
+// while every step wraps, so the sum is formed step by step in that order (such words come from
+// products with a single Barrett correction and are rare).
+__device__ __noinline__ uint64_t baby_b_sum(const uint64_t* key_b, size_t key_stride, const uint64_t* a,
+                                            const uint64_t* digit, size_t part_stride, int parts, int own_part,
+                                            uint64_t b, uint64_t q, uint64_t qninv) {
+    for (int p = 0; p < parts; ++p)
+        b = add_mod(b, mont_mul(p == own_part ? *a : digit[p * part_stride], key_b[p * key_stride], q, qninv), q);
+    return b;
+}
+
+// Ciphertexts [c0, c0 + NC) of the job.  NC is a compile-time count so that every digit load of a part
+// is unconditional and all of them are in flight at once; FP: sums in FP64; passes as in mac_group.
+template <int NC, bool FP>
+__device__ __forceinline__ void baby_step(const BabyJob* j, int c0, const Modulus& m, const CtRef* __restrict__ cts,
                                           const uint64_t* __restrict__ digits, uint64_t* __restrict__ babies,
-                                          const Modulus* mods, int nq, int L, int K, int parts, int alpha,
-                                          int nslots, int logN) {
+                                          int L, int K, int parts, int alpha, int nslots, int logN) {
     const size_t N = size_t{1} << logN;
     const uint32_t x = blockIdx.x * kT + threadIdx.x;
     const int i = j->i;
     const int T = L + K;
     const bool is_p = i >= L;
-    const Modulus& m = mods[is_p ? nq + (i - L) : i];
     const uint64_t q = m.q, qninv = m.qninv;
+    const double qd = m.qd, inv_q = m.inv_q;
     const size_t key_limbs = (size_t)j->key_level + 1 + K;
     const size_t klimb = is_p ? (size_t)j->key_level + 1 + (i - L) : (size_t)i;
     const size_t part_stride = (size_t)T * N;
     const size_t limb = (size_t)i * N + x;
-    const CtRef* ct = cts + j->c0;
+    const CtRef* ct = cts + c0;
     uint64_t acc_a[NC], acc_b[NC];
+    double sum_a[NC], sum_b[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         acc_a[c] = 0;
-        acc_b[c] = is_p ? 0 : ct[c].b[limb];
+        acc_b[c] = is_p || FP ? 0 : ct[c].b[limb];
+        sum_a[c] = sum_b[c] = 0.0;
     }
     for (int p = 0; p < parts; ++p) {
         const int s0 = p * alpha, s1 = s0 + alpha < L ? s0 + alpha : L;
@@ -153,20 +165,57 @@ __device__ __forceinline__ void baby_step(const BabyJob* j, const CtRef* __restr
         uint64_t d[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-            d[c] = own ? ct[c].a[limb] : digits[((size_t)(j->c0 + c) * parts + p) * part_stride + limb];
+            d[c] = own ? ct[c].a[limb] : digits[((size_t)(c0 + c) * parts + p) * part_stride + limb];
+        if (FP) {
+            const fp::Factor fa = fp::key_factor(ka, inv_q), fb = fp::key_factor(kb, inv_q);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            acc_a[c] = add_mod(acc_a[c], mont_mul(d[c], ka, q, qninv), q);
-            acc_b[c] = add_mod(acc_b[c], mont_mul(d[c], kb, q, qninv), q);
+            for (int c = 0; c < NC; ++c) {
+                const double w = fp::from_word(d[c]);
+                sum_a[c] = fp::mont_sum_bound(dadd(sum_a[c], fp::mulmod(w, fa.w, fa.wq, qd)), p, m);
+                sum_b[c] = fp::mont_sum_bound(dadd(sum_b[c], fp::mulmod(w, fb.w, fb.wq, qd)), p, m);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                acc_a[c] = add_mod(acc_a[c], mont_mul(d[c], ka, q, qninv), q);
+                acc_b[c] = add_mod(acc_b[c], mont_mul(d[c], kb, q, qninv), q);
+            }
         }
     }
     const uint32_t dst = automorphism_src(x, j->galois_inv, logN);
     const size_t slot_words = 2 * (size_t)T * N;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        uint64_t* o = babies + ((size_t)(j->c0 + c) * nslots + j->slot) * slot_words + (size_t)i * N;
+        if (FP) {
+            acc_a[c] = fp::mont_sum_word(sum_a[c], m);
+            acc_b[c] = fp::mont_sum_word(sum_b[c], m);
+            if (!is_p) {
+                const uint64_t b = ct[c].b[limb];
+                acc_b[c] = b < q ? add_mod(b, acc_b[c], q)
+                                 : baby_b_sum(j->key + (key_limbs + klimb) * N + x, 2 * key_limbs * N, ct[c].a + limb,
+                                              digits + (size_t)(c0 + c) * parts * part_stride + limb, part_stride,
+                                              parts, i / alpha, b, q, qninv);
+            }
+        }
+        uint64_t* o = babies + ((size_t)(c0 + c) * nslots + j->slot) * slot_words + (size_t)i * N;
         o[dst] = acc_a[c];
         o[(size_t)T * N + dst] = acc_b[c];
+    }
+}
+
+template <bool FP>
+__device__ __forceinline__ void baby_passes(const BabyJob* j, const Modulus& m, const CtRef* __restrict__ cts,
+                                            const uint64_t* __restrict__ digits, uint64_t* __restrict__ babies, int L,
+                                            int K, int parts, int alpha, int nslots, int logN) {
+    static_assert(kMacPass == 4, "one case per pass size");
+    const int end = j->c0 + j->nc;
+    for (int c0 = j->c0; c0 < end; c0 += kMacPass) {
+        switch (end - c0) {  // the same for every thread of the block
+            case 1: baby_step<1, FP>(j, c0, m, cts, digits, babies, L, K, parts, alpha, nslots, logN); break;
+            case 2: baby_step<2, FP>(j, c0, m, cts, digits, babies, L, K, parts, alpha, nslots, logN); break;
+            case 3: baby_step<3, FP>(j, c0, m, cts, digits, babies, L, K, parts, alpha, nslots, logN); break;
+            default: baby_step<4, FP>(j, c0, m, cts, digits, babies, L, K, parts, alpha, nslots, logN); break;
+        }
     }
 }
 
@@ -176,19 +225,11 @@ __global__ void __launch_bounds__(kT, 3) kb_baby(const BabyJob* jobs, int n, con
                                                  int nslots, int logN) {
     const BabyJob* j = job_of(jobs, n);
     if (!j) return;
-    static_assert(kGiantBatch == 8, "one case per batch size");
-#define WG_BABY(NC) baby_step<NC>(j, cts, digits, babies, mods, nq, L, K, parts, alpha, nslots, logN)
-    switch (j->nc) {  // the same for every thread of the block
-        case 1: WG_BABY(1); break;
-        case 2: WG_BABY(2); break;
-        case 3: WG_BABY(3); break;
-        case 4: WG_BABY(4); break;
-        case 5: WG_BABY(5); break;
-        case 6: WG_BABY(6); break;
-        case 7: WG_BABY(7); break;
-        default: WG_BABY(8); break;
-    }
-#undef WG_BABY
+    const Modulus& m = mods[j->i >= L ? nq + (j->i - L) : j->i];
+    if (m.q < fp::kLimit)
+        baby_passes<true>(j, m, cts, digits, babies, L, K, parts, alpha, nslots, logN);
+    else
+        baby_passes<false>(j, m, cts, digits, babies, L, K, parts, alpha, nslots, logN);
 }
 
 // Adds one term's products to the accumulator pair of its giant step.  g is the same for every
@@ -217,31 +258,64 @@ __device__ __forceinline__ void giant_add(int g, uint64_t pa, uint64_t pb, uint6
     }
 }
 
+// The same in FP64 for moduli below fp::kNoReduce: the terms' factors x (baby-step words) and d (a
+// diagonal word, Montgomery form), exact sums with one reduction at the end.
+__device__ __forceinline__ void giant_add_fp(int g, double xa, double xb, double d, fp::Dot* sum_a, fp::Dot* sum_b) {
+    switch (g) {
+#define WG_GIANT_ADD(G)      \
+    case G:                  \
+        sum_a[G].add(xa, d); \
+        sum_b[G].add(xb, d); \
+        break;
+        WG_GIANT_ADD(0)
+        WG_GIANT_ADD(1)
+        WG_GIANT_ADD(2)
+        WG_GIANT_ADD(3)
+        WG_GIANT_ADD(4)
+        WG_GIANT_ADD(5)
+        WG_GIANT_ADD(6)
+        WG_GIANT_ADD(7)
+#undef WG_GIANT_ADD
+        default:
+            break;
+    }
+}
+
 // Giant-step inner sums: inner[c][g] = sum over the terms (g, slot) of diag x baby[c][slot], in
 // QP.  Montgomery products and modular additions of canonical residues, so the order of the
 // terms does not change the canonical sums.
 // The terms go kGiantUnroll at a time: their table entries, then all their diagonal and baby-step
 // words, then the products, so each warp has that many HBM loads in flight rather than one
 // dependent chain per term (a baby-step word shared by consecutive terms is read again from L1).
+// A term costs two products: about 66 integer instructions, or 8 FP64 ones plus 6 for the words'
+// conversion (moduli below fp::kNoReduce), which is what bounds the kernel.
 constexpr int kGiantUnroll = 4;
+static_assert(fp::kDotTerms % kGiantUnroll == 0, "a giant step's sums are carried over between unrolled groups");
 
-__global__ void __launch_bounds__(kT, 3) kb_giant(const GiantJob* jobs, int n, const TermRef* __restrict__ term_table,
-                                                  const Modulus* mods, int nq, int L, int T, int nslots, int ngiants,
-                                                  size_t N) {
-    const GiantJob* j = job_of(jobs, n);
-    if (!j) return;
+template <bool FP>
+__device__ __forceinline__ void giant_sums(const GiantJob* j, const Modulus& m, const TermRef* __restrict__ term_table,
+                                           int T, int nslots, int ngiants, size_t N) {
     const size_t x = (size_t)blockIdx.x * kT + threadIdx.x;
-    const int i = j->i;
-    const Modulus& m = mods[i < L ? i : nq + (i - L)];
     const uint64_t q = m.q, qninv = m.qninv;
-    const size_t limb = (size_t)i * N + x;
+    const size_t limb = (size_t)j->i * N + x;
     const size_t slot_words = 2 * (size_t)T * N;
     uint64_t acc_a[kGiantGroup], acc_b[kGiantGroup];
+    fp::Dot sum_a[kGiantGroup], sum_b[kGiantGroup];
 #pragma unroll
-    for (int g = 0; g < kGiantGroup; ++g) acc_a[g] = acc_b[g] = 0;
+    for (int g = 0; g < kGiantGroup; ++g) {
+        acc_a[g] = acc_b[g] = 0;
+        sum_a[g].clear();
+        sum_b[g].clear();
+    }
     const uint64_t* babies = j->babies + (size_t)j->c * nslots * slot_words + limb;
     const TermRef* terms = term_table + j->term0;
     const int nterms = j->nterms;
+    auto add = [&](const TermRef& tr, uint64_t d, uint64_t ba, uint64_t bb) {
+        if (FP)
+            giant_add_fp(tr.g, fp::from_word(ba), fp::from_word(bb), fp::from_word(d), sum_a, sum_b);
+        else
+            giant_add(tr.g, mont_mul(ba, d, q, qninv), mont_mul(bb, d, q, qninv), q, acc_a, acc_b);
+    };
     int t = 0;
     for (; t + kGiantUnroll <= nterms; t += kGiantUnroll) {
         TermRef tr[kGiantUnroll];
@@ -256,22 +330,40 @@ __global__ void __launch_bounds__(kT, 3) kb_giant(const GiantJob* jobs, int n, c
             bb[u] = bs[(size_t)T * N];
         }
 #pragma unroll
-        for (int u = 0; u < kGiantUnroll; ++u)
-            giant_add(tr[u].g, mont_mul(ba[u], d[u], q, qninv), mont_mul(bb[u], d[u], q, qninv), q, acc_a, acc_b);
+        for (int u = 0; u < kGiantUnroll; ++u) add(tr[u], d[u], ba[u], bb[u]);
+        // every sum holds at most one term per table entry since it was carried over last
+        if (FP && (t + kGiantUnroll) % fp::kDotTerms == 0) {
+#pragma unroll
+            for (int g = 0; g < kGiantGroup; ++g) {
+                sum_a[g].carry(m.qd, m.inv_q);
+                sum_b[g].carry(m.qd, m.inv_q);
+            }
+        }
     }
     for (; t < nterms; ++t) {
         const TermRef tr = terms[t];
         const uint64_t* bs = babies + (size_t)tr.slot * slot_words;
-        const uint64_t d = tr.diag[limb];
-        giant_add(tr.g, mont_mul(bs[0], d, q, qninv), mont_mul(bs[(size_t)T * N], d, q, qninv), q, acc_a, acc_b);
+        add(tr, tr.diag[limb], bs[0], bs[(size_t)T * N]);
     }
 #pragma unroll
     for (int g = 0; g < kGiantGroup; ++g) {
         if (g >= j->ng) break;
         uint64_t* o = j->inner + ((size_t)j->c * ngiants + j->g0 + g) * slot_words;
-        o[limb] = acc_a[g];
-        o[(size_t)T * N + limb] = acc_b[g];
+        o[limb] = FP ? fp::mont_sum_word(sum_a[g].value(m.qd, m.inv_q), m) : acc_a[g];
+        o[(size_t)T * N + limb] = FP ? fp::mont_sum_word(sum_b[g].value(m.qd, m.inv_q), m) : acc_b[g];
     }
+}
+
+__global__ void __launch_bounds__(kT, 2) kb_giant(const GiantJob* jobs, int n, const TermRef* __restrict__ term_table,
+                                                  const Modulus* mods, int nq, int L, int T, int nslots, int ngiants,
+                                                  size_t N) {
+    const GiantJob* j = job_of(jobs, n);
+    if (!j) return;
+    const Modulus& m = mods[j->i < L ? j->i : nq + (j->i - L)];
+    if (m.q < fp::kNoReduce)
+        giant_sums<true>(j, m, term_table, T, nslots, ngiants, N);
+    else
+        giant_sums<false>(j, m, term_table, T, nslots, ngiants, N);
 }
 
 __global__ void __launch_bounds__(kT) kb_moddown_single(const ModDownJob* jobs, int n, const Modulus* mods, int nq,

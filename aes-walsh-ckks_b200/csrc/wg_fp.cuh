@@ -99,6 +99,25 @@ WG_HD void factor_of(uint64_t w, double q, double inv_q, double& fw, double& fwq
     fwq = dmul(fw, inv_q);
 }
 
+// Sums of Montgomery products (key inner products): each term x k, k a stored word in [0, q) (the
+// factor times 2^64) and x a word below 2 q, is formed without the 2^-64, which one product per sum
+// puts back.  wq = k inv_q is off by at most 2^-52, so a term is at most 1.1 q in magnitude; sums
+// of the moduli from kNoReduce up are brought to q / 2 after every fourth term.
+struct Factor {
+    double w, wq;
+};
+WG_HD Factor key_factor(uint64_t k, double inv_q) {
+    const double w = from_word(k);
+    return {w, dmul(w, inv_q)};
+}
+WG_HD double mont_sum_bound(double acc, int term, const Modulus& m) {
+    return m.q >= kNoReduce && (term & 3) == 3 ? reduce(acc, m.qd, m.inv_q) : acc;
+}
+WG_HD uint64_t mont_sum_word(double acc, const Modulus& m) {
+    if (m.q >= kNoReduce) acc = reduce(acc, m.qd, m.inv_q);
+    return to_word(lift(mulmod(acc, m.r_inv_w, m.r_inv_wq, m.qd), m.qd));
+}
+
 // Sums of many products a w for moduli below kNoReduce, 4 FP64 instructions a term and one reduction
 // a sum: h collects the products rounded to multiples of 2^40 (it stays in the binade of kDot, whose
 // spacing that is), l the exact remainders (and any small value carried along).  Factors below 2^43
@@ -116,6 +135,11 @@ struct Dot {
         const double t = dfma(a, w, h);
         l = dadd(l, dfma(a, w, -dadd(t, -h)));
         h = t;
+    }
+    // the sum so far as one term, so that kDotTerms more may follow
+    WG_HD void carry(double q, double inv_q) {
+        l = value(q, inv_q);
+        h = kDot;
     }
     // a representative in [-q / 2, q / 2]: the quotient is at most 32 factors of 43 bits, below 2^48
     // and off by less than one part in 2^51 of itself, so the remainder of h is an integer below q

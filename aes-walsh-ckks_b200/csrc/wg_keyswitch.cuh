@@ -14,6 +14,7 @@
 #include <cstdint>
 
 #include "wg_arith.cuh"
+#include "wg_fp.cuh"
 
 namespace wg {
 
@@ -163,6 +164,29 @@ WG_HD void mac_accumulate(const Modulus& m, int L, int K, int parts, int alpha, 
     }
 }
 
+// The same sums from zero in FP64 (m.q < fp::kLimit), as canonical words: the key words stay in
+// Montgomery form, one product by 2^-64 per sum takes it out again.
+WG_HD void mac_words_fp(const Modulus& m, int L, int K, int parts, int alpha, const uint64_t* __restrict__ key,
+                        int key_level, const uint64_t* __restrict__ key_term, const uint64_t* __restrict__ digits,
+                        size_t part_stride, size_t N, int i, size_t coeff, uint64_t& out_a, uint64_t& out_b) {
+    const bool is_p = i >= L;
+    const size_t key_limbs = (size_t)key_level + 1 + K;
+    const size_t klimb = is_p ? (size_t)key_level + 1 + (i - L) : (size_t)i;
+    double acc_a = 0.0, acc_b = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < parts; ++j) {
+        const int s0 = j * alpha, s1 = s0 + alpha < L ? s0 + alpha : L;
+        const double d = fp::from_word((!is_p && i >= s0 && i < s1) ? key_term[(size_t)i * N + coeff]
+                                                                    : digits[j * part_stride + (size_t)i * N + coeff]);
+        const fp::Factor ka = fp::key_factor(key[(((size_t)j * 2 + 0) * key_limbs + klimb) * N + coeff], m.inv_q);
+        const fp::Factor kb = fp::key_factor(key[(((size_t)j * 2 + 1) * key_limbs + klimb) * N + coeff], m.inv_q);
+        acc_a = fp::mont_sum_bound(dadd(acc_a, fp::mulmod(d, ka.w, ka.wq, m.qd)), j, m);
+        acc_b = fp::mont_sum_bound(dadd(acc_b, fp::mulmod(d, kb.w, kb.wq, m.qd)), j, m);
+    }
+    out_a = fp::mont_sum_word(acc_a, m);
+    out_b = fp::mont_sum_word(acc_b, m);
+}
+
 // Key inner product for QP limb i at one coefficient:
 //   acc_{a,b}[i] = sum_parts REDC(digit_part[i] * key_part_{a,b}[i]).
 // Source limbs of a digit use the evaluation-form key term itself (as the reference does).
@@ -173,7 +197,10 @@ WG_HD void mac_coeff(const Modulus* __restrict__ mods, int nq, int L, int K, int
     const int T = L + K;
     const Modulus& m = mods[i >= L ? nq + (i - L) : i];
     uint64_t acc_a = 0, acc_b = 0;
-    mac_accumulate(m, L, K, parts, alpha, key, key_level, key_term, digits, part_stride, N, i, coeff, acc_a, acc_b);
+    if (m.q < fp::kLimit)
+        mac_words_fp(m, L, K, parts, alpha, key, key_level, key_term, digits, part_stride, N, i, coeff, acc_a, acc_b);
+    else
+        mac_accumulate(m, L, K, parts, alpha, key, key_level, key_term, digits, part_stride, N, i, coeff, acc_a, acc_b);
     acc[(size_t)i * N + coeff] = acc_a;
     acc[(size_t)(T + i) * N + coeff] = acc_b;
 }

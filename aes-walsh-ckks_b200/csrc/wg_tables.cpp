@@ -81,6 +81,7 @@ HostTables build_tables(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
         md.inv_q = 1.0 / (double)m;
         md.qd = (double)m;
         fp::factor(md.n_inv, m, md.n_inv_w, md.n_inv_wq);
+        fp::factor(host::inverse((uint64_t)(((unsigned __int128)1 << 64) % m), m), m, md.r_inv_w, md.r_inv_wq);
     }
 
     TableImage img{H.words};
