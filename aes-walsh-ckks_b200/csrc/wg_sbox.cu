@@ -147,6 +147,25 @@ __global__ void __launch_bounds__(kT, 2) kb_walsh_products(const WalshJob* jobs,
         lb[t] = j->low[0][t][k];
         la[t] = j->low[1][t][k];
     }
+    if (m.q < fp::kNoReduce) {
+        WalshFp f;
+        walsh_load_fp(lb, la, pt_i, m, f);
+        double xb, xa;
+        walsh_pair_fp(f, *cf, 0, j->limb, m, xb, xa);
+        j->out[0][k] = walsh_word(xb, m);
+        j->out[1][k] = walsh_word(xa, m);
+        WalshRaw raw;
+        raw.b.clear();
+        raw.a.clear();
+        raw.c.clear();
+#pragma unroll 1
+        for (int hm = 1; hm < (int)kNibble; ++hm)
+            walsh_product_fp(f, *cf, hm, j->limb, m, j->high[0][hm][k], j->high[1][hm][k], raw);
+        j->out[2][k] = walsh_word(raw.b.value(m.qd, m.inv_q), m);
+        j->out[3][k] = walsh_word(raw.a.value(m.qd, m.inv_q), m);
+        j->out[4][k] = walsh_word(raw.c.value(m.qd, m.inv_q), m);
+        return;
+    }
     WalshLow w;
     walsh_load_low(lb, la, w);
     uint64_t acc_b, acc_a;
@@ -542,6 +561,8 @@ private:
                     throw std::runtime_error("ckks_walsh_sbox: missing low-sign multiple");
                 reinterpret_cast<uint8_t*>(cf[0].cw[0][hm])[lm] = (uint8_t)((lm ? rcm : 0) + kWalshBias);
                 reinterpret_cast<uint8_t*>(cf[0].cw[1][hm])[lm] = (uint8_t)((lm ? icm : 0) + kWalshBias);
+                cf[0].cd[hm][lm][0] = lm ? (double)rcm : 0.0;
+                cf[0].cd[hm][lm][1] = lm ? (double)icm : 0.0;
             }
             for (size_t l = 0; l < L; ++l) {
                 cf[0].c0[0][hm][l] = int_const(table_[rb][0][hm], scale, c_.q[l]);

@@ -641,6 +641,8 @@ static Modulus emu_modulus(uint64_t q) {
     m.q = q;
     m.mu_lo = (uint64_t)mu;
     m.mu_hi = (uint64_t)(mu >> 64);
+    m.inv_q = 1.0 / (double)q;
+    m.qd = (double)q;
     return m;
 }
 
@@ -682,8 +684,31 @@ void emu_walsh_products(uint64_t q, size_t n, const uint64_t* low_b, const uint6
     for (int i = 0; i < 2 * 16 * 16; ++i) biased[i] = (uint8_t)(coefs[i] + kWalshBias);
     std::memcpy(cf.cw, biased, sizeof(cf.cw));
     for (int r = 0; r < 2; ++r)
-        for (int hm = 0; hm < kWalshMasks; ++hm) cf.c0[r][hm][0] = c0[r * kWalshMasks + hm];
+        for (int hm = 0; hm < kWalshMasks; ++hm) {
+            cf.c0[r][hm][0] = c0[r * kWalshMasks + hm];
+            for (int lm = 1; lm < kWalshMasks; ++lm)
+                cf.cd[hm][lm][r] = coefs[(r * kWalshMasks + hm) * kWalshMasks + lm];
+        }
     for (size_t i = 0; i < n; ++i) {
+        if (q < fp::kNoReduce) {
+            WalshFp f;
+            walsh_load_fp(low_b + i * 16, low_a + i * 16, pt_i[i], m, f);
+            uint64_t* o = out + i * 5;
+            double xb, xa;
+            walsh_pair_fp(f, cf, 0, 0, m, xb, xa);
+            o[0] = walsh_word(xb, m);
+            o[1] = walsh_word(xa, m);
+            WalshRaw raw;
+            raw.b.clear();
+            raw.a.clear();
+            raw.c.clear();
+            for (int hm = 1; hm < kWalshMasks; ++hm)
+                walsh_product_fp(f, cf, hm, 0, m, high_b[i * 16 + hm], high_a[i * 16 + hm], raw);
+            o[2] = walsh_word(raw.b.value(m.qd, m.inv_q), m);
+            o[3] = walsh_word(raw.a.value(m.qd, m.inv_q), m);
+            o[4] = walsh_word(raw.c.value(m.qd, m.inv_q), m);
+            continue;
+        }
         WalshLow w;
         walsh_load_low(low_b + i * 16, low_a + i * 16, w);
         uint64_t* o = out + i * 5;

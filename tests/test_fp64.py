@@ -9,7 +9,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from test_emulation import emu, u64p  # noqa: F401
+from test_emulation import emu, test_walsh_products_exact as _walsh_exact, u64p  # noqa: F401
 
 f64p = np.ctypeslib.ndpointer(dtype=np.float64, flags="C_CONTIGUOUS")
 
@@ -148,6 +148,13 @@ def test_emulated_mixed_key_switches(oracle_mod, emu, prm):  # noqa: F811
     finally:
         emu.emu_set_keyswitch_fusion(0)
         emu.emu_destroy(h)
+
+
+@pytest.mark.parametrize("q", [_prime(1 << 42, 1 << 15), _prime(1 << 42, 1 << 15, 1), 12289, _prime(1 << 55, 1 << 15, 1)])
+def test_walsh_products_at_the_edges(emu, q):  # noqa: F811
+    """The Walsh products on both sides of the FP64 limit, at a small modulus (coefficients and signs
+    up to 12 bits wrap) and just above the limit of the one-word sums."""
+    _walsh_exact(emu, q)
 
 
 @pytest.mark.gpu
