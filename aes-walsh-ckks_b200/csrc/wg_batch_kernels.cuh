@@ -112,23 +112,24 @@ __global__ void __launch_bounds__(kT) kb_mac(const MacJob* jobs, int n, const Mo
 // a group of more than kMacPass switches takes two passes, the second finding the key words in L1,
 // which keeps the sums in 64 registers and four blocks on an SM.
 // FP: the modulus is below fp::kLimit and the sums run in FP64 (mac_words_fp); 16 FP64 instructions
-// per part and switch against two Montgomery products, which leaves the kernel to its loads.
+// per part and switch against two Montgomery products, which leaves the kernel to its loads.  Larger
+// moduli sum their products as integers and reduce once (WideSum).
 constexpr int kMacPass = 4;
 template <int NC, bool FP>
 __device__ __forceinline__ void mac_group(const MacGroupJob* j, int c0, const Modulus& m, size_t N) {
     const size_t coeff = (size_t)blockIdx.x * kT + threadIdx.x;
     const int i = j->i, L = j->L, K = j->K, T = L + K;
     const bool is_p = i >= L;
-    const uint64_t q = m.q, qninv = m.qninv;
     const double qd = m.qd, inv_q = m.inv_q;
     const size_t key_limbs = (size_t)j->key_level + 1 + K;
     const size_t klimb = is_p ? (size_t)j->key_level + 1 + (i - L) : (size_t)i;
     const size_t at = (size_t)i * N + coeff;
-    uint64_t acc_a[NC], acc_b[NC];
+    WideSum acc_a[NC], acc_b[NC];
     double sum_a[NC], sum_b[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        acc_a[c] = acc_b[c] = 0;
+        acc_a[c].clear();
+        acc_b[c].clear();
         sum_a[c] = sum_b[c] = 0.0;
     }
     for (int p = 0; p < j->parts; ++p) {
@@ -150,15 +151,15 @@ __device__ __forceinline__ void mac_group(const MacGroupJob* j, int c0, const Mo
         } else {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                acc_a[c] = add_mod(acc_a[c], mont_mul(d[c], ka, q, qninv), q);
-                acc_b[c] = add_mod(acc_b[c], mont_mul(d[c], kb, q, qninv), q);
+                acc_a[c].add(d[c], ka, m);
+                acc_b[c].add(d[c], kb, m);
             }
         }
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        j->acc[c0 + c][at] = FP ? fp::mont_sum_word(sum_a[c], m) : acc_a[c];
-        j->acc[c0 + c][(size_t)T * N + at] = FP ? fp::mont_sum_word(sum_b[c], m) : acc_b[c];
+        j->acc[c0 + c][at] = FP ? fp::mont_sum_word(sum_a[c], m) : acc_a[c].mont_value(m);
+        j->acc[c0 + c][(size_t)T * N + at] = FP ? fp::mont_sum_word(sum_b[c], m) : acc_b[c].mont_value(m);
     }
 }
 template <bool FP>
@@ -174,7 +175,7 @@ __device__ __forceinline__ void mac_passes(const MacGroupJob* j, const Modulus& 
     }
 }
 
-__global__ void __launch_bounds__(kT, 3) kb_mac_group(const MacGroupJob* jobs, int n, const Modulus* mods, int nq,
+__global__ void __launch_bounds__(kT, 4) kb_mac_group(const MacGroupJob* jobs, int n, const Modulus* mods, int nq,
                                                       size_t N) {
     const MacGroupJob* j = job_of(jobs, n);
     if (!j) return;

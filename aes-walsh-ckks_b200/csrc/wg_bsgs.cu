@@ -123,7 +123,7 @@ struct AccumJob {
 // The b sum of a baby step whose input word b is not below q: add_mod keeps such a word's excess
 // while every step wraps, so the sum is formed step by step in that order (such words come from
 // products with a single Barrett correction and are rare).
-__device__ __noinline__ uint64_t baby_b_sum(const uint64_t* key_b, size_t key_stride, const uint64_t* a,
+__device__ __forceinline__ uint64_t baby_b_sum(const uint64_t* key_b, size_t key_stride, const uint64_t* a,
                                             const uint64_t* digit, size_t part_stride, int parts, int own_part,
                                             uint64_t b, uint64_t q, uint64_t qninv) {
     for (int p = 0; p < parts; ++p)
@@ -142,19 +142,19 @@ __device__ __forceinline__ void baby_step(const BabyJob* j, int c0, const Modulu
     const int i = j->i;
     const int T = L + K;
     const bool is_p = i >= L;
-    const uint64_t q = m.q, qninv = m.qninv;
+    const uint64_t q = m.q;
     const double qd = m.qd, inv_q = m.inv_q;
     const size_t key_limbs = (size_t)j->key_level + 1 + K;
     const size_t klimb = is_p ? (size_t)j->key_level + 1 + (i - L) : (size_t)i;
     const size_t part_stride = (size_t)T * N;
     const size_t limb = (size_t)i * N + x;
     const CtRef* ct = cts + c0;
-    uint64_t acc_a[NC], acc_b[NC];
+    WideSum acc_a[NC], acc_b[NC];
     double sum_a[NC], sum_b[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        acc_a[c] = 0;
-        acc_b[c] = is_p || FP ? 0 : ct[c].b[limb];
+        acc_a[c].clear();
+        acc_b[c].clear();
         sum_a[c] = sum_b[c] = 0.0;
     }
     for (int p = 0; p < parts; ++p) {
@@ -177,8 +177,8 @@ __device__ __forceinline__ void baby_step(const BabyJob* j, int c0, const Modulu
         } else {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                acc_a[c] = add_mod(acc_a[c], mont_mul(d[c], ka, q, qninv), q);
-                acc_b[c] = add_mod(acc_b[c], mont_mul(d[c], kb, q, qninv), q);
+                acc_a[c].add(d[c], ka, m);
+                acc_b[c].add(d[c], kb, m);
             }
         }
     }
@@ -186,20 +186,21 @@ __device__ __forceinline__ void baby_step(const BabyJob* j, int c0, const Modulu
     const size_t slot_words = 2 * (size_t)T * N;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        if (FP) {
-            acc_a[c] = fp::mont_sum_word(sum_a[c], m);
-            acc_b[c] = fp::mont_sum_word(sum_b[c], m);
-            if (!is_p) {
-                const uint64_t b = ct[c].b[limb];
-                acc_b[c] = b < q ? add_mod(b, acc_b[c], q)
-                                 : baby_b_sum(j->key + (key_limbs + klimb) * N + x, 2 * key_limbs * N, ct[c].a + limb,
-                                              digits + (size_t)(c0 + c) * parts * part_stride + limb, part_stride,
-                                              parts, i / alpha, b, q, qninv);
-            }
-        }
+        const uint64_t ra = FP ? fp::mont_sum_word(sum_a[c], m) : acc_a[c].mont_value(m);
+        const uint64_t rb = FP ? fp::mont_sum_word(sum_b[c], m) : acc_b[c].mont_value(m);
         uint64_t* o = babies + ((size_t)(c0 + c) * nslots + j->slot) * slot_words + (size_t)i * N;
-        o[dst] = acc_a[c];
-        o[(size_t)T * N + dst] = acc_b[c];
+        o[dst] = ra;
+        o[(size_t)T * N + dst] = is_p ? rb : add_mod(ct[c].b[limb], rb, q);
+    }
+    // words not below q, after the stores so that the sums are out of the registers
+    if (is_p) return;
+#pragma unroll 1
+    for (int c = 0; c < NC; ++c) {
+        const uint64_t b = ct[c].b[limb];
+        if (b < q) continue;
+        babies[((size_t)(c0 + c) * nslots + j->slot) * slot_words + (size_t)(T + i) * N + dst] =
+            baby_b_sum(j->key + (key_limbs + klimb) * N + x, 2 * key_limbs * N, ct[c].a + limb,
+                       digits + (size_t)(c0 + c) * parts * part_stride + limb, part_stride, parts, i / alpha, b, q, m.qninv);
     }
 }
 
@@ -219,7 +220,7 @@ __device__ __forceinline__ void baby_passes(const BabyJob* j, const Modulus& m, 
     }
 }
 
-__global__ void __launch_bounds__(kT, 3) kb_baby(const BabyJob* jobs, int n, const CtRef* __restrict__ cts,
+__global__ void __launch_bounds__(kT, 4) kb_baby(const BabyJob* jobs, int n, const CtRef* __restrict__ cts,
                                                  const uint64_t* __restrict__ digits, uint64_t* __restrict__ babies,
                                                  const Modulus* mods, int nq, int L, int K, int parts, int alpha,
                                                  int nslots, int logN) {
@@ -232,40 +233,62 @@ __global__ void __launch_bounds__(kT, 3) kb_baby(const BabyJob* jobs, int n, con
         baby_passes<false>(j, m, cts, digits, babies, L, K, parts, alpha, nslots, logN);
 }
 
-// Adds one term's products to the accumulator pair of its giant step.  g is the same for every
-// thread of the block (one job per block), so this is a uniform branch to that pair; the
-// accumulators keep constant indices and stay in registers.
-__device__ __forceinline__ void giant_add(int g, uint64_t pa, uint64_t pb, uint64_t q, uint64_t* acc_a,
-                                          uint64_t* acc_b) {
+// The sums of a giant step, by modulus: terms x d of a baby-step word x and a diagonal word d
+// (Montgomery form), the 2^-64 taken out once a sum.
+//   below fp::kNoReduce: exact FP64 sums, 4 FP64 instructions a product (of the same words in
+//     Montgomery products: two high and two low 64-bit products, 0.4 SM clocks a lane against 0.06);
+//   below fp::kLimit: FP64 products, reduced as they are added;
+//   larger: 128-bit integer sums (WideSum), half the 64-bit products.
+// The giant sums of a Walsh AES evaluation take 58.5 ms, 61.7 with Montgomery products from
+// fp::kNoReduce up; those of the CoeffToSlot of eight ciphertexts 1.83 ms against 1.91.
+struct GiantDot {
+    using X = double;
+    using D = double;
+    fp::Dot s;
+    static __device__ X baby(uint64_t w) { return fp::from_word(w); }
+    static __device__ D diag(uint64_t w, const Modulus&) { return fp::from_word(w); }
+    __device__ void clear() { s.clear(); }
+    __device__ void add(X x, D d, const Modulus&) { s.add(x, d); }
+    __device__ void carry(const Modulus& m) { s.carry(m.qd, m.inv_q); }
+    __device__ uint64_t word(const Modulus& m) const { return fp::mont_sum_word(s.value(m.qd, m.inv_q), m); }
+};
+struct GiantFp {
+    using X = double;
+    using D = fp::Factor;
+    double s;
+    static __device__ X baby(uint64_t w) { return fp::from_word(w); }
+    static __device__ D diag(uint64_t w, const Modulus& m) { return fp::key_factor(w, m.inv_q); }
+    __device__ void clear() { s = 0.0; }
+    __device__ void add(X x, const D& d, const Modulus& m) {
+        s = fp::reduce(dadd(s, fp::mulmod(x, d.w, d.wq, m.qd)), m.qd, m.inv_q);
+    }
+    __device__ void carry(const Modulus&) {}
+    __device__ uint64_t word(const Modulus& m) const { return fp::mont_sum_word(s, m); }
+};
+struct GiantWide {
+    using X = uint64_t;
+    using D = uint64_t;
+    WideSum s;
+    static __device__ X baby(uint64_t w) { return w; }
+    static __device__ D diag(uint64_t w, const Modulus&) { return w; }
+    __device__ void clear() { s.clear(); }
+    __device__ void add(X x, D d, const Modulus& m) { s.add(x, d, m); }
+    __device__ void carry(const Modulus&) {}
+    __device__ uint64_t word(const Modulus& m) const { return s.mont_value(m); }
+};
+
+// Adds one term's products to the sum pair of its giant step.  g is the same for every thread of the
+// block (one job per block), so this is a uniform branch to that pair; the sums keep constant
+// indices and stay in registers.
+template <class S>
+__device__ __forceinline__ void giant_add(int g, typename S::X xa, typename S::X xb, const typename S::D& d,
+                                          const Modulus& m, S* sum_a, S* sum_b) {
     static_assert(kGiantGroup == 8, "one case per giant step of a group");
     switch (g) {
-#define WG_GIANT_ADD(G)                          \
-    case G:                                      \
-        acc_a[G] = add_mod(acc_a[G], pa, q);     \
-        acc_b[G] = add_mod(acc_b[G], pb, q);     \
-        break;
-        WG_GIANT_ADD(0)
-        WG_GIANT_ADD(1)
-        WG_GIANT_ADD(2)
-        WG_GIANT_ADD(3)
-        WG_GIANT_ADD(4)
-        WG_GIANT_ADD(5)
-        WG_GIANT_ADD(6)
-        WG_GIANT_ADD(7)
-#undef WG_GIANT_ADD
-        default:
-            break;
-    }
-}
-
-// The same in FP64 for moduli below fp::kNoReduce: the terms' factors x (baby-step words) and d (a
-// diagonal word, Montgomery form), exact sums with one reduction at the end.
-__device__ __forceinline__ void giant_add_fp(int g, double xa, double xb, double d, fp::Dot* sum_a, fp::Dot* sum_b) {
-    switch (g) {
-#define WG_GIANT_ADD(G)      \
-    case G:                  \
-        sum_a[G].add(xa, d); \
-        sum_b[G].add(xb, d); \
+#define WG_GIANT_ADD(G)         \
+    case G:                     \
+        sum_a[G].add(xa, d, m); \
+        sum_b[G].add(xb, d, m); \
         break;
         WG_GIANT_ADD(0)
         WG_GIANT_ADD(1)
@@ -282,40 +305,28 @@ __device__ __forceinline__ void giant_add_fp(int g, double xa, double xb, double
 }
 
 // Giant-step inner sums: inner[c][g] = sum over the terms (g, slot) of diag x baby[c][slot], in
-// QP.  Montgomery products and modular additions of canonical residues, so the order of the
-// terms does not change the canonical sums.
+// QP.  Canonical residues of exact sums, so the order of the terms does not change them.
 // The terms go kGiantUnroll at a time: their table entries, then all their diagonal and baby-step
 // words, then the products, so each warp has that many HBM loads in flight rather than one
 // dependent chain per term (a baby-step word shared by consecutive terms is read again from L1).
-// A term costs two products: about 66 integer instructions, or 8 FP64 ones plus 6 for the words'
-// conversion (moduli below fp::kNoReduce), which is what bounds the kernel.
 constexpr int kGiantUnroll = 4;
 static_assert(fp::kDotTerms % kGiantUnroll == 0, "a giant step's sums are carried over between unrolled groups");
 
-template <bool FP>
+template <class S>
 __device__ __forceinline__ void giant_sums(const GiantJob* j, const Modulus& m, const TermRef* __restrict__ term_table,
                                            int T, int nslots, int ngiants, size_t N) {
     const size_t x = (size_t)blockIdx.x * kT + threadIdx.x;
-    const uint64_t q = m.q, qninv = m.qninv;
     const size_t limb = (size_t)j->i * N + x;
     const size_t slot_words = 2 * (size_t)T * N;
-    uint64_t acc_a[kGiantGroup], acc_b[kGiantGroup];
-    fp::Dot sum_a[kGiantGroup], sum_b[kGiantGroup];
+    S sum_a[kGiantGroup], sum_b[kGiantGroup];
 #pragma unroll
     for (int g = 0; g < kGiantGroup; ++g) {
-        acc_a[g] = acc_b[g] = 0;
         sum_a[g].clear();
         sum_b[g].clear();
     }
     const uint64_t* babies = j->babies + (size_t)j->c * nslots * slot_words + limb;
     const TermRef* terms = term_table + j->term0;
     const int nterms = j->nterms;
-    auto add = [&](const TermRef& tr, uint64_t d, uint64_t ba, uint64_t bb) {
-        if (FP)
-            giant_add_fp(tr.g, fp::from_word(ba), fp::from_word(bb), fp::from_word(d), sum_a, sum_b);
-        else
-            giant_add(tr.g, mont_mul(ba, d, q, qninv), mont_mul(bb, d, q, qninv), q, acc_a, acc_b);
-    };
     int t = 0;
     for (; t + kGiantUnroll <= nterms; t += kGiantUnroll) {
         TermRef tr[kGiantUnroll];
@@ -330,27 +341,28 @@ __device__ __forceinline__ void giant_sums(const GiantJob* j, const Modulus& m, 
             bb[u] = bs[(size_t)T * N];
         }
 #pragma unroll
-        for (int u = 0; u < kGiantUnroll; ++u) add(tr[u], d[u], ba[u], bb[u]);
+        for (int u = 0; u < kGiantUnroll; ++u)
+            giant_add<S>(tr[u].g, S::baby(ba[u]), S::baby(bb[u]), S::diag(d[u], m), m, sum_a, sum_b);
         // every sum holds at most one term per table entry since it was carried over last
-        if (FP && (t + kGiantUnroll) % fp::kDotTerms == 0) {
+        if ((t + kGiantUnroll) % fp::kDotTerms == 0) {
 #pragma unroll
             for (int g = 0; g < kGiantGroup; ++g) {
-                sum_a[g].carry(m.qd, m.inv_q);
-                sum_b[g].carry(m.qd, m.inv_q);
+                sum_a[g].carry(m);
+                sum_b[g].carry(m);
             }
         }
     }
     for (; t < nterms; ++t) {
         const TermRef tr = terms[t];
         const uint64_t* bs = babies + (size_t)tr.slot * slot_words;
-        add(tr, tr.diag[limb], bs[0], bs[(size_t)T * N]);
+        giant_add<S>(tr.g, S::baby(bs[0]), S::baby(bs[(size_t)T * N]), S::diag(tr.diag[limb], m), m, sum_a, sum_b);
     }
 #pragma unroll
     for (int g = 0; g < kGiantGroup; ++g) {
         if (g >= j->ng) break;
         uint64_t* o = j->inner + ((size_t)j->c * ngiants + j->g0 + g) * slot_words;
-        o[limb] = FP ? fp::mont_sum_word(sum_a[g].value(m.qd, m.inv_q), m) : acc_a[g];
-        o[(size_t)T * N + limb] = FP ? fp::mont_sum_word(sum_b[g].value(m.qd, m.inv_q), m) : acc_b[g];
+        o[limb] = sum_a[g].word(m);
+        o[(size_t)T * N + limb] = sum_b[g].word(m);
     }
 }
 
@@ -361,9 +373,11 @@ __global__ void __launch_bounds__(kT, 2) kb_giant(const GiantJob* jobs, int n, c
     if (!j) return;
     const Modulus& m = mods[j->i < L ? j->i : nq + (j->i - L)];
     if (m.q < fp::kNoReduce)
-        giant_sums<true>(j, m, term_table, T, nslots, ngiants, N);
+        giant_sums<GiantDot>(j, m, term_table, T, nslots, ngiants, N);
+    else if (m.q < fp::kLimit)
+        giant_sums<GiantFp>(j, m, term_table, T, nslots, ngiants, N);
     else
-        giant_sums<false>(j, m, term_table, T, nslots, ngiants, N);
+        giant_sums<GiantWide>(j, m, term_table, T, nslots, ngiants, N);
 }
 
 __global__ void __launch_bounds__(kT) kb_moddown_single(const ModDownJob* jobs, int n, const Modulus* mods, int nq,
@@ -626,9 +640,9 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
                         ntt_dig2.push_back({dg2 + j * T * N + l * N, dg2 + j * T * N + l * N, modq(l), 0});
             }
         }
+    double mac2_bytes = 0.0;
     // the giant's key inner products, up to kMacGroup ciphertexts per job so each key word is
     // loaded once for all of them
-    double mac2_bytes = 0.0;
     for (size_t gk = 0; gk < ng; ++gk) {
         if (giants[gk] == 0) continue;
         const KeyEntry& key = rot_key(giants[gk] * st.baby);

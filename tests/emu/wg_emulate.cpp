@@ -654,6 +654,30 @@ void emu_mont_mul(uint64_t q, const uint64_t* x, const uint64_t* y, size_t n, ui
     for (size_t i = 0; i < n; ++i) out[i] = mont_mul(x[i], y[i], q, 0 - inv);
 }
 
+// WideSum and the exact FP64 sum (fp::Dot, q < fp::kNoReduce) of n products x[i] y[i], times 2^-64
+// modulo q (qninv as in emu_mont_mul): out[0] and out[1].
+void emu_mont_sums(uint64_t q, const uint64_t* x, const uint64_t* y, size_t n, uint64_t* out) {
+    Modulus m = emu_modulus(q);
+    uint64_t inv = q;
+    for (int k = 0; k < 5; ++k) inv *= 2 - q * inv;
+    m.qninv = 0 - inv;
+    uint64_t r_inv = mont_mul(1, 1, q, m.qninv);  // 2^-64 mod q
+    fp::factor(r_inv, q, m.r_inv_w, m.r_inv_wq);
+    WideSum w;
+    w.clear();
+    fp::Dot d;
+    d.clear();
+    for (size_t i = 0; i < n; ++i) {
+        w.add(x[i], y[i], m);
+        if (q < fp::kNoReduce) {
+            d.add(fp::from_word(x[i]), fp::from_word(y[i]));
+            if ((i + 1) % fp::kDotTerms == 0) d.carry(m.qd, m.inv_q);
+        }
+    }
+    out[0] = w.mont_value(m);
+    out[1] = q < fp::kNoReduce ? fp::mont_sum_word(d.value(m.qd, m.inv_q), m) : out[0];
+}
+
 // fp::mulmod on n pairs (a[i] any integer-valued double, w[i] a residue): the representative and,
 // in word[i], the canonical word of it.
 void emu_fp_mulmod(uint64_t q, const double* a, const uint64_t* w, size_t n, double* out, uint64_t* word) {

@@ -51,6 +51,22 @@ def test_product_is_exact_and_bounded(emu, q):  # noqa: F811
         assert int(word[i]) == a[i] * w[i] % q
 
 
+@pytest.mark.parametrize("q", [_prime(1 << 42, 1 << 15), 274876334081, 12289, _prime(1 << 61, 1 << 15), _prime(1 << 62, 1 << 15)])
+@pytest.mark.parametrize("n", [1, 3, 32, 33, 500])
+def test_sums_of_products(emu, q, n):  # noqa: F811
+    """Long sums of products (exact FP64 sums carried over every 32 terms, 128-bit integer sums folded
+    on the way) with words up to 2 q - 1 times words up to q - 1, at their largest and at random."""
+    emu.emu_mont_sums.argtypes = [C.c_uint64, u64p, u64p, C.c_size_t, u64p]
+    rng = np.random.default_rng(n)
+    out = np.zeros(2, np.uint64)
+    for x, y in ((np.full(n, 2 * q - 1, np.uint64), np.full(n, q - 1, np.uint64)),
+                 (rng.integers(0, 2 * q, n, dtype=np.uint64), rng.integers(0, q, n, dtype=np.uint64)),
+                 (np.zeros(n, np.uint64), np.full(n, q - 1, np.uint64))):
+        emu.emu_mont_sums(q, x, y, n, out)
+        want = sum(int(a) * int(b) for a, b in zip(x, y)) * pow(1 << 64, -1, q) % q
+        assert [int(v) for v in out] == [want, want]
+
+
 def _extreme_polys(q, N, rng):
     """Residue polynomials that drive the lazy sums to their bounds, with words up to 4q - 1."""
     top = np.full(N, q - 1, np.uint64)
