@@ -38,8 +38,9 @@ struct KsPlan {
     int n_modup;
     const NttJob* ntt_digits;
     int n_ntt_digits;
-    const MacGroupJob* mac;
-    int n_mac;
+    const MacGroupJob *mac, *rows_mac;
+    bool rows_words;  // MacLists::words
+    int n_mac, n_rows_mac;
     const NttJob* intt_p;
     int n_intt_p;
     const ModDownJob* moddown;
@@ -53,7 +54,7 @@ struct KsPlan {
     const NttEpiJob* contrib_epi;  // fused: forward row phase of the contributions + combine
     int n_contrib_epi;
     double contrib_epi_bytes;
-    double mac_bytes, modup_bytes, moddown_bytes, combine_bytes;
+    double mac_bytes, rows_mac_bytes, modup_bytes, moddown_bytes, combine_bytes;
     bool fused;   // ModUp / ModDown fused with the NTT column phases (Context::ntt_fusion)
     int max_src;  // widest digit (fused ModUp shared memory)
     int max_dst;  // most destination limbs of a digit
@@ -70,7 +71,6 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     const size_t N = c.N, K = c.np, nq = c.nq;
     std::vector<NttJob> intt_in, ntt_digits, intt_p, ntt_contrib;
     std::vector<ModUpJob> modup;
-    std::vector<MacGroupJob> mac;
     std::vector<ModDownJob> moddown;
     std::vector<CombineJob> combine;
     std::vector<GatherJob> gather;
@@ -79,6 +79,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     p.fused = c.fuse();
     // MAC groups: consecutive switches with the same key, level and digit layout (up to
     // kMacGroup), one job per QP limb; [group_begin, it) is the open group
+    MacLists mac(c, n, n ? items[0].level + 1 + K : 0);
     size_t group_begin = 0;
     std::vector<uint64_t*> group_digits, group_acc;
     auto close_group = [&](size_t end) {
@@ -101,9 +102,8 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
                 jb.digits[k - group_begin] = group_digits[k - group_begin];
                 jb.acc[k - group_begin] = group_acc[k - group_begin];
             }
-            mac.push_back(jb);
+            mac.add(c, jb, i < L ? i : nq + (i - L));
         }
-        p.mac_bytes += 8.0 * N * T * (2.0 * B + (double)(end - group_begin) * (B + 2.0));
         group_begin = end;
         group_digits.clear();
         group_acc.clear();
@@ -129,9 +129,10 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
             p.modup_bytes += 8.0 * N * (d.src_count + d.dst_count);
             const size_t s0 = j * c.alpha, s1 = std::min(s0 + c.alpha, L);
             for (size_t l = 0; l < T; ++l) {
-                if (l >= s0 && l < s1) continue;
+                const size_t mod = l < L ? l : nq + (l - L);
+                if ((l >= s0 && l < s1) || mac.in_rows(c, mod)) continue;  // k_rows_mac transforms the latter
                 uint64_t* ptr = digits + j * T * N + l * N;
-                ntt_digits.push_back({ptr, ptr, (int)(l < L ? l : nq + (l - L)), 0});
+                ntt_digits.push_back({ptr, ptr, (int)mod, 0});
             }
         }
         if (it > group_begin) {
@@ -142,6 +143,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
         group_acc.push_back(acc);
         for (int poly = 0; poly < 2; ++poly)
             for (size_t pi = 0; pi < K; ++pi) {
+                if (mac.in_rows(c, nq + pi)) continue;
                 uint64_t* ptr = acc + (poly * T + L + pi) * N;
                 intt_p.push_back({ptr, ptr, (int)(nq + pi), 0});
             }
@@ -182,8 +184,13 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     p.n_modup = (int)modup.size();
     p.ntt_digits = t.add(ntt_digits);
     p.n_ntt_digits = (int)ntt_digits.size();
-    p.mac = t.add(mac);
-    p.n_mac = (int)mac.size();
+    p.mac = t.add(mac.sums);
+    p.n_mac = (int)mac.sums.size();
+    p.mac_bytes = mac.sums_bytes;
+    p.rows_mac = t.add(mac.rows);
+    p.n_rows_mac = (int)mac.rows.size();
+    p.rows_mac_bytes = mac.rows_bytes;
+    p.rows_words = mac.words;
     p.intt_p = t.add(intt_p);
     p.n_intt_p = (int)intt_p.size();
     p.moddown = t.add(moddown);
@@ -203,12 +210,14 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
 static void run_keyswitch(const Context& c, const KsPlan& p, const JobTable& t, cudaStream_t s) {
     const size_t N = c.N;
     if (p.fused) {
-        // inverse row phase -> [inverse column phase, ModUp, forward column phase] -> forward
-        // row phase; the same around ModDown (wg_ksfuse.cu)
+        // inverse row phase -> [inverse column phase, ModUp, forward column phase] -> [forward row
+        // phase, key product, inverse row phase of the P limbs] -> [the same around ModDown]
+        // -> forward row phase and combine (wg_ksfuse.cu, k_rows_mac, k_ntt_rows_epi)
         ntt_jobs_phase(c, t.at(p.intt_in), p.n_intt_in, false, false, s);
         modup_ntt_jobs(c, t.at(p.modup), p.n_modup, p.max_src, p.max_dst, p.modup_bytes, s);
+        rows_mac_jobs(c, t.at(p.rows_mac), p.n_rows_mac, p.rows_words, p.rows_mac_bytes, s);
         ntt_jobs_phase(c, t.at(p.ntt_digits), p.n_ntt_digits, true, false, s);
-        {
+        if (p.n_mac) {
             Probe probe(kClsKeyMac, p.mac_bytes, s);
             kb_mac_group<<<grid_for(c, p.n_mac), kT, 0, s>>>(t.at(p.mac), p.n_mac, c.d_mod, (int)c.nq, N);
         }

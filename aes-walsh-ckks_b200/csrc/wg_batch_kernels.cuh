@@ -26,17 +26,6 @@ struct MacJob {
     size_t part_stride;
     int L, K, parts, alpha, key_level, i;
 };
-// Key inner product of up to kMacGroup switches that share the key, the level and the digit
-// layout, for one QP limb: the key words of a coefficient are loaded once for all of them.
-constexpr int kMacGroup = 8;
-struct MacGroupJob {
-    const uint64_t* key;
-    const uint64_t* key_term[kMacGroup];
-    const uint64_t* digits[kMacGroup];
-    uint64_t* acc[kMacGroup];
-    size_t part_stride;
-    int L, K, parts, alpha, key_level, i, n, pad;
-};
 struct CombineJob {
     const uint64_t* acc;
     const uint64_t* contrib;

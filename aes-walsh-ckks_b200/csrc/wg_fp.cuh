@@ -100,8 +100,8 @@ WG_HD void factor_of(uint64_t w, double q, double inv_q, double& fw, double& fwq
 }
 
 // Sums of Montgomery products (key inner products): each term x k, k a stored word in [0, q) (the
-// factor times 2^64) and x a word below 2 q, is formed without the 2^-64, which one product per sum
-// puts back.  wq = k inv_q is off by at most 2^-52, so a term is at most 1.1 q in magnitude; sums
+// factor times 2^64) and x a word below 2 q (or any |x| < 2^48 where q < kNoReduce), is formed
+// without the 2^-64, which one product per sum puts back.  wq = k inv_q is off by at most 2^-52, so a term is at most 1.1 q in magnitude; sums
 // of the moduli from kNoReduce up are brought to q / 2 after every fourth term.
 struct Factor {
     double w, wq;
@@ -113,10 +113,11 @@ WG_HD Factor key_factor(uint64_t k, double inv_q) {
 WG_HD double mont_sum_bound(double acc, int term, const Modulus& m) {
     return m.q >= kNoReduce && (term & 3) == 3 ? reduce(acc, m.qd, m.inv_q) : acc;
 }
-WG_HD uint64_t mont_sum_word(double acc, const Modulus& m) {
+WG_HD double mont_sum_value(double acc, const Modulus& m) {
     if (m.q >= kNoReduce) acc = reduce(acc, m.qd, m.inv_q);
-    return to_word(lift(mulmod(acc, m.r_inv_w, m.r_inv_wq, m.qd), m.qd));
+    return mulmod(acc, m.r_inv_w, m.r_inv_wq, m.qd);
 }
+WG_HD uint64_t mont_sum_word(double acc, const Modulus& m) { return to_word(lift(mont_sum_value(acc, m), m.qd)); }
 
 // Sums of many products a w for moduli below kNoReduce, 4 FP64 instructions a term and one reduction
 // a sum: h collects the products rounded to multiples of 2^40 (it stays in the binade of kDot, whose

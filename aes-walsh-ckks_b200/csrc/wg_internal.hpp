@@ -335,6 +335,32 @@ struct RescaleNttJob {
     int words;
     uint64_t* keep;
 };
+// Key inner product of up to kMacGroup switches that share the key, the level and the digit
+// layout, for one QP limb: the key words of a coefficient are loaded once for all of them.
+constexpr int kMacGroup = 8;
+struct MacGroupJob {
+    const uint64_t* key;
+    const uint64_t* key_term[kMacGroup];
+    const uint64_t* digits[kMacGroup];
+    uint64_t* acc[kMacGroup];
+    size_t part_stride;
+    int L, K, parts, alpha, key_level, i, n, pad;
+};
+// The digits' forward row phase and the key inner product in one launch (k_rows_mac, wg_ntt.cu):
+// digits as the fused ModUp leaves them, accumulators as kb_mac_group's; p_rows: the accumulators' P
+// limbs go on through the inverse row phase, as the fused ModDown takes them.
+void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, bool words, double bytes, cudaStream_t s);
+// The key products of one batched step: `rows` for rows_mac_jobs, `sums` for kb_mac_group.
+struct MacLists {
+    std::vector<MacGroupJob> rows, sums;
+    double rows_bytes = 0.0, sums_bytes = 0.0;
+    bool words;  // whether limbs of word moduli (from fp::kLimit up) go to `rows` too
+    int group;   // switches a job of `rows` takes
+    MacLists(const Context& c, size_t switches, size_t T);
+    bool in_rows(const Context& c, size_t mod) const;
+    void add(const Context& c, const MacGroupJob& job, size_t mod);
+};
+
 // The forward row phase of job-table limbs with an element-wise epilogue (NttEpiJob, wg_ntt.cuh).
 using ntt::NttEpiJob;
 using ntt::kEpiRescale;

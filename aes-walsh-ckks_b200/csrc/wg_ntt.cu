@@ -445,6 +445,183 @@ __global__ void __launch_bounds__(Phase<LOGN, true, false, EB, STAGED>::THREADS,
     }
 }
 
+// The forward row phase of a switch's digits with the key inner product on it, for one QP limb's
+// row tile: a digit's transformed words meet the key words in the registers of the last round, where a
+// thread has 8 consecutive coefficients, and only the two accumulators are stored; with p_rows an
+// accumulator's P limb goes straight on through its inverse row phase, whose first round has the
+// thread's same 8 coefficients.  Against the separate launches a digit limb is read once instead of
+// written and read again twice over, and a switch takes two launches less.  The switches of a job
+// follow one another, so a tile's key words (parts x 32 KiB) come from L1 after the first.
+// One rotation takes 95 us, 104 with the separate launches; 64 mixed operations 4.23 ms against 4.49; the
+// 16 S-boxes of an XBOOT SubBytes layer 84.9 ms against 89.6.  Two blocks of 256 threads an SM (128
+// registers: the sums, the residues and the next digit's): latency, not the FP64 pipe, bounds it.
+template <int LOGN>
+struct RowsMac {
+    using P = Phase<LOGN, true, false, 3, false>;
+    using Begin = Round<LOGN, true, false, 3, false, 0>;
+    using End = Round<LOGN, true, false, 3, false, P::ROUNDS - 1>;
+    using InvEnd = Round<LOGN, false, false, 3, false, P::ROUNDS - 1>;
+    static constexpr auto rounds() { return std::make_integer_sequence<int, P::ROUNDS>{}; }
+    static constexpr size_t smem() { return 8 * (size_t)(P::TILE + P::TILE / 16); }
+};
+// One switch in FP64: |transformed word| <= 27 q where the modulus needs no reduction (FpArith), so its
+// product with a key word (key_factor) has |a wq| < 2^47.
+template <int LOGN>
+__device__ __forceinline__ void rows_mac_fp(uint64_t* sm, const MacGroupJob* j, int c, const Modulus& m, bool rows,
+                                            size_t at, size_t key_at, size_t key_stride, int own_part, size_t T, int tile,
+                                            int sub, int o, const TwPair* tw) {
+    using R = RowsMac<LOGN>;
+    const size_t N = R::P::N;
+    const int eb = R::Begin::element(sub, o), ee = R::End::element(sub, o), parts = j->parts;
+    const uint64_t* digits = j->digits[c] + at;
+    const uint64_t* own = j->key_term[c] + at + ee;
+    const bool red = m.q >= fp::kNoReduce;
+    uint64_t w[8];
+    auto fetch = [&](int p) {
+        if (p == own_part)
+            load_words<typename R::End>(own, w);
+        else
+            load_words<typename R::Begin>(digits + p * j->part_stride + eb, w);
+    };
+    double sa[8], sb[8], v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sa[k] = sb[k] = 0.0;
+    fetch(0);
+    for (int p = 0; p < parts; ++p) {
+        if (p == own_part) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = fp::from_word(w[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = fp::bits_double(w[k]);
+            ntt_rounds<LOGN, true, false, 3, false, kMaxTile>(R::rounds(), sm, v, sub, o, tile, fp_arith(m), tw);
+            if (red) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = fp::reduce(v[k], m.qd, m.inv_q);
+            }
+        }
+        if (p + 1 < parts) fetch(p + 1);
+        uint64_t k8[8];
+        const uint64_t* key = j->key + p * 2 * key_stride + key_at + ee;
+        load_words<typename R::End>(key, k8);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const fp::Factor f = fp::key_factor(k8[k], m.inv_q);
+            sa[k] = fp::mont_sum_bound(dadd(sa[k], fp::mulmod(v[k], f.w, f.wq, m.qd)), p, m);
+        }
+        load_words<typename R::End>(key + key_stride, k8);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const fp::Factor f = fp::key_factor(k8[k], m.inv_q);
+            sb[k] = fp::mont_sum_bound(dadd(sb[k], fp::mulmod(v[k], f.w, f.wq, m.qd)), p, m);
+        }
+    }
+#pragma unroll
+    for (int poly = 0; poly < 2; ++poly) {
+        double* s = poly ? sb : sa;
+        uint64_t* out = j->acc[c] + poly * T * N + at;
+        if (rows) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s[k] = fp::mont_sum_value(s[k], m);
+            ntt_rounds<LOGN, false, false, 3, false, kMaxTile>(R::rounds(), sm, s, sub, o, tile, fp_arith(m), tw + N);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = fp_store(false, false, fp::double_bits(s[k]), m);
+            store_words<typename R::InvEnd>(out + R::InvEnd::element(sub, o), w);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = fp::mont_sum_word(s[k], m);
+            store_words<typename R::End>(out + ee, w);
+        }
+    }
+}
+// The same in words.
+template <int LOGN, bool LAZY>
+__device__ __forceinline__ void rows_mac_words(uint64_t* sm, const MacGroupJob* j, int c, const Modulus& m, bool rows,
+                                               size_t at, size_t key_at, size_t key_stride, int own_part, size_t T,
+                                               int tile, int sub, int o, const TwPair* tw) {
+    using R = RowsMac<LOGN>;
+    const size_t N = R::P::N;
+    const int eb = R::Begin::element(sub, o), ee = R::End::element(sub, o), parts = j->parts;
+    WideSum sa[8], sb[8];
+    uint64_t w[8], k8[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        sa[k].clear();
+        sb[k].clear();
+    }
+    for (int p = 0; p < parts; ++p) {
+        if (p == own_part) {
+            load_words<typename R::End>(j->key_term[c] + at + ee, w);
+        } else {
+            load_words<typename R::Begin>(j->digits[c] + p * j->part_stride + at + eb, w);
+            ntt_rounds<LOGN, true, false, 3, false, kMaxTile>(R::rounds(), sm, w, sub, o, tile, WordArith<LAZY>{m.q}, tw);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = word_store(true, true, w[k], m);
+        }
+        const uint64_t* key = j->key + p * 2 * key_stride + key_at + ee;
+        load_words<typename R::End>(key, k8);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sa[k].add(w[k], k8[k], m);
+        load_words<typename R::End>(key + key_stride, k8);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sb[k].add(w[k], k8[k], m);
+    }
+#pragma unroll
+    for (int poly = 0; poly < 2; ++poly) {
+        uint64_t* out = j->acc[c] + poly * T * N + at;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w[k] = (poly ? sb[k] : sa[k]).mont_value(m);
+        if (rows) {
+            ntt_rounds<LOGN, false, false, 3, false, kMaxTile>(R::rounds(), sm, w, sub, o, tile, WordArith<false>{m.q},
+                                                              tw + N);
+            store_words<typename R::InvEnd>(out + R::InvEnd::element(sub, o), w);
+        } else {
+            store_words<typename R::End>(out + ee, w);
+        }
+    }
+}
+
+template <int LOGN, bool WORDS>
+__global__ void __launch_bounds__(RowsMac<LOGN>::P::THREADS, 2)
+    k_rows_mac(const MacGroupJob* __restrict__ jobs, int njobs, const Modulus* __restrict__ mods, int nq,
+               const TwPair* __restrict__ tw_base) {
+    using P = typename RowsMac<LOGN>::P;
+    const int jn = blockIdx.y + 65535 * blockIdx.z;
+    if (jn >= njobs) return;
+    extern __shared__ __align__(16) uint64_t smem[];
+    const MacGroupJob* j = jobs + jn;
+    const int i = j->i, L = j->L, K = j->K, tile = blockIdx.x, t = threadIdx.x;
+    const bool is_p = i >= L;
+    const int mi = is_p ? nq + (i - L) : i;
+    const Modulus m = mods[mi];
+    const TwPair* tw = tw_base + (size_t)mi * 2 * P::N;
+    const size_t key_limbs = (size_t)j->key_level + 1 + K, key_stride = key_limbs * P::N;
+    const size_t klimb = is_p ? (size_t)j->key_level + 1 + (i - L) : (size_t)i;
+    const size_t at = (size_t)i * P::N + (size_t)tile * P::TILE, key_at = klimb * P::N + (size_t)tile * P::TILE;
+    const int own_part = is_p ? -1 : i / j->alpha, sub = P::sub_of(t), o = P::o_of(t);
+    const size_t T = L + K;
+    for (int c = 0; c < j->n; ++c) {
+        if (!WORDS || m.q < fp::kLimit)
+            rows_mac_fp<LOGN>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw);
+        else if (m.q < kLazyForwardLimit)
+            rows_mac_words<LOGN, true>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw);
+        else
+            rows_mac_words<LOGN, false>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw);
+    }
+}
+
+template <int LOGN>
+void launch_rows_mac(const Context& c, const MacGroupJob* jobs, int njobs, bool words, cudaStream_t s) {
+    using P = typename RowsMac<LOGN>::P;
+    const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
+    if (words)
+        k_rows_mac<LOGN, true><<<grid, P::THREADS, RowsMac<LOGN>::smem(), s>>>(jobs, njobs, c.d_mod, (int)c.nq,
+                                                                               c.twiddles(3));
+    else
+        k_rows_mac<LOGN, false><<<grid, P::THREADS, RowsMac<LOGN>::smem(), s>>>(jobs, njobs, c.d_mod, (int)c.nq,
+                                                                                c.twiddles(3));
+}
+
 template <int LOGN, int EB, bool STAGED>
 void launch_rows_epi(const Context& c, const NttEpiJob* jobs, int njobs, cudaStream_t s) {
     using P = Phase<LOGN, true, false, EB, STAGED>;
@@ -600,6 +777,61 @@ void ntt_jobs_phase(const Context& c, const NttJob* d_jobs, int njobs, bool forw
     phase_dispatch(c, forward, cols, c.ntt_variant[forward ? 0 : 1][cols ? 1 : 0], nullptr, 0, 0, 0, LimbMap{0, 0, 0},
                    d_jobs, njobs, s);
     check_cuda(cudaGetLastError(), "ntt launch");
+}
+
+// Word moduli take k_rows_mac only in small steps, where its two launches less count (one bootstrap
+// 7.58 ms, 7.81 with the word limbs apart): their rounds keep its
+// registers, and so its two blocks an SM, busy for longer than the separate launches take (the Walsh
+// AES's transforms and key products 333 ms apart, 340 ms together).  Four waves is the line.
+// Two switches a job share the key words in L1 where that leaves as many waves; longer jobs lose in the
+// last wave what they read less (XBOOT S-box layer: 34.8, 33.5 and 32.9 ms at 1, 2 and 4 a job, a
+// bootstrap's 13.2, 13.2 and 13.4).
+MacLists::MacLists(const Context& c, size_t switches, size_t T) {
+    const size_t tiles = std::max<size_t>(1, c.N / kMaxTile), ctas = switches * tiles;
+    const size_t waves4 = 4 * 2 * (size_t)c.sm_count;
+    words = ctas * (c.np + 1) <= waves4;
+    group = ctas * T >= 2 * waves4 ? 2 : 1;
+}
+
+bool MacLists::in_rows(const Context& c, size_t mod) const {
+    return c.fuse() && (words || c.mods[mod].q < fp::kLimit);
+}
+
+void MacLists::add(const Context& c, const MacGroupJob& job, size_t mod) {
+    const double bytes = 8.0 * (double)c.N * (2.0 * job.parts + (double)job.n * (job.parts + 2.0));
+    if (!in_rows(c, mod)) {
+        sums.push_back(job);
+        sums_bytes += bytes;
+        return;
+    }
+    rows_bytes += bytes;
+    for (int k0 = 0; k0 < job.n; k0 += group) {
+        MacGroupJob j = job;
+        j.n = std::min(group, job.n - k0);
+        for (int k = 0; k < j.n; ++k) {
+            j.key_term[k] = job.key_term[k0 + k];
+            j.digits[k] = job.digits[k0 + k];
+            j.acc[k] = job.acc[k0 + k];
+        }
+        rows.push_back(j);
+    }
+}
+
+void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, bool words, double bytes,
+                   cudaStream_t s) {
+    if (njobs <= 0) return;
+    Probe probe(kClsKeyMac, bytes, s);
+    switch (c.logN) {
+        case 10: launch_rows_mac<10>(c, d_jobs, njobs, words, s); break;
+        case 11: launch_rows_mac<11>(c, d_jobs, njobs, words, s); break;
+        case 12: launch_rows_mac<12>(c, d_jobs, njobs, words, s); break;
+        case 13: launch_rows_mac<13>(c, d_jobs, njobs, words, s); break;
+        case 14: launch_rows_mac<14>(c, d_jobs, njobs, words, s); break;
+        case 15: launch_rows_mac<15>(c, d_jobs, njobs, words, s); break;
+        case 16: launch_rows_mac<16>(c, d_jobs, njobs, words, s); break;
+        default: fail(kInvalid, "ntt: ring degree must be 2^10 .. 2^16");
+    }
+    check_cuda(cudaGetLastError(), "key inner product launch");
 }
 
 void ntt_rows_epilogue_jobs(const Context& c, const NttEpiJob* d_jobs, int njobs, double bytes, cudaStream_t s) {

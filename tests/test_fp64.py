@@ -234,3 +234,32 @@ def test_mixed_key_switches(wg, oracle_mod, prm, fusion):
         (ref,) = o.rescale(level, [r0])
         torch.cuda.synchronize()
         assert (wg.to_host(e0)[: level * N] == ref).all(), level
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 7, 601])
+@pytest.mark.parametrize("prm", MIXED)
+def test_fused_key_products_of_many(wg, oracle_mod, prm, count):
+    """The fused steps against the separate launches: word limbs in the fused key product (small
+    counts) or apart (601 at 2^10 is past its line), one or two switches a job and an odd one left."""
+    import torch
+
+    O, N = oracle_mod, 1 << 10
+    p, q = O.find_primes(prm["p_bits"], prm["q_bits"], N)
+    ctx, o, L = wg.Context(N, q, p, prm["dnum"]), O.OracleCtx(N, q, p, prm["dnum"]), len(q)
+    s = o.ternary(64, 3)
+    ctx.set_key(wg.WG_KEY_RELIN, o.relin_key(s, 13))
+    ctx.set_key(wg.WG_KEY_ROTATION, o.rotation_key(s, 3, 11), rotation=3)
+    rng = np.random.default_rng(count)
+    host = (rng.integers(0, 1 << 63, (4, count, L, N), dtype=np.uint64) % np.asarray(q, np.uint64)[:, None]).reshape(-1)
+    levels = [1 + i % (L - 1) if i % 50 == 0 else L - 1 for i in range(count)]
+    got = []
+    for fusion in (0, 1):
+        ctx.set_ntt_fusion(fusion)
+        x = wg.to_device(host).reshape(4, count, L * N)
+        ctx.batch_mul_relin_rescale_rotate(levels, list(x[0]), list(x[1]), list(x[2]), list(x[3]), [3] * count)
+        torch.cuda.synchronize()
+        got.append(wg.to_host(x.reshape(-1)))
+    out = [g.reshape(4, count, L, N) for g in got]
+    for i, level in enumerate(levels):
+        assert (out[0][:2, i, :level] == out[1][:2, i, :level]).all(), i
