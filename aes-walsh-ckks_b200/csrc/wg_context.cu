@@ -284,6 +284,7 @@ Context* create_context(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
     c->alpha = (nq + dnum - 1) / dnum;
     c->q.assign(q, q + nq);
     c->p.assign(p, p + np);
+    for (size_t i = 0; i < nq + np; ++i) c->word_moduli |= (i < nq ? q[i] : p[i - nq]) >= fp::kLimit;
     check_cuda(cudaSetDevice(device), "cudaSetDevice");
     {
         // The batched operations draw their temporaries from this process's stream-ordered

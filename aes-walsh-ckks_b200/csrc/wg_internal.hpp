@@ -142,6 +142,7 @@ struct Context {
     int logN = 0;
     size_t nq = 0, np = 0, dnum = 0, alpha = 0;
     std::vector<uint64_t> q, p;
+    bool word_moduli = false;        // some modulus is fp::kLimit or more
     std::vector<Modulus> mods;       // nq + np entries (P after Q)
     Modulus* d_mod = nullptr;
     // twiddle pairs [mod][2][N] (forward, inverse; ntt::twiddle_pairs) for 8 and 16 residues per thread
@@ -347,8 +348,8 @@ struct MacGroupJob {
     int L, K, parts, alpha, key_level, i, n, pad;
 };
 // The digits' forward row phase and the key inner product in one launch (k_rows_mac, wg_ntt.cu):
-// digits as the fused ModUp leaves them, accumulators as kb_mac_group's; p_rows: the accumulators' P
-// limbs go on through the inverse row phase, as the fused ModDown takes them.
+// digits as the fused ModUp leaves them, accumulators as kb_mac_group's, with the P limbs gone on through
+// the inverse row phase, as the fused ModDown takes them.  words: some job is of a word modulus.
 void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, bool words, double bytes, cudaStream_t s);
 // The key products of one batched step: `rows` for rows_mac_jobs, `sums` for kb_mac_group.
 struct MacLists {

@@ -22,7 +22,7 @@
 // The butterflies, reductions and FP64 sums are those of the unfused kernels in the same
 // order, so the words written equal the ones the separate launches write.
 //
-// A thread owns the same 8 elements of the tile in the inverse phase's last round as in the forward
+// A thread owns the same elements of the tile in the inverse phase's last round as in the forward
 // phase's first (make_plan), so between the two transforms everything is its own: the finished
 // source limbs wait in shared memory slots that only their thread touches (slot k * THREADS + t: no
 // barrier, no bank conflict, no padding), and a base change's values go from registers straight
@@ -42,22 +42,34 @@
 namespace wg {
 namespace ksf {
 
-// Column tile of the fused kernels: 1024 elements (8 per thread, 128 threads), so the
-// source tiles of a digit or of the P limbs fit in shared memory several CTAs per SM.
+// Column tile of the fused kernels: 1024 elements, so the source tiles of a digit or of the P limbs fit
+// in shared memory several CTAs per SM.
 constexpr int kTile = 1024;
 
-template <int LOGN>
+// EB: a thread carries 2^EB residues, 8 or 4 (128 or 256 threads a tile).  Four hold 64 registers, so the
+// same tiles keep twice the warps on an SM, at one round's exchange more and half the sums per table
+// entry read: measured (us) against eight, the ModUp of a Walsh AES takes 97400 against 105000, its
+// ModDown 120500 against 122700, and in one bootstrap 1140 against 1273 and 1070 against 1171 (61-bit
+// words: long serial chains of integer products); on the all-FP64 XBOOT chain the ModUp of a bootstrap
+// takes 5510 against 4910 but the ModDown 3205 against 3434, and a rescale is 2 to 10 % slower.
+constexpr int kModUpBits = 2;    // chains with word moduli (from fp::kLimit up)
+constexpr int kModUpFpBits = 3;  // chains without
+constexpr int kModDownBits = 2;
+constexpr int kRescaleBits = 3;
+
+template <int LOGN, int EB>
 struct Geom {
-    using Fwd = ntt::Phase<LOGN, true, true, 3, false, kTile>;
-    using Inv = ntt::Phase<LOGN, false, true, 3, false, kTile>;
+    using Fwd = ntt::Phase<LOGN, true, true, EB, false, kTile>;
+    using Inv = ntt::Phase<LOGN, false, true, EB, false, kTile>;
     template <int RD>
-    using FwdRound = ntt::Round<LOGN, true, true, 3, false, RD, kTile>;
+    using FwdRound = ntt::Round<LOGN, true, true, EB, false, RD, kTile>;
     template <int RD>
-    using InvRound = ntt::Round<LOGN, false, true, 3, false, RD, kTile>;
+    using InvRound = ntt::Round<LOGN, false, true, EB, false, RD, kTile>;
+    static constexpr int LOG = LOGN, BITS = EB;
     static constexpr int N = 1 << LOGN;
     static constexpr int TILE = Fwd::TILE;
     static constexpr int THREADS = Fwd::THREADS;
-    static constexpr int E = 8;
+    static constexpr int E = 1 << EB;
     static constexpr int PAD = TILE + TILE / 16;  // words of the padded exchange tile
     static constexpr int TILES = N / TILE;
     static constexpr int ROUNDS = Fwd::ROUNDS;
@@ -76,9 +88,8 @@ WG_HD size_t limb_offset(int tile, int t) {
 // Thread t's elements (first inverse round) of one limb into its slots, as asynchronous copies
 // (cp.async, 8 bytes each) that pass no register, so a CTA can have all its source limbs in flight at
 // once; completion is awaited per commit group (cp_async_wait_upto), by the thread alone.
-template <int LOGN>
+template <class G>
 __device__ __forceinline__ void load_slots_async(uint64_t* slots, const uint64_t* __restrict__ limb, int tile, int t) {
-    using G = Geom<LOGN>;
     using R = typename G::template InvRound<0>;
     const uint64_t* p = limb + limb_offset<R>(tile, t);
 #pragma unroll
@@ -137,40 +148,42 @@ WG_HD uint64_t slot_word(uint64_t x, bool fp64) { return fp64 ? fp::to_word(fp::
 
 // Last step of an FP64 inverse transform: multiply by the factor pair (N^-1, or N^-1 with a base
 // change's constant) to the canonical residue.
+template <int E>
 WG_HD void scale_fp(double* v, double w, double wq, double q) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = fp::lift(fp::mulmod(v[k], w, wq, q), q);
+    for (int k = 0; k < E; ++k) v[k] = fp::lift(fp::mulmod(v[k], w, wq, q), q);
 }
 
 // Last step of the inverse transform: multiply by N^-1 (canonical).
+template <int E>
 WG_HD void scale_n_inv(uint64_t* v, const Modulus& m) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = mul_shoup(v[k], m.n_inv, m.n_inv_shoup, m.q);
+    for (int k = 0; k < E; ++k) v[k] = mul_shoup(v[k], m.n_inv, m.n_inv_shoup, m.q);
 }
 
 // ModUp, source limb i of the digit (canonical coefficients): scale by qhat_inv_i in place and add
 // the FP64 estimate term to the alpha sums, in the order of modup_coeff_w.  (modup_coeff_w first
 // reduces its input below q; the inverse transform's N^-1 step already leaves it canonical, so that
 // reduction is the identity here.)
-template <class Desc>
+template <class G, class Desc>
 WG_HD void modup_scale(uint64_t* v, const Desc& d, int i, uint64_t qi, double* alpha) {
     const uint64_t w = WG_LDG(d.qhat_inv + i), ws = WG_LDG(d.qhat_inv_s + i);
     const double inv = WG_LDG(d.src_inv + i);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < G::E; ++k) {
         v[k] = mul_shoup(v[k], w, ws, qi);
         alpha[k] = dadd(alpha[k], dmul(u2d(v[k]), inv));
     }
 }
 
 // The same for an FP64 source, from the inverse rounds' values: N^-1 and qhat_inv_i in one factor.
-template <class Desc>
+template <class G, class Desc>
 WG_HD void modup_scale_fp(double* v, const Desc& d, int i, double qi, double* alpha) {
     const ntt::TwPair f = d.scale_fp[i];
-    scale_fp(v, fp::bits_double(f.w), fp::bits_double(f.ws), qi);
+    scale_fp<G::E>(v, fp::bits_double(f.w), fp::bits_double(f.ws), qi);
     const double inv = WG_LDG(d.src_inv + i);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) alpha[k] = dadd(alpha[k], dmul(v[k], inv));
+    for (int k = 0; k < G::E; ++k) alpha[k] = dadd(alpha[k], dmul(v[k], inv));
 }
 
 WG_HD uint32_t hps_count(double alpha, int n) {
@@ -179,32 +192,24 @@ WG_HD uint32_t hps_count(double alpha, int n) {
 }
 
 // ModUp destination dst of the digit: thread t's coefficients.
-// src holds the n scaled sources' slots (TILE words each); W >= n bounds the digit width so the
-// dst row of constants stays in registers.
-template <int LOGN, int W, class Desc>
+// src holds the n scaled sources' slots (TILE words each).
+template <class G, class Desc>
 WG_HD void modup_value(uint64_t* v, const uint64_t* src, int t, const Desc& d, int dst, uint64_t m, const uint32_t* hps,
                        unsigned fp_src) {
-    using G = Geom<LOGN>;
     const int n = d.src_count;
     const uint64_t* row = d.qhat + (size_t)dst * n;
     const uint64_t* row_s = d.qhat_s + (size_t)dst * n;
     const uint64_t* corr = d.corr + (size_t)dst * (n + 1);
-    uint64_t w[W], ws[W];
 #pragma unroll
-    for (int i = 0; i < W; ++i) {
-        w[i] = i < n ? WG_LDG(row + i) : 0;
-        ws[i] = i < n ? WG_LDG(row_s + i) : 0;
+    for (int k = 0; k < G::E; ++k) v[k] = 0;
+    for (int i = 0; i < n; ++i) {
+        const uint64_t w = WG_LDG(row + i), ws = WG_LDG(row_s + i);
+#pragma unroll
+        for (int k = 0; k < G::E; ++k)
+            v[k] = add_mod(v[k], mul_shoup(slot_word(src[i * G::TILE + k * G::THREADS + t], fp_src >> i & 1), w, ws, m), m);
     }
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        uint64_t acc = 0;
-#pragma unroll
-        for (int i = 0; i < W; ++i)
-            if (i < n)
-                acc = add_mod(acc, mul_shoup(slot_word(src[i * G::TILE + k * G::THREADS + t], fp_src >> i & 1), w[i], ws[i], m),
-                              m);
-        v[k] = sub_mod(acc, WG_LDG(corr + hps[k]), m);
-    }
+    for (int k = 0; k < G::E; ++k) v[k] = sub_mod(v[k], WG_LDG(corr + hps[k]), m);
 }
 
 // Sums of products s w of thread t's source elements s, modulo a destination q of the FP64 path.
@@ -215,17 +220,16 @@ WG_HD void modup_value(uint64_t* v, const uint64_t* src, int t, const Desc& d, i
 //     source a lazy Shoup product in [0, 2q), centred; each term adds at most q in magnitude, and the
 //     sum is brought back to q / 2 after every fourth, so it stays below 5.5 q < 2^53.
 // `f` is the term's table entry: (w, w / q), or (w, 2^31 w) for a word source (fp::kWordSplit).
+template <class G>
 struct SumFp {
-    fp::Dot d[8];
+    fp::Dot d[G::E];
     WG_HD void start(int k, double v) {
         d[k].clear();
         d[k].l = v;
     }
-    template <int LOGN>
     WG_HD void add(const uint64_t* slots, int t, bool fp64, bool wide, ntt::TwPair f, uint64_t w, uint64_t ws, int term,
                    const Modulus& m) {
-        using G = Geom<LOGN>;
-        const double f0 = fp::bits_double(f.w), f1 = fp::bits_double(f.ws);
+            const double f0 = fp::bits_double(f.w), f1 = fp::bits_double(f.ws);
         const bool dot = m.q < fp::kNoReduce;
         slots += t;
         if (fp64 && dot && !wide) {
@@ -257,24 +261,23 @@ struct SumFp {
     WG_HD void finish(double* v, const Modulus& m) const {
         const bool dot = m.q < fp::kNoReduce;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = dot ? d[k].value(m.qd, m.inv_q) : d[k].l;
+        for (int k = 0; k < G::E; ++k) v[k] = dot ? d[k].value(m.qd, m.inv_q) : d[k].l;
     }
 };
 static_assert(2 * kMaxDigitWidth <= fp::kDotTerms && 2 * kMaxPLimbs <= fp::kDotTerms, "a base change is one exact sum");
 
 // ModUp destination dst of the FP64 path: thread t's coefficients, unreduced.
-template <int LOGN, class Desc>
+template <class G, class Desc>
 WG_HD void modup_value_fp(double* v, const uint64_t* src, int t, const Desc& d, int dst, const Modulus& m,
                           const uint32_t* hps, SourceKinds kinds) {
-    using G = Geom<LOGN>;
     const int n = d.src_count;
     const uint64_t* corr = d.corr + (size_t)dst * (n + 1);
-    SumFp sum;
+    SumFp<G> sum;
 #pragma unroll
     for (int k = 0; k < G::E; ++k) sum.start(k, -fp::from_word(WG_LDG(corr + hps[k])));
     for (int i = 0; i < n; ++i) {
         const size_t at = (size_t)dst * n + i;
-        sum.add<LOGN>(src + i * G::TILE, t, kinds.fp64 >> i & 1, kinds.wide >> i & 1, d.qhat_fp[at], d.qhat[at],
+        sum.add(src + i * G::TILE, t, kinds.fp64 >> i & 1, kinds.wide >> i & 1, d.qhat_fp[at], d.qhat[at],
                       d.qhat_s[at], i, m);
     }
     sum.finish(v, m);
@@ -284,73 +287,62 @@ WG_HD void modup_value_fp(double* v, const uint64_t* src, int t, const Desc& d, 
 // moddown_all_limbs_k; FMA: rounded as a fused multiply-add (the pair ModDown's compiled form)
 // or as a multiply then an add (the single-polynomial ModDown's).  The slots hold canonical
 // residues (the inverse transform's N^-1 step), so moddown_all_limbs_k's reduction of its input
-// below p is the identity here and is left out.  KW >= K keeps the constants in registers.
-template <int LOGN, int KW, bool FMA = true>
+// below p is the identity here and is left out.
+template <class G, bool FMA = true>
 WG_HD void moddown_hps(const uint64_t* src, int t, const Modulus* __restrict__ pmods, int K, uint32_t* hps,
                        unsigned fp_src) {
-    using G = Geom<LOGN>;
-    double inv[KW];
+    double alpha[G::E];
 #pragma unroll
-    for (int pi = 0; pi < KW; ++pi) inv[pi] = pi < K ? pmods[pi].inv_q : 0.0;
+    for (int k = 0; k < G::E; ++k) alpha[k] = 0.0;
+    for (int pi = 0; pi < K; ++pi) {
+        const double inv = pmods[pi].inv_q;
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        double alpha = 0.0;
-#pragma unroll
-        for (int pi = 0; pi < KW; ++pi)
-            if (pi < K) {
-                const uint64_t x = src[pi * G::TILE + k * G::THREADS + t];
-                const double s = fp_src >> pi & 1 ? fp::bits_double(x) : u2d(x);
-                alpha = FMA ? dfma(s, inv[pi], alpha) : dadd(alpha, dmul(s, inv[pi]));
-            }
-        hps[k] = hps_count(alpha, K);
+        for (int k = 0; k < G::E; ++k) {
+            const uint64_t x = src[pi * G::TILE + k * G::THREADS + t];
+            const double s = fp_src >> pi & 1 ? fp::bits_double(x) : u2d(x);
+            alpha[k] = FMA ? dfma(s, inv, alpha[k]) : dadd(alpha[k], dmul(s, inv));
+        }
     }
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) hps[k] = hps_count(alpha[k], K);
 }
 
 // ModDown contribution for Q limb qi: thread t's coefficients (canonical P residues as for
-// moddown_hps; KW >= K).
-template <int LOGN, int KW>
+// moddown_hps).
+template <class G>
 WG_HD void moddown_value(uint64_t* v, const uint64_t* src, int t, int K, uint64_t q, const uint64_t* __restrict__ iv,
                          const uint64_t* __restrict__ ivs, const uint32_t* hps, unsigned fp_src) {
-    using G = Geom<LOGN>;
-    uint64_t w[KW], ws[KW];
 #pragma unroll
-    for (int pi = 0; pi < KW; ++pi) {
-        w[pi] = pi < K ? WG_LDG(iv + pi) : 0;
-        ws[pi] = pi < K ? WG_LDG(ivs + pi) : 0;
+    for (int k = 0; k < G::E; ++k) v[k] = 0;
+    for (int pi = 0; pi < K; ++pi) {
+        const uint64_t w = WG_LDG(iv + pi), ws = WG_LDG(ivs + pi);
+#pragma unroll
+        for (int k = 0; k < G::E; ++k)
+            v[k] = add_mod(v[k], mul_shoup(slot_word(src[pi * G::TILE + k * G::THREADS + t], fp_src >> pi & 1), w, ws, q), q);
     }
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) {
-        uint64_t acc = 0;
-#pragma unroll
-        for (int pi = 0; pi < KW; ++pi)
-            if (pi < K)
-                acc = add_mod(acc, mul_shoup(slot_word(src[pi * G::TILE + k * G::THREADS + t], fp_src >> pi & 1), w[pi],
-                                             ws[pi], q), q);
-        v[k] = sub_mod(acc, (uint64_t)hps[k], q);
-    }
+    for (int k = 0; k < G::E; ++k) v[k] = sub_mod(v[k], (uint64_t)hps[k], q);
 }
 
 // The same for a Q limb of the FP64 path, unreduced.
-template <int LOGN>
+template <class G>
 WG_HD void moddown_value_fp(double* v, const uint64_t* src, int t, int K, const Modulus& m,
                             const uint64_t* __restrict__ iv, const uint64_t* __restrict__ ivs,
                             const ntt::TwPair* __restrict__ ivf, const uint32_t* hps, SourceKinds kinds) {
-    using G = Geom<LOGN>;
-    SumFp sum;
+    SumFp<G> sum;
 #pragma unroll
     for (int k = 0; k < G::E; ++k) sum.start(k, -fp::from_word(hps[k]));
     for (int pi = 0; pi < K; ++pi)
-        sum.add<LOGN>(src + pi * G::TILE, t, kinds.fp64 >> pi & 1, kinds.wide >> pi & 1, ivf[pi], iv[pi], ivs[pi], pi, m);
+        sum.add(src + pi * G::TILE, t, kinds.fp64 >> pi & 1, kinds.wide >> pi & 1, ivf[pi], iv[pi], ivs[pi], pi, m);
     sum.finish(v, m);
 }
 
 // Rescale: thread t's rounded remainders of the dropped limb (slots, canonical, modulus p) for
 // target limb q, as kb_rescale_prep forms them
 // (ckks_rescale, src/ckks/operations/arith/ckks_rescale.cpp:68-148).
-template <int LOGN>
+template <class G>
 WG_HD void rescale_value(uint64_t* v, const uint64_t* drop, int t, uint64_t p, uint64_t q, uint64_t one_s, uint64_t half,
                          bool fp_drop) {
-    using G = Geom<LOGN>;
 #pragma unroll
     for (int k = 0; k < G::E; ++k) {
         uint64_t shift = slot_word(drop[k * G::THREADS + t], fp_drop) + (p >> 1);
@@ -360,10 +352,9 @@ WG_HD void rescale_value(uint64_t* v, const uint64_t* drop, int t, uint64_t p, u
 }
 
 // The same for a target limb of the FP64 path: unreduced, at most 2 q in magnitude.
-template <int LOGN>
+template <class G>
 WG_HD void rescale_value_fp(double* v, const uint64_t* drop, int t, uint64_t p, const Modulus& m, uint64_t one_s,
                             uint64_t half, bool fp_drop) {
-    using G = Geom<LOGN>;
     const double h = fp::from_word(half);
     const double pd = u2d(p), hp = u2d(p >> 1);
 #pragma unroll

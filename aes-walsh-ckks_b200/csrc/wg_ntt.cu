@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(Phase<LOGN, true, false, EB, STAGED>::THREADS,
 
 // The forward row phase of a switch's digits with the key inner product on it, for one QP limb's
 // row tile: a digit's transformed words meet the key words in the registers of the last round, where a
-// thread has 8 consecutive coefficients, and only the two accumulators are stored; with p_rows an
+// thread has 8 consecutive coefficients, and only the two accumulators are stored; an
 // accumulator's P limb goes straight on through its inverse row phase, whose first round has the
 // thread's same 8 coefficients.  Against the separate launches a digit limb is read once instead of
 // written and read again twice over, and a switch takes two launches less.  The switches of a job

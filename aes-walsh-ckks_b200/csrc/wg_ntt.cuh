@@ -99,7 +99,7 @@ struct Phase {
     // entries.
     static constexpr int TW = COLS ? (1 << NB1) : (TILE - SUBS);
     static_assert(MB >= EB, "transform too small for this round radix");
-    static_assert(EB == 3 || EB == 4, "rounds of 8 or 16 residues per thread");
+    static_assert(EB >= 2 && EB <= 4, "rounds of 4, 8 or 16 residues per thread");
 };
 
 // Table index of staged twiddle t (see Phase::TW).  Row-stage k occupies staged entries

@@ -164,25 +164,23 @@ int g_fused = 0;
 
 bool is_fp(const Emu& E, int mi) { return E.H.mods[mi].q < fp::kLimit; }
 
-template <int LOGN, bool FWD, class Arith>
-void columns(Lanes<Arith, 8>& v, int tile, const Arith& ar, const ntt::TwPair* tw) {
-    using G = ksf::Geom<LOGN>;
+template <class G, bool FWD, class Arith>
+void columns(Lanes<Arith, G::E>& v, int tile, const Arith& ar, const ntt::TwPair* tw) {
     std::vector<uint64_t> sm(G::PAD);
-    rounds<LOGN, FWD, true, 3, false, ksf::kTile>(std::make_integer_sequence<int, G::ROUNDS>{}, sm.data(), v, tile, ar, tw);
+    rounds<G::LOG, FWD, true, G::BITS, false, ksf::kTile>(std::make_integer_sequence<int, G::ROUNDS>{}, sm.data(), v, tile, ar, tw);
 }
 
 // inverse_slots (wg_ksfuse.cu) of one source limb whose words thread t has at slots[k * THREADS + t].
-template <int LOGN, class ScaleFp, class ScaleWords>
+template <class G, class ScaleFp, class ScaleWords>
 void inverse_slots(const Emu& E, uint64_t* slots, int tile, int mi, ScaleFp scale_f, ScaleWords scale_w) {
-    using G = ksf::Geom<LOGN>;
     const Modulus& m = E.H.mods[mi];
     const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * G::N + G::N;
     auto run = [&](const auto& ar, auto scale) {
         using A = std::decay_t<decltype(ar)>;
-        Lanes<A, 8> v(G::THREADS);
+        Lanes<A, G::E> v(G::THREADS);
         for (int t = 0; t < G::THREADS; ++t)
             for (int k = 0; k < G::E; ++k) v[t][k] = A::of_bits(slots[k * G::THREADS + t]);
-        columns<LOGN, false>(v, tile, ar, tw);
+        columns<G, false>(v, tile, ar, tw);
         for (int t = 0; t < G::THREADS; ++t) {
             scale(v[t].data(), t);
             for (int k = 0; k < G::E; ++k) slots[k * G::THREADS + t] = A::bits(v[t][k]);
@@ -193,29 +191,27 @@ void inverse_slots(const Emu& E, uint64_t* slots, int tile, int mi, ScaleFp scal
     else
         run(ntt::WordArith<false>{m.q}, scale_w);
 }
-template <int LOGN>
+template <class G>
 void load_slots(uint64_t* slots, const uint64_t* limb, int tile) {
-    using G = ksf::Geom<LOGN>;
     for (int t = 0; t < G::THREADS; ++t) {
-        uint64_t w[8];
+        uint64_t w[G::E];
         ksf::load_limb<typename G::template InvRound<0>>(w, limb, tile, t);
         for (int k = 0; k < G::E; ++k) slots[k * G::THREADS + t] = w[k];
     }
 }
 // forward_limb (wg_ksfuse.cu).
-template <int LOGN, class ValueFp, class ValueWords>
+template <class G, class ValueFp, class ValueWords>
 void forward_limb(const Emu& E, uint64_t* limb, int tile, int mi, ValueFp value_f, ValueWords value_w) {
-    using G = ksf::Geom<LOGN>;
     using End = typename G::template FwdRound<G::ROUNDS - 1>;
     const Modulus& m = E.H.mods[mi];
     const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * G::N;
     auto run = [&](const auto& ar, auto value) {
         using A = std::decay_t<decltype(ar)>;
-        Lanes<A, 8> v(G::THREADS);
+        Lanes<A, G::E> v(G::THREADS);
         for (int t = 0; t < G::THREADS; ++t) value(v[t].data(), t);
-        columns<LOGN, true>(v, tile, ar, tw);
+        columns<G, true>(v, tile, ar, tw);
         for (int t = 0; t < G::THREADS; ++t) {
-            uint64_t w[8];
+            uint64_t w[G::E];
             for (int k = 0; k < G::E; ++k) w[k] = A::bits(v[t][k]);
             ksf::store_limb<End>(w, limb, tile, t);
         }
@@ -229,9 +225,8 @@ void forward_limb(const Emu& E, uint64_t* limb, int tile, int mi, ValueFp value_
 }
 
 // k_modup_ntt over every column tile of one digit.
-template <int LOGN>
-void modup_fused(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t* digit) {
-    using G = ksf::Geom<LOGN>;
+template <class G>
+void modup_fused_g(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t* digit) {
     const int n = d.src_count;
     std::vector<uint64_t> slots((size_t)n * G::TILE);
     for (int tile = 0; tile < G::TILES; ++tile) {
@@ -242,13 +237,13 @@ void modup_fused(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t
             const Modulus& m = E.H.mods[mi];
             uint64_t* sl = slots.data() + (size_t)i * G::TILE;
             kinds.set(i, m.q);
-            load_slots<LOGN>(sl, src + (size_t)mi * G::N, tile);
-            inverse_slots<LOGN>(
+            load_slots<G>(sl, src + (size_t)mi * G::N, tile);
+            inverse_slots<G>(
                 E, sl, tile, mi,
-                [&](double* v, int t) { ksf::modup_scale_fp(v, d, i, m.qd, alpha.data() + (size_t)t * G::E); },
+                [&](double* v, int t) { ksf::modup_scale_fp<G>(v, d, i, m.qd, alpha.data() + (size_t)t * G::E); },
                 [&](uint64_t* v, int t) {
-                    ksf::scale_n_inv(v, m);
-                    ksf::modup_scale(v, d, i, m.q, alpha.data() + (size_t)t * G::E);
+                    ksf::scale_n_inv<G::E>(v, m);
+                    ksf::modup_scale<G>(v, d, i, m.q, alpha.data() + (size_t)t * G::E);
                 });
         }
         std::vector<uint32_t> hps((size_t)G::THREADS * G::E);
@@ -256,23 +251,32 @@ void modup_fused(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t
         for (int dst = 0; dst < d.dst_count; ++dst) {
             const int mi = d.dst_mod[dst];
             const Modulus& m = E.H.mods[mi];
-            forward_limb<LOGN>(
+            forward_limb<G>(
                 E, digit + (size_t)d.dst_limb[dst] * G::N, tile, mi,
                 [&](double* v, int t) {
-                    ksf::modup_value_fp<LOGN>(v, slots.data(), t, d, dst, m, hps.data() + (size_t)t * G::E, kinds);
+                    ksf::modup_value_fp<G>(v, slots.data(), t, d, dst, m, hps.data() + (size_t)t * G::E, kinds);
                 },
                 [&](uint64_t* v, int t) {
-                    ksf::modup_value<LOGN, 16>(v, slots.data(), t, d, dst, m.q, hps.data() + (size_t)t * G::E, kinds.fp64);
+                    ksf::modup_value<G>(v, slots.data(), t, d, dst, m.q, hps.data() + (size_t)t * G::E, kinds.fp64);
                 });
         }
     }
+}
+template <int LOGN>
+void modup_fused(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t* digit) {
+    bool words = false;  // Context::word_moduli
+    for (const Modulus& m : E.H.mods) words |= m.q >= fp::kLimit;
+    if (words)
+        modup_fused_g<ksf::Geom<LOGN, ksf::kModUpBits>>(E, d, src, digit);
+    else
+        modup_fused_g<ksf::Geom<LOGN, ksf::kModUpFpBits>>(E, d, src, digit);
 }
 
 // k_moddown_ntt over every column tile of one accumulator polynomial.
 template <int LOGN>
 void moddown_fused(const Emu& E, const uint64_t* src_p, uint64_t* out, int L, const uint64_t* inv,
                    const uint64_t* inv_s, const ntt::TwPair* inv_fp) {
-    using G = ksf::Geom<LOGN>;
+    using G = ksf::Geom<LOGN, ksf::kModDownBits>;
     const int K = (int)E.H.np, nq = (int)E.H.nq;
     const Modulus* pmods = E.H.mods.data() + nq;
     std::vector<uint64_t> slots((size_t)K * G::TILE);
@@ -282,25 +286,25 @@ void moddown_fused(const Emu& E, const uint64_t* src_p, uint64_t* out, int L, co
         for (int pi = 0; pi < K; ++pi) {
             const Modulus& m = pmods[pi];
             uint64_t* sl = slots.data() + (size_t)pi * G::TILE;
-            load_slots<LOGN>(sl, src_p + (size_t)pi * G::N, tile);
-            inverse_slots<LOGN>(
-                E, sl, tile, nq + pi, [&](double* v, int) { ksf::scale_fp(v, m.n_inv_w, m.n_inv_wq, m.qd); },
-                [&](uint64_t* v, int) { ksf::scale_n_inv(v, m); });
+            load_slots<G>(sl, src_p + (size_t)pi * G::N, tile);
+            inverse_slots<G>(
+                E, sl, tile, nq + pi, [&](double* v, int) { ksf::scale_fp<G::E>(v, m.n_inv_w, m.n_inv_wq, m.qd); },
+                [&](uint64_t* v, int) { ksf::scale_n_inv<G::E>(v, m); });
         }
         std::vector<uint32_t> hps((size_t)G::THREADS * G::E);
         for (int t = 0; t < G::THREADS; ++t)
-            ksf::moddown_hps<LOGN, 16>(slots.data(), t, pmods, K, hps.data() + (size_t)t * G::E, kinds.fp64);
+            ksf::moddown_hps<G>(slots.data(), t, pmods, K, hps.data() + (size_t)t * G::E, kinds.fp64);
         for (int qi = 0; qi < L; ++qi) {
             const Modulus& m = E.H.mods[qi];
             const uint64_t *iv = inv + (size_t)qi * K, *ivs = inv_s + (size_t)qi * K;
-            forward_limb<LOGN>(
+            forward_limb<G>(
                 E, out + (size_t)qi * G::N, tile, qi,
                 [&](double* v, int t) {
-                    ksf::moddown_value_fp<LOGN>(v, slots.data(), t, K, m, iv, ivs, inv_fp + (size_t)qi * K,
+                    ksf::moddown_value_fp<G>(v, slots.data(), t, K, m, iv, ivs, inv_fp + (size_t)qi * K,
                                                 hps.data() + (size_t)t * G::E, kinds);
                 },
                 [&](uint64_t* v, int t) {
-                    ksf::moddown_value<LOGN, 16>(v, slots.data(), t, K, m.q, iv, ivs, hps.data() + (size_t)t * G::E, kinds.fp64);
+                    ksf::moddown_value<G>(v, slots.data(), t, K, m.q, iv, ivs, hps.data() + (size_t)t * G::E, kinds.fp64);
                 });
         }
     }
@@ -328,23 +332,23 @@ void rows_epi(const Emu& E, const ntt::NttEpiJob& j) {
 // phase); rc: the rescale constants of level lv (one_s, inv_p, inv_p_s, half).
 template <int LOGN>
 void rescale_fused(const Emu& E, const uint64_t* drop, uint64_t* rem, int lv, const uint64_t* rc) {
-    using G = ksf::Geom<LOGN>;
+    using G = ksf::Geom<LOGN, ksf::kRescaleBits>;
     std::vector<uint64_t> slots(G::TILE);
     const Modulus& mp = E.H.mods[lv];
     for (int tile = 0; tile < G::TILES; ++tile) {
-        load_slots<LOGN>(slots.data(), drop, tile);
-        inverse_slots<LOGN>(
-            E, slots.data(), tile, lv, [&](double* v, int) { ksf::scale_fp(v, mp.n_inv_w, mp.n_inv_wq, mp.qd); },
-            [&](uint64_t* v, int) { ksf::scale_n_inv(v, mp); });
+        load_slots<G>(slots.data(), drop, tile);
+        inverse_slots<G>(
+            E, slots.data(), tile, lv, [&](double* v, int) { ksf::scale_fp<G::E>(v, mp.n_inv_w, mp.n_inv_wq, mp.qd); },
+            [&](uint64_t* v, int) { ksf::scale_n_inv<G::E>(v, mp); });
         for (int qi = 0; qi < lv; ++qi) {
             const Modulus& m = E.H.mods[qi];
-            forward_limb<LOGN>(
+            forward_limb<G>(
                 E, rem + (size_t)qi * G::N, tile, qi,
                 [&](double* v, int t) {
-                    ksf::rescale_value_fp<LOGN>(v, slots.data(), t, mp.q, m, rc[qi], rc[3 * lv + qi], is_fp(E, lv));
+                    ksf::rescale_value_fp<G>(v, slots.data(), t, mp.q, m, rc[qi], rc[3 * lv + qi], is_fp(E, lv));
                 },
                 [&](uint64_t* v, int t) {
-                    ksf::rescale_value<LOGN>(v, slots.data(), t, mp.q, m.q, rc[qi], rc[3 * lv + qi], is_fp(E, lv));
+                    ksf::rescale_value<G>(v, slots.data(), t, mp.q, m.q, rc[qi], rc[3 * lv + qi], is_fp(E, lv));
                 });
         }
     }
