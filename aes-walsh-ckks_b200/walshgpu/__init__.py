@@ -728,11 +728,13 @@ class Context:
         pb, pa = arr([x[0] for x in cts]), arr([x[1] for x in cts])
         sc = np.ascontiguousarray(scales, dtype=np.float64)
         sec = np.ascontiguousarray(secret, dtype=np.int8)
-        re = np.zeros((len(cts), self.N // 2))
-        im = np.zeros((len(cts), self.N // 2))
+        re = np.empty((len(cts), self.N // 2))
+        im = np.empty((len(cts), self.N // 2))
         _check(lib().wg_decrypt_decode(self.h, len(cts), int(level), sc.ctypes.data, pb.ctypes.data, pa.ctypes.data,
                                        None, sec.ctypes.data, re.ctypes.data, im.ctypes.data, _stream(stream)))
-        return re + 1j * im
+        out = np.empty(re.shape, np.complex128)  # two strided copies, not a complex product and a sum
+        out.real, out.imag = re, im
+        return out
 
     def encode_slots_device(self, limbs, scale, re, im, outs, eval_form=False, stream=None):
         """CKKS encoding on the device (wg_encode_slots_device) of slot vectors re / im ([count][N/2]
