@@ -38,9 +38,8 @@ struct KsPlan {
     int n_modup;
     const NttJob* ntt_digits;
     int n_ntt_digits;
-    const MacGroupJob *mac, *rows_mac;
-    bool rows_words;  // MacLists::words
-    int n_mac, n_rows_mac;
+    const MacGroupJob* mac;
+    int n_mac;
     const NttJob* intt_p;
     int n_intt_p;
     const ModDownJob* moddown;
@@ -54,7 +53,7 @@ struct KsPlan {
     const NttEpiJob* contrib_epi;  // fused: forward row phase of the contributions + combine
     int n_contrib_epi;
     double contrib_epi_bytes;
-    double mac_bytes, rows_mac_bytes, modup_bytes, moddown_bytes, combine_bytes;
+    double mac_bytes, modup_bytes, moddown_bytes, combine_bytes;
     bool fused;   // ModUp / ModDown fused with the NTT column phases (Context::ntt_fusion)
     int max_src;  // widest digit (fused ModUp shared memory)
     int max_dst;  // most destination limbs of a digit
@@ -78,8 +77,9 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     KsPlan p{};
     p.fused = c.fuse();
     // MAC groups: consecutive switches with the same key, level and digit layout (up to
-    // kMacGroup), one job per QP limb; [group_begin, it) is the open group
-    MacLists mac(c, n, n ? items[0].level + 1 + K : 0);
+    // mac_group), one job per QP limb; [group_begin, it) is the open group
+    std::vector<MacGroupJob> mac;
+    const size_t mac_group = p.fused && n ? rows_mac_group(c, n, items[0].level + 1 + K) : kMacGroup;
     size_t group_begin = 0;
     std::vector<uint64_t*> group_digits, group_acc;
     auto close_group = [&](size_t end) {
@@ -102,8 +102,9 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
                 jb.digits[k - group_begin] = group_digits[k - group_begin];
                 jb.acc[k - group_begin] = group_acc[k - group_begin];
             }
-            mac.add(c, jb, i < L ? i : nq + (i - L));
+            mac.push_back(jb);
         }
+        p.mac_bytes += 8.0 * N * T * (2.0 * B + (double)(end - group_begin) * (B + 2.0));
         group_begin = end;
         group_digits.clear();
         group_acc.clear();
@@ -128,22 +129,20 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
             p.max_dst = std::max(p.max_dst, d.dst_count);
             p.modup_bytes += 8.0 * N * (d.src_count + d.dst_count);
             const size_t s0 = j * c.alpha, s1 = std::min(s0 + c.alpha, L);
-            for (size_t l = 0; l < T; ++l) {
-                const size_t mod = l < L ? l : nq + (l - L);
-                if ((l >= s0 && l < s1) || mac.in_rows(c, mod)) continue;  // k_rows_mac transforms the latter
+            for (size_t l = 0; l < T && !p.fused; ++l) {  // fused: k_rows_mac transforms them
+                if (l >= s0 && l < s1) continue;
                 uint64_t* ptr = digits + j * T * N + l * N;
-                ntt_digits.push_back({ptr, ptr, (int)mod, 0});
+                ntt_digits.push_back({ptr, ptr, (int)(l < L ? l : nq + (l - L)), 0});
             }
         }
         if (it > group_begin) {
             const KsItem& g = items[group_begin];
-            if (it - group_begin == (size_t)kMacGroup || g.key != x.key || g.level != x.level) close_group(it);
+            if (it - group_begin == mac_group || g.key != x.key || g.level != x.level) close_group(it);
         }
         group_digits.push_back(digits);
         group_acc.push_back(acc);
-        for (int poly = 0; poly < 2; ++poly)
+        for (int poly = 0; poly < 2 && !p.fused; ++poly)
             for (size_t pi = 0; pi < K; ++pi) {
-                if (mac.in_rows(c, nq + pi)) continue;
                 uint64_t* ptr = acc + (poly * T + L + pi) * N;
                 intt_p.push_back({ptr, ptr, (int)(nq + pi), 0});
             }
@@ -184,13 +183,8 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     p.n_modup = (int)modup.size();
     p.ntt_digits = t.add(ntt_digits);
     p.n_ntt_digits = (int)ntt_digits.size();
-    p.mac = t.add(mac.sums);
-    p.n_mac = (int)mac.sums.size();
-    p.mac_bytes = mac.sums_bytes;
-    p.rows_mac = t.add(mac.rows);
-    p.n_rows_mac = (int)mac.rows.size();
-    p.rows_mac_bytes = mac.rows_bytes;
-    p.rows_words = mac.words;
+    p.mac = t.add(mac);
+    p.n_mac = (int)mac.size();
     p.intt_p = t.add(intt_p);
     p.n_intt_p = (int)intt_p.size();
     p.moddown = t.add(moddown);
@@ -215,13 +209,7 @@ static void run_keyswitch(const Context& c, const KsPlan& p, const JobTable& t, 
         // -> forward row phase and combine (wg_ksfuse.cu, k_rows_mac, k_ntt_rows_epi)
         ntt_jobs_phase(c, t.at(p.intt_in), p.n_intt_in, false, false, s);
         modup_ntt_jobs(c, t.at(p.modup), p.n_modup, p.max_src, p.max_dst, p.modup_bytes, s);
-        rows_mac_jobs(c, t.at(p.rows_mac), p.n_rows_mac, p.rows_words, p.rows_mac_bytes, s);
-        ntt_jobs_phase(c, t.at(p.ntt_digits), p.n_ntt_digits, true, false, s);
-        if (p.n_mac) {
-            Probe probe(kClsKeyMac, p.mac_bytes, s);
-            kb_mac_group<<<grid_for(c, p.n_mac), kT, 0, s>>>(t.at(p.mac), p.n_mac, c.d_mod, (int)c.nq, N);
-        }
-        ntt_jobs_phase(c, t.at(p.intt_p), p.n_intt_p, false, false, s);
+        rows_mac_jobs(c, t.at(p.mac), p.n_mac, p.mac_bytes, s);
         moddown_ntt_jobs(c, t.at(p.moddown), p.n_moddown, p.max_limbs, p.moddown_bytes, s);
         ntt_rows_epilogue_jobs(c, t.at(p.contrib_epi), p.n_contrib_epi, p.contrib_epi_bytes, s);
         if (p.n_gather) {

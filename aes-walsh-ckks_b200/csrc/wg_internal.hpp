@@ -349,18 +349,10 @@ struct MacGroupJob {
 };
 // The digits' forward row phase and the key inner product in one launch (k_rows_mac, wg_ntt.cu):
 // digits as the fused ModUp leaves them, accumulators as kb_mac_group's, with the P limbs gone on through
-// the inverse row phase, as the fused ModDown takes them.  words: some job is of a word modulus.
-void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, bool words, double bytes, cudaStream_t s);
-// The key products of one batched step: `rows` for rows_mac_jobs, `sums` for kb_mac_group.
-struct MacLists {
-    std::vector<MacGroupJob> rows, sums;
-    double rows_bytes = 0.0, sums_bytes = 0.0;
-    bool words;  // whether limbs of word moduli (from fp::kLimit up) go to `rows` too
-    int group;   // switches a job of `rows` takes
-    MacLists(const Context& c, size_t switches, size_t T);
-    bool in_rows(const Context& c, size_t mod) const;
-    void add(const Context& c, const MacGroupJob& job, size_t mod);
-};
+// the inverse row phase, as the fused ModDown takes them.
+void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, double bytes, cudaStream_t s);
+// How many of `switches` equal switches of T limbs a job of rows_mac_jobs takes.
+int rows_mac_group(const Context& c, size_t switches, size_t T);
 
 // The forward row phase of job-table limbs with an element-wise epilogue (NttEpiJob, wg_ntt.cuh).
 using ntt::NttEpiJob;

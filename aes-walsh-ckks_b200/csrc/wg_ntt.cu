@@ -454,7 +454,10 @@ __global__ void __launch_bounds__(Phase<LOGN, true, false, EB, STAGED>::THREADS,
 // follow one another, so a tile's key words (parts x 32 KiB) come from L1 after the first.
 // One rotation takes 95 us, 104 with the separate launches; 64 mixed operations 4.23 ms against 4.49; the
 // 16 S-boxes of an XBOOT SubBytes layer 84.9 ms against 89.6.  Two blocks of 256 threads an SM (128
-// registers: the sums, the residues and the next digit's): latency, not the FP64 pipe, bounds it.
+// registers: the sums, the residues and the next digit's): latency, not the FP64 pipe, bounds it.  Limbs of
+// word moduli spill some of them here and still gain: with theirs in the separate launches the
+// transforms and key products of a Walsh AES take 334 ms, with them 325, of 64 mixed operations 2.08 and
+// 1.89.
 template <int LOGN>
 struct RowsMac {
     using P = Phase<LOGN, true, false, 3, false>;
@@ -611,10 +614,10 @@ __global__ void __launch_bounds__(RowsMac<LOGN>::P::THREADS, 2)
 }
 
 template <int LOGN>
-void launch_rows_mac(const Context& c, const MacGroupJob* jobs, int njobs, bool words, cudaStream_t s) {
+void launch_rows_mac(const Context& c, const MacGroupJob* jobs, int njobs, cudaStream_t s) {
     using P = typename RowsMac<LOGN>::P;
     const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
-    if (words)
+    if (c.word_moduli)
         k_rows_mac<LOGN, true><<<grid, P::THREADS, RowsMac<LOGN>::smem(), s>>>(jobs, njobs, c.d_mod, (int)c.nq,
                                                                                c.twiddles(3));
     else
@@ -779,56 +782,25 @@ void ntt_jobs_phase(const Context& c, const NttJob* d_jobs, int njobs, bool forw
     check_cuda(cudaGetLastError(), "ntt launch");
 }
 
-// Word moduli take k_rows_mac only in small steps, where its two launches less count (one bootstrap
-// 7.58 ms, 7.81 with the word limbs apart): their rounds keep its
-// registers, and so its two blocks an SM, busy for longer than the separate launches take (the Walsh
-// AES's transforms and key products 333 ms apart, 340 ms together).  Four waves is the line.
-// Two switches a job share the key words in L1 where that leaves as many waves; longer jobs lose in the
-// last wave what they read less (XBOOT S-box layer: 34.8, 33.5 and 32.9 ms at 1, 2 and 4 a job, a
-// bootstrap's 13.2, 13.2 and 13.4).
-MacLists::MacLists(const Context& c, size_t switches, size_t T) {
-    const size_t tiles = std::max<size_t>(1, c.N / kMaxTile), ctas = switches * tiles;
-    const size_t waves4 = 4 * 2 * (size_t)c.sm_count;
-    words = ctas * (c.np + 1) <= waves4;
-    group = ctas * T >= 2 * waves4 ? 2 : 1;
+// Two switches a job share the key words in L1 where that leaves eight waves of two blocks an SM; longer
+// jobs lose in the last wave what they read less (XBOOT S-box layer: 34.8, 33.5 and 32.9 ms at 1, 2 and
+// 4 a job, a bootstrap's 13.2, 13.2 and 13.4; a Walsh AES's 339, 340 and 367 at 1, 2 and 8).
+int rows_mac_group(const Context& c, size_t switches, size_t T) {
+    const size_t tiles = std::max<size_t>(1, c.N / kMaxTile);
+    return switches * T * tiles >= 16 * (size_t)c.sm_count ? 2 : 1;
 }
 
-bool MacLists::in_rows(const Context& c, size_t mod) const {
-    return c.fuse() && (words || c.mods[mod].q < fp::kLimit);
-}
-
-void MacLists::add(const Context& c, const MacGroupJob& job, size_t mod) {
-    const double bytes = 8.0 * (double)c.N * (2.0 * job.parts + (double)job.n * (job.parts + 2.0));
-    if (!in_rows(c, mod)) {
-        sums.push_back(job);
-        sums_bytes += bytes;
-        return;
-    }
-    rows_bytes += bytes;
-    for (int k0 = 0; k0 < job.n; k0 += group) {
-        MacGroupJob j = job;
-        j.n = std::min(group, job.n - k0);
-        for (int k = 0; k < j.n; ++k) {
-            j.key_term[k] = job.key_term[k0 + k];
-            j.digits[k] = job.digits[k0 + k];
-            j.acc[k] = job.acc[k0 + k];
-        }
-        rows.push_back(j);
-    }
-}
-
-void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, bool words, double bytes,
-                   cudaStream_t s) {
+void rows_mac_jobs(const Context& c, const MacGroupJob* d_jobs, int njobs, double bytes, cudaStream_t s) {
     if (njobs <= 0) return;
     Probe probe(kClsKeyMac, bytes, s);
     switch (c.logN) {
-        case 10: launch_rows_mac<10>(c, d_jobs, njobs, words, s); break;
-        case 11: launch_rows_mac<11>(c, d_jobs, njobs, words, s); break;
-        case 12: launch_rows_mac<12>(c, d_jobs, njobs, words, s); break;
-        case 13: launch_rows_mac<13>(c, d_jobs, njobs, words, s); break;
-        case 14: launch_rows_mac<14>(c, d_jobs, njobs, words, s); break;
-        case 15: launch_rows_mac<15>(c, d_jobs, njobs, words, s); break;
-        case 16: launch_rows_mac<16>(c, d_jobs, njobs, words, s); break;
+        case 10: launch_rows_mac<10>(c, d_jobs, njobs, s); break;
+        case 11: launch_rows_mac<11>(c, d_jobs, njobs, s); break;
+        case 12: launch_rows_mac<12>(c, d_jobs, njobs, s); break;
+        case 13: launch_rows_mac<13>(c, d_jobs, njobs, s); break;
+        case 14: launch_rows_mac<14>(c, d_jobs, njobs, s); break;
+        case 15: launch_rows_mac<15>(c, d_jobs, njobs, s); break;
+        case 16: launch_rows_mac<16>(c, d_jobs, njobs, s); break;
         default: fail(kInvalid, "ntt: ring degree must be 2^10 .. 2^16");
     }
     check_cuda(cudaGetLastError(), "key inner product launch");

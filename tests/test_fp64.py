@@ -240,8 +240,8 @@ def test_mixed_key_switches(wg, oracle_mod, prm, fusion):
 @pytest.mark.parametrize("count", [1, 7, 601])
 @pytest.mark.parametrize("prm", MIXED)
 def test_fused_key_products_of_many(wg, oracle_mod, prm, count):
-    """The fused steps against the separate launches: word limbs in the fused key product (small
-    counts) or apart (601 at 2^10 is past its line), one or two switches a job and an odd one left."""
+    """The fused steps against the separate launches: one switch a job, or (601 at 2^10) two and an odd
+    one left."""
     import torch
 
     O, N = oracle_mod, 1 << 10
