@@ -50,6 +50,14 @@ WG_HD uint64_t umulhi(uint64_t a, uint64_t b) {
 #endif
 }
 
+WG_HD int clz64(uint64_t x) {
+#if defined(__CUDA_ARCH__)
+    return __clzll((long long)x);
+#else
+    return __builtin_clzll(x);
+#endif
+}
+
 // IEEE double helpers with explicit rounding, so no multiply-add is contracted unless asked.
 WG_HD double u2d(uint64_t x) {
 #if defined(__CUDA_ARCH__)

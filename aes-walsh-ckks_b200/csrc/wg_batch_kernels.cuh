@@ -7,6 +7,7 @@
 #include "wg_batch.hpp"
 #include "wg_internal.hpp"
 #include "wg_keyswitch.cuh"
+#include "wg_tensor.cuh"
 
 namespace wg {
 namespace bk {
@@ -200,38 +201,12 @@ __global__ void __launch_bounds__(kT) kb_gather(const GatherJob* jobs, int n, in
     j->a[i] = j->src_a[s];
 }
 
-// One coefficient of the tensor (c2, b1, a1) in place of (xa, xb).
-__device__ __forceinline__ void tensor_words(uint64_t& xa, uint64_t& xb, uint64_t ya, uint64_t yb, uint64_t& c2,
-                                             const Modulus& m) {
-    c2 = barrett_mul(xa, ya, m);
-    const uint64_t tmp = barrett_mul(xb, ya, m);
-    xb = barrett_mul(xb, yb, m);
-    xa = add_mod(barrett_mul(xa, yb, m), tmp, m.q);
-}
-// The same in FP64 for moduli below fp::kNoReduce and words below 2^43, where the four Barrett
-// products (eight 64-bit high products, 3.2 SM clocks a lane) bound the kernel.  The Barrett product's
-// one correction leaves q in place of 0 where its quotient estimate is two short, which takes
-// z mod q < z q 2^-128 < 1 (z < 2^86): for a zero residue alone.  Returns false for the caller to form
-// the products in words there.
-__device__ __forceinline__ bool tensor_fp(uint64_t& xa, uint64_t& xb, uint64_t ya, uint64_t yb, uint64_t& c2,
-                                          const Modulus& m) {
-    if ((xa | xb | ya | yb) >> 43) return false;
-    const double a = fp::from_word(xa), b = fp::from_word(xb);
-    const fp::Factor fa = fp::key_factor(ya, m.inv_q), fb = fp::key_factor(yb, m.inv_q);
-    const double aa = fp::mulmod(a, fa.w, fa.wq, m.qd), ba = fp::mulmod(b, fa.w, fa.wq, m.qd);
-    const double bb = fp::mulmod(b, fb.w, fb.wq, m.qd), ab = fp::mulmod(a, fb.w, fb.wq, m.qd);
-    if (aa == 0.0 || ba == 0.0 || bb == 0.0 || ab == 0.0) return false;
-    c2 = fp::to_word(fp::lift(aa, m.qd));
-    xb = fp::to_word(fp::lift(bb, m.qd));
-    xa = fp::canonical(dadd(ab, ba), m.qd, m.inv_q);
-    return true;
-}
-
 __global__ void __launch_bounds__(kT) kb_tensor(const TensorJob* jobs, int n, const Modulus* mods) {
     const TensorJob* j = job_of(jobs, n);
     if (!j) return;
     const Modulus m = mods[j->mod];
     const bool fp64 = m.q < fp::kNoReduce;
+    const int shift = tensor_shift(m);
     uint64_t xa[kWide], xb[kWide], ya[kWide], yb[kWide];
 #pragma unroll
     for (int r = 0; r < kWide; ++r) {
@@ -242,7 +217,7 @@ __global__ void __launch_bounds__(kT) kb_tensor(const TensorJob* jobs, int n, co
     for (int r = 0; r < kWide; ++r) {
         const size_t k = wide_index(r);
         uint64_t c2;
-        if (!fp64 || !tensor_fp(xa[r], xb[r], ya[r], yb[r], c2, m)) tensor_words(xa[r], xb[r], ya[r], yb[r], c2, m);
+        if (!fp64 || !tensor_fp(xa[r], xb[r], ya[r], yb[r], c2, m, shift)) tensor_words(xa[r], xb[r], ya[r], yb[r], c2, m);
         j->c2[k] = c2;
         j->b1[k] = xb[r];
         j->a1[k] = xa[r];

@@ -53,14 +53,6 @@ WG_HD void walsh_coef_words(const WalshCoefs& cf, int r, int hm, uint32_t* w) {
 #endif
 }
 
-WG_HD int clz64(uint64_t x) {
-#if defined(__CUDA_ARCH__)
-    return __clzll((long long)x);
-#else
-    return __builtin_clzll(x);
-#endif
-}
-
 // The low signs of one residue position and polynomial (masks 1..15 at their index; index 0 is
 // zero), and the sums of their low and high 32-bit halves.
 struct WalshSigns {

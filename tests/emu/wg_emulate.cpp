@@ -16,6 +16,7 @@
 #include "wg_ksfuse.cuh"
 #include "wg_ntt.cuh"
 #include "wg_tables.hpp"
+#include "wg_tensor.cuh"
 #include "wg_walsh.cuh"
 #include "wg_ring.hpp"
 #include "wg_bundle.hpp"
@@ -691,6 +692,23 @@ void emu_fp_mulmod(uint64_t q, const double* a, const uint64_t* w, size_t n, dou
         out[i] = fp::mulmod(a[i], fw, fwq, (double)q);
         word[i] = fp::canonical(out[i], (double)q, 1.0 / (double)q);
     }
+}
+
+// The tensor of n coefficients as kb_tensor forms it (out: c2, b1, a1 of each) and in words (ref);
+// returns how many went through FP64.
+size_t emu_tensor(uint64_t q, const uint64_t* xa, const uint64_t* xb, const uint64_t* ya, const uint64_t* yb, size_t n,
+                  uint64_t* out, uint64_t* ref) {
+    const Modulus m = emu_modulus(q);
+    size_t taken = 0;
+    for (size_t i = 0; i < n; ++i, out += 3, ref += 3) {
+        out[2] = ref[2] = xa[i];
+        out[1] = ref[1] = xb[i];
+        const bool fp64 = q < fp::kNoReduce && tensor_fp(out[2], out[1], ya[i], yb[i], out[0], m, tensor_shift(m));
+        if (!fp64) tensor_words(out[2], out[1], ya[i], yb[i], out[0], m);
+        tensor_words(ref[2], ref[1], ya[i], yb[i], ref[0], m);
+        taken += fp64;
+    }
+    return taken;
 }
 
 // reduce128 on n values (hi[i], lo[i]) modulo q

@@ -67,6 +67,29 @@ def test_sums_of_products(emu, q, n):  # noqa: F811
         assert [int(v) for v in out] == [want, want]
 
 
+@pytest.mark.parametrize("q", [_prime(1 << 27, 1 << 14), _prime(1 << 38, 1 << 15), _prime(1 << 42, 1 << 15), _prime(1 << 42, 1 << 15, 1)])
+def test_tensor_takes_words_of_any_size(emu, q):  # noqa: F811
+    """The tensor's FP64 products give the words of the Barrett products for residues (0, 1, q - 1 and
+    zero products among them), for words in [q, 2 q), and for larger ones, which have to go through
+    the words: beyond a few q the FP64 quotient no longer fits its rounding."""
+    emu.emu_tensor.argtypes = [C.c_uint64] + [u64p] * 4 + [C.c_size_t] + [u64p] * 2
+    emu.emu_tensor.restype = C.c_size_t
+    rng = np.random.default_rng(q % 1000003)
+    edge = [0, 1, q // 2, q - 1, q, q + 1, 2 * q - 1, 2 * q, 3 * q, 4 * q - 1, 4 * q, 1 << 40, (1 << 43) - 1, 1 << 43, (1 << 52) + 5, (1 << 64) - 1]
+    pairs = np.array([(a, b, c, d) for a in edge for b in edge for c in edge for d in (0, q - 1, 2 * q - 1, (1 << 43) - 1)], np.uint64)
+    blocks = [pairs] + [rng.integers(0, hi, (4000, 4), dtype=np.uint64) for hi in (q, 2 * q, 1 << 40, 1 << 43, 1 << 63)]
+    for k, v in enumerate(blocks):
+        xa, xb, ya, yb = (np.ascontiguousarray(v[:, i]) for i in range(4))
+        out, ref = np.zeros(3 * len(v), np.uint64), np.zeros(3 * len(v), np.uint64)
+        taken = emu.emu_tensor(q, xa, xb, ya, yb, len(v), out, ref)
+        assert (out == ref).all(), k
+        if k in (1, 2):  # words below 2 q
+            assert taken >= 3990 if q < 1 << 42 else taken == 0
+        for i in rng.integers(0, len(v), 200):
+            a, b, c, d = (int(w) for w in v[i])
+            assert [int(w) % q for w in out[3 * i:3 * i + 3]] == [a * c % q, b * d % q, (a * d + b * c) % q]
+
+
 def _extreme_polys(q, N, rng):
     """Residue polynomials that drive the lazy sums to their bounds, with words up to 4q - 1."""
     top = np.full(N, q - 1, np.uint64)
