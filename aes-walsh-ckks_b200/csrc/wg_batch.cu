@@ -244,23 +244,24 @@ static void run_keyswitch(const Context& c, const KsPlan& p, const JobTable& t, 
     check_cuda(cudaGetLastError(), "batched keyswitch launch");
 }
 
-void batch_keyswitch(Context& c, const KsItem* items, size_t n, cudaStream_t s) {
+void batch_keyswitch(Context& c, const KsItem* items, size_t n, cudaStream_t s, uint64_t* ws) {
     WG_SPAN("keyswitch");
     if (n == 0) return;
-    uint64_t* ws = c.batch_buffers(s).arena(c, batch_keyswitch_words(c, items, n), s);
+    if (!ws) ws = c.batch_buffers(s).arena(c, batch_keyswitch_words(c, items, n), s);
     JobTable t;
     KsPlan p = plan_keyswitch(c, items, n, ws, t);
     t.upload(c, s);
     run_keyswitch(c, p, t, s);
 }
 
-void batch_rescale(Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, cudaStream_t s) {
+void batch_rescale(Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, uint64_t* ws,
+                   size_t ws_words, cudaStream_t s) {
     if (level == 0 || level >= c.nq) fail(kInvalid, "ckks_rescale: invalid level");
-    constexpr size_t kChunk = 64;  // bounds the scratch for the remainders
-    for (size_t k0 = 0; k0 < npolys; k0 += kChunk) {
-        const size_t n = std::min(kChunk, npolys - k0);
-        const size_t words = (level + 1) * c.N;  // the remainders and the dropped limb's row phase
-        uint64_t* ws = c.batch_buffers(s).arena(c, n * words, s);
+    const size_t words = (level + 1) * c.N;  // a polynomial's remainders and its dropped limb's row phase
+    const size_t chunk = ws_words / words;
+    if (chunk == 0) fail(kRuntime, "ckks_rescale: scratch too small");
+    for (size_t k0 = 0; k0 < npolys; k0 += chunk) {
+        const size_t n = std::min(chunk, npolys - k0);
         RescaleJobs rs;
         rs.dropped = RescaleJobs::kCoefficients;
         for (size_t k = 0; k < n; ++k)

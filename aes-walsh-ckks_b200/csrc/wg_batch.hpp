@@ -48,9 +48,12 @@ struct JobTable {
 };
 
 size_t batch_keyswitch_words(const Context& c, const KsItem* items, size_t n);
-void batch_keyswitch(Context& c, const KsItem* items, size_t n, cudaStream_t s);
-// Rescale of npolys polynomials at one level, `stride` words apart.
-void batch_rescale(Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, cudaStream_t s);
+// ws: batch_keyswitch_words words of scratch on s, or null for the stream's batch arena.
+void batch_keyswitch(Context& c, const KsItem* items, size_t n, cudaStream_t s, uint64_t* ws = nullptr);
+// Rescale of npolys polynomials at one level, `stride` words apart, in the ws_words words of ws (at least
+// one polynomial's level + 1 limbs).
+void batch_rescale(Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, uint64_t* ws,
+                   size_t ws_words, cudaStream_t s);
 void batch_mul_relin_rescale_rotate(Context& c, size_t count, const size_t* levels, uint64_t* const* xb,
                                     uint64_t* const* xa, const uint64_t* const* yb, const uint64_t* const* ya,
                                     const int64_t* rots, const uint64_t* galois, const KeyEntry* relin,

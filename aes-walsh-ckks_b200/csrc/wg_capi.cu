@@ -80,11 +80,12 @@ bool stream_capturing(cudaStream_t s) {
 }
 
 // One key switch of one ciphertext.  Outside stream capture it runs as a batch of one (each
-// stage of the switch, all digits included, in a single launch); under capture, stage by stage
-// on the stream's reserved workspace (the batched path stages a job table per call).
+// stage of the switch, all digits included, in a single launch), in the batch arena or in `ws`;
+// under capture, stage by stage on the stream's reserved workspace (the batched path stages a job
+// table per call).
 void switch_one(wg::Context& c, size_t level, const uint64_t* key_term, const wg::KeyEntry& k, const uint64_t* b_in,
                 const uint64_t* a_in, uint64_t* b, uint64_t* a, bool b_add, bool a_add, uint64_t galois,
-                cudaStream_t s) {
+                uint64_t* ws, cudaStream_t s) {
     if (stream_capturing(s)) {
         wg::keyswitch(c, level, key_term, k, b_in, a_in, b, a, b_add, a_add, galois, c.workspace(s), s);
         return;
@@ -100,19 +101,19 @@ void switch_one(wg::Context& c, size_t level, const uint64_t* key_term, const wg
     it.b_add = b_add ? 1 : 0;
     it.a_add = a_add ? 1 : 0;
     it.galois = galois;
-    wg::batch_keyswitch(c, &it, 1, s);
+    wg::batch_keyswitch(c, &it, 1, s, ws);
 }
 
 void do_rotate(wg::Context& c, size_t level, uint64_t* b, uint64_t* a, int64_t rotation, cudaStream_t s) {
     const int64_t r = normalize_rotation(c, rotation);
     if (r == 0) return;
     const wg::KeyEntry& k = c.key(WG_KEY_ROTATION, r);
-    switch_one(c, level, a, k, b, a, b, a, true, false, rotation_galois(c, r), s);
+    switch_one(c, level, a, k, b, a, b, a, true, false, rotation_galois(c, r), nullptr, s);
 }
 
 void do_relin(wg::Context& c, size_t level, uint64_t* c0, uint64_t* c1, const uint64_t* c2, cudaStream_t s) {
     const wg::KeyEntry& k = c.key(WG_KEY_RELIN, 0);
-    switch_one(c, level, c2, k, c0, c1, c0, c1, true, true, 0, s);
+    switch_one(c, level, c2, k, c0, c1, c0, c1, true, true, 0, nullptr, s);
 }
 
 uint64_t* scratch_after_switch(wg::Context& c, cudaStream_t s) {
@@ -121,7 +122,7 @@ uint64_t* scratch_after_switch(wg::Context& c, cudaStream_t s) {
 
 void do_rescale(wg::Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, cudaStream_t s) {
     if (!stream_capturing(s)) {
-        wg::batch_rescale(c, level, polys, npolys, stride, s);
+        wg::batch_rescale(c, level, polys, npolys, stride, c.workspace(s), c.workspace_words(), s);
         return;
     }
     uint64_t* ws = scratch_after_switch(c, s);
@@ -232,7 +233,11 @@ int wg_ctx_has_key(const wg_context* ctx, int kind, int64_t rotation) {
 }
 
 int wg_ctx_reserve(wg_context* ctx, void* stream) {
-    return guard([&] { C(ctx).workspace(S(stream)); });
+    return guard([&] {
+        wg::Context& c = C(ctx);
+        c.workspace(S(stream));
+        if (!stream_capturing(S(stream))) c.batch_buffers(S(stream)).ensure_ring(c, 1, S(stream));
+    });
 }
 
 size_t wg_ctx_workspace_words(const wg_context* ctx) { return ctx && ctx->c ? ctx->c->workspace_words() : 0; }
@@ -374,7 +379,8 @@ int wg_keyswitch(wg_context* ctx, size_t level, const uint64_t* key_term, int ki
         check_ptr(a, "ckks_hybrid_keyswitch");
         const int64_t r = kind == WG_KEY_ROTATION ? normalize_rotation(c, rotation) : 0;
         const wg::KeyEntry& k = c.key(kind, r);
-        switch_one(c, level, key_term, k, b, a, b, a, b_add != 0, a_add != 0, 0, S(stream));
+        // the workspace in either form of the call: one call outside a capture makes the next capturable
+        switch_one(c, level, key_term, k, b, a, b, a, b_add != 0, a_add != 0, 0, c.workspace(S(stream)), S(stream));
     });
 }
 
@@ -401,7 +407,7 @@ int wg_conjugate(wg_context* ctx, size_t level, uint64_t* b, uint64_t* a, void* 
         const uint64_t g = 2 * c.N - 1;
         wg::automorphism(c, b, pb, (int)(level + 1), 1, 0, g, S(stream));
         wg::automorphism(c, a, pa, (int)(level + 1), 1, 0, g, S(stream));
-        switch_one(c, level, pa, k, pb, pa, b, a, true, false, 0, S(stream));
+        switch_one(c, level, pa, k, pb, pa, b, a, true, false, 0, c.workspace(S(stream)), S(stream));
     });
 }
 

@@ -32,30 +32,34 @@ void* BatchBuffers::stage(const Context& c, const void* data, size_t bytes, cuda
     return commit(off, bytes, s);
 }
 
+void BatchBuffers::ensure_ring(const Context& c, size_t bytes, cudaStream_t s) {
+    const size_t need = (std::max<size_t>(bytes, 1) + 255) & ~size_t{255};
+    if (need <= ring_bytes) return;
+    // grow: everything queued on the stream may still read the old device ring
+    check_cuda(cudaSetDevice(c.device), "cudaSetDevice");
+    check_cuda(cudaStreamSynchronize(s), "staging ring resize");
+    for (Flight& f : flights) spare_events.push_back(f.done);
+    flights.clear();
+    cudaFree(d_ring);
+    cudaFreeHost(h_ring);
+    d_ring = h_ring = nullptr;
+    ring_bytes = 0;
+    const size_t cap = std::max<size_t>(need * 2, size_t{64} << 20);
+    if (cudaMalloc((void**)&d_ring, cap) != cudaSuccess || cudaMallocHost((void**)&h_ring, cap) != cudaSuccess) {
+        cudaGetLastError();
+        fail(kNoMemory, "staging ring allocation failed");
+    }
+    ring_bytes = cap;
+    head = 0;
+}
+
 size_t BatchBuffers::reserve(const Context& c, size_t bytes, cudaStream_t s) {
     g_stage_calls.fetch_add(1, std::memory_order_relaxed);
     g_stage_bytes.fetch_add(bytes, std::memory_order_relaxed);
     if (capturing(s))
         fail(kRuntime, "batched calls cannot be captured into a graph (their staging is reused); use wg_batch_plan_*");
+    ensure_ring(c, bytes, s);
     const size_t need = (std::max<size_t>(bytes, 1) + 255) & ~size_t{255};
-    if (need > ring_bytes) {
-        // grow: everything queued on the stream may still read the old device ring
-        check_cuda(cudaSetDevice(c.device), "cudaSetDevice");
-        check_cuda(cudaStreamSynchronize(s), "staging ring resize");
-        for (Flight& f : flights) spare_events.push_back(f.done);
-        flights.clear();
-        cudaFree(d_ring);
-        cudaFreeHost(h_ring);
-        d_ring = h_ring = nullptr;
-        ring_bytes = 0;
-        const size_t cap = std::max<size_t>(need * 2, size_t{64} << 20);
-        if (cudaMalloc((void**)&d_ring, cap) != cudaSuccess || cudaMallocHost((void**)&h_ring, cap) != cudaSuccess) {
-            cudaGetLastError();
-            fail(kNoMemory, "staging ring allocation failed");
-        }
-        ring_bytes = cap;
-        head = 0;
-    }
     // wait for the uploads whose host bytes this region still holds (ring_place: the newest
     // overlapping one, which completes every older one too; all of them are then released)
     size_t wait = 0;

@@ -117,6 +117,8 @@ struct BatchBuffers {
     // Copy `bytes` of host data into the ring and onto the device (stream order); returns the
     // device address, valid for kernels queued on `s` before the ring wraps back over it.
     void* stage(const Context& c, const void* data, size_t bytes, cudaStream_t s);
+    // allocates or grows the ring to hold a region of `bytes` (stage() and reserve() do so as needed)
+    void ensure_ring(const Context& c, size_t bytes, cudaStream_t s);
     // The same in two steps, for callers that write the bytes in place: reserve() makes a
     // region of `bytes` free (waiting for old uploads as stage() does) and returns its offset;
     // the caller fills h_ring + offset; commit() uploads it and returns d_ring + offset.

@@ -104,7 +104,9 @@ int wg_keygen_switch_key(wg_context* ctx, int kind, int64_t rotation, const int8
 int wg_keygen_secret_switch(wg_context* ctx, int kind, const int8_t* source, const int8_t* target, const uint64_t* a,
                             const int64_t* e, uint64_t seed, double sigma, uint64_t* out, void* stream);
 int wg_ctx_has_key(const wg_context* ctx, int kind, int64_t rotation);
-/* Allocate the scratch of `stream` now (required before capturing the stream in a graph). */
+/* Allocate the scratch and the staging ring (64 MiB pinned, mirrored on the device) of `stream` now.
+ * Required before a single operation on the stream is captured in a graph, unless a wg_keyswitch,
+ * wg_conjugate or wg_rescale on it has run outside a capture before. */
 int wg_ctx_reserve(wg_context* ctx, void* stream);
 /* Give back the device memory the context holds for `stream` beyond its tables and keys (the
  * stream's scratch and staging buffers) and its cache of reusable scratch chunks, after the
