@@ -292,7 +292,7 @@ struct NttJob {
 };
 void ntt_jobs(const Context& c, const NttJob* d_jobs, int njobs, bool forward, cudaStream_t s);
 // Time every NTT geometry on the context's device and keep the fastest per direction and phase
-// (cached per device and ring degree for the process).
+// (cached per device, ring degree and share of word moduli for the process).
 void ntt_autotune(Context& c);
 // One phase (cols: the high-bit phase) of a strided batch with a given geometry.
 void ntt_phase_geometry(const Context& c, bool forward, bool cols, int variant, uint64_t* data, int limbs,

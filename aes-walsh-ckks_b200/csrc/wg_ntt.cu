@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 #include "wg_internal.hpp"
@@ -751,11 +752,19 @@ void dispatch(const Context& c, uint64_t* data, int limbs, int polys, size_t str
     check_cuda(cudaGetLastError(), "ntt launch");
 }
 
-// Tuned choices per (device, ring degree), shared by every context of the process.
+// Tuned choices per (device, ring degree, share of word moduli in quarters, rounded up), shared by the
+// process's contexts: FP64 and integer limbs favour different geometries, and a chain's launches mix
+// them as its timing batch does.
 struct TuneKey {
-    int device, logN;
-    bool operator<(const TuneKey& o) const { return device != o.device ? device < o.device : logN < o.logN; }
+    int device, logN, words;
+    bool operator<(const TuneKey& o) const {
+        return std::tie(device, logN, words) < std::tie(o.device, o.logN, o.words);
+    }
 };
+TuneKey tune_key(const Context& c) {
+    const auto n = std::count_if(c.mods.begin(), c.mods.end(), [](const Modulus& m) { return m.q >= fp::kLimit; });
+    return {c.device, c.logN, (int)((4 * n + c.mods.size() - 1) / c.mods.size())};
+}
 std::mutex g_tune_mutex;
 std::map<TuneKey, NttTuning> g_tuned;
 
@@ -846,7 +855,7 @@ void ntt_phase_geometry(const Context& c, bool forward, bool cols, int variant, 
 void ntt_autotune(Context& c) {
     {
         std::lock_guard<std::mutex> g(g_tune_mutex);
-        auto it = g_tuned.find({c.device, c.logN});
+        auto it = g_tuned.find(tune_key(c));
         if (it != g_tuned.end()) {
             c.tuning = it->second;
             for (int d = 0; d < 2; ++d)
@@ -921,7 +930,7 @@ void ntt_autotune(Context& c) {
     for (int d = 0; d < 2; ++d)
         for (int p = 0; p < 2; ++p) c.ntt_variant[d][p] = tn.chosen[d][p];
     std::lock_guard<std::mutex> g(g_tune_mutex);
-    g_tuned[{c.device, c.logN}] = tn;
+    g_tuned[tune_key(c)] = tn;
 }
 
 }  // namespace wg

@@ -145,8 +145,8 @@ int wg_evalmod_k_bound(size_t coefficients, size_t hamming_weight, double log2_f
  * order, ntt.cpp:235-386).  Four geometries compute the same words: 0 = 8 residues per thread
  * with twiddles staged in shared memory, 1 = 8 residues, twiddles read from the table,
  * 2 = 16 residues, staged, 3 = 16 residues, from the table.  wg_ctx_create times each one per
- * direction and phase on the device (once per device and ring degree in the process) and
- * keeps the fastest.  wg_ntt_tuning reports chosen[direction][phase] (direction 0 forward,
+ * direction and phase on the device (once in the process per device, ring degree and share of
+ * moduli of 2^50 and more, in quarters) and keeps the fastest.  wg_ntt_tuning reports chosen[direction][phase] (direction 0 forward,
  * 1 inverse; phase 0 rows = low index bits, 1 columns = high bits; 4 ints), the timings
  * ms[direction][phase][geometry] (16 floats, best of three launches over a batch of `limbs`
  * limb-transforms) and that batch size.  Either output pointer may be null. */

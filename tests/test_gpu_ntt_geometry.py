@@ -84,3 +84,15 @@ def test_tuning_report(wg, oracle_mod):
     for d, dn in enumerate(("forward", "inverse")):
         for ph, pn in enumerate(("rows", "columns")):
             print(f"  {dn} {pn}: " + ", ".join(f"{ms[d, ph, g]:.4f}" for g in range(4)))
+
+
+def test_tuning_is_kept_per_arithmetic(wg, oracle_mod):
+    """FP64 and word chains of one ring are timed apart (two timings never agree to the last bit), and
+    a second chain of the same arithmetic takes the first one's."""
+    def ms(bits):
+        p, q = oracle_mod.find_primes([bits], [bits] * 3, 1 << 12)
+        return wg.Context(1 << 12, q, p, 1).ntt_tuning()["ms"]
+
+    fp64, words = ms(40), ms(58)
+    assert (fp64 != words).any()
+    assert (ms(41) == fp64).all() and (ms(59) == words).all()
