@@ -722,18 +722,19 @@ void phase_dispatch(const Context& c, bool fwd, bool cols, int variant, uint64_t
     }
 }
 
+// The geometry of one phase over `words` residues: the caller's where it is pinned, else by the tuned one.
+int phase_geometry(const Context& c, int direction, bool cols, size_t words) {
+    const int v = c.ntt_variant[direction][cols ? 1 : 0];
+    return c.ntt_pinned[direction] >> (cols ? 1 : 0) & 1 ? v : launch_geometry(v, words, c.sm_count, c.word_moduli);
+}
+
 void dispatch(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,
               const NttJob* jobs, int njobs, bool fwd, cudaStream_t s) {
     if (jobs ? njobs <= 0 : (limbs <= 0 || polys <= 0)) return;
     if (!jobs && (polys > 65535 || limbs > 65535)) fail(kInvalid, "ntt: too many limbs or polynomials in one batch");
     const int d = fwd ? 0 : 1;
-    // One launch per transform for the rings whose limb a cluster of small CTAs covers, while the batch
-    // is about one wave of clusters.  Measured at 38-bit moduli, one launch / two phases, in us: 2^14:
-    // 10 / 12 (32 limbs), 14 / 16 (64), 20 / 20 (96), 42 / 38 (256); 2^13: 9 / 12 (64), 13 / 17 (128),
-    // 22 / 24 (256); 2^12: 9 / 12 (128), 18 / 22 (512).  At 2^15 clusters of 8 CTAs of 512 threads
-    // leave most SMs waiting (29 / 24 at 64 limbs, 189 / 132 at 512), so larger rings take the phases.
-    const size_t words = (size_t)(jobs ? njobs : limbs * (size_t)polys) * c.N;
-    if (!c.ntt_pinned[d] && (c.logN <= 12 || (c.logN <= kWholeMaxLog && words <= ((size_t)1 << 20)))) {
+    const size_t transforms = jobs ? (size_t)njobs : limbs * (size_t)polys, words = transforms * c.N;
+    if (!c.ntt_pinned[d] && whole_launch(c.logN, transforms, c.sm_count, c.word_moduli)) {
         switch (c.logN) {
             case 10: whole_dispatch<10>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
             case 11: whole_dispatch<11>(c, data, limbs, polys, stride, map, jobs, njobs, fwd, s); break;
@@ -745,10 +746,10 @@ void dispatch(const Context& c, uint64_t* data, int limbs, int polys, size_t str
     }
     // forward: columns then rows; inverse: rows then columns
     const bool first_cols = fwd;
-    phase_dispatch(c, fwd, first_cols, c.ntt_variant[d][first_cols ? 1 : 0], data, limbs, polys, stride, map, jobs,
+    phase_dispatch(c, fwd, first_cols, phase_geometry(c, d, first_cols, words), data, limbs, polys, stride, map, jobs,
                    njobs, s);
-    phase_dispatch(c, fwd, !first_cols, c.ntt_variant[d][first_cols ? 0 : 1], data, limbs, polys, stride, map, jobs,
-                   njobs, s);
+    phase_dispatch(c, fwd, !first_cols, phase_geometry(c, d, !first_cols, words), data, limbs, polys, stride, map,
+                   jobs, njobs, s);
     check_cuda(cudaGetLastError(), "ntt launch");
 }
 
@@ -786,8 +787,8 @@ void ntt_jobs(const Context& c, const NttJob* d_jobs, int njobs, bool forward, c
 
 void ntt_jobs_phase(const Context& c, const NttJob* d_jobs, int njobs, bool forward, bool cols, cudaStream_t s) {
     if (njobs <= 0) return;
-    phase_dispatch(c, forward, cols, c.ntt_variant[forward ? 0 : 1][cols ? 1 : 0], nullptr, 0, 0, 0, LimbMap{0, 0, 0},
-                   d_jobs, njobs, s);
+    phase_dispatch(c, forward, cols, phase_geometry(c, forward ? 0 : 1, cols, njobs * c.N), nullptr, 0, 0, 0,
+                   LimbMap{0, 0, 0}, d_jobs, njobs, s);
     check_cuda(cudaGetLastError(), "ntt launch");
 }
 

@@ -401,6 +401,35 @@ WG_HD HandOver hand_over(int tile, int e) {
     return {c / W::COLUMNS, h * W::COLUMNS + c % W::COLUMNS};
 }
 
+// Whether `transforms` limbs of a ring go in one launch each way (Whole) or in two phases: one launch for
+// the rings whose limb a cluster of small CTAs covers, while the batch is about one wave of clusters.
+// Forward at 38-bit moduli, one launch / two phases, as calls one after the other, in us: 2^14: 8 / 12 (12
+// limbs), 10 / 12 (32), 14 / 17 (64); 2^13: 9 / 12 (64), 12 / 14 (128), 21 / 21 (256).  Device time alone:
+// 2^14: 5.6 / 6.2 (12), 7.7 / 6.3 (16), 7.9 / 8.4 (24), 12.8 / 13.0 (64), 20.5 / 20.5 (128); 2^13: 7.3 / 7.9 (64);
+// 2^12: 6.4 / 7.5 (128), 54 / 59 (2048); 2^10: 3.2 / 4.4 (64), 12.8 / 17.2 (2048).  At 60 bits: 2^14: 7.3 / 7.7 (12),
+// 10.7 / 7.8 (16), 10.8 / 11.4 (24), 14.5 / 15.0 (48), 19.0 / 18.3 (64); 2^13: 17.0 / 17.3 (128); 2^12: 90.7 / 90.8 (2048);
+// 2^10: 20.5 / 22.8 (2048).  So chains with word moduli stop at 48 limbs of 2^14 and leave out the launches
+// that fit one CTA an SM where the clusters of 8 do not (13 to 18 limbs; with 38 bits there the call with
+// one launch is still the shorter one, 10 / 12).  At 2^15 clusters of 8 CTAs of 512 threads leave most
+// SMs waiting (29 / 24 at 64 limbs, 189 / 132 at 512), so larger rings take the phases.
+inline bool whole_launch(int logN, size_t transforms, int sm_count, bool word_moduli) {
+    if (logN <= 12) return true;
+    if (logN > kWholeMaxLog || transforms << logN > (size_t{1} << 20)) return false;
+    if (logN < kWholeMaxLog || !word_moduli) return true;
+    const size_t ctas = (transforms << logN) / kMaxTile;
+    return transforms <= 12 || (ctas > (size_t)sm_count && transforms <= 48);
+}
+
+// The geometry (kNttGeometries order) of one phase over `words` residues where `tuned` is the best of
+// large batches: in small launches 8 residues a thread in place of 16, which halve the threads.
+// Forward transforms of 60-bit moduli, 8 and 16 residues in the row phase, device time in us: 2^15, 4
+// limbs 7.9 and 8.8, 8 limbs 8.0 and 9.3, 24 limbs 15.7 and 16.2, 64 limbs 30.9 and 31.1; 38-bit
+// moduli, 8 limbs 6.3 and 6.2, 12 limbs 8.5 and 8.3.
+inline int launch_geometry(int tuned, size_t words, int sm_count, bool word_moduli) {
+    const size_t small = (size_t)sm_count * kMaxTile * (word_moduli ? 4 : 1);
+    return tuned >= 2 && words <= small ? tuned - 2 : tuned;
+}
+
 // The place of twiddle x of a row (of the 2^kr of row-stage kr = NB2 - 1 - b) in the table.  In the
 // round of a row's lowest bits thread o uses the 2^(eb-1-b) consecutive twiddles from o << (eb-1-b),
 // so over a warp each of these loads would touch a 128-byte line per lane; there they stand
