@@ -75,7 +75,7 @@ static KsPlan plan_keyswitch(const Context& c, const KsItem* items, size_t n, ui
     std::vector<GatherJob> gather;
     std::vector<NttEpiJob> contrib_epi;
     KsPlan p{};
-    p.fused = c.fuse();
+    p.fused = c.fuse_switch(2 * n);  // the ModDown launch has two jobs per switch
     // MAC groups: consecutive switches with the same key, level and digit layout (up to
     // mac_group), one job per QP limb; [group_begin, it) is the open group
     std::vector<MacGroupJob> mac;

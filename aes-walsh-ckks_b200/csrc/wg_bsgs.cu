@@ -543,7 +543,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
 
     JobTable t;
     // 1. hoist
-    const bool fused = c.fuse();
+    const bool fused = c.fuse_switch(2 * count);  // the pair ModDown launch: two jobs per ciphertext
     int max_src = 1;
     for (size_t j = 0; j < B; ++j) max_src = std::max(max_src, c.modup[level][j].src_count);
     std::vector<NttJob> intt_a, ntt_dig;
@@ -868,7 +868,7 @@ void rotate_many_batch(Context& c, size_t level, size_t count, const uint64_t* c
     uint64_t* arena = c.batch_buffers(s).arena(c, count * per_ct, s);
     auto modq = [&](size_t limb) { return (int)(limb < L ? limb : nq + (limb - L)); };
 
-    const bool fused = c.fuse();
+    const bool fused = c.fuse_switch(count * B);  // the ModUp launch: one job per digit
     int max_src = 1;
     for (size_t j = 0; j < B; ++j) max_src = std::max(max_src, c.modup[level][j].src_count);
     std::vector<NttJob> intt_a, ntt_dig, intt_p, ntt_c;

@@ -289,6 +289,12 @@ Context* create_context(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
     c->q.assign(q, q + nq);
     c->p.assign(p, p + np);
     for (size_t i = 0; i < nq + np; ++i) c->word_moduli |= (i < nq ? q[i] : p[i - nq]) >= fp::kLimit;
+    const auto within = [](const uint64_t* m, size_t n) {
+        const size_t words = std::count_if(m, m + n, [](uint64_t x) { return x >= fp::kLimit; });
+        return n <= Context::kFusedSources && words <= Context::kFusedWordSources;
+    };
+    c->narrow = within(p, np);
+    for (size_t s0 = 0; s0 < nq; s0 += c->alpha) c->narrow &= within(q + s0, std::min(c->alpha, nq - s0));
     check_cuda(cudaSetDevice(device), "cudaSetDevice");
     {
         // The batched operations draw their temporaries from this process's stream-ordered

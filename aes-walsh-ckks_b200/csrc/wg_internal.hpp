@@ -159,11 +159,22 @@ struct Context {
     // k_ntt_rows_epi).  0: the separate launches; 1, 2: fused.  The words are the same in every mode.
     int ntt_fusion = 1;
     int sm_count = 148;  // multiprocessors of the device
-    // Whether the batched steps run fused.  Launches too small to fill the device divide their
-    // jobs' output limbs over several CTAs (split_of, wg_ksfuse.cu), so the fused sequence is the
-    // shorter one at every size.
+    // Whether a rescale runs fused.  Launches too small to fill the device divide their jobs'
+    // output limbs over several CTAs (split_of, wg_ksfuse.cu), so the fused sequence is the shorter
+    // one at every size.
     bool fuse() const { return ntt_fusion != 0; }
-    // Whether a step over `jobs` jobs counts as one that fills the device (RescaleJobs).
+    // Whether a key switch whose base changes have `jobs` jobs runs fused.  In launches that do not
+    // fill the device a block walks its sources' column phases one after the other, and so does every
+    // block that shares the job: past kFusedSources sources, or kFusedWordSources of word moduli (three
+    // to four times the time of an FP64 one), the separate launches are shorter.  Fused and separate,
+    // time against separate launches in integer words throughout: one relinearisation of 2^14 with
+    // 60-bit moduli, 4 + 4 sources 0.78 and 0.86, 5 + 5 0.90 and 0.80, 8 + 8 0.95 and 0.90, 16 + 16
+    // 1.41 and 0.96; with 50-bit moduli, 8 + 8 0.74 and 0.78, 12 + 12 0.72 and 0.85, 16 + 16 1.05 and
+    // 0.88; 4 hoisted rotations at 60 bits, 4 + 4 0.98 and 0.91, 5 + 5 1.08 and 0.93, 16 + 16 1.30 and 1.00.
+    bool fuse_switch(size_t jobs) const { return ntt_fusion != 0 && (narrow || fills(jobs)); }
+    static constexpr size_t kFusedSources = 12, kFusedWordSources = 4;
+    bool narrow = true;  // no digit and not the P limbs are beyond them
+    // Whether a step over `jobs` jobs counts as one that fills the device.
     bool fills(size_t jobs) const {
         return ntt_fusion == 2 || (ntt_fusion == 1 && jobs * (N >= 1024 ? N / 1024 : 1) >= 2 * (size_t)sm_count);
     }

@@ -301,3 +301,42 @@ def test_fused_key_products_of_many(wg, oracle_mod, prm, count):
     out = [g.reshape(4, count, L, N) for g in got]
     for i, level in enumerate(levels):
         assert (out[0][:2, i, :level] == out[1][:2, i, :level]).all(), i
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits,width,fused", [(60, 4, True), (60, 5, False), (50, 12, True), (50, 13, False)])
+def test_wide_base_changes_take_the_separate_launches(wg, oracle_mod, bits, width, fused):
+    """Small launches fuse the base changes up to 12 sources, 4 of word moduli; launches that fill the
+    device fuse them at any width.  The route shows in the launch counts, the words are the same."""
+    import torch
+
+    O, N, count = oracle_mod, 1 << 10, 160
+    p, q = O.find_primes([bits] * width, [bits] * width, N)
+    ctx, o = wg.Context(N, q, p, 1), O.OracleCtx(N, q, p, 1)
+    s = o.ternary(64, 3)
+    key = o.rotation_key(s, 3, 11)
+    ctx.set_key(wg.WG_KEY_ROTATION, key, rotation=3)
+    ctx.set_key(wg.WG_KEY_RELIN, o.relin_key(s, 13))
+    n = width * N
+    b, a = o.uniform(width, 9), o.uniform(width, 10)
+    want = o.rotate(width - 1, b, a, key, 3)
+    launches, batch = [], []
+    for mode in (0, 1, 2):
+        ctx.set_ntt_fusion(mode)
+        db, da, out = wg.to_device(b), wg.to_device(a), torch.empty(2 * n, dtype=torch.int64, device="cuda")
+        n0 = wg.launch_count()
+        ctx.rotate_many(width - 1, db, da, [3], out)
+        n1 = wg.launch_count()
+        ctx.rotate(width - 1, db, da, 3)
+        n2 = wg.launch_count()
+        x = [wg.to_device(b).repeat(count).reshape(count, n) for _ in range(2)]
+        ctx.batch_mul_relin_rescale_rotate([width - 1] * count, list(x[0]), list(x[1]), [wg.to_device(b)] * count,
+                                           [wg.to_device(a)] * count, [3] * count)
+        batch.append((wg.launch_count() - n2, wg.to_host(x[0][:, : n - N].reshape(-1))))
+        torch.cuda.synchronize()
+        launches.append((n1 - n0, n2 - n1))
+        assert (wg.to_host(db) == want[0]).all() and (wg.to_host(da) == want[1]).all(), mode
+        assert (wg.to_host(out) == np.concatenate(want)).all(), mode
+    assert launches[0] != launches[2] and launches[1] == launches[2 if fused else 0], launches
+    assert batch[1][0] == batch[2][0] < batch[0][0]
+    assert (batch[1][1] == batch[0][1]).all() and (batch[2][1] == batch[0][1]).all()
