@@ -82,11 +82,13 @@ bool stream_capturing(cudaStream_t s) {
 // One key switch of one ciphertext.  Outside stream capture it runs as a batch of one (each
 // stage of the switch, all digits included, in a single launch), in the batch arena or in `ws`;
 // under capture, stage by stage on the stream's reserved workspace (the batched path stages a job
-// table per call).
+// table per call).  With `ws`, a switch of one or two limbs that would not run fused goes stage by
+// stage as well: there the call waits on the host's launches, and the table is one more copy (2 + 4
+// limbs of 60 bits at 2^15: 76 us against 81, but 16 + 16 limbs at 2^14 165 against 150).
 void switch_one(wg::Context& c, size_t level, const uint64_t* key_term, const wg::KeyEntry& k, const uint64_t* b_in,
                 const uint64_t* a_in, uint64_t* b, uint64_t* a, bool b_add, bool a_add, uint64_t galois,
                 uint64_t* ws, cudaStream_t s) {
-    if (stream_capturing(s)) {
+    if (stream_capturing(s) || (ws && level <= 1 && !c.fuse_switch(2))) {
         wg::keyswitch(c, level, key_term, k, b_in, a_in, b, a, b_add, a_add, galois, c.workspace(s), s);
         return;
     }
@@ -121,7 +123,13 @@ uint64_t* scratch_after_switch(wg::Context& c, cudaStream_t s) {
 }
 
 void do_rescale(wg::Context& c, size_t level, uint64_t* polys, size_t npolys, size_t stride, cudaStream_t s) {
-    if (!stream_capturing(s)) {
+    // One or two polynomials of many word limbs stage by stage: the fused step's blocks walk several
+    // output limbs one after the other there (two of 13 limbs of 60 bits at 2^15: 43 us against 46, of 12
+    // limbs 43 and 43; one of 18 limbs at 2^16 50 and 53).  The stages take two polynomials at a time, so
+    // from three on the batch is shorter (1.3 times and more).
+    const size_t words = std::count_if(c.q.begin(), c.q.begin() + level + 1, [](uint64_t q) { return q >= wg::fp::kLimit; });
+    const bool staged = c.ntt_fusion != 2 && npolys <= 2 && words * npolys * c.N > (size_t{24} << 15);
+    if (!stream_capturing(s) && !staged) {
         wg::batch_rescale(c, level, polys, npolys, stride, c.workspace(s), c.workspace_words(), s);
         return;
     }

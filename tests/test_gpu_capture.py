@@ -110,3 +110,39 @@ def test_reserve_covers_the_single_calls(wg, oracle_mod):
     torch.cuda.synchronize()
     got = wg.to_host(many.reshape(-1)).reshape(60, -1)[:, : level * N]
     assert (got == want).all()
+
+
+def test_routes_of_single_calls(wg, oracle_mod):
+    """Outside a capture: a key switch of one or two limbs whose base changes are too wide to fuse goes
+    stage by stage (nothing is staged for it), a rescale of one or two polynomials of many word limbs too
+    (six launches, not three)."""
+    import torch
+
+    N = 1 << 10
+    p, q = oracle_mod.find_primes([60] * 5, [60] * 3, N)
+    o, ctx = oracle_mod.OracleCtx(N, q, p, 1), wg.Context(N, q, p, 1)
+    key = o.rotation_key(o.ternary(64, 3), 3, 11)
+    ctx.set_key(wg.WG_KEY_ROTATION, key, rotation=3)
+    for level, staged in ((0, 0), (1, 0), (2, 1)):
+        x = [o.uniform(level + 1, 70 + i) for i in range(3)]
+        d = [wg.to_device(v) for v in x]
+        calls = wg.host_stats()["stages"]
+        ctx.keyswitch(level, d[2], wg.WG_KEY_ROTATION, d[0], d[1], True, False, rotation=3)
+        torch.cuda.synchronize()
+        assert wg.host_stats()["stages"] - calls == staged, level
+        wb, wa = o.keyswitch(level, x[2], key, x[0], x[1], 1, 0)
+        assert (wg.to_host(d[0]) == wb).all() and (wg.to_host(d[1]) == wa).all(), level
+
+    N = 1 << 15
+    p, q = oracle_mod.find_primes([60], [60] * 13, N)
+    o, ctx = oracle_mod.OracleCtx(N, q, p, 13), wg.Context(N, q, p, 13)
+    poly = o.uniform(13, 80)
+    for level, polys, launches in ((12, 2, 6), (11, 2, 3), (12, 1, 3), (12, 3, 3)):
+        n = (level + 1) * N
+        d = wg.to_device(poly[:n]).repeat(polys)
+        n0 = wg.launch_count()
+        ctx.rescale(level, d, npolys=polys, stride=n)
+        torch.cuda.synchronize()
+        assert wg.launch_count() - n0 == launches, (level, polys)
+        (want,) = o.rescale(level, [poly[:n]])
+        assert (wg.to_host(d).reshape(polys, n)[:, : level * N] == want).all(), (level, polys)
