@@ -363,7 +363,9 @@ WG_HD uint64_t fp_epilogue_value(const NttEpiJob& j, const FpEpilogue& c, uint64
                                  const Modulus& m) {
     const double v = fp::reduce(fp::bits_double(x), m.qd, m.inv_q);
     if (j.kind == kEpiRescale) {
-        // |in - v| <= 2.5 q < 2^52: the product is below q in magnitude (factor_of)
+        // |in - v| <= 2^51 + q / 2 (any larger word is reduced first): the product stays below q in
+        // magnitude (1/2 + |in - v| 2^-53, factor_of)
+        if (in >> 51) in = reduce64(in, m);
         const double d = dadd(fp::from_word(in), -v);
         return fp::to_word(fp::lift(fp::mulmod(d, c.w, c.wq, m.qd), m.qd));
     }

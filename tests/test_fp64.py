@@ -204,6 +204,33 @@ def test_emulated_mixed_key_switches(oracle_mod, emu, prm):  # noqa: F811
         emu.emu_destroy(h)
 
 
+def test_emulated_rescale_of_unreduced_words(oracle_mod, emu):  # noqa: F811
+    """The limbs a rescale keeps may hold words of any size (only the dropped one is transformed): both
+    sequences give the rescale of their residues."""
+    N = 1 << 10
+    q = np.array([_prime(1 << 27, N), _prime(1 << 42, N), _prime(1 << 50, N), _prime(1 << 50, N, 1), _prime(1 << 36, N)], np.uint64)
+    p = np.array([_prime(1 << 60, N)], np.uint64)
+    o = oracle_mod.OracleCtx(N, q, p, 1)
+    h = emu.emu_create(N, q, len(q), p, 1, 1)
+    try:
+        rng = np.random.default_rng(8)
+        qs = np.repeat(q[:4], N)
+        for hi in (1 << 51, 1 << 52, 1 << 63):
+            kept = rng.integers(0, hi, 4 * N, dtype=np.uint64)
+            kept[::7] = hi - 1
+            kept[1::7] = qs[1::7] * (hi // qs[1::7]) - 1
+            drop = rng.integers(0, int(q[4]), N, dtype=np.uint64)
+            (want,) = o.rescale(4, [np.concatenate([kept % qs, drop])])
+            for fused in (0, 1):
+                emu.emu_set_keyswitch_fusion(fused)
+                x = np.concatenate([kept, drop])
+                emu.emu_rescale(h, 4, x)
+                assert (x[: 4 * N] == want).all(), (hi, fused)
+    finally:
+        emu.emu_set_keyswitch_fusion(0)
+        emu.emu_destroy(h)
+
+
 @pytest.mark.parametrize("q", [_prime(1 << 42, 1 << 15), _prime(1 << 42, 1 << 15, 1), 12289, _prime(1 << 55, 1 << 15, 1)])
 def test_walsh_products_at_the_edges(emu, q):  # noqa: F811
     """The Walsh products on both sides of the FP64 limit, at a small modulus (coefficients and signs
