@@ -120,15 +120,19 @@ struct AccumJob {
     int ngiants, i, pad0, pad1;
 };
 
-// The b sum of a baby step whose input word b is not below q: add_mod keeps such a word's excess
-// while every step wraps, so the sum is formed step by step in that order (such words come from
-// products with a single Barrett correction and are rare).
-__device__ __forceinline__ uint64_t baby_b_sum(const uint64_t* key_b, size_t key_stride, const uint64_t* a,
-                                            const uint64_t* digit, size_t part_stride, int parts, int own_part,
-                                            uint64_t b, uint64_t q, uint64_t qninv) {
-    for (int p = 0; p < parts; ++p)
-        b = add_mod(b, mont_mul(p == own_part ? *a : digit[p * part_stride], key_b[p * key_stride], q, qninv), q);
-    return b;
+// A word of a ciphertext as the giant sums take it: canonical, whatever its size.
+__device__ __forceinline__ uint64_t baby_word(uint64_t b, const Modulus& m) { return b < m.q ? b : reduce64(b, m); }
+
+// Baby step 0, the ciphertexts themselves in QP: job (c, i) is limb i of ciphertext c, zero for P limbs.
+__global__ void __launch_bounds__(kT) kb_baby0(const CtRef* __restrict__ cts, int n, uint64_t* __restrict__ babies,
+                                               const Modulus* mods, int L, int T, int nslots, size_t N) {
+    const int j = blockIdx.y + 65535 * blockIdx.z;
+    if (j >= n) return;
+    const int c = j / T, i = j % T;
+    const size_t at = (size_t)i * N + (size_t)blockIdx.x * kT + threadIdx.x;
+    uint64_t* o = babies + (size_t)c * nslots * 2 * T * N + at;
+    o[0] = i < L ? baby_word(cts[c].a[at], mods[i]) : 0;
+    o[(size_t)T * N] = i < L ? baby_word(cts[c].b[at], mods[i]) : 0;
 }
 
 // Ciphertexts [c0, c0 + NC) of the job.  NC is a compile-time count so that every digit load of a part
@@ -142,7 +146,6 @@ __device__ __forceinline__ void baby_step(const BabyJob* j, int c0, const Modulu
     const int i = j->i;
     const int T = L + K;
     const bool is_p = i >= L;
-    const uint64_t q = m.q;
     const double qd = m.qd, inv_q = m.inv_q;
     const size_t key_limbs = (size_t)j->key_level + 1 + K;
     const size_t klimb = is_p ? (size_t)j->key_level + 1 + (i - L) : (size_t)i;
@@ -190,17 +193,7 @@ __device__ __forceinline__ void baby_step(const BabyJob* j, int c0, const Modulu
         const uint64_t rb = FP ? fp::mont_sum_word(sum_b[c], m) : acc_b[c].mont_value(m);
         uint64_t* o = babies + ((size_t)(c0 + c) * nslots + j->slot) * slot_words + (size_t)i * N;
         o[dst] = ra;
-        o[(size_t)T * N + dst] = is_p ? rb : add_mod(ct[c].b[limb], rb, q);
-    }
-    // words not below q, after the stores so that the sums are out of the registers
-    if (is_p) return;
-#pragma unroll 1
-    for (int c = 0; c < NC; ++c) {
-        const uint64_t b = ct[c].b[limb];
-        if (b < q) continue;
-        babies[((size_t)(c0 + c) * nslots + j->slot) * slot_words + (size_t)(T + i) * N + dst] =
-            baby_b_sum(j->key + (key_limbs + klimb) * N + x, 2 * key_limbs * N, ct[c].a + limb,
-                       digits + (size_t)(c0 + c) * parts * part_stride + limb, part_stride, parts, i / alpha, b, q, m.qninv);
+        o[(size_t)T * N + dst] = is_p ? rb : add_mod(baby_word(ct[c].b[limb], m), rb, m.q);
     }
 }
 
@@ -559,7 +552,7 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
                 if (l < s0 || l >= s1) ntt_dig.push_back({dg + j * T * N + l * N, dg + j * T * N + l * N, modq(l), 0});
         }
     }
-    // 2. babies: baby 0 as a copy (P limbs zeroed below), others by MAC + scatter
+    // 2. babies: baby 0 the ciphertext itself (slot 0, kb_baby0), others by MAC + scatter
     std::vector<BabyJob> baby_jobs;
     std::vector<CtRef> ct_refs;
     for (size_t ci = 0; ci < count; ++ci) ct_refs.push_back({a[ci], b[ci]});
@@ -710,15 +703,6 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
             }
     }
 
-    // Baby slot 0 holds (a, b) with zero P limbs: copy Q limbs, clear P limbs.
-    for (size_t ci = 0; ci < count && baby0; ++ci) {
-        uint64_t* slot = babybuf + (ci * ns + 0) * slotw;
-        check_cuda(cudaMemcpyAsync(slot, a[ci], L * N * 8, cudaMemcpyDeviceToDevice, s), "baby 0");
-        check_cuda(cudaMemcpyAsync(slot + T * N, b[ci], L * N * 8, cudaMemcpyDeviceToDevice, s), "baby 0");
-        check_cuda(cudaMemsetAsync(slot + L * N, 0, K * N * 8, s), "baby 0");
-        check_cuda(cudaMemsetAsync(slot + T * N + L * N, 0, K * N * 8, s), "baby 0");
-    }
-
     const NttJob* j_intt_a = t.add(intt_a);
     const ModUpJob* j_modup = t.add(modup);
     const NttJob* j_ntt_dig = t.add(ntt_dig);
@@ -759,6 +743,11 @@ void lt_stage_apply(Context& c, const LtStage& st, size_t count, uint64_t* const
         ntt_jobs(c, t.at(j_ntt_dig), (int)ntt_dig.size(), true, s);
     }
     // 2.
+    if (baby0) {
+        Probe probe(kClsElementwise, 8.0 * N * (double)(count * (2 * L + 2 * T)), s);
+        kb_baby0<<<grid_for(c, count * T), kT, 0, s>>>(t.at(j_cts), (int)(count * T), babybuf, c.d_mod, (int)L, (int)T,
+                                                       (int)ns, N);
+    }
     if (!baby_jobs.empty()) {
         double bytes = 0;
         for (const BabyJob& bj : baby_jobs) bytes += 8.0 * N * (2.0 * B + bj.nc * (B + 3.0));

@@ -367,3 +367,31 @@ def test_wide_base_changes_take_the_separate_launches(wg, oracle_mod, bits, widt
     assert launches[0] != launches[2] and launches[1] == launches[2 if fused else 0], launches
     assert batch[1][0] == batch[2][0] < batch[0][0]
     assert (batch[1][1] == batch[0][1]).all() and (batch[2][1] == batch[0][1]).all()
+
+
+@pytest.mark.gpu
+def test_linear_transform_of_unreduced_words(wg, oracle_mod):
+    """The b polynomial of a linear transform's input may hold words of any size (only a is transformed):
+    the result is that of its residues, in every arithmetic of the giant sums."""
+    import torch
+
+    N = 1 << 10
+    q = np.array([_prime(1 << 30, N), _prime(1 << 42, N), _prime(1 << 50, N), _prime(1 << 61, N)], np.uint64)
+    p = np.array([_prime(1 << 60, N)], np.uint64)
+    ctx, o = wg.Context(N, q, p, 2), oracle_mod.OracleCtx(N, q, p, 2)
+    s = o.ternary(64, 3)
+    for r in (1, 2):
+        ctx.set_key(wg.WG_KEY_ROTATION, o.rotation_key(s, r, 11 + r), rotation=r)
+    rng = np.random.default_rng(9)
+    diags = np.concatenate([rng.integers(0, int(m), N, dtype=np.uint64) for _ in range(4) for m in (*q, *p)])
+    stage = wg.LtStage(ctx, 3, [0, 1, 2, 3], diags, 2)
+    b, a = o.uniform(4, 5), o.uniform(4, 6)
+    room = ((1 << 63) - 1 - b) // np.repeat(q, N)
+    big = b + np.repeat(q, N) * rng.integers(0, room, dtype=np.uint64)
+    out = []
+    for words in (b, big):
+        db, da = wg.to_device(words), wg.to_device(a)
+        stage.apply([db], [da])
+        torch.cuda.synchronize()
+        out.append((wg.to_host(db), wg.to_host(da)))
+    assert (out[0][0] == out[1][0]).all() and (out[0][1] == out[1][1]).all()
