@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <deque>
@@ -293,6 +294,17 @@ struct Probe {
 // ---------------------------------------------------------------------------------------
 // Kernel launchers.
 // ---------------------------------------------------------------------------------------
+// Opts a kernel in to `bytes` of dynamic shared memory (from 48 KiB up that is needed), once per device:
+// the attribute belongs to the kernel on the current device, which a launch has made the context's.
+template <auto Kernel>
+void allow_shared(int device, size_t bytes) {
+    static std::atomic<uint64_t> done{0};
+    const uint64_t bit = device < 64 ? uint64_t{1} << device : 0;
+    if (done.load(std::memory_order_acquire) & bit) return;
+    cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    done.fetch_or(bit, std::memory_order_release);
+}
+
 // One limb of a job-table NTT: the first phase reads src and writes dst, the second phase
 // works in place on dst (src == dst for an in-place transform).
 struct NttJob {

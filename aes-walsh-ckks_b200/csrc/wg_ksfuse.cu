@@ -277,12 +277,7 @@ void launch_rescale(const Context& c, const RescaleNttJob* jobs, int njobs, int 
 
 template <class G>
 void launch_modup_g(const Context& c, const ModUpNttJob* jobs, int njobs, int max_src, int max_out, cudaStream_t s) {
-    static const bool opted = [] {
-        cudaFuncSetAttribute(k_modup_ntt<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)fused_smem<G>(kMaxDigitWidth));
-        return true;
-    }();
-    (void)opted;
+    allow_shared<k_modup_ntt<G>>(c.device, fused_smem<G>(kMaxDigitWidth));
     const dim3 grid(G::TILES * split_of(c, njobs, G::TILES, kResident, max_src, max_out),
                     njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
     k_modup_ntt<G><<<grid, G::THREADS, fused_smem<G>(max_src), s>>>(jobs, njobs, c.d_mod, c.twiddles(3));
@@ -299,12 +294,7 @@ void launch_modup(const Context& c, const ModUpNttJob* jobs, int njobs, int max_
 template <int LOGN, bool FMA>
 void launch_moddown_f(const Context& c, const ModDownNttJob* jobs, int njobs, int max_out, cudaStream_t s) {
     using G = Geom<LOGN, kModDownBits>;
-    static const bool opted = [] {
-        cudaFuncSetAttribute(k_moddown_ntt<G, FMA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)fused_smem<G>(kMaxPLimbs));
-        return true;
-    }();
-    (void)opted;
+    allow_shared<k_moddown_ntt<G, FMA>>(c.device, fused_smem<G>(kMaxPLimbs));
     const dim3 grid(G::TILES * split_of(c, njobs, G::TILES, kResident, (int)c.np, max_out),
                     njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
     k_moddown_ntt<G, FMA><<<grid, G::THREADS, fused_smem<G>((int)c.np), s>>>(

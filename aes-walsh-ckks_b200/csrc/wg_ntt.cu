@@ -307,12 +307,7 @@ template <int LOGN, bool FWD, bool TABLE>
 void launch_whole(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,
                   const NttJob* jobs, int njobs, cudaStream_t s) {
     using W = Whole<LOGN>;
-    static const bool opted = [] {
-        cudaFuncSetAttribute(k_ntt_whole<LOGN, FWD, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)whole_smem<LOGN>());
-        return true;
-    }();
-    (void)opted;
+    static_assert(whole_smem<LOGN>() <= size_t{48} << 10, "no opt-in");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = TABLE ? dim3(W::CTAS, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535)
                         : dim3(W::CTAS, limbs, polys);
@@ -630,11 +625,7 @@ template <int LOGN, int EB, bool STAGED>
 void launch_rows_epi(const Context& c, const NttEpiJob* jobs, int njobs, cudaStream_t s) {
     using P = Phase<LOGN, true, false, EB, STAGED>;
     constexpr size_t sm = rows_epi_smem<LOGN, EB, STAGED>();
-    static const bool opted = [] {
-        cudaFuncSetAttribute(k_ntt_rows_epi<LOGN, EB, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        return true;
-    }();
-    (void)opted;
+    allow_shared<k_ntt_rows_epi<LOGN, EB, STAGED>>(c.device, sm);
     const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
     k_ntt_rows_epi<LOGN, EB, STAGED><<<grid, P::THREADS, sm, s>>>(jobs, njobs, c.d_mod, c.twiddles(EB));
 }
@@ -649,17 +640,6 @@ void rows_epi_variant(const Context& c, int variant, const NttEpiJob* jobs, int 
     }
 }
 
-template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, bool TABLE>
-void enable_smem() {
-    // opt in to more than 48 KiB of dynamic shared memory once per kernel instance
-    static const bool done = [] {
-        cudaFuncSetAttribute(k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, TABLE>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<LOGN, FWD, COLS, EB, STAGED>());
-        return true;
-    }();
-    (void)done;
-}
-
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED>
 void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,
                  const NttJob* jobs, int njobs, cudaStream_t s) {
@@ -667,7 +647,7 @@ void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t 
     constexpr size_t sm = smem_bytes<LOGN, FWD, COLS, EB, STAGED>();
     const TwPair* tw = c.twiddles(EB);
     if (jobs) {
-        enable_smem<LOGN, FWD, COLS, EB, STAGED, true>();
+        allow_shared<k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, true>>(c.device, sm);
         const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
         // algorithmic bytes: every residue read once and written once per transform, i.e. 8 B
         // per residue for each of the two phases (16 N B per limb-transform)
@@ -676,7 +656,7 @@ void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t 
                                                                                    c.d_mod, tw,
                                                                                    c.d_tw_words + (EB - 3) * c.nq * c.N);
     } else {
-        enable_smem<LOGN, FWD, COLS, EB, STAGED, false>();
+        allow_shared<k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, false>>(c.device, sm);
         const dim3 grid(P::N / P::TILE, limbs, polys);
         Probe probe(kClsNtt, 8.0 * P::N * limbs * polys, s);
         k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, false><<<grid, P::THREADS, sm, s>>>(data, stride, map, nullptr, 0,

@@ -93,3 +93,16 @@ def test_every_launch_matches_the_kernel_grid():
                     continue  # an argument of launch_jobs<true> (checked above)
                 bad.append((fname, kernel, "named outside a checked launch"))
     assert not bad, bad
+
+
+def test_shared_memory_opt_in_is_per_device():
+    """The attribute of a kernel belongs to the device that is current: every opt-in goes through
+    allow_shared, which keeps a flag per device, not one for the process."""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*")) + glob.glob(os.path.join(CSRC, "*.hpp"))):
+        text = open(path).read()
+        calls = text.count("cudaFuncSetAttribute")
+        if os.path.basename(path) == "wg_internal.hpp":
+            body = _body(text, text.index("void allow_shared(int device"))
+            assert calls == 1 == body.count("cudaFuncSetAttribute") and "<< device" in body
+        else:
+            assert calls == 0, path
