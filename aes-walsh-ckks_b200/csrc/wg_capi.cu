@@ -358,6 +358,7 @@ int wg_ntt_set_geometry(wg_context* ctx, int direction, int phase, int geometry)
         wg::Context& c = C(ctx);
         if (direction < 0 || direction > 1 || phase < 0 || phase > 1) wg::fail(wg::kInvalid, "ntt: invalid direction or phase");
         if (geometry >= wg::kNttGeometries) wg::fail(wg::kInvalid, "ntt: unknown geometry");
+        if (phase == 0 && geometry >= 2) c.rows16(true);
         if (geometry < 0)
             c.ntt_pinned[direction] &= ~(1 << phase);
         else

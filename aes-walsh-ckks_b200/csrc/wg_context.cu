@@ -11,6 +11,28 @@
 #include "wg_tables.hpp"
 
 namespace wg {
+namespace {
+
+// Table blockIdx.y for 8 residues a thread from the (w, Shoup w) pairs [mod][2][N]: those of 2 nm tables,
+// then the inverse ones of the Q limbs as words.
+__global__ void __launch_bounds__(256) k_twiddles_8(const ntt::TwPair* __restrict__ in, ntt::TwPair* __restrict__ out,
+                                                    const Modulus* __restrict__ mods, int nm, int logN) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const int t = blockIdx.y;
+    const bool words = t >= 2 * nm;
+    const int from = words ? 2 * (t - 2 * nm) + 1 : t;
+    const ntt::TwPair p = in[((size_t)from << logN) + i];
+    out[((size_t)t << logN) + ntt::twiddle_place(logN, 3, i)] = ntt::twiddle_pair(p.w, p.ws, mods[from / 2].q, words);
+}
+
+// The tables for 16 residues a thread: those for 8 in another order.
+__global__ void __launch_bounds__(256) k_twiddles_16(const ntt::TwPair* __restrict__ in, ntt::TwPair* __restrict__ out,
+                                                     int logN) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x, table = (size_t)blockIdx.y << logN;
+    out[table + ntt::twiddle_place(logN, 4, i)] = in[table + ntt::twiddle_place(logN, 3, i)];
+}
+
+}  // namespace
 
 static bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -231,9 +253,39 @@ Context::~Context() {
     for (auto& kv : batches) kv.second.release();
     cudaFree(d_modup);
     cudaFree(d_mod);
-    for (uint64_t* t : d_tw) cudaFree(t);
-    cudaFree(d_tw_words);
+    for (ntt::TwPair* t : d_tw) cudaFree(t);
     cudaFree(d_tables);
+}
+
+void Context::rows16(bool keep) {
+    if (keep == (d_tw[1] != nullptr)) return;
+    if (!keep) {
+        cudaFree(d_tw[1]);
+        d_tw[1] = nullptr;
+        return;
+    }
+    // a caller may pin a geometry while one of its streams is capturing
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    ntt::TwPair* d = nullptr;
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&d, table_pairs() * sizeof(ntt::TwPair));
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) {
+        k_twiddles_16<<<dim3((unsigned)(N / 256), (unsigned)(table_pairs() / N)), 256, 0, s>>>(d_tw[0], d, logN);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+    if (s) cudaStreamDestroy(s);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(d);
+        if (e == cudaErrorMemoryAllocation) fail(kNoMemory, "ntt: no room for the 16-residue twiddles");
+        check_cuda(e, "ntt: 16-residue twiddles");
+    }
+    d_tw[1] = d;
 }
 
 size_t Context::workspace_words() const {
@@ -325,28 +377,21 @@ Context* create_context(uint64_t N, const uint64_t* q, size_t nq, const uint64_t
     dev_alloc((void**)&c->d_tables, c->tables_words * 8);
     check_cuda(cudaMemcpy(c->d_mod, c->mods.data(), nm * sizeof(Modulus), cudaMemcpyHostToDevice), "upload moduli");
     {
-        // twiddle pairs per modulus and direction, as the NTT kernels read them
+        // interleaved (w, Shoup w) pairs per modulus and direction; the tables are made of them on the device
         std::vector<ntt::TwPair> pairs(nm * 2 * N);
-        auto upload = [&](uint64_t*& d, int eb) {
-            for (size_t i = 0; i < nm; ++i)
-                for (size_t dir = 0; dir < 2; ++dir) {
-                    const uint64_t* w = H.tw.data() + (i * 4 + 2 * dir) * N;
-                    ntt::twiddle_pairs(N, H.mods[i].q, w, w + N, eb, false, pairs.data() + (i * 2 + dir) * N);
-                }
-            dev_alloc((void**)&d, pairs.size() * sizeof(ntt::TwPair));
-            check_cuda(cudaMemcpy(d, pairs.data(), pairs.size() * sizeof(ntt::TwPair), cudaMemcpyHostToDevice),
-                       "upload twiddles");
-        };
-        upload(c->d_tw[0], 3);
-        upload(c->d_tw[1], 4);
-        for (int eb = 3; eb <= 4; ++eb)
-            for (size_t i = 0; i < nq; ++i) {
-                const uint64_t* w = H.tw.data() + (i * 4 + 2) * N;
-                ntt::twiddle_pairs(N, H.mods[i].q, w, w + N, eb, true, pairs.data() + ((eb - 3) * nq + i) * N);
-            }
-        dev_alloc((void**)&c->d_tw_words, 2 * nq * N * sizeof(ntt::TwPair));
-        check_cuda(cudaMemcpy(c->d_tw_words, pairs.data(), 2 * nq * N * sizeof(ntt::TwPair), cudaMemcpyHostToDevice),
+        for (size_t t = 0; t < 2 * nm; ++t) {
+            const uint64_t* w = H.tw.data() + 2 * t * N;
+            for (size_t i = 0; i < N; ++i) pairs[t * N + i] = {w[i], w[N + i]};
+        }
+        for (ntt::TwPair*& d : c->d_tw) dev_alloc((void**)&d, c->table_pairs() * sizeof(ntt::TwPair));
+        check_cuda(cudaMemcpy(c->d_tw[1], pairs.data(), pairs.size() * sizeof(ntt::TwPair), cudaMemcpyHostToDevice),
                    "upload twiddles");
+        k_twiddles_8<<<dim3((unsigned)(N / 256), (unsigned)(2 * nm + nq)), 256>>>(c->d_tw[1], c->d_tw[0], c->d_mod, (int)nm,
+                                                                                 c->logN);
+        check_cuda(cudaGetLastError(), "twiddle tables");
+        check_cuda(cudaStreamSynchronize(nullptr), "twiddle tables");
+        cudaFree(c->d_tw[1]);
+        c->d_tw[1] = nullptr;
     }
     check_cuda(cudaMemcpy(c->d_tables, H.words.data(), H.words.size() * 8, cudaMemcpyHostToDevice),
                "upload tables");

@@ -78,8 +78,8 @@ WG_HD double reduce(double x, double q, double inv_q) {
 WG_HD double lift(double x, double q) { return x < 0.0 ? dadd(x, q) : x; }
 WG_HD uint64_t canonical(double x, double q, double inv_q) { return to_word(lift(reduce(x, q, inv_q), q)); }
 
-// The factor pair of a residue w in [0, q).
-inline void factor(uint64_t w, uint64_t q, double& fw, double& fwq) {
+// The factor pair of a residue w in [0, q), q < kLimit.
+WG_HD void factor(uint64_t w, uint64_t q, double& fw, double& fwq) {
     fw = w > q / 2 ? -(double)(q - w) : (double)w;
     fwq = fw / (double)q;
 }

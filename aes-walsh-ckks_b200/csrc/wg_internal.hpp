@@ -148,11 +148,15 @@ struct Context {
     bool word_moduli = false;        // some modulus is fp::kLimit or more
     std::vector<Modulus> mods;       // nq + np entries (P after Q)
     Modulus* d_mod = nullptr;
-    // twiddle pairs [mod][2][N] (forward, inverse; ntt::twiddle_pairs) for 8 and 16 residues per thread
-    uint64_t* d_tw[2] = {nullptr, nullptr};
-    // [8 / 16 residues][Q limb][N]: the inverse's (w, Shoup w) pairs of every Q limb (NttJob::words)
-    ntt::TwPair* d_tw_words = nullptr;
-    const ntt::TwPair* twiddles(int eb) const { return reinterpret_cast<const ntt::TwPair*>(d_tw[eb - 3]); }
+    // twiddle pairs [mod][2][N] (forward, inverse; ntt::twiddle_pair) in the orders for 8 and 16 residues
+    // per thread (ntt::twiddle_place), then the inverse's (w, Shoup w) pairs [Q limb][N] of every Q limb
+    // (NttJob::words) in the same order.  The orders differ in the row phase's part alone; the second
+    // exists while a row phase uses it (rows16).
+    ntt::TwPair* d_tw[2] = {nullptr, nullptr};
+    const ntt::TwPair* twiddles(int eb) const { return d_tw[eb - 3]; }
+    const ntt::TwPair* word_twiddles(int eb) const { return twiddles(eb) + 2 * (nq + np) * N; }
+    size_t table_pairs() const { return (2 * (nq + np) + nq) * N; }
+    void rows16(bool keep);  // makes the tables for 16 residues, or gives them back
     int ntt_variant[2][2] = {{0, 0}, {0, 0}};  // NTT geometry per [direction][phase: rows, columns]
     int ntt_pinned[2] = {0, 0};                // phases of the direction whose geometry the caller pinned (bits)
     // Key switches and rescales can run their base changes fused with the adjacent NTT column
@@ -317,9 +321,6 @@ void ntt_jobs(const Context& c, const NttJob* d_jobs, int njobs, bool forward, c
 // Time every NTT geometry on the context's device and keep the fastest per direction and phase
 // (cached per device, ring degree and share of word moduli for the process).
 void ntt_autotune(Context& c);
-// One phase (cols: the high-bit phase) of a strided batch with a given geometry.
-void ntt_phase_geometry(const Context& c, bool forward, bool cols, int variant, uint64_t* data, int limbs,
-                        int polys, size_t poly_stride, LimbMap map, cudaStream_t s);
 
 // One phase of a job-table NTT (cols: the high-bit phase) with the context's geometry; the
 // inverse transform is rows then columns, the forward one columns then rows, and the first

@@ -630,22 +630,12 @@ void launch_rows_epi(const Context& c, const NttEpiJob* jobs, int njobs, cudaStr
     k_ntt_rows_epi<LOGN, EB, STAGED><<<grid, P::THREADS, sm, s>>>(jobs, njobs, c.d_mod, c.twiddles(EB));
 }
 
-template <int LOGN>
-void rows_epi_variant(const Context& c, int variant, const NttEpiJob* jobs, int njobs, cudaStream_t s) {
-    switch (variant) {
-        case 0: launch_rows_epi<LOGN, 3, true>(c, jobs, njobs, s); break;
-        case 1: launch_rows_epi<LOGN, 3, false>(c, jobs, njobs, s); break;
-        case 2: launch_rows_epi<LOGN, 4, true>(c, jobs, njobs, s); break;
-        default: launch_rows_epi<LOGN, 4, false>(c, jobs, njobs, s); break;
-    }
-}
-
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED>
 void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,
                  const NttJob* jobs, int njobs, cudaStream_t s) {
     using P = Phase<LOGN, FWD, COLS, EB, STAGED>;
     constexpr size_t sm = smem_bytes<LOGN, FWD, COLS, EB, STAGED>();
-    const TwPair* tw = c.twiddles(EB);
+    const TwPair* tw = c.twiddles(COLS ? 3 : EB);  // column phases read the part that all orders share
     if (jobs) {
         allow_shared<k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, true>>(c.device, sm);
         const dim3 grid(P::N / P::TILE, njobs < 65535 ? njobs : 65535, (njobs + 65534) / 65535);
@@ -654,7 +644,7 @@ void launch_geom(const Context& c, uint64_t* data, int limbs, int polys, size_t 
         Probe probe(kClsNtt, 8.0 * P::N * njobs, s);
         k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, true><<<grid, P::THREADS, sm, s>>>(nullptr, 0, map, jobs, njobs,
                                                                                    c.d_mod, tw,
-                                                                                   c.d_tw_words + (EB - 3) * c.nq * c.N);
+                                                                                   c.word_twiddles(COLS ? 3 : EB));
     } else {
         allow_shared<k_ntt_phase<LOGN, FWD, COLS, EB, STAGED, false>>(c.device, sm);
         const dim3 grid(P::N / P::TILE, limbs, polys);
@@ -749,6 +739,16 @@ TuneKey tune_key(const Context& c) {
 std::mutex g_tune_mutex;
 std::map<TuneKey, NttTuning> g_tuned;
 
+void take_tuning(Context& c) {
+    bool rows16 = false;
+    for (int d = 0; d < 2; ++d)
+        for (int p = 0; p < 2; ++p) {
+            c.ntt_variant[d][p] = c.tuning.chosen[d][p];
+            rows16 |= p == 0 && c.tuning.chosen[d][p] >= 2;
+        }
+    c.rows16(rows16);
+}
+
 }  // namespace
 
 void ntt_forward(const Context& c, uint64_t* data, int limbs, int polys, size_t poly_stride, LimbMap map,
@@ -803,26 +803,17 @@ void ntt_rows_epilogue_jobs(const Context& c, const NttEpiJob* d_jobs, int njobs
     // 8 residues per thread with twiddles from the table whatever the tuner chose for the plain
     // row phase: the prefetched operands take 32 KiB of shared memory, which leaves 4 blocks per
     // SM only in this geometry
-    const int v = 1;
     switch (c.logN) {
-        case 10: rows_epi_variant<10>(c, v, d_jobs, njobs, s); break;
-        case 11: rows_epi_variant<11>(c, v, d_jobs, njobs, s); break;
-        case 12: rows_epi_variant<12>(c, v, d_jobs, njobs, s); break;
-        case 13: rows_epi_variant<13>(c, v, d_jobs, njobs, s); break;
-        case 14: rows_epi_variant<14>(c, v, d_jobs, njobs, s); break;
-        case 15: rows_epi_variant<15>(c, v, d_jobs, njobs, s); break;
-        case 16: rows_epi_variant<16>(c, v, d_jobs, njobs, s); break;
+        case 10: launch_rows_epi<10, 3, false>(c, d_jobs, njobs, s); break;
+        case 11: launch_rows_epi<11, 3, false>(c, d_jobs, njobs, s); break;
+        case 12: launch_rows_epi<12, 3, false>(c, d_jobs, njobs, s); break;
+        case 13: launch_rows_epi<13, 3, false>(c, d_jobs, njobs, s); break;
+        case 14: launch_rows_epi<14, 3, false>(c, d_jobs, njobs, s); break;
+        case 15: launch_rows_epi<15, 3, false>(c, d_jobs, njobs, s); break;
+        case 16: launch_rows_epi<16, 3, false>(c, d_jobs, njobs, s); break;
         default: fail(kInvalid, "ntt: ring degree must be 2^10 .. 2^16");
     }
     check_cuda(cudaGetLastError(), "ntt epilogue launch");
-}
-
-void ntt_phase_geometry(const Context& c, bool forward, bool cols, int variant, uint64_t* data, int limbs, int polys,
-                        size_t poly_stride, LimbMap map, cudaStream_t s) {
-    if (variant < 0 || variant >= kNttGeometries) fail(kInvalid, "ntt: unknown geometry");
-    if (limbs <= 0 || polys <= 0) return;
-    phase_dispatch(c, forward, cols, variant, data, limbs, polys, poly_stride, map, nullptr, 0, s);
-    check_cuda(cudaGetLastError(), "ntt launch");
 }
 
 // Time every geometry of every (direction, phase) the way the batched circuits launch the
@@ -839,8 +830,7 @@ void ntt_autotune(Context& c) {
         auto it = g_tuned.find(tune_key(c));
         if (it != g_tuned.end()) {
             c.tuning = it->second;
-            for (int d = 0; d < 2; ++d)
-                for (int p = 0; p < 2; ++p) c.ntt_variant[d][p] = it->second.chosen[d][p];
+            take_tuning(c);
             return;
         }
     }
@@ -856,6 +846,13 @@ void ntt_autotune(Context& c) {
         // no room for the timing batch: keep the default geometry (tuning.limbs = 0 says so)
         cudaGetLastError();
         cudaFree(buf);
+        return;
+    }
+    try {
+        c.rows16(true);
+    } catch (const Error&) {
+        cudaFree(buf);
+        cudaFree(d_jobs);
         return;
     }
     cudaStream_t s = nullptr;
@@ -908,8 +905,7 @@ void ntt_autotune(Context& c) {
     }
     release();
     c.tuning = tn;
-    for (int d = 0; d < 2; ++d)
-        for (int p = 0; p < 2; ++p) c.ntt_variant[d][p] = tn.chosen[d][p];
+    take_tuning(c);
     std::lock_guard<std::mutex> g(g_tune_mutex);
     g_tuned[tune_key(c)] = tn;
 }

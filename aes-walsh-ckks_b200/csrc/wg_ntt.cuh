@@ -14,9 +14,9 @@ namespace ntt {
 constexpr int kMaxTile = 2048;
 
 // One entry of the interleaved twiddle table: the twiddle and its Shoup constant (for the moduli of
-// the FP64 path: the doubles w and w / q, twiddle_pairs) side by side, so a butterfly fetches both
+// the FP64 path: the doubles w and w / q, twiddle_pair) side by side, so a butterfly fetches both
 // with one 16-byte load.  Table layout per modulus:
-// [forward pairs (N)][inverse pairs (N)], one table per residues-per-thread (twiddle_pairs).
+// [forward pairs (N)][inverse pairs (N)], one order per residues-per-thread (twiddle_place).
 struct alignas(16) TwPair {
     uint64_t w, ws;
 };
@@ -436,32 +436,30 @@ inline int launch_geometry(int tuned, size_t words, int sm_count, bool word_modu
 // round of a row's lowest bits thread o uses the 2^(eb-1-b) consecutive twiddles from o << (eb-1-b),
 // so over a warp each of these loads would touch a 128-byte line per lane; there they stand
 // thread-minor.
-inline size_t row_order(int nb2, int eb, int b, size_t x) {
+WG_HD size_t row_order(int nb2, int eb, int b, size_t x) {
     const int last = nb2 - eb * ((nb2 + eb - 1) / eb - 1);  // stages of that round
     if (b >= last) return x;
     const int kb = eb - 1 - b, ob = nb2 - eb;
     return ((x & (((size_t)1 << kb) - 1)) << ob) | (x >> kb);
 }
 
-// The table a modulus q is transformed with by the geometries of 2^eb residues per thread, one
-// direction, from the split (w, Shoup w) words: the factor pairs (w, w / q) as bits of doubles for the
-// moduli of the FP64 path (unless `words`), the words otherwise; rows in row_order.
-inline void twiddle_pairs(size_t N, uint64_t q, const uint64_t* w, const uint64_t* ws, int eb, bool words, TwPair* out) {
-    const bool fp64 = q < fp::kLimit && !words;
-    const int n = floor_log2((unsigned)N), nb1 = n / 2, nb2 = n - nb1;
-    auto put = [&](size_t to, size_t from) {
-        double f = 0, fq = 0;
-        if (fp64) fp::factor(w[from], q, f, fq);
-        out[to] = fp64 ? TwPair{fp::double_bits(f), fp::double_bits(fq)} : TwPair{w[from], ws[from]};
-    };
-    for (size_t i = 0; i < ((size_t)1 << nb1); ++i) put(i, i);
-    for (int kr = 0; kr < nb2; ++kr) {
-        const size_t stage = (size_t)1 << (nb1 + kr);
-        for (size_t i = 0; i < stage; ++i) {
-            const size_t row = i >> kr, x = i & (((size_t)1 << kr) - 1);
-            put(stage + (row << kr) + row_order(nb2, eb, nb2 - 1 - kr, x), stage + i);
-        }
-    }
+// The place of twiddle i of a ring of 2^n in the table of the geometries of 2^eb residues per thread: rows
+// in row_order.
+WG_HD size_t twiddle_place(int n, int eb, size_t i) {
+    const int nb1 = n / 2, nb2 = n - nb1;
+    if (i < ((size_t)1 << nb1)) return i;
+    const int kr = floor_log2((unsigned)i) - nb1;
+    const size_t stage = (size_t)1 << (nb1 + kr), row = (i - stage) >> kr, x = i & (((size_t)1 << kr) - 1);
+    return stage + (row << kr) + row_order(nb2, eb, nb2 - 1 - kr, x);
+}
+
+// An entry of a modulus's table from its split (w, Shoup w) words: the factor pair (w, w / q) as bits of
+// doubles for the moduli of the FP64 path (unless `words`), the words otherwise.
+WG_HD TwPair twiddle_pair(uint64_t w, uint64_t ws, uint64_t q, bool words) {
+    if (q >= fp::kLimit || words) return TwPair{w, ws};
+    double f, fq;
+    fp::factor(w, q, f, fq);
+    return TwPair{fp::double_bits(f), fp::double_bits(fq)};
 }
 
 }  // namespace ntt

@@ -44,6 +44,13 @@ struct Emu {
     std::vector<ntt::TwPair> tw;  // twiddle pairs of every modulus: [mod][fwd N, inv N]
 };
 
+// A modulus's table of one direction as the device makes it (k_twiddles_8, k_twiddles_16), from its split
+// words (w at i, its Shoup companion at N + i).
+void twiddle_table(int logN, uint64_t q, const uint64_t* w, int eb, ntt::TwPair* out) {
+    const size_t N = (size_t)1 << logN;
+    for (size_t i = 0; i < N; ++i) out[ntt::twiddle_place(logN, eb, i)] = ntt::twiddle_pair(w[i], w[N + i], q, false);
+}
+
 // The rounds of one phase over a CTA: v[t] are thread t's elements, exchanged through the padded tile
 // where the kernels do (ntt_round, wg_ntt.cu).
 template <class Arith, int E>
@@ -102,7 +109,7 @@ void phase(const Emu& E, uint64_t* x, int mi, bool epilogue) {
     const size_t N = P::N;
     std::vector<ntt::TwPair> table(N);
     const uint64_t* w = E.H.tw.data() + ((size_t)mi * 4 + (FWD ? 0 : 2)) * N;
-    ntt::twiddle_pairs(N, E.H.mods[mi].q, w, w + N, EB, false, table.data());
+    twiddle_table(E.logN, E.H.mods[mi].q, w, EB, table.data());
     const ntt::TwPair* tw = table.data();
     const Modulus& md = E.H.mods[mi];
     const bool fp64 = md.q < fp::kLimit, lazy = FWD && md.q < ntt::kLazyForwardLimit;
@@ -473,7 +480,7 @@ void* emu_create(uint64_t N, const uint64_t* q, size_t nq, const uint64_t* p, si
     for (size_t m = 0; m < nq + np; ++m)
         for (size_t dir = 0; dir < 2; ++dir) {
             const uint64_t* w = E->H.tw.data() + (m * 4 + 2 * dir) * N;
-            ntt::twiddle_pairs(N, E->H.mods[m].q, w, w + N, 3, false, E->tw.data() + (m * 2 + dir) * N);
+            twiddle_table(E->logN, E->H.mods[m].q, w, 3, E->tw.data() + (m * 2 + dir) * N);
         }
     return E;
 }
