@@ -121,16 +121,9 @@ int split_of(const Context& c, int njobs, int tiles, int resident, int sources, 
     const int most = (2 * outputs + sources - 1) / std::max(1, sources);
     return std::max(1, std::min({room, most, outputs}));
 }
-// The outputs begin, begin + step, ... of a block: gridDim.x = TILES * split.  (Every step-th and not
-// a run, so that the word moduli, which cost several times an FP64 one and stand together at the end,
-// spread over the blocks.)
-struct Share {
-    int tile, begin, step;
-};
 template <class G>
 __device__ __forceinline__ Share block_share() {
-    constexpr int tiles = G::TILES;
-    return {(int)(blockIdx.x % tiles), (int)(blockIdx.x / tiles), (int)(gridDim.x / tiles)};
+    return share_of(blockIdx.x, gridDim.x, G::TILES);
 }
 
 // Block (tile and share of the outputs, job): one digit's column tile.

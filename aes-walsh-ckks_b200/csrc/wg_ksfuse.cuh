@@ -76,6 +76,16 @@ struct Geom {
     static_assert(Fwd::TILE == Inv::TILE && Fwd::THREADS == Inv::THREADS, "one tile shape for both directions");
 };
 
+// The column tile of block `x` of a job's `blocks` = TILES * split and the outputs begin, begin + step, ...
+// it makes.  (Every step-th and not a run, so that the word moduli, which cost several times an FP64
+// one and stand together at the end, spread over the blocks.)
+struct Share {
+    int tile, begin, step;
+};
+WG_HD Share share_of(unsigned x, unsigned blocks, unsigned tiles) {
+    return {(int)(x % tiles), (int)(x / tiles), (int)(blocks / tiles)};
+}
+
 // Offset in the limb of thread t's element 0 in a round; element k is limb_step(k) further.
 template <class R>
 WG_HD size_t limb_offset(int tile, int t) {

@@ -90,13 +90,6 @@ __device__ __forceinline__ void store_words(uint64_t* __restrict__ p, const uint
     }
 }
 
-// Words of a word-arithmetic limb on their way out of its last phase.
-__device__ __forceinline__ uint64_t word_store(bool last, bool fwd, uint64_t v, const Modulus& m) {
-    if (!last) return v;
-    if (!fwd) return mul_shoup(v, m.n_inv, m.n_inv_shoup, m.q);
-    return m.q < kLazyForwardLimit ? reduce64(v, m) : red4q(v, m.q);
-}
-
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED>
 constexpr size_t smem_bytes() {
     using P = Phase<LOGN, FWD, COLS, EB, STAGED>;
@@ -463,118 +456,57 @@ struct RowsMac {
     static constexpr auto rounds() { return std::make_integer_sequence<int, P::ROUNDS>{}; }
     static constexpr size_t smem() { return 8 * (size_t)(P::TILE + P::TILE / 16); }
 };
-// One switch in FP64: |transformed word| <= 27 q where the modulus needs no reduction (FpArith), so its
-// product with a key word (key_factor) has |a wq| < 2^47.
-template <int LOGN>
-__device__ __forceinline__ void rows_mac_fp(uint64_t* sm, const MacGroupJob* j, int c, const Modulus& m, bool rows,
-                                            size_t at, size_t key_at, size_t key_stride, int own_part, size_t T, int tile,
-                                            int sub, int o, const TwPair* tw) {
+// One switch (c) of a job: Sums is the modulus's arithmetic (MacSumsFp, MacSumsWords), `fwd` and `inv` the
+// rounds' (FP64: one for both).  AHEAD: the next digit is loaded before the products with this one's key words.
+template <int LOGN, bool AHEAD, class Sums, class Fwd, class Inv>
+__device__ __forceinline__ void rows_mac(uint64_t* sm, const MacGroupJob* j, int c, const Modulus& m, bool rows,
+                                         size_t at, size_t key_at, size_t key_stride, int own_part, size_t T, int tile,
+                                         int sub, int o, const TwPair* tw, const Fwd& fwd, const Inv& inv) {
     using R = RowsMac<LOGN>;
     const size_t N = R::P::N;
     const int eb = R::Begin::element(sub, o), ee = R::End::element(sub, o), parts = j->parts;
-    const uint64_t* digits = j->digits[c] + at;
-    const uint64_t* own = j->key_term[c] + at + ee;
-    const bool red = m.q >= fp::kNoReduce;
-    uint64_t w[8];
+    uint64_t w[8], k8[8];
     auto fetch = [&](int p) {
         if (p == own_part)
-            load_words<typename R::End>(own, w);
-        else
-            load_words<typename R::Begin>(digits + p * j->part_stride + eb, w);
-    };
-    double sa[8], sb[8], v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) sa[k] = sb[k] = 0.0;
-    fetch(0);
-    for (int p = 0; p < parts; ++p) {
-        if (p == own_part) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = fp::from_word(w[k]);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = fp::bits_double(w[k]);
-            ntt_rounds<LOGN, true, false, 3, false, kMaxTile>(R::rounds(), sm, v, sub, o, tile, fp_arith(m), tw);
-            if (red) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = fp::reduce(v[k], m.qd, m.inv_q);
-            }
-        }
-        if (p + 1 < parts) fetch(p + 1);
-        uint64_t k8[8];
-        const uint64_t* key = j->key + p * 2 * key_stride + key_at + ee;
-        load_words<typename R::End>(key, k8);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const fp::Factor f = fp::key_factor(k8[k], m.inv_q);
-            sa[k] = fp::mont_sum_bound(dadd(sa[k], fp::mulmod(v[k], f.w, f.wq, m.qd)), p, m);
-        }
-        load_words<typename R::End>(key + key_stride, k8);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const fp::Factor f = fp::key_factor(k8[k], m.inv_q);
-            sb[k] = fp::mont_sum_bound(dadd(sb[k], fp::mulmod(v[k], f.w, f.wq, m.qd)), p, m);
-        }
-    }
-#pragma unroll
-    for (int poly = 0; poly < 2; ++poly) {
-        double* s = poly ? sb : sa;
-        uint64_t* out = j->acc[c] + poly * T * N + at;
-        if (rows) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) s[k] = fp::mont_sum_value(s[k], m);
-            ntt_rounds<LOGN, false, false, 3, false, kMaxTile>(R::rounds(), sm, s, sub, o, tile, fp_arith(m), tw + N);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) w[k] = fp_store(false, false, fp::double_bits(s[k]), m);
-            store_words<typename R::InvEnd>(out + R::InvEnd::element(sub, o), w);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) w[k] = fp::mont_sum_word(s[k], m);
-            store_words<typename R::End>(out + ee, w);
-        }
-    }
-}
-// The same in words.
-template <int LOGN, bool LAZY>
-__device__ __forceinline__ void rows_mac_words(uint64_t* sm, const MacGroupJob* j, int c, const Modulus& m, bool rows,
-                                               size_t at, size_t key_at, size_t key_stride, int own_part, size_t T,
-                                               int tile, int sub, int o, const TwPair* tw) {
-    using R = RowsMac<LOGN>;
-    const size_t N = R::P::N;
-    const int eb = R::Begin::element(sub, o), ee = R::End::element(sub, o), parts = j->parts;
-    WideSum sa[8], sb[8];
-    uint64_t w[8], k8[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        sa[k].clear();
-        sb[k].clear();
-    }
-    for (int p = 0; p < parts; ++p) {
-        if (p == own_part) {
             load_words<typename R::End>(j->key_term[c] + at + ee, w);
-        } else {
+        else
             load_words<typename R::Begin>(j->digits[c] + p * j->part_stride + at + eb, w);
-            ntt_rounds<LOGN, true, false, 3, false, kMaxTile>(R::rounds(), sm, w, sub, o, tile, WordArith<LAZY>{m.q}, tw);
+    };
+    Sums sums;
+    sums.clear();
+    typename Sums::V v[8];
+    if (AHEAD) fetch(0);
+    for (int p = 0; p < parts; ++p) {
+        if (!AHEAD) fetch(p);
+        if (p == own_part) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) w[k] = word_store(true, true, w[k], m);
+            for (int k = 0; k < 8; ++k) v[k] = Sums::own(w[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = Sums::digit(w[k]);
+            ntt_rounds<LOGN, true, false, 3, false, kMaxTile>(R::rounds(), sm, v, sub, o, tile, fwd, tw);
+            Sums::transformed(v, m);
         }
+        if (AHEAD && p + 1 < parts) fetch(p + 1);
         const uint64_t* key = j->key + p * 2 * key_stride + key_at + ee;
         load_words<typename R::End>(key, k8);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sa[k].add(w[k], k8[k], m);
+        sums.add(0, v, k8, p, m);
         load_words<typename R::End>(key + key_stride, k8);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sb[k].add(w[k], k8[k], m);
+        sums.add(1, v, k8, p, m);
     }
 #pragma unroll
     for (int poly = 0; poly < 2; ++poly) {
         uint64_t* out = j->acc[c] + poly * T * N + at;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] = (poly ? sb[k] : sa[k]).mont_value(m);
         if (rows) {
-            ntt_rounds<LOGN, false, false, 3, false, kMaxTile>(R::rounds(), sm, w, sub, o, tile, WordArith<false>{m.q},
-                                                              tw + N);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = sums.value(poly, k, m);
+            ntt_rounds<LOGN, false, false, 3, false, kMaxTile>(R::rounds(), sm, v, sub, o, tile, inv, tw + N);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = Sums::row_word(v[k], m);
             store_words<typename R::InvEnd>(out + R::InvEnd::element(sub, o), w);
         } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = sums.word(poly, k, m);
             store_words<typename R::End>(out + ee, w);
         }
     }
@@ -600,12 +532,17 @@ __global__ void __launch_bounds__(RowsMac<LOGN>::P::THREADS, 2)
     const int own_part = is_p ? -1 : i / j->alpha, sub = P::sub_of(t), o = P::o_of(t);
     const size_t T = L + K;
     for (int c = 0; c < j->n; ++c) {
-        if (!WORDS || m.q < fp::kLimit)
-            rows_mac_fp<LOGN>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw);
-        else if (m.q < kLazyForwardLimit)
-            rows_mac_words<LOGN, true>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw);
-        else
-            rows_mac_words<LOGN, false>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw);
+        if (!WORDS || m.q < fp::kLimit) {
+            const FpArith ar = fp_arith(m);
+            rows_mac<LOGN, true, MacSumsFp>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw, ar, ar);
+        } else if (m.q < kLazyForwardLimit) {
+            rows_mac<LOGN, false, MacSumsWords>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw,
+                                                WordArith<true>{m.q}, WordArith<false>{m.q});
+        } else {
+            const WordArith<false> ar{m.q};
+            rows_mac<LOGN, false, MacSumsWords>(smem, j, c, m, is_p, at, key_at, key_stride, own_part, T, tile, sub, o, tw, ar,
+                                                ar);
+        }
     }
 }
 

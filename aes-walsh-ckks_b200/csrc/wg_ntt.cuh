@@ -337,6 +337,71 @@ WG_HD void ntt_epilogue(const NttEpiJob& j, size_t off, uint64_t v, uint64_t q) 
     j.out[off] = epilogue_value(j, acc, in, v, q);
 }
 
+// Words of a word-arithmetic limb on their way out of its last phase.
+WG_HD uint64_t word_store(bool last, bool fwd, uint64_t v, const Modulus& m) {
+    if (!last) return v;
+    if (!fwd) return mul_shoup(v, m.n_inv, m.n_inv_shoup, m.q);
+    return m.q < kLazyForwardLimit ? reduce64(v, m) : red4q(v, m.q);
+}
+
+// Key products on 8 coefficients of a thread, between the rounds of k_rows_mac (wg_ntt.cu): `own` and
+// `digit` take a key-term word and a digit's word before its row phase, `transformed` what its rounds
+// leave, `add` the products with the key words of one of the two polynomials; `value` is the sum as
+// the inverse row phase starts from it and `row_word` a word that phase ends with, `words` the
+// canonical sum.
+// FP64: |transformed word| <= 27 q where the modulus needs no reduction (FpArith), so its product with a
+// key word (key_factor) has |a wq| < 2^47.
+struct MacSumsFp {
+    using V = double;
+    double s[2][8];
+    WG_HD void clear() {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[0][k] = s[1][k] = 0.0;
+    }
+    WG_HD static V own(uint64_t w) { return fp::from_word(w); }
+    WG_HD static V digit(uint64_t w) { return fp::bits_double(w); }
+    WG_HD static void transformed(V* v, const Modulus& m) {
+        if (m.q < fp::kNoReduce) return;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = fp::reduce(v[k], m.qd, m.inv_q);
+    }
+    WG_HD void add(int poly, const V* v, const uint64_t* key, int part, const Modulus& m) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const fp::Factor f = fp::key_factor(key[k], m.inv_q);
+            s[poly][k] = fp::mont_sum_bound(dadd(s[poly][k], fp::mulmod(v[k], f.w, f.wq, m.qd)), part, m);
+        }
+    }
+    WG_HD V value(int poly, int k, const Modulus& m) const { return fp::mont_sum_value(s[poly][k], m); }
+    WG_HD static uint64_t row_word(V v, const Modulus& m) { return fp_store(false, false, fp::double_bits(v), m); }
+    WG_HD uint64_t word(int poly, int k, const Modulus& m) const { return fp::mont_sum_word(s[poly][k], m); }
+};
+// The same in words.
+struct MacSumsWords {
+    using V = uint64_t;
+    WideSum s[2][8];
+    WG_HD void clear() {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            s[0][k].clear();
+            s[1][k].clear();
+        }
+    }
+    WG_HD static V own(uint64_t w) { return w; }
+    WG_HD static V digit(uint64_t w) { return w; }
+    WG_HD static void transformed(V* v, const Modulus& m) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = word_store(true, true, v[k], m);
+    }
+    WG_HD void add(int poly, const V* v, const uint64_t* key, int, const Modulus& m) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[poly][k].add(v[k], key[k], m);
+    }
+    WG_HD V value(int poly, int k, const Modulus& m) const { return s[poly][k].mont_value(m); }
+    WG_HD static uint64_t row_word(V v, const Modulus&) { return v; }
+    WG_HD uint64_t word(int poly, int k, const Modulus& m) const { return s[poly][k].mont_value(m); }
+};
+
 // Global offset (within one limb) of tile element e.
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, int TL = kMaxTile>
 WG_HD size_t tile_offset(int tile, int e) {

@@ -93,11 +93,7 @@ void tile_phase(uint64_t* x, int tile, const Arith& ar, const ntt::TwPair* tw, I
     }
 }
 
-uint64_t word_store(bool last, bool fwd, uint64_t v, const Modulus& m) {
-    if (!last) return v;
-    if (!fwd) return mul_shoup(v, m.n_inv, m.n_inv_shoup, m.q);
-    return m.q < ntt::kLazyForwardLimit ? reduce64(v, m) : red4q(v, m.q);
-}
+using ntt::word_store;
 
 // NTT geometry the emulated phases use (the device's kNttGeometries order: 0 = 8 residues per
 // thread, staged twiddles; 1 = 8, table; 2 = 16, staged; 3 = 16, table).
@@ -167,7 +163,8 @@ void ntt_one(const Emu& E, uint64_t* x, int mi, bool fwd) {
     }
 }
 
-// Key switches and rescales run the fused sequences of wg_ksfuse.cu (Context::ntt_fusion).
+// Key switches and rescales run the fused sequences of wg_ksfuse.cu (Context::ntt_fusion), each job's
+// outputs over g_fused blocks a column tile (split_of).
 int g_fused = 0;
 
 bool is_fp(const Emu& E, int mi) { return E.H.mods[mi].q < fp::kLimit; }
@@ -237,7 +234,9 @@ template <class G>
 void modup_fused_g(const Emu& E, const HostModUp& d, const uint64_t* src, uint64_t* digit) {
     const int n = d.src_count;
     std::vector<uint64_t> slots((size_t)n * G::TILE);
-    for (int tile = 0; tile < G::TILES; ++tile) {
+    for (int block = 0; block < G::TILES * g_fused; ++block) {
+        const ksf::Share sh = ksf::share_of(block, G::TILES * g_fused, G::TILES);
+        const int tile = sh.tile;
         std::vector<double> alpha((size_t)G::THREADS * G::E, 0.0);
         ksf::SourceKinds kinds;
         for (int i = 0; i < n; ++i) {
@@ -256,7 +255,7 @@ void modup_fused_g(const Emu& E, const HostModUp& d, const uint64_t* src, uint64
         }
         std::vector<uint32_t> hps((size_t)G::THREADS * G::E);
         for (size_t k = 0; k < hps.size(); ++k) hps[k] = ksf::hps_count(alpha[k], n);
-        for (int dst = 0; dst < d.dst_count; ++dst) {
+        for (int dst = sh.begin; dst < d.dst_count; dst += sh.step) {
             const int mi = d.dst_mod[dst];
             const Modulus& m = E.H.mods[mi];
             forward_limb<G>(
@@ -290,7 +289,9 @@ void moddown_fused(const Emu& E, const uint64_t* src_p, uint64_t* out, int L, co
     std::vector<uint64_t> slots((size_t)K * G::TILE);
     ksf::SourceKinds kinds;
     for (int pi = 0; pi < K; ++pi) kinds.set(pi, pmods[pi].q);
-    for (int tile = 0; tile < G::TILES; ++tile) {
+    for (int block = 0; block < G::TILES * g_fused; ++block) {
+        const ksf::Share sh = ksf::share_of(block, G::TILES * g_fused, G::TILES);
+        const int tile = sh.tile;
         for (int pi = 0; pi < K; ++pi) {
             const Modulus& m = pmods[pi];
             uint64_t* sl = slots.data() + (size_t)pi * G::TILE;
@@ -302,7 +303,7 @@ void moddown_fused(const Emu& E, const uint64_t* src_p, uint64_t* out, int L, co
         std::vector<uint32_t> hps((size_t)G::THREADS * G::E);
         for (int t = 0; t < G::THREADS; ++t)
             ksf::moddown_hps<G>(slots.data(), t, pmods, K, hps.data() + (size_t)t * G::E, kinds.fp64);
-        for (int qi = 0; qi < L; ++qi) {
+        for (int qi = sh.begin; qi < L; qi += sh.step) {
             const Modulus& m = E.H.mods[qi];
             const uint64_t *iv = inv + (size_t)qi * K, *ivs = inv_s + (size_t)qi * K;
             forward_limb<G>(
@@ -315,6 +316,81 @@ void moddown_fused(const Emu& E, const uint64_t* src_p, uint64_t* out, int L, co
                     ksf::moddown_value<G>(v, slots.data(), t, K, m.q, iv, ivs, hps.data() + (size_t)t * G::E, kinds.fp64);
                 });
         }
+    }
+}
+
+// k_rows_mac for one switch: QP limb i of both accumulators from the digits as the fused ModUp leaves
+// them (key limb klimb of key_limbs).
+template <int LOGN, class Sums, class Fwd, class Inv>
+void rows_mac_limb(const Emu& E, const Modulus& m, int mi, int parts, int own_part, const uint64_t* key_term,
+                   const uint64_t* digits, size_t part_stride, const uint64_t* key, size_t key_stride, uint64_t* acc_a,
+                   uint64_t* acc_b, bool rows, const Fwd& fwd, const Inv& inv) {
+    using P = ntt::Phase<LOGN, true, false, 3, false>;
+    using Begin = ntt::Round<LOGN, true, false, 3, false, 0>;
+    using End = ntt::Round<LOGN, true, false, 3, false, P::ROUNDS - 1>;
+    using InvEnd = ntt::Round<LOGN, false, false, 3, false, P::ROUNDS - 1>;
+    constexpr auto all = std::make_integer_sequence<int, P::ROUNDS>{};
+    const ntt::TwPair* tw = E.tw.data() + (size_t)mi * 2 * P::N;
+    std::vector<uint64_t> sm(P::TILE + P::TILE / 16);
+    for (int tile = 0; tile < P::N / P::TILE; ++tile) {
+        const size_t at = (size_t)tile * P::TILE;
+        std::vector<Sums> sums(P::THREADS);
+        for (auto& s : sums) s.clear();
+        Lanes<Fwd, 8> v(P::THREADS);
+        auto element = [&](auto round, int t) { return at + decltype(round)::element(P::sub_of(t), P::o_of(t)); };
+        for (int p = 0; p < parts; ++p) {
+            const uint64_t* d = digits + p * part_stride;
+            for (int t = 0; t < P::THREADS; ++t)
+                for (int k = 0; k < 8; ++k)
+                    v[t][k] = p == own_part ? Sums::own(key_term[element(End{}, t) + End::limb_step(k)])
+                                            : Sums::digit(d[element(Begin{}, t) + Begin::limb_step(k)]);
+            if (p != own_part) {
+                rounds<LOGN, true, false, 3, false, ntt::kMaxTile>(all, sm.data(), v, tile, fwd, tw);
+                for (auto& x : v) Sums::transformed(x.data(), m);
+            }
+            for (int t = 0; t < P::THREADS; ++t)
+                for (int poly = 0; poly < 2; ++poly) {
+                    uint64_t k8[8];
+                    for (int k = 0; k < 8; ++k)
+                        k8[k] = key[(2 * p + poly) * key_stride + element(End{}, t) + End::limb_step(k)];
+                    sums[t].add(poly, v[t].data(), k8, p, m);
+                }
+        }
+        for (int poly = 0; poly < 2; ++poly) {
+            uint64_t* out = poly ? acc_b : acc_a;
+            if (rows) {
+                for (int t = 0; t < P::THREADS; ++t)
+                    for (int k = 0; k < 8; ++k) v[t][k] = sums[t].value(poly, k, m);
+                rounds<LOGN, false, false, 3, false, ntt::kMaxTile>(all, sm.data(), v, tile, inv, tw + P::N);
+                for (int t = 0; t < P::THREADS; ++t)
+                    for (int k = 0; k < 8; ++k)
+                        out[element(InvEnd{}, t) + InvEnd::limb_step(k)] = Sums::row_word(v[t][k], m);
+            } else {
+                for (int t = 0; t < P::THREADS; ++t)
+                    for (int k = 0; k < 8; ++k) out[element(End{}, t) + End::limb_step(k)] = sums[t].word(poly, k, m);
+            }
+        }
+    }
+}
+template <int LOGN>
+void rows_mac(const Emu& E, size_t L, size_t B, const uint64_t* key, size_t key_level, const uint64_t* key_term,
+              const uint64_t* digits, uint64_t* acc) {
+    const size_t N = E.H.N, K = E.H.np, T = L + K;
+    for (size_t i = 0; i < T; ++i) {
+        const bool rows = i >= L;
+        const int mi = (int)(rows ? E.H.nq + i - L : i), own = rows ? -1 : (int)(i / E.H.alpha);
+        const size_t klimb = rows ? key_level + 1 + (i - L) : i, stride = (key_level + 1 + K) * N;
+        const Modulus& m = E.H.mods[mi];
+        auto run = [&](auto sums, const auto& fwd, const auto& inv) {
+            rows_mac_limb<LOGN, decltype(sums)>(E, m, mi, (int)B, own, key_term + (rows ? 0 : i * N), digits + i * N, T * N,
+                                               key + klimb * N, stride, acc + i * N, acc + (T + i) * N, rows, fwd, inv);
+        };
+        if (is_fp(E, mi))
+            run(ntt::MacSumsFp{}, ntt::fp_arith(m), ntt::fp_arith(m));
+        else if (m.q < ntt::kLazyForwardLimit)
+            run(ntt::MacSumsWords{}, ntt::WordArith<true>{m.q}, ntt::WordArith<false>{m.q});
+        else
+            run(ntt::MacSumsWords{}, ntt::WordArith<false>{m.q}, ntt::WordArith<false>{m.q});
     }
 }
 
@@ -343,12 +419,14 @@ void rescale_fused(const Emu& E, const uint64_t* drop, uint64_t* rem, int lv, co
     using G = ksf::Geom<LOGN, ksf::kRescaleBits>;
     std::vector<uint64_t> slots(G::TILE);
     const Modulus& mp = E.H.mods[lv];
-    for (int tile = 0; tile < G::TILES; ++tile) {
+    for (int block = 0; block < G::TILES * g_fused; ++block) {
+        const ksf::Share sh = ksf::share_of(block, G::TILES * g_fused, G::TILES);
+        const int tile = sh.tile;
         load_slots<G>(slots.data(), drop, tile);
         inverse_slots<G>(
             E, slots.data(), tile, lv, [&](double* v, int) { ksf::scale_fp<G::E>(v, mp.n_inv_w, mp.n_inv_wq, mp.qd); },
             [&](uint64_t* v, int) { ksf::scale_n_inv<G::E>(v, mp); });
-        for (int qi = 0; qi < lv; ++qi) {
+        for (int qi = sh.begin; qi < lv; qi += sh.step) {
             const Modulus& m = E.H.mods[qi];
             forward_limb<G>(
                 E, rem + (size_t)qi * G::N, tile, qi,
@@ -529,7 +607,7 @@ void emu_keyswitch(void* h, size_t level, const uint64_t* key_term, const uint64
     const Modulus* mods = E.H.mods.data();
     std::memcpy(coeff, key_term, L * N * 8);
     if (g_fused) {
-        // inverse row phase, fused [inverse columns, ModUp, forward columns], forward row phase
+        // inverse row phase, fused [inverse columns, ModUp, forward columns]
         for (size_t l = 0; l < L; ++l) EMU_LOGN_SWITCH(E.logN, phase_one<LG>(E, coeff + l * N, (int)l, false, false));
         for (size_t j = 0; j < B; ++j)
             EMU_LOGN_SWITCH(E.logN, modup_fused<LG>(E, E.modup[level][j], coeff, digits + j * T * N));
@@ -538,26 +616,22 @@ void emu_keyswitch(void* h, size_t level, const uint64_t* key_term, const uint64
         for (size_t j = 0; j < B; ++j)
             for (size_t c = 0; c < N; ++c) modup_coeff(E.modup[level][j], mods, coeff, digits + j * T * N, N, c);
     }
-    for (size_t j = 0; j < B; ++j) {
-        const size_t s0 = j * alpha, s1 = std::min(s0 + alpha, L);
-        for (size_t l = 0; l < T; ++l) {
-            if (l >= s0 && l < s1) continue;
-            const int mi = (int)(l < L ? l : nq + (l - L));
-            if (g_fused)
-                EMU_LOGN_SWITCH(E.logN, phase_one<LG>(E, digits + j * T * N + l * N, mi, true, false));
-            else
-                ntt_one(E, digits + j * T * N + l * N, mi, true);
+    if (g_fused) {
+        // fused [forward row phase, key product, inverse row phase of the P limbs]
+        EMU_LOGN_SWITCH(E.logN, rows_mac<LG>(E, L, B, key, key_level, key_term, digits, acc));
+    } else {
+        for (size_t j = 0; j < B; ++j) {
+            const size_t s0 = j * alpha, s1 = std::min(s0 + alpha, L);
+            for (size_t l = 0; l < T; ++l)
+                if (l < s0 || l >= s1) ntt_one(E, digits + j * T * N + l * N, (int)(l < L ? l : nq + (l - L)), true);
         }
+        for (size_t i = 0; i < T; ++i)
+            for (size_t c = 0; c < N; ++c)
+                mac_coeff(mods, (int)nq, (int)L, (int)K, (int)B, (int)alpha, key, (int)key_level, key_term, digits, T * N,
+                          acc, N, (int)i, c);
     }
-    for (size_t i = 0; i < T; ++i)
-        for (size_t c = 0; c < N; ++c)
-            mac_coeff(mods, (int)nq, (int)L, (int)K, (int)B, (int)alpha, key, (int)key_level, key_term, digits, T * N,
-                      acc, N, (int)i, c);
     const uint64_t* W = E.H.words.data();
     if (g_fused) {
-        for (int poly = 0; poly < 2; ++poly)
-            for (size_t pi = 0; pi < K; ++pi)
-                EMU_LOGN_SWITCH(E.logN, phase_one<LG>(E, acc + (poly * T + L + pi) * N, (int)(nq + pi), false, false));
         for (int poly = 0; poly < 2; ++poly)
             EMU_LOGN_SWITCH(E.logN, moddown_fused<LG>(E, acc + (poly * T + L) * N, contrib + poly * L * N, (int)L,
                                                       W + E.H.fold_inv[level], W + E.H.fold_inv_s[level],

@@ -42,13 +42,14 @@ def emu(tmp_path_factory):
 MANY_DIGITS = dict(logN=10, q_bits=[40, 45, 45, 45, 50, 50, 50, 50], p_bits=[55], dnum=8, h=64)
 
 
-@pytest.mark.parametrize("fused", [0, 1])
+@pytest.mark.parametrize("fused", [0, 1, 3])
 @pytest.mark.parametrize("prm", SMALL + [MANY_DIGITS])
 def test_emulated_kernels_match_oracle(oracle_mod, emu, prm, fused):
     """NTT, key switch (rotation, relinearisation) and rescale at three levels; fused = 1 runs
     them as the device does by default: ModUp, ModDown and the rescale remainders inside the NTT
-    column phases (wg_ksfuse.cuh), the combine and the rescale finish as the epilogue of the last
-    row phase."""
+    column phases (wg_ksfuse.cuh), the digits' row phase, the key product and the P limbs' row phase
+    as one step, the combine and the rescale finish as the epilogue of the last row phase; fused = 3
+    with each job's outputs divided over three blocks, as small launches do."""
     O = oracle_mod
     N = 1 << prm["logN"]
     p, q = O.find_primes(prm["p_bits"], prm["q_bits"], N)

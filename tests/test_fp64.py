@@ -187,7 +187,7 @@ def test_emulated_mixed_key_switches(oracle_mod, emu, prm):  # noqa: F811
     try:
         L = len(q)
         rk = o.rotation_key(o.ternary(64, 3), 3, 11)
-        for fused in (0, 1):
+        for fused in (0, 1, 2):  # 2: each job's outputs divided over two blocks
             emu.emu_set_keyswitch_fusion(fused)
             for level in (L - 1, L // 2, 1):
                 b, a = o.uniform(level + 1, 9), o.uniform(level + 1, 10)
