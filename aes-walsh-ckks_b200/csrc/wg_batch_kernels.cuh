@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kT) kb_mac(const MacJob* jobs, int n, const Mo
 // group, parts accumulated in order as in mac_accumulate (wg_keyswitch.cuh).  NC is a compile-time
 // count so that every digit load of a part is unconditional and all of them are in flight at once;
 // a group of more than kMacPass switches takes two passes, the second finding the key words in L1,
-// which keeps the sums in 64 registers and four blocks on an SM.
+// which keeps the FP64 sums in the 64 registers of four blocks an SM (the integer sums of word moduli
+// spill a few of theirs; two blocks an SM without spills, or two switches a pass, were not tried).
 // FP: the modulus is below fp::kLimit and the sums run in FP64 (mac_words_fp); 16 FP64 instructions
 // per part and switch against two Montgomery products, which leaves the kernel to its loads.  Larger
 // moduli sum their products as integers and reduce once (WideSum).

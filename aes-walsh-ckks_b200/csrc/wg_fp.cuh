@@ -67,8 +67,9 @@ WG_HD double mulmod(double a, double w, double wq, double q) {
     return dadd(dfma(-k, q, h), l);
 }
 
-// The representative of x nearest zero, |x| <= 2^53 (|result| <= q / 2 up to the rounding of
-// x inv_q, far below one part in 2^30 for the |x| <= 2^11 q the callers pass).
+// The representative of an integer x nearest zero, |x| <= 2^53 and q >= 4: |x inv_q| <= 2^51 rounds to an
+// integer as above, inv_q is off by at most 2^-53 of itself and so the quotient by at most 2^-53 |x / q| <= 1 / q
+// before its rounding: |result| <= q / 2 + 1, and the subtraction is exact.
 WG_HD double reduce(double x, double q, double inv_q) {
     const double k = dadd(dfma(x, inv_q, kRound), -kRound);
     return dfma(-k, q, x);

@@ -102,8 +102,9 @@ __device__ __forceinline__ void forward_limb(uint64_t* sm, uint64_t* limb, int t
 }
 
 // Shared memory: the sources' slots (TILE words each), then the exchange tile.  Four blocks an SM: up to
-// five sources (50 KB) leave room for them, and four residues a thread take 64 registers, eight 128.  A
-// rescale has one source and takes 80 registers.
+// five sources (50 KB) leave room for them, and four residues a thread take 64 registers, eight 128 (with
+// more sources fewer blocks fit, and split_of, which counts four, divides a small launch further than one
+// wave).  A rescale has one source and takes 80 registers.
 constexpr int kResident = 4;
 constexpr int kRescaleResident = 6;
 template <class G>

@@ -239,7 +239,7 @@ struct SumFp {
     }
     WG_HD void add(const uint64_t* slots, int t, bool fp64, bool wide, ntt::TwPair f, uint64_t w, uint64_t ws, int term,
                    const Modulus& m) {
-            const double f0 = fp::bits_double(f.w), f1 = fp::bits_double(f.ws);
+        const double f0 = fp::bits_double(f.w), f1 = fp::bits_double(f.ws);
         const bool dot = m.q < fp::kNoReduce;
         slots += t;
         if (fp64 && dot && !wide) {
@@ -287,8 +287,8 @@ WG_HD void modup_value_fp(double* v, const uint64_t* src, int t, const Desc& d, 
     for (int k = 0; k < G::E; ++k) sum.start(k, -fp::from_word(WG_LDG(corr + hps[k])));
     for (int i = 0; i < n; ++i) {
         const size_t at = (size_t)dst * n + i;
-        sum.add(src + i * G::TILE, t, kinds.fp64 >> i & 1, kinds.wide >> i & 1, d.qhat_fp[at], d.qhat[at],
-                      d.qhat_s[at], i, m);
+        sum.add(src + i * G::TILE, t, kinds.fp64 >> i & 1, kinds.wide >> i & 1, d.qhat_fp[at], d.qhat[at], d.qhat_s[at], i,
+                m);
     }
     sum.finish(v, m);
 }

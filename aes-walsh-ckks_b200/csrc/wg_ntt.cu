@@ -13,8 +13,9 @@
 //     round, from device memory into the first round and from the last one back;
 //   * between rounds the CTA exchanges them in shared memory with one pad word every 16 words, so
 //     strided 64-bit accesses stay at two wavefronts per warp;
-//   * twiddles come as (w, Shoup w) pairs, one 16-byte load each, either staged in shared
-//     memory per CTA or read from the L2-resident table directly (the geometry's STAGED);
+//   * twiddles come as pairs (w, Shoup w), or (w, w / q) for the FP64 moduli below, one 16-byte load
+//     each, either staged in shared memory per CTA or read from the L2-resident table directly
+//     (the geometry's STAGED);
 //   * grid.y indexes limbs and grid.z polynomials, so one launch covers a whole ciphertext
 //     batch; each limb picks its modulus through a LimbMap (Q limbs, P limbs or a mix).
 // Moduli below 2^50 (fp::kLimit) run in FP64: signed integers in doubles, exact products through
@@ -96,12 +97,8 @@ constexpr size_t smem_bytes() {
     return 8 * (size_t)(P::TILE + P::TILE / 16) + (STAGED ? 16 * (size_t)P::TW : 0);
 }
 
-// Registers: 8-residue rounds fit 64 registers (4 CTAs of 256 threads per SM); 16-residue
-// rounds get up to 128 (4 CTAs of 128 threads).
-template <int EB>
-constexpr int min_blocks() {
-    return 4;
-}
+// CTAs per SM: 8-residue rounds fit 64 registers (256 threads), 16-residue ones get up to 128 (128 threads).
+constexpr int kMinBlocks = 4;
 
 // The twiddle pairs a CTA reads, copied to shared memory in twiddle_src order.
 template <int LOGN, bool FWD, bool COLS, int EB>
@@ -128,7 +125,7 @@ __device__ __forceinline__ void stage_twiddles(const TwPair* __restrict__ tw, Tw
 // first phase may read from a different buffer than it writes (src -> dst); the second phase
 // works in place on dst.
 template <int LOGN, bool FWD, bool COLS, int EB, bool STAGED, bool TABLE>
-__global__ void __launch_bounds__(Phase<LOGN, FWD, COLS, EB, STAGED>::THREADS, min_blocks<EB>())
+__global__ void __launch_bounds__(Phase<LOGN, FWD, COLS, EB, STAGED>::THREADS, kMinBlocks)
     k_ntt_phase(uint64_t* __restrict__ data, size_t poly_stride, LimbMap map, const NttJob* __restrict__ jobs,
                 int njobs, const Modulus* __restrict__ mods, const TwPair* __restrict__ tw_base,
                 const TwPair* __restrict__ tw_words) {
@@ -354,7 +351,7 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
 }
 
 template <int LOGN, int EB, bool STAGED>
-__global__ void __launch_bounds__(Phase<LOGN, true, false, EB, STAGED>::THREADS, min_blocks<EB>())
+__global__ void __launch_bounds__(Phase<LOGN, true, false, EB, STAGED>::THREADS, kMinBlocks)
     k_ntt_rows_epi(const NttEpiJob* __restrict__ jobs, int njobs, const Modulus* __restrict__ mods,
                    const TwPair* __restrict__ tw_base) {
     using P = Phase<LOGN, true, false, EB, STAGED>;

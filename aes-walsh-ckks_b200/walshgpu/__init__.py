@@ -675,7 +675,7 @@ class Context:
     def set_ntt_fusion(self, mode):
         """Key switches and rescales with their base changes fused into the NTT column phases
         and their last element-wise steps into the row-phase epilogue: 0 never, 1 (default; True
-        maps here) and 2 always; the words are the same."""
+        maps here) except small launches with wide base changes, 2 always; the words are the same."""
         _check(lib().wg_set_ntt_fusion(self.h, int(mode)))
 
     def keyswitch(self, level, key_term, kind, b, a, b_add=True, a_add=False, rotation=0, stream=None):

@@ -163,8 +163,10 @@ int wg_ntt_set_geometry(wg_context* ctx, int direction, int phase, int geometry)
  * (src/ckks/operations/keyswitch/ckks_keyswitch.cpp:1330-1641) and ckks_rescale
  * (src/ckks/operations/arith/ckks_rescale.cpp:68-148) compute the same words step by step.
  * Launches too small to fill the device divide a job's output limbs over several blocks.  mode 1
- * (the default) and mode 2 fuse, mode 0 runs the separate launches.  The words are identical in
- * every mode. */
+ * (the default) fuses except where such a launch is shorter unfused (base changes of more than 12
+ * limbs, or of more than 4 moduli of 2^50 and more; rescales of one or two polynomials of many such
+ * limbs), mode 2 always fuses, mode 0 runs the separate launches.  The words are identical in every
+ * mode. */
 int wg_set_ntt_fusion(wg_context* ctx, int mode);
 
 /* Hybrid key switch of key_term at `level` with the installed key (kind, rotation):

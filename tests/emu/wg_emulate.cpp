@@ -792,6 +792,10 @@ size_t emu_tensor(uint64_t q, const uint64_t* xa, const uint64_t* xb, const uint
     return taken;
 }
 
+void emu_fp_reduce(uint64_t q, const double* x, size_t n, double* out) {
+    for (size_t i = 0; i < n; ++i) out[i] = fp::reduce(x[i], (double)q, 1.0 / (double)q);
+}
+
 // reduce128 on n values (hi[i], lo[i]) modulo q
 void emu_reduce128(uint64_t q, const uint64_t* hi, const uint64_t* lo, size_t n, uint64_t* out) {
     const Modulus m = emu_modulus(q);

@@ -51,6 +51,23 @@ def test_product_is_exact_and_bounded(emu, q):  # noqa: F811
         assert int(word[i]) == a[i] * w[i] % q
 
 
+@pytest.mark.parametrize("q", [12289, _prime(1 << 27, 1 << 15), _prime(1 << 42, 1 << 15), _prime(1 << 50, 1 << 15)])
+def test_reduce_over_its_whole_domain(emu, q):  # noqa: F811
+    """fp::reduce is a representative within q / 2 + 1 for every |x| <= 2^53: at random, next to multiples of q
+    and half-way between them, from the smallest NTT modulus (2^39 q and more) up."""
+    emu.emu_fp_reduce.argtypes = [C.c_uint64, f64p, C.c_size_t, f64p]
+    rng = np.random.default_rng(q % 1000003)
+    top = (1 << 53) // q
+    x = [int(v) for v in rng.integers(-(1 << 53), 1 << 53, 4000)]
+    for k in [0, 1, top - 1, top // 2] + [int(v) for v in rng.integers(0, top, 500)]:
+        x += [s * (k * q + d) for s in (1, -1) for d in (0, 1, -1, q // 2, q // 2 + 1, q - 1)]
+    x = [v for v in x + [1 << 53, -(1 << 53)] if abs(v) <= 1 << 53]
+    out = np.zeros(len(x))
+    emu.emu_fp_reduce(q, np.array(x, np.float64), len(x), out)
+    for v, r in zip(x, out):
+        assert r == int(r) and (int(r) - v) % q == 0 and 2 * abs(int(r)) <= q + 2, v
+
+
 @pytest.mark.parametrize("q", [_prime(1 << 42, 1 << 15), 274876334081, 12289, _prime(1 << 61, 1 << 15), _prime(1 << 62, 1 << 15)])
 @pytest.mark.parametrize("n", [1, 3, 32, 33, 500])
 def test_sums_of_products(emu, q, n):  # noqa: F811

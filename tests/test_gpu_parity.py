@@ -96,12 +96,12 @@ def _oracle_setup(O, wg, prm, rotations, seed=5):
     return N, o, ctx, keys, conj, relin
 
 
-@pytest.mark.parametrize("fusion", [1, 2])
+@pytest.mark.parametrize("fusion", [0, 1, 2])
 @pytest.mark.parametrize("prm", SMALL)
 def test_small_sets_against_oracle(wg, oracle_mod, prm, fusion):
-    """Every operation on one ciphertext at several levels against the oracle; fusion 1 (the
-    default) runs single ciphertexts through the separate launches, 2 forces the fused
-    key-switch and rescale kernels."""
+    """Every operation on one ciphertext at several levels against the oracle; fusion 0 runs the
+    separate launches, 1 (the default) the fused key-switch and rescale kernels except where a small
+    launch's base changes are wide, 2 the fused kernels always."""
     import torch
 
     O = oracle_mod
