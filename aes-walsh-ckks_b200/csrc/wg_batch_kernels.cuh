@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kT) kb_modup(const ModUpJob* jobs, int n, cons
     modup_coeff(*j->desc, mods, j->src, j->digit, N, coeff);
 }
 
-__global__ void __launch_bounds__(kT) kb_mac(const MacJob* jobs, int n, const Modulus* mods, int nq, size_t N) {
+__global__ void __launch_bounds__(kT, 4) kb_mac(const MacJob* jobs, int n, const Modulus* mods, int nq, size_t N) {
     const MacJob* j = job_of(jobs, n);
     if (!j) return;
     const size_t coeff = (size_t)blockIdx.x * kT + threadIdx.x;
