@@ -462,16 +462,23 @@ __device__ __forceinline__ void rows_mac(uint64_t* sm, const MacGroupJob* j, int
     using R = RowsMac<LOGN>;
     const size_t N = R::P::N;
     const int eb = R::Begin::element(sub, o), ee = R::End::element(sub, o), parts = j->parts;
+    const uint64_t* digits = j->digits[c] + at + eb;
+    const uint64_t* own = j->key_term[c] + at + ee;
     uint64_t w[8], k8[8];
+    // (the word sums leave no registers for the two pointers: read again from the job)
     auto fetch = [&](int p) {
         if (p == own_part)
-            load_words<typename R::End>(j->key_term[c] + at + ee, w);
+            load_words<typename R::End>(AHEAD ? own : j->key_term[c] + at + ee, w);
         else
-            load_words<typename R::Begin>(j->digits[c] + p * j->part_stride + at + eb, w);
+            load_words<typename R::Begin>((AHEAD ? digits : j->digits[c] + at + eb) + p * j->part_stride, w);
     };
     Sums sums;
     sums.clear();
-    typename Sums::V v[8];
+    typename Sums::V ahead[8], *v;  // the residues: beside the next digit's words, or in their place
+    if constexpr (AHEAD)
+        v = ahead;
+    else
+        v = w;
     if (AHEAD) fetch(0);
     for (int p = 0; p < parts; ++p) {
         if (!AHEAD) fetch(p);
@@ -494,17 +501,21 @@ __device__ __forceinline__ void rows_mac(uint64_t* sm, const MacGroupJob* j, int
 #pragma unroll
     for (int poly = 0; poly < 2; ++poly) {
         uint64_t* out = j->acc[c] + poly * T * N + at;
-        if (rows) {
+        if (!AHEAD || rows) {
 #pragma unroll
             for (int k = 0; k < 8; ++k) v[k] = sums.value(poly, k, m);
+        }
+        if (rows) {
             ntt_rounds<LOGN, false, false, 3, false, kMaxTile>(R::rounds(), sm, v, sub, o, tile, inv, tw + N);
 #pragma unroll
             for (int k = 0; k < 8; ++k) w[k] = Sums::row_word(v[k], m);
             store_words<typename R::InvEnd>(out + R::InvEnd::element(sub, o), w);
         } else {
+            if constexpr (AHEAD) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) w[k] = sums.word(poly, k, m);
-            store_words<typename R::End>(out + ee, w);
+                for (int k = 0; k < 8; ++k) w[k] = sums.word(poly, k, m);
+            }
+            store_words<typename R::End>(out + ee, w);  // (word sums: v is w, and the value the word)
         }
     }
 }
