@@ -79,6 +79,17 @@ bool stream_capturing(cudaStream_t s) {
     return cs != cudaStreamCaptureStatusNone;
 }
 
+// Scratch of a call outside a capture that reserves the stream's workspace, so that the next may be
+// captured: `words` words of the batch arena where it has them already (the call before left them in
+// the L2: one multiply, relinearise and rescale 196 us in the workspace, 194 in the arena), else the
+// workspace.
+uint64_t* call_scratch(wg::Context& c, size_t words, cudaStream_t s) {
+    uint64_t* ws = c.workspace(s);
+    if (stream_capturing(s)) return ws;
+    const wg::BatchBuffers& b = c.batch_buffers(s);
+    return b.arena_words >= words ? b.d_arena : ws;
+}
+
 // One key switch of one ciphertext.  Outside stream capture it runs as a batch of one (each
 // stage of the switch, all digits included, in a single launch), in the batch arena or in `ws`;
 // under capture, stage by stage on the stream's reserved workspace (the batched path stages a job
@@ -130,7 +141,9 @@ void do_rescale(wg::Context& c, size_t level, uint64_t* polys, size_t npolys, si
     const size_t words = std::count_if(c.q.begin(), c.q.begin() + level + 1, [](uint64_t q) { return q >= wg::fp::kLimit; });
     const bool staged = c.ntt_fusion != 2 && npolys <= 2 && words * npolys * c.N > (size_t{24} << 15);
     if (!stream_capturing(s) && !staged) {
-        wg::batch_rescale(c, level, polys, npolys, stride, c.workspace(s), c.workspace_words(), s);
+        const size_t all = npolys * (level + 1) * c.N;
+        uint64_t* ws = call_scratch(c, all, s);
+        wg::batch_rescale(c, level, polys, npolys, stride, ws, ws == c.workspace(s) ? c.workspace_words() : all, s);
         return;
     }
     uint64_t* ws = scratch_after_switch(c, s);
@@ -389,7 +402,8 @@ int wg_keyswitch(wg_context* ctx, size_t level, const uint64_t* key_term, int ki
         const int64_t r = kind == WG_KEY_ROTATION ? normalize_rotation(c, rotation) : 0;
         const wg::KeyEntry& k = c.key(kind, r);
         // the workspace in either form of the call: one call outside a capture makes the next capturable
-        switch_one(c, level, key_term, k, b, a, b, a, b_add != 0, a_add != 0, 0, c.workspace(S(stream)), S(stream));
+        switch_one(c, level, key_term, k, b, a, b, a, b_add != 0, a_add != 0, 0,
+                   call_scratch(c, wg::keyswitch_workspace_words(c, level), S(stream)), S(stream));
     });
 }
 
@@ -416,7 +430,8 @@ int wg_conjugate(wg_context* ctx, size_t level, uint64_t* b, uint64_t* a, void* 
         const uint64_t g = 2 * c.N - 1;
         wg::automorphism(c, b, pb, (int)(level + 1), 1, 0, g, S(stream));
         wg::automorphism(c, a, pa, (int)(level + 1), 1, 0, g, S(stream));
-        switch_one(c, level, pa, k, pb, pa, b, a, true, false, 0, c.workspace(S(stream)), S(stream));
+        switch_one(c, level, pa, k, pb, pa, b, a, true, false, 0,
+                   call_scratch(c, wg::keyswitch_workspace_words(c, level), S(stream)), S(stream));
     });
 }
 
