@@ -640,7 +640,7 @@ void phase_dispatch(const Context& c, bool fwd, bool cols, int variant, uint64_t
 // The geometry of one phase over `words` residues: the caller's where it is pinned, else by the tuned one.
 int phase_geometry(const Context& c, int direction, bool cols, size_t words) {
     const int v = c.ntt_variant[direction][cols ? 1 : 0];
-    return c.ntt_pinned[direction] >> (cols ? 1 : 0) & 1 ? v : launch_geometry(v, words, c.sm_count, c.word_moduli);
+    return c.ntt_pinned[direction] >> (cols ? 1 : 0) & 1 ? v : launch_geometry(v, cols, words, c.sm_count, c.word_moduli);
 }
 
 void dispatch(const Context& c, uint64_t* data, int limbs, int polys, size_t stride, LimbMap map,

@@ -489,11 +489,12 @@ inline bool whole_launch(int logN, size_t transforms, int sm_count, bool word_mo
 
 // The geometry (kNttGeometries order) of one phase over `words` residues where `tuned` is the best of
 // large batches: in small launches 8 residues a thread in place of 16, which halve the threads.
-// Forward transforms of 60-bit moduli, 8 and 16 residues in the row phase, device time in us: 2^15, 4
-// limbs 7.9 and 8.8, 8 limbs 8.0 and 9.3, 24 limbs 15.7 and 16.2, 64 limbs 30.9 and 31.1; 38-bit
-// moduli, 8 limbs 6.3 and 6.2, 12 limbs 8.5 and 8.3.
-inline int launch_geometry(int tuned, size_t words, int sm_count, bool word_moduli) {
-    const size_t small = (size_t)sm_count * kMaxTile * (word_moduli ? 4 : 1);
+// Device time with 8 and 16 in us: forward row phases of 60-bit moduli at 2^15, 4 limbs 7.9 and 8.8, 8
+// limbs 8.0 and 9.3, 24 limbs 15.7 and 16.2, 32 limbs 19.3 and 19.1; inverse ones of 38-bit moduli, 8
+// limbs 6.4 and 6.8, 17 limbs 8.3 and 8.8, 34 limbs 12.6 and 12.8, 68 limbs 21.3 and 21.2; inverse column
+// phases of the walsh15 chain, 13 limbs 9.4 and 9.8, 26 limbs 11.6 and 11.6, 52 limbs 19.3 and 18.2.
+inline int launch_geometry(int tuned, bool cols, size_t words, int sm_count, bool word_moduli) {
+    const size_t small = (size_t)sm_count * kMaxTile * (word_moduli && !cols ? 3 : 2);
     return tuned >= 2 && words <= small ? tuned - 2 : tuned;
 }
 

@@ -850,8 +850,8 @@ void emu_walsh_products(uint64_t q, size_t n, const uint64_t* low_b, const uint6
 }
 
 int emu_whole_launch(int logN, size_t transforms, int sms, int words) { return ntt::whole_launch(logN, transforms, sms, words != 0); }
-int emu_launch_geometry(int tuned, size_t residues, int sms, int words) {
-    return ntt::launch_geometry(tuned, residues, sms, words != 0);
+int emu_launch_geometry(int tuned, int cols, size_t residues, int sms, int words) {
+    return ntt::launch_geometry(tuned, cols != 0, residues, sms, words != 0);
 }
 
 // The staging ring's placement (wg_ring.hpp) over `steps` seeded uploads of mixed sizes (1 in 100

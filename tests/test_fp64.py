@@ -177,15 +177,17 @@ def test_launch_rules(emu):  # noqa: F811
     """On 148 SMs: one launch or two phases on both sides of every line, and 8 residues a thread in small
     launches whatever large ones were tuned to."""
     emu.emu_whole_launch.argtypes = [C.c_int, C.c_size_t, C.c_int, C.c_int]
-    emu.emu_launch_geometry.argtypes = [C.c_int, C.c_size_t, C.c_int, C.c_int]
+    emu.emu_launch_geometry.argtypes = [C.c_int, C.c_int, C.c_size_t, C.c_int, C.c_int]
     whole = lambda logN, n, words: emu.emu_whole_launch(logN, n, 148, words)
     assert all(whole(logN, n, words) for logN in (10, 11, 12) for n in (1, 5000) for words in (0, 1))
     assert all(whole(13, 128, words) and not whole(13, 129, words) and not whole(15, 1, words) for words in (0, 1))
     assert [n for n in range(1, 80) if whole(14, n, 0)] == list(range(1, 65))
     assert [n for n in range(1, 80) if whole(14, n, 1)] == list(range(1, 13)) + list(range(19, 49))
-    tuned = lambda words, residues: [emu.emu_launch_geometry(v, residues, 148, words) for v in range(4)]
-    for words, line in ((0, 148 * 2048), (1, 4 * 148 * 2048)):
-        assert tuned(words, line) == [0, 1, 0, 1] and tuned(words, line + 1) == [0, 1, 2, 3]
+    tuned = lambda words, cols, ctas: [emu.emu_launch_geometry(v, cols, ctas * 2048, 148, words) for v in range(4)]
+    for words in (0, 1):
+        for cols in (0, 1):
+            line = 148 * (3 if words and not cols else 2)
+            assert tuned(words, cols, line) == [0, 1, 0, 1] and tuned(words, cols, line + 1) == [0, 1, 2, 3]
 
 
 # digits of eight 50-bit limbs over nine 50-bit P limbs (the sums' bound, every width of the ModDown);
