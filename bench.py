@@ -1524,7 +1524,7 @@ def summary_keys(line):
         return d
 
     out = {"blocks_per_s": line["value"], "e2e_blocks_per_s": get(line, "e2e", "value"),
-           "ntt_frac_of_hbm": get(line, "roofline", "frac"),
+           "ntt_frac_of_hbm": ratio(get(line, "kernels", "ntt", "gbs"), get(line, "roofline", "peak")),
            "max_error": get(line, "correctness", "max_error"),
            "average_error": get(line, "correctness", "average_error"),
            "mismatches": get(line, "correctness", "mismatches")}
