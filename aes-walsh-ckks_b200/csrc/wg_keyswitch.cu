@@ -20,7 +20,6 @@ namespace wg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMaxParts = 16;
 
 struct ModUpBatch {
     ModUpDesc d[kMaxParts];

@@ -20,6 +20,7 @@ namespace wg {
 
 constexpr int kMaxDigitWidth = 16;  // largest alpha (Q limbs per digit) the kernels support
 constexpr int kMaxPLimbs = 16;
+constexpr int kMaxParts = 16;  // digits of a switch that runs stage by stage
 
 // Galois automorphism on the bit-reversed evaluation layout
 // (build_ntt_automorphism_map, src/ckks/context/rotation_key_generation.cpp:80-90):

@@ -146,3 +146,24 @@ def test_routes_of_single_calls(wg, oracle_mod):
         assert wg.launch_count() - n0 == launches, (level, polys)
         (want,) = o.rescale(level, [poly[:n]])
         assert (wg.to_host(d).reshape(polys, n)[:, : level * N] == want).all(), (level, polys)
+
+
+def test_more_digits_than_a_switch_takes_are_refused(wg, oracle_mod):
+    """wg_keyswitch and wg_conjugate take 16 digits, outside a capture as under it."""
+    import torch
+
+    N = 1 << 10
+    p, q = oracle_mod.find_primes([50], [40] * 17, N)
+    o, ctx = oracle_mod.OracleCtx(N, q, p, 17), wg.Context(N, q, p, 17)
+    secret = o.ternary(64, 3)
+    ctx.keygen_switch_key(wg.WG_KEY_CONJ, 0, secret, seed=7)
+    for level in (15, 16):
+        x = [wg.to_device(o.uniform(level + 1, 90 + i)) for i in range(3)]
+        calls = [lambda: ctx.keyswitch(level, x[2], wg.WG_KEY_CONJ, x[0], x[1]), lambda: ctx.conjugate(level, x[0], x[1])]
+        for call in calls:
+            if level == 15:
+                call()
+                continue
+            with pytest.raises(wg.InvalidArgument):
+                call()
+        torch.cuda.synchronize()
